@@ -211,7 +211,15 @@ struct CompressJob {
     std::chrono::steady_clock::time_point t_begin;
 };
 
-constexpr size_t kStageBytes = 4096;      // pinned staging for the small headers of a device-resident object
+constexpr size_t kStageBytes = 4096;      // pinned staging for the small headers of a device-resident object on its way in
+
+// What goes into a device-resident object, gathered while the stages are enqueued and moved by one kernel at the end.
+struct DevicePack {
+    CopySegment seg[kMaxCopySegments];
+    int segments = 0;
+    PackHeaders heads;
+    int head_bytes = 0;
+};
 
 struct Runtime {
     bool initialized = false;
@@ -231,8 +239,8 @@ struct Runtime {
     TopkBufs outlier, err;
     SvdWorkspace *svd = nullptr;
     unsigned *h_status = nullptr;                        // pinned mirror of the device status words
-    uint8_t *h_stage = nullptr;                          // pinned: section headers on their way to / from a device-resident object
-    size_t stage_used = 0;
+    uint8_t *h_stage = nullptr;                          // pinned: section headers of a device-resident object on their way in
+    DevicePack pack;
     CompressJob job;
     bool decompress_active = false;
     unsigned inject_status = 0;                          // test hook: OR-ed into the status word of the next call
@@ -436,23 +444,27 @@ void bitsqz_llm_decompress_release() {
 // ================================================================================================
 namespace {
 
-// Where the bytes of a packed object go: `base` is the start of the payload, in a pinned host block or in a device
-// buffer.  Device-produced bytes are copied there by the stream either way; host-known bytes (section headers) are
-// written directly into a host block and travel through the runtime's pinned staging area into a device buffer.
-bool put_small(Runtime &rt, const CompressJob &job, uint8_t *dst, const void *src, size_t bytes) {
+// Where the bytes of a packed object go: into a pinned host block (device-produced bytes copied there by the stream,
+// host-known bytes written directly) or into a device buffer (both noted in the runtime's DevicePack, whose kernel
+// runs after the last stage).  put_small: `d_patch` (nullable) is a device word that replaces the four bytes at `patch_at`.
+bool put_small(Runtime &rt, const CompressJob &job, uint8_t *dst, const void *src, size_t bytes, const void *d_patch = nullptr,
+               size_t patch_at = 0) {
     if (!job.to_device) {
         std::memcpy(dst, src, bytes);
-        return true;
+        return !d_patch || cudaMemcpyAsync(dst + patch_at, d_patch, 4, cudaMemcpyDefault, rt.stream) == cudaSuccess;
     }
-    const size_t need = (bytes + 15) & ~(size_t)15;
-    if (rt.stage_used + need > kStageBytes) return false;
-    uint8_t *stage = rt.h_stage + rt.stage_used;
-    rt.stage_used += need;
-    std::memcpy(stage, src, bytes);
-    return cudaMemcpyAsync(dst, stage, bytes, cudaMemcpyHostToDevice, rt.stream) == cudaSuccess;
+    PackHeaders &h = rt.pack.heads;
+    if (h.pieces >= kMaxHeads || rt.pack.head_bytes + bytes > sizeof(h.bytes)) return false;
+    std::memcpy(h.bytes + rt.pack.head_bytes, src, bytes);
+    h.piece[h.pieces++] = PackHeaders::Piece{dst, d_patch, (uint16_t)rt.pack.head_bytes, (uint16_t)bytes, (uint16_t)patch_at};
+    rt.pack.head_bytes += (int)bytes;
+    return true;
 }
-bool put_device(Runtime &rt, uint8_t *dst, const void *d_src, size_t bytes) {
-    return cudaMemcpyAsync(dst, d_src, bytes, cudaMemcpyDefault, rt.stream) == cudaSuccess;
+bool put_device(Runtime &rt, const CompressJob &job, uint8_t *dst, const void *d_src, size_t bytes) {
+    if (!job.to_device) return cudaMemcpyAsync(dst, d_src, bytes, cudaMemcpyDefault, rt.stream) == cudaSuccess;
+    if (rt.pack.segments >= kMaxCopySegments) return false;
+    rt.pack.seg[rt.pack.segments++] = CopySegment{dst, d_src, bytes};
+    return true;
 }
 
 // One quantised section into its final place: the host-known 48-byte header (quantization_cuda.cu:736-807), then
@@ -466,24 +478,23 @@ bool emit_quant_section(Runtime &rt, const CompressJob &job, const QuantBufs &q,
     h.num_elements = n;
     h.num_blocks = nb;
     h.block_size = 64;
-    if (!put_small(rt, job, dst, &h, sizeof(h))) return false;
+    if (!put_small(rt, job, dst, &h, sizeof(h), method == NF4 ? nullptr : q.dq.p, offsetof(QuantHeader, dq_scale))) return false;
     uint8_t *scales_dst = dst + sizeof(h);
     if (method == NF4) {
-        if (!put_device(rt, scales_dst, q.scales_f32.p, nb * 4)) return false;
+        if (!put_device(rt, job, scales_dst, q.scales_f32.p, nb * 4)) return false;
         scales_dst += nb * 4;
     } else {
-        if (!put_device(rt, dst + offsetof(QuantHeader, dq_scale), q.dq.p, 4)) return false;
-        if (!put_device(rt, scales_dst, q.scale_codes.p, nb)) return false;
+        if (!put_device(rt, job, scales_dst, q.scale_codes.p, nb)) return false;
         scales_dst += nb;
     }
-    return put_device(rt, scales_dst, q.data.p, (n + 1) / 2);
+    return put_device(rt, job, scales_dst, q.data.p, (n + 1) / 2);
 }
 
 bool emit_topk_section(Runtime &rt, const CompressJob &job, const TopkBufs &t, uint8_t *dst) {
     TopkHeader h{rt.rows, rt.cols, (uint16_t)t.k, 0};
     if (!put_small(rt, job, dst, &h, sizeof(h))) return false;
     const size_t cnt = (size_t)rt.rows * t.k;
-    return put_device(rt, dst + 8, t.idx.p, cnt * 2) && put_device(rt, dst + 8 + cnt * 2, t.val.p, cnt * 4);
+    return put_device(rt, job, dst + 8, t.idx.p, cnt * 2) && put_device(rt, job, dst + 8 + cnt * 2, t.val.p, cnt * 4);
 }
 
 // Quantise `d_src` (n elements) into q; d_deq (nullable, may alias d_src) receives the dequantised values.
@@ -543,6 +554,35 @@ void abandon_job(Runtime &rt) {
     job = CompressJob{};
 }
 
+// The 200-byte header of the object (src/bitsqz_llm.cu:1253-1271).
+bitsqz_llm_array_t object_header(const Runtime &rt, const CompressJob &job, bool has_error_topk) {
+    bitsqz_llm_array_t hdr;
+    std::memset(&hdr, 0, sizeof(hdr));
+    hdr.num_rows = rt.rows;
+    hdr.num_columns = rt.cols;
+    hdr.num_elements = (uint32_t)rt.rows * rt.cols;
+    hdr.outlier_topk_ratio = rt.outlier_ratio;
+    hdr.error_correction_topk_ratio = rt.error_ratio;
+    hdr.svd_ranks = (int16_t)rt.svd_ranks;
+    hdr.svd_niters = (int16_t)rt.svd_niters;
+    hdr.effective_rank = (int16_t)(job.has_svd ? rt.rank : 0);
+    hdr.svd_uv_format = (quantization_method_t)rt.uv_format;
+    hdr.svd_s_format = (quantization_method_t)rt.s_format;
+    hdr.quantization_only_format = (quantization_method_t)rt.q_format;
+    hdr.flags = (job.has_svd ? kFlagSvd : 0u) | (rt.outlier.k > 0 ? kFlagOutlier : 0u) | (has_error_topk ? kFlagError : 0u);
+    auto put = [](bitsqz_section_t &dst, const SectionPlan &s) {
+        dst.offset = s.offset; dst.size = s.size; dst.storage = s.storage;
+    };
+    put(hdr.section_u, job.sec_u);
+    put(hdr.section_s, job.sec_s);
+    put(hdr.section_v, job.sec_v);
+    put(hdr.section_direct, job.sec_direct);
+    put(hdr.section_outlier_topk, job.sec_out);
+    if (has_error_topk) put(hdr.section_error_topk, job.sec_err);
+    hdr.payload = job.block + sizeof(bitsqz_llm_array_t);
+    return hdr;
+}
+
 // Enqueue one compress call on the runtime's stream: staging of a host input, every stage, and the copies of the
 // results into their final place.  d_packed == nullptr: the object goes to a pinned host block; otherwise into the
 // caller's device buffer of `capacity` bytes.  Returns without waiting; compress_end finishes the call.
@@ -576,7 +616,7 @@ int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_p
         std::memset(job.block, 0, sizeof(bitsqz_llm_array_t));
     }
     job.active = true;
-    rt.stage_used = 0;
+    rt.pack.segments = rt.pack.heads.pieces = rt.pack.head_bytes = 0;
     auto fail = [&]() {
         abandon_job(rt);
         return 1;
@@ -666,27 +706,40 @@ int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_p
         // FP32 factors are stored as computed; when they were quantised the device copies now hold
         // the dequantised values and the payload takes the quantised form instead
         if (rt.uv_format != quantization_NONE) ok = ok && emit_quant_section(rt, job, rt.q_u, rt.uv_format, payload + job.sec_u.offset);
-        else ok = ok && put_device(rt, payload + job.sec_u.offset, rt.u.p, ub);
+        else ok = ok && put_device(rt, job, payload + job.sec_u.offset, rt.u.p, ub);
         if (rt.s_format != quantization_NONE) ok = ok && emit_quant_section(rt, job, rt.q_s, rt.s_format, payload + job.sec_s.offset);
-        else ok = ok && put_device(rt, payload + job.sec_s.offset, rt.s.p, sb);
+        else ok = ok && put_device(rt, job, payload + job.sec_s.offset, rt.s.p, sb);
         if (rt.uv_format != quantization_NONE) ok = ok && emit_quant_section(rt, job, rt.q_v, rt.uv_format, payload + job.sec_v.offset);
-        else ok = ok && put_device(rt, payload + job.sec_v.offset, rt.v.p, vb);
+        else ok = ok && put_device(rt, job, payload + job.sec_v.offset, rt.v.p, vb);
     } else if (rt.q_format != quantization_NONE) {
         ok = ok && emit_quant_section(rt, job, rt.q_direct, rt.q_format, payload + job.sec_direct.offset);
     } else {
-        ok = ok && put_device(rt, payload + job.sec_direct.offset, d_src, (size_t)n * 4);
+        ok = ok && put_device(rt, job, payload + job.sec_direct.offset, d_src, (size_t)n * 4);
     }
     if (ko > 0) ok = ok && emit_topk_section(rt, job, rt.outlier, payload + job.sec_out.offset);
     if (error_path) ok = ok && emit_topk_section(rt, job, rt.err, payload + job.sec_err.offset);
-    ok = ok && cudaMemcpyAsync(rt.h_status, d_status, 64, cudaMemcpyDeviceToHost, st) == cudaSuccess;
+    if (job.to_device) {
+        PackHeaders &h = rt.pack.heads;
+        const bitsqz_llm_array_t hdr = object_header(rt, job, error_path);
+        static_assert(sizeof(hdr) == sizeof(h.object), "the object's header");
+        std::memcpy(h.object, &hdr, sizeof(hdr));
+        h.object_dst = job.block;
+        h.flags_at = offsetof(bitsqz_llm_array_t, flags);                 // (little-endian: the flags' low byte)
+        h.error_flag = kFlagError;
+        h.error_entry_at = offsetof(bitsqz_llm_array_t, section_error_topk);
+        h.error_entry_length = sizeof(hdr.section_error_topk);
+        ok = ok && pack_object(rt.pack.seg, rt.pack.segments, h, d_status, rt.h_status, st) == cudaSuccess;
+    } else {
+        ok = ok && cudaMemcpyAsync(rt.h_status, d_status, 4 * kStatusWords, cudaMemcpyDeviceToHost, st) == cudaSuccess;
+    }
     mark();                                                               // last event: copies done
     if (!ok) return fail();
     return 0;
 }
 
 // Wait for the call begun by compress_begin and finish the object: status check, header (src/bitsqz_llm.cu:1253-1271).
-// Host object: *out receives the block.  Device object: the 200-byte header is copied to the front of the caller's
-// buffer and into *header_out (nullable), whose `payload` is then a DEVICE pointer.
+// Host object: *out receives the block.  Device object: the sections and the 200-byte header are in the caller's buffer
+// by then, and *header_out (nullable) receives a copy of the header, whose `payload` is a DEVICE pointer.
 int compress_end(Runtime &rt, bitsqz_llm_array_t **out, bitsqz_llm_array_t *header_out, uint64_t *packed_size,
                  bitsqz_llm_compress_profile_t *profile) {
     CompressJob &job = rt.job;
@@ -696,40 +749,10 @@ int compress_end(Runtime &rt, bitsqz_llm_array_t **out, bitsqz_llm_array_t *head
         abandon_job(rt);
         return 1;
     }
-    const bool has_svd = job.has_svd;
     const bool has_error_topk = job.error_path && rt.h_status[1] != 0;      // src/bitsqz_llm.cu:1160-1178
-    bitsqz_llm_array_t hdr;
-    std::memset(&hdr, 0, sizeof(hdr));
-    hdr.num_rows = rt.rows;
-    hdr.num_columns = rt.cols;
-    hdr.num_elements = (uint32_t)rt.rows * rt.cols;
-    hdr.outlier_topk_ratio = rt.outlier_ratio;
-    hdr.error_correction_topk_ratio = rt.error_ratio;
-    hdr.svd_ranks = (int16_t)rt.svd_ranks;
-    hdr.svd_niters = (int16_t)rt.svd_niters;
-    hdr.effective_rank = (int16_t)(has_svd ? rt.rank : 0);
-    hdr.svd_uv_format = (quantization_method_t)rt.uv_format;
-    hdr.svd_s_format = (quantization_method_t)rt.s_format;
-    hdr.quantization_only_format = (quantization_method_t)rt.q_format;
-    hdr.flags = (has_svd ? kFlagSvd : 0u) | (rt.outlier.k > 0 ? kFlagOutlier : 0u) | (has_error_topk ? kFlagError : 0u);
-    auto put = [](bitsqz_section_t &dst, const SectionPlan &s) {
-        dst.offset = s.offset; dst.size = s.size; dst.storage = s.storage;
-    };
-    put(hdr.section_u, job.sec_u);
-    put(hdr.section_s, job.sec_s);
-    put(hdr.section_v, job.sec_v);
-    put(hdr.section_direct, job.sec_direct);
-    put(hdr.section_outlier_topk, job.sec_out);
-    if (has_error_topk) put(hdr.section_error_topk, job.sec_err);
-    hdr.payload = job.block + sizeof(bitsqz_llm_array_t);
+    const bitsqz_llm_array_t hdr = object_header(rt, job, has_error_topk);
     if (job.to_device) {
-        std::memcpy(rt.h_stage, &hdr, sizeof(hdr));
-        if (cudaMemcpyAsync(job.block, rt.h_stage, sizeof(hdr), cudaMemcpyHostToDevice, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess) {
-            abandon_job(rt);
-            return 1;
-        }
-        if (header_out) *header_out = hdr;
+        if (header_out) *header_out = hdr;                    // (the device copy was written with the sections)
     } else {
         std::memcpy(job.block, &hdr, sizeof(hdr));
         if (out) *out = reinterpret_cast<bitsqz_llm_array_t *>(job.block);
@@ -793,7 +816,7 @@ bool section_method_ok(const bitsqz_section_t &s, int method) {                 
 }
 
 // The small headers that sit inside the payload, fetched before anything is decided from them: straight reads for a
-// host payload, one batch of small device-to-host copies (and one wait) for a device-resident payload.
+// host payload, one small kernel (and one wait) for a device-resident payload, which also clears the status words.
 struct SectionHeads {
     QuantHeader u, s, v, direct;
     TopkHeader outlier, err;
@@ -811,8 +834,8 @@ bool fetch_heads(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_devic
         {&c->section_outlier_topk, &heads->outlier, sizeof(TopkHeader), BITSQZ_SECTION_TOPK},
         {&c->section_error_topk, &heads->err, sizeof(TopkHeader), BITSQZ_SECTION_TOPK},
     };
-    size_t used = 0;
-    uint8_t *staged[6] = {};
+    HeadList list{};
+    void *into[kMaxHeads] = {};
     for (int i = 0; i < 6; ++i) {
         const Want &w = wants[i];
         if (w.sec->storage != w.storage || w.sec->size < w.bytes) continue;     // absent, FP32, or too short (rejected later)
@@ -820,14 +843,14 @@ bool fetch_heads(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_devic
             std::memcpy(w.dst, payload + w.sec->offset, w.bytes);
             continue;
         }
-        staged[i] = rt.h_stage + used;
-        used += 64;
-        if (cudaMemcpyAsync(staged[i], payload + w.sec->offset, w.bytes, cudaMemcpyDeviceToHost, rt.stream) != cudaSuccess) return false;
+        list.src[list.count] = payload + w.sec->offset;
+        list.length[list.count] = (int)w.bytes;
+        into[list.count++] = w.dst;
     }
     if (payload_on_device) {
-        if (cudaStreamSynchronize(rt.stream) != cudaSuccess) return false;
-        for (int i = 0; i < 6; ++i)
-            if (staged[i]) std::memcpy(wants[i].dst, staged[i], wants[i].bytes);
+        if (fetch_heads(list, rt.h_stage, rt.status.as<unsigned>(), rt.stream) != cudaSuccess) return false;
+        if (list.count > 0 && cudaStreamSynchronize(rt.stream) != cudaSuccess) return false;
+        for (int i = 0; i < list.count; ++i) std::memcpy(into[i], rt.h_stage + 64 * i, list.length[i]);
     }
     return true;
 }
@@ -882,10 +905,17 @@ bool validate_header(const Runtime &rt, const bitsqz_llm_array_t *c) {
     return true;
 }
 
-// Checks of one quantised section against its 48-byte header (quantization_cuda.cu:691-734,809-876); uploads its
-// scales and nibbles into the runtime's aligned buffers.
-bool upload_quant(Runtime &rt, const bitsqz_llm_array_t *c, const bitsqz_section_t &s, const QuantHeader &h, int method,
-                  uint64_t expected_count, QuantBufs *q) {
+// The pieces of a quantised section where the dequantise kernels read them.
+struct QuantSource {
+    const float *scales_f32 = nullptr, *dq = nullptr;
+    const uint8_t *scale_codes = nullptr, *data = nullptr;
+};
+bool aligned_to(const void *p, size_t a) { return reinterpret_cast<uintptr_t>(p) % a == 0; }
+
+// Checks of one quantised section against its 48-byte header (quantization_cuda.cu:691-734,809-876).  A device-resident
+// section whose pieces are 4-byte aligned is read where it lies; others go into the runtime's aligned buffers first.
+bool locate_quant(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, const bitsqz_section_t &s, const QuantHeader &h, int method,
+                  uint64_t expected_count, QuantBufs *q, QuantSource *where) {
     if (s.storage != BITSQZ_SECTION_QUANT || method == quantization_NONE || !q || q->cap < expected_count) return false;
     q->n = expected_count;
     if (s.size < sizeof(QuantHeader)) return false;
@@ -894,46 +924,77 @@ bool upload_quant(Runtime &rt, const bitsqz_llm_array_t *c, const bitsqz_section
         h.block_size != 64 || h.num_blocks != nb || s.size != quant_section_bytes(method, expected_count))
         return false;
     const uint8_t *src = static_cast<const uint8_t *>(c->payload) + s.offset;
-    const uint8_t *scales = src + sizeof(QuantHeader);
-    cudaStream_t st = rt.stream;
-    if (method == NF4) {
-        return cudaMemcpyAsync(q->scales_f32.p, scales, nb * 4, cudaMemcpyDefault, st) == cudaSuccess &&
-               cudaMemcpyAsync(q->data.p, scales + nb * 4, (expected_count + 1) / 2, cudaMemcpyDefault, st) == cudaSuccess;
+    const uint8_t *scales = src + sizeof(QuantHeader), *dq = src + offsetof(QuantHeader, dq_scale);
+    const uint64_t scale_bytes = method == NF4 ? nb * 4 : nb, data_bytes = (expected_count + 1) / 2;
+    if (on_device && aligned_to(src, 4) && aligned_to(scales + scale_bytes, 4)) {
+        if (method == NF4) {
+            where->scales_f32 = reinterpret_cast<const float *>(scales);
+        } else {
+            where->dq = reinterpret_cast<const float *>(dq);
+            where->scale_codes = scales;
+        }
+        where->data = scales + scale_bytes;
+        return true;
     }
-    return cudaMemcpyAsync(q->dq.p, src + offsetof(QuantHeader, dq_scale), 4, cudaMemcpyDefault, st) == cudaSuccess &&
-           cudaMemcpyAsync(q->scale_codes.p, scales, nb, cudaMemcpyDefault, st) == cudaSuccess &&
-           cudaMemcpyAsync(q->data.p, scales + nb, (expected_count + 1) / 2, cudaMemcpyDefault, st) == cudaSuccess;
+    CopySegment seg[3];
+    int count = 0;
+    if (method == NF4) {
+        seg[count++] = CopySegment{q->scales_f32.p, scales, scale_bytes};
+        where->scales_f32 = q->scales_f32.as<float>();
+    } else {
+        seg[count++] = CopySegment{q->dq.p, dq, 4};
+        seg[count++] = CopySegment{q->scale_codes.p, scales, scale_bytes};
+        where->dq = q->dq.as<float>();
+        where->scale_codes = q->scale_codes.as<uint8_t>();
+    }
+    seg[count++] = CopySegment{q->data.p, scales + scale_bytes, data_bytes};
+    where->data = q->data.as<uint8_t>();
+    if (on_device) return copy_segments(seg, count, rt.stream) == cudaSuccess;
+    for (int i = 0; i < count; ++i)
+        if (cudaMemcpyAsync(seg[i].dst, seg[i].src, seg[i].bytes, cudaMemcpyDefault, rt.stream) != cudaSuccess) return false;
+    return true;
 }
 
-// One section -> `d_out` (expected_count floats).  FP32: plain copy.  QUANT: upload, then the dequantise kernel.
-bool decode_section(Runtime &rt, const bitsqz_llm_array_t *c, const bitsqz_section_t &s, const QuantHeader &h, int method,
+// One section -> `d_out` (expected_count floats).  FP32: plain copy.  QUANT: the dequantise kernel.
+bool decode_section(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, const bitsqz_section_t &s, const QuantHeader &h, int method,
                     uint64_t expected_count, QuantBufs *q, float *d_out) {
     const uint8_t *src = static_cast<const uint8_t *>(c->payload) + s.offset;
     if (s.storage == BITSQZ_SECTION_FP32) {
         if (s.size != expected_count * 4) return false;
         return cudaMemcpyAsync(d_out, src, s.size, cudaMemcpyDefault, rt.stream) == cudaSuccess;
     }
-    if (!upload_quant(rt, c, s, h, method, expected_count, q)) return false;
-    if (method == NF4)
-        return nf4_dequantize(q->scales_f32.as<float>(), q->data.as<uint8_t>(), expected_count, d_out, rt.sm_count, rt.stream) == cudaSuccess;
-    return nf4dq_dequantize(q->dq.as<float>(), q->scale_codes.as<uint8_t>(), q->data.as<uint8_t>(), expected_count, d_out,
-                            rt.sm_count, rt.stream) == cudaSuccess;
+    QuantSource from;
+    if (!locate_quant(rt, c, on_device, s, h, method, expected_count, q, &from)) return false;
+    if (method == NF4) return nf4_dequantize(from.scales_f32, from.data, expected_count, d_out, rt.sm_count, rt.stream) == cudaSuccess;
+    return nf4dq_dequantize(from.dq, from.scale_codes, from.data, expected_count, d_out, rt.sm_count, rt.stream) == cudaSuccess;
 }
 
-bool upload_topk(Runtime &rt, const bitsqz_llm_array_t *c, const bitsqz_section_t &s, const TopkHeader &h, TopkBufs &bufs) {
-    const uint8_t *src = static_cast<const uint8_t *>(c->payload) + s.offset;
+// The two arrays of a top-k section: where they lie (device-resident and aligned) or copied into `bufs`.
+bool locate_topk(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, const bitsqz_section_t &s, const TopkHeader &h, TopkBufs &bufs,
+                 const uint16_t **idx, const float **val) {
+    const uint8_t *src = static_cast<const uint8_t *>(c->payload) + s.offset + sizeof(TopkHeader);
     const size_t cnt = (size_t)h.num_rows * h.num_topk_columns;
+    if (on_device && aligned_to(src, 2) && aligned_to(src + cnt * 2, 4)) {
+        *idx = reinterpret_cast<const uint16_t *>(src);
+        *val = reinterpret_cast<const float *>(src + cnt * 2);
+        return true;
+    }
+    *idx = bufs.idx.as<uint16_t>();
+    *val = bufs.val.as<float>();
     if (cnt == 0) return true;
-    return cudaMemcpyAsync(bufs.idx.p, src + 8, cnt * 2, cudaMemcpyDefault, rt.stream) == cudaSuccess &&
-           cudaMemcpyAsync(bufs.val.p, src + 8 + cnt * 2, cnt * 4, cudaMemcpyDefault, rt.stream) == cudaSuccess;
+    const CopySegment seg[2] = {{bufs.idx.p, src, cnt * 2}, {bufs.val.p, src + cnt * 2, cnt * 4}};
+    if (on_device) return copy_segments(seg, 2, rt.stream) == cudaSuccess;
+    return cudaMemcpyAsync(bufs.idx.p, src, cnt * 2, cudaMemcpyDefault, rt.stream) == cudaSuccess &&
+           cudaMemcpyAsync(bufs.val.p, src + cnt * 2, cnt * 4, cudaMemcpyDefault, rt.stream) == cudaSuccess;
 }
 
-bool apply_topk_section(Runtime &rt, const bitsqz_llm_array_t *c, const bitsqz_section_t &s, const TopkHeader &h, TopkBufs &bufs,
-                        float *d_dst) {
+bool apply_topk_section(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, const bitsqz_section_t &s, const TopkHeader &h,
+                        TopkBufs &bufs, float *d_dst) {
     if ((size_t)h.num_rows * h.num_topk_columns == 0) return true;
-    if (!upload_topk(rt, c, s, h, bufs)) return false;
-    return topk_apply(bufs.idx.as<uint16_t>(), bufs.val.as<float>(), h.num_rows, h.num_columns, h.num_topk_columns, d_dst,
-                      rt.status.as<unsigned>(), rt.stream) == cudaSuccess;
+    const uint16_t *idx = nullptr;
+    const float *val = nullptr;
+    if (!locate_topk(rt, c, on_device, s, h, bufs, &idx, &val)) return false;
+    return topk_apply(idx, val, h.num_rows, h.num_columns, h.num_topk_columns, d_dst, rt.status.as<unsigned>(), rt.stream) == cudaSuccess;
 }
 
 // Enqueue one decompress call (src/bitsqz_llm.cu:1304-1393).  `c` is the 200-byte header in host memory; its payload
@@ -952,7 +1013,7 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
     const bool has_out = c->flags & kFlagOutlier, has_err = c->flags & kFlagError;
     if (has_out && !topk_section_ok(rt.outlier, c, c->section_outlier_topk, heads.outlier)) return 1;
     if (has_err && !topk_section_ok(rt.err, c, c->section_error_topk, heads.err)) return 1;
-    if (cudaMemsetAsync(rt.status.p, 0, 64, st) != cudaSuccess) return fail();
+    if (!payload_on_device && cudaMemsetAsync(rt.status.p, 0, 64, st) != cudaSuccess) return fail();
     if (rt.inject_status) {
         rt.h_status[8] = rt.inject_status;
         rt.inject_status = 0;
@@ -962,9 +1023,9 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
     bool lists_done = false;
     if (c->flags & kFlagSvd) {
         const uint32_t rank = (uint16_t)c->effective_rank;
-        if (!decode_section(rt, c, c->section_u, heads.u, c->svd_uv_format, (uint64_t)c->num_rows * rank, &rt.q_direct, rt.u.as<float>())) return fail();
-        if (!decode_section(rt, c, c->section_s, heads.s, c->svd_s_format, rank, &rt.q_direct, rt.s.as<float>())) return fail();
-        if (!decode_section(rt, c, c->section_v, heads.v, c->svd_uv_format, (uint64_t)c->num_columns * rank, &rt.q_direct, rt.v.as<float>())) return fail();
+        if (!decode_section(rt, c, payload_on_device, c->section_u, heads.u, c->svd_uv_format, (uint64_t)c->num_rows * rank, &rt.q_direct, rt.u.as<float>())) return fail();
+        if (!decode_section(rt, c, payload_on_device, c->section_s, heads.s, c->svd_s_format, rank, &rt.q_direct, rt.s.as<float>())) return fail();
+        if (!decode_section(rt, c, payload_on_device, c->section_v, heads.v, c->svd_uv_format, (uint64_t)c->num_columns * rank, &rt.q_direct, rt.v.as<float>())) return fail();
         if (reconstruct_lowrank(rt.u.as<float>(), rt.s.as<float>(), rt.v.as<float>(), c->num_rows, c->num_columns, (int)rank,
                                 nullptr, d_dst, nullptr, d_status, rt.recon_ws.as<float>(), rt.recon_ws_bytes, rt.sm_count, st) != cudaSuccess)
             return fail();
@@ -975,26 +1036,26 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
         TopkBufs &tb = has_out ? rt.outlier : rt.err;
         const bitsqz_section_t &ts = has_out ? c->section_outlier_topk : c->section_error_topk;
         const int method = c->quantization_only_format;
-        if (!upload_quant(rt, c, c->section_direct, heads.direct, method, c->num_elements, &rt.q_direct)) return fail();
         if ((size_t)th.num_rows * th.num_topk_columns == 0) {
-            if (!decode_section(rt, c, c->section_direct, heads.direct, method, c->num_elements, &rt.q_direct, d_dst)) return fail();
+            if (!decode_section(rt, c, payload_on_device, c->section_direct, heads.direct, method, c->num_elements, &rt.q_direct, d_dst)) return fail();
         } else {
-            if (!upload_topk(rt, c, ts, th, tb)) return fail();
-            QuantBufs &q = rt.q_direct;
-            if (nf4_dequantize_add_topk(method == NF4 ? q.scales_f32.as<float>() : nullptr, method == NF4 ? nullptr : q.dq.as<float>(),
-                                        method == NF4 ? nullptr : q.scale_codes.as<uint8_t>(), q.data.as<uint8_t>(), c->num_rows,
-                                        c->num_columns, tb.idx.as<uint16_t>(), tb.val.as<float>(), th.num_topk_columns, d_dst,
-                                        d_status, rt.sm_count, st) != cudaSuccess)
+            QuantSource q;
+            const uint16_t *idx = nullptr;
+            const float *val = nullptr;
+            if (!locate_quant(rt, c, payload_on_device, c->section_direct, heads.direct, method, c->num_elements, &rt.q_direct, &q)) return fail();
+            if (!locate_topk(rt, c, payload_on_device, ts, th, tb, &idx, &val)) return fail();
+            if (nf4_dequantize_add_topk(q.scales_f32, q.dq, q.scale_codes, q.data, c->num_rows, c->num_columns, idx, val,
+                                        th.num_topk_columns, d_dst, d_status, rt.sm_count, st) != cudaSuccess)
                 return fail();
         }
         lists_done = true;
     } else {
-        if (!decode_section(rt, c, c->section_direct, heads.direct, c->quantization_only_format, c->num_elements, &rt.q_direct, d_dst)) return fail();
+        if (!decode_section(rt, c, payload_on_device, c->section_direct, heads.direct, c->quantization_only_format, c->num_elements, &rt.q_direct, d_dst)) return fail();
     }
     if (!lists_done) {
         // error first, outliers second (src/bitsqz_llm.cu:1372-1387)
-        if (has_err && !apply_topk_section(rt, c, c->section_error_topk, heads.err, rt.err, d_dst)) return fail();
-        if (has_out && !apply_topk_section(rt, c, c->section_outlier_topk, heads.outlier, rt.outlier, d_dst)) return fail();
+        if (has_err && !apply_topk_section(rt, c, payload_on_device, c->section_error_topk, heads.err, rt.err, d_dst)) return fail();
+        if (has_out && !apply_topk_section(rt, c, payload_on_device, c->section_outlier_topk, heads.outlier, rt.outlier, d_dst)) return fail();
     }
     if (cudaMemcpyAsync(rt.h_status, rt.status.p, 64, cudaMemcpyDeviceToHost, st) != cudaSuccess) return fail();
     rt.decompress_active = true;

@@ -66,6 +66,41 @@ cudaError_t frontend_quantize(int method, const float *d_in, uint32_t rows, uint
 cudaError_t residual_error(const float *d_a, const float *d_b, uint64_t n, float *d_e, unsigned *d_flag, int sm_count,
                            cudaStream_t stream);
 
+// ---- device-resident objects (bsq_pack.cu) ---------------------------------------------------
+constexpr int kMaxCopySegments = 12, kMaxHeads = 6;
+constexpr int kStatusWords = 16;                             // [0] kernel status bits, [1] error-nonzero flag, [8] bound of the SVD's products
+struct CopySegment {
+    void *dst;
+    const void *src;
+    uint64_t bytes;
+};
+// Headers that the host knows, on their way into a device-resident object.
+struct PackHeaders {
+    struct Piece {
+        uint8_t *dst;
+        const void *patch;                                   // nullable: device word that replaces the four bytes at patch_at
+        uint16_t at, length, patch_at;
+    } piece[kMaxHeads];
+    int pieces;
+    uint8_t bytes[256];                                      // the pieces' contents
+    uint8_t object[200];                                     // the object's header as it is with an error section
+    uint8_t *object_dst;
+    int flags_at, error_entry_at, error_entry_length;        // cleared where status word 1 says that there is none
+    uint8_t error_flag;
+};
+struct HeadList {
+    const uint8_t *src[kMaxHeads];
+    int length[kMaxHeads];                                   // at most 64
+    int count;
+};
+// Copies up to kMaxCopySegments pieces of device memory, of any alignment, in one launch.
+cudaError_t copy_segments(const CopySegment *segments, int count, cudaStream_t stream);
+// The same together with the headers and, into page-locked `mirror`, the status words.
+cudaError_t pack_object(const CopySegment *segments, int count, const PackHeaders &headers, const unsigned *d_status, unsigned *mirror,
+                        cudaStream_t stream);
+// Small headers out of a device-resident payload into page-locked `host`, 64 bytes apart; clears the status words.
+cudaError_t fetch_heads(const HeadList &heads, uint8_t *host, unsigned *d_status, cudaStream_t stream);
+
 int device_sm_count();
 // A block for a packed object that the caller will release with bitsqz_llm_free: page-locked from the library's pool
 // when one can be had, plain heap memory otherwise (bsq_api.cu).

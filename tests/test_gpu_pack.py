@@ -1,0 +1,90 @@
+"""Device-resident objects are assembled and read back by kernels of their own (csrc/bsq_pack.cu): the same bytes as the host
+object, whatever the alignment of the caller's buffer and of the sections inside it, and the same matrix when they are read."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+# rows, cols, outlier, error, rank, uv, s, q: sections that end on every alignment (odd list lengths, odd code counts), objects
+# of less than one 16-byte unit per piece and of more than one CTA's share (32 KB) per piece, with and without an error list
+CASES = [
+    (1, 1, 0.0, 0.0, -1, -1, -1, 11),
+    (3, 5, 0.3, 0.3, -1, -1, -1, 10),
+    (7, 64, 0.02, 0.0, -1, -1, -1, 10),
+    (33, 77, 0.04, 0.04, -1, -1, -1, 11),
+    (256, 1024, 0.01, 0.0, -1, -1, -1, 10),
+    (515, 1001, 0.0, 0.0, -1, -1, -1, -1),
+    (129, 203, 0.02, 0.02, 13, 10, 11, -1),
+    (512, 640, 0.01, 0.0, 32, -1, -1, -1),
+    (300, 257, 0.01, 0.01, 21, 11, -1, -1),
+]
+
+
+@pytest.mark.parametrize("case", CASES)
+@pytest.mark.parametrize("off", [0, 1, 6, 12])
+def test_device_object_equals_host_object_at_any_alignment(pkg, lib, case, off):
+    rows, cols, outlier, error, rank, uv, s, q = case
+    g = torch.Generator(device="cuda").manual_seed(rows * 7 + cols)
+    x = torch.randn(rows, cols, device="cuda", generator=g)
+    lane = lib.bsq_lane_create(rows, cols, outlier, error, rank, 2, uv, s, q)
+    assert lane
+    try:
+        cap = int(lib.bsq_lane_packed_capacity(lane))
+        buf = torch.full((cap + 64,), 0xA5, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        hdr, size, out = pkg.Array(), C.c_uint64(0), C.c_void_p(None)
+        assert lib.bsq_lane_compress_begin(lane, x.data_ptr(), 1, buf.data_ptr() + off, cap) == 0
+        assert lib.bsq_lane_compress_end(lane, None, C.byref(hdr), C.byref(size)) == 0
+        assert lib.bsq_lane_compress_begin(lane, x.data_ptr(), 1, None, 0) == 0
+        assert lib.bsq_lane_compress_end(lane, C.byref(out), None, None) == 0
+        n = int(lib.bsq_get_packed_size(out))
+        host = np.frombuffer(C.string_at(out.value, n), np.uint8).copy()
+        assert int(size.value) == n <= cap
+        got = buf.cpu().numpy()
+        assert (got[:off] == 0xA5).all() and (got[off + cap:] == 0xA5).all()       # nothing outside the object
+        dev = got[off: off + n].copy()
+        assert dev[192:200].view(np.uint64)[0] == buf.data_ptr() + off + 200
+        dev[192:200] = 0
+        host[192:200] = 0
+        assert np.array_equal(dev, host)
+        y_dev = torch.empty_like(x)
+        y_host = torch.empty_like(x)
+        torch.cuda.synchronize()
+        assert lib.bsq_lane_decompress_begin(lane, C.byref(hdr), 1, y_dev.data_ptr(), rows * cols) == 0
+        assert lib.bsq_lane_decompress_end(lane) == 0
+        assert lib.bsq_lane_decompress_begin(lane, out, 0, y_host.data_ptr(), rows * cols) == 0
+        assert lib.bsq_lane_decompress_end(lane) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(y_dev.view(torch.int32), y_host.view(torch.int32))
+        lib.bsq_free(out)
+    finally:
+        lib.bsq_lane_destroy(lane)
+
+
+def test_damaged_device_object_is_refused(pkg, lib):
+    """The headers inside a device-resident payload are checked as those of a host object are, before anything is decoded."""
+    rows, cols = 64, 128
+    x = torch.randn(rows, cols, device="cuda")
+    lane = lib.bsq_lane_create(rows, cols, 0.02, 0.0, -1, 1, -1, -1, 11)
+    try:
+        cap = int(lib.bsq_lane_packed_capacity(lane))
+        buf = torch.empty(cap, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        hdr = pkg.Array()
+        assert lib.bsq_lane_compress_begin(lane, x.data_ptr(), 1, buf.data_ptr(), cap) == 0
+        assert lib.bsq_lane_compress_end(lane, None, C.byref(hdr), None) == 0
+        y = torch.empty_like(x)
+        for at in (200 + hdr.section_direct.offset, 200 + hdr.section_outlier_topk.offset + 4):      # magic number, list length
+            good = int(buf[at])
+            buf[at] = good ^ 0x80
+            torch.cuda.synchronize()
+            assert lib.bsq_lane_decompress_begin(lane, C.byref(hdr), 1, y.data_ptr(), rows * cols) == 1
+            buf[at] = good
+        torch.cuda.synchronize()
+        assert lib.bsq_lane_decompress_begin(lane, C.byref(hdr), 1, y.data_ptr(), rows * cols) == 0
+        assert lib.bsq_lane_decompress_end(lane) == 0
+    finally:
+        lib.bsq_lane_destroy(lane)
