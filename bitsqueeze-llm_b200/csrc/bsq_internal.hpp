@@ -105,7 +105,6 @@ int device_sm_count();
 // A block for a packed object that the caller will release with bitsqz_llm_free: page-locked from the library's pool
 // when one can be had, plain heap memory otherwise (bsq_api.cu).
 void *host_block_take(size_t bytes);
-bool topk_rows_fit_smem(const void *d_in, const void *d_residual, uint32_t cols, uint32_t k);
 
 // ---- randomized low-rank SVD and reconstruction (bsq_svd.cu, bsq_gemm.cu) -------------------
 // Replaces svd_lowrank_cuda_initialize / svd_lowrank_cuda / svd_lowrank_cuda_release

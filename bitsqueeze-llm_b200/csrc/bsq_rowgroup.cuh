@@ -238,7 +238,7 @@ __device__ __noinline__ void group_topk_exact(const RowGroup<G> &g, GroupCtl &c,
     group_rank_emit<G>(g, c, row, min(c.count, (unsigned)kCandCap), k, out_idx, out_val, zero_selected);
 }
 
-// Selection on a shared-memory row (cols % 4 == 0, 16-byte aligned, k <= kCandCap).
+// Selection on a shared-memory row (16-byte aligned, +0 from cols up to a multiple of four, k <= kCandCap).
 //   hint : a guess of a bound slightly below the k-th largest |x| (0 = none), normally from the row
 //          the group did before.  Any bound that between k and kCandCap elements reach gives the exact
 //          answer, so a bad guess only costs a second sweep.
@@ -255,7 +255,7 @@ __device__ __forceinline__ float group_topk_row(const RowGroup<G> &g, GroupCtl &
                                                 uint16_t *out_idx, float *out_val, bool zero_selected, float hint,
                                                 bool *special_out, RowFree row_free) {
     constexpr int L = RowGroup<G>::L;
-    const unsigned f4 = cols >> 2;
+    const unsigned f4 = (cols + 3) >> 2;
     const float4 *row4 = reinterpret_cast<const float4 *>(row);
     if (g.lane == 0) { c.count = 0; c.nhits = 0; c.flags = 0; }
     if (g.lane < 8) c.seen[g.lane] = 0u;
