@@ -233,7 +233,7 @@ struct Runtime {
     int sm_count = 148;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[8] = {};
-    DevBuf input_stage, residual, recon, error, u, s, v, scratch, status, recon_ws;
+    DevBuf input_stage, residual, error, u, s, v, scratch, status, recon_ws;
     size_t recon_ws_bytes = 0;
     QuantBufs q_direct, q_u, q_s, q_v;
     TopkBufs outlier, err;
@@ -247,7 +247,7 @@ struct Runtime {
 
     void release() {
         if (stream) cudaStreamSynchronize(stream);
-        input_stage.release(); residual.release(); recon.release(); error.release();
+        input_stage.release(); residual.release(); error.release();
         u.release(); s.release(); v.release(); scratch.release(); status.release(); recon_ws.release();
         q_direct.release(); q_u.release(); q_s.release(); q_v.release();
         outlier.release(); err.release();
@@ -327,7 +327,7 @@ bool setup_runtime(Runtime &rt, bool compress, uint16_t rows, uint16_t cols, flo
     if (compress) {
         if (input_location == BITSQZ_LLM_INPUT_HOST && !rt.input_stage.alloc(n * 4)) return false;
         if (!rt.residual.alloc(n * 4)) return false;
-        if (ke > 0 && (!rt.recon.alloc(n * 4) || !rt.error.alloc(n * 4))) return false;
+        if (ke > 0 && !rt.error.alloc(n * 4)) return false;
     }
     if (has_svd) {
         const size_t r = (size_t)rt.rank;
@@ -497,14 +497,15 @@ bool emit_topk_section(Runtime &rt, const CompressJob &job, const TopkBufs &t, u
     return put_device(rt, job, dst + 8, t.idx.p, cnt * 2) && put_device(rt, job, dst + 8 + cnt * 2, t.val.p, cnt * 4);
 }
 
-// Quantise `d_src` (n elements) into q; d_deq (nullable, may alias d_src) receives the dequantised values.
-bool run_quantize(Runtime &rt, int method, const float *d_src, QuantBufs &q, float *d_deq) {
+// Quantise `d_src` (n elements) into q; d_deq (nullable, may alias d_src) receives the dequantised values, or, with
+// d_error_flag, what they are off by.
+bool run_quantize(Runtime &rt, int method, const float *d_src, QuantBufs &q, float *d_deq, unsigned *d_error_flag = nullptr) {
     cudaError_t err;
     if (method == NF4)
-        err = nf4_quantize(d_src, q.n, q.scales_f32.as<float>(), q.data.as<uint8_t>(), d_deq, rt.sm_count, rt.stream);
+        err = nf4_quantize(d_src, q.n, q.scales_f32.as<float>(), q.data.as<uint8_t>(), d_deq, rt.sm_count, rt.stream, d_error_flag);
     else
         err = nf4dq_quantize(d_src, q.n, q.dq.as<float>(), q.scale_codes.as<uint8_t>(), q.data.as<uint8_t>(), d_deq,
-                             rt.scratch.p, rt.sm_count, rt.stream);
+                             rt.scratch.p, rt.sm_count, rt.stream, d_error_flag);
     return err == cudaSuccess;
 }
 
@@ -686,11 +687,10 @@ int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_p
             mark(); job.ev_recon = job.nev - 1;
         }
     } else if (rt.q_format != quantization_NONE && !fused_front) {
-        if (!run_quantize(rt, rt.q_format, d_src, rt.q_direct, error_path ? rt.recon.as<float>() : nullptr)) return fail();
+        // (the error stage's input comes out of the quantiser: no dequantised matrix, no pass to subtract it)
+        if (!run_quantize(rt, rt.q_format, d_src, rt.q_direct, error_path ? rt.error.as<float>() : nullptr, error_path ? d_status + 1 : nullptr))
+            return fail();
         mark(); job.ev_quant = job.nev - 1;
-        if (error_path)
-            if (residual_error(d_src, rt.recon.as<float>(), n, rt.error.as<float>(), d_status + 1, rt.sm_count, st) != cudaSuccess)
-                return fail();
     }
     if (error_path) {
         if (topk_rows(rt.error.as<float>(), nullptr, rows, cols, ke, rt.err.idx.as<uint16_t>(), rt.err.val.as<float>(),

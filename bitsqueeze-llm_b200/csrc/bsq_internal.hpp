@@ -11,12 +11,13 @@ namespace bsq {
 
 // ---- NF4 / NF4_DQ over a flat array (bsq_quant.cu) ----------------------------------------
 // d_deq_out (nullable): also write the dequantised values, which is what the reference's
-// compress path feeds into its error-correction stage (src/bitsqz_llm.cu:506-511).
+// compress path feeds into its error-correction stage (src/bitsqz_llm.cu:506-511).  With d_error_flag (a device word) the
+// second output is x - dequantised instead, and the word is set to 1 when some |difference| > FLT_EPSILON.
 cudaError_t nf4_quantize(const float *d_x, uint64_t n, float *d_scales, uint8_t *d_data, float *d_deq_out, int sm_count,
-                         cudaStream_t stream);
+                         cudaStream_t stream, unsigned *d_error_flag = nullptr);
 size_t nf4dq_scratch_bytes(uint64_t n);
 cudaError_t nf4dq_quantize(const float *d_x, uint64_t n, float *d_dq, uint8_t *d_scale_codes, uint8_t *d_data,
-                           float *d_deq_out, void *d_scratch, int sm_count, cudaStream_t stream);
+                           float *d_deq_out, void *d_scratch, int sm_count, cudaStream_t stream, unsigned *d_error_flag = nullptr);
 // Variant for callers that must not allocate: scratch is a fixed array inside the library.
 uint64_t nf4dq_static_max_elements();
 cudaError_t nf4dq_quantize_static(const float *d_x, uint64_t n, float *d_dq, uint8_t *d_scale_codes, uint8_t *d_data,

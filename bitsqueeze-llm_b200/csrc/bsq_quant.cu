@@ -101,12 +101,17 @@ __global__ void __launch_bounds__(kThreads) absmax_flat_kernel(const float *__re
 }
 
 // ---- encode: NF4 (DQ == false: computes its own absmax) or NF4_DQ pass 2 -----------------
-template <bool DQ, bool WRITE_DEQ>
+// What the encoder writes beside codes and scales: nothing, the dequantised values, or what the quantiser got wrong,
+// x - dequantised, with *flag |= any(|.| > FLT_EPSILON) (the reference's subtract_kernel + has_nonzero_kernel,
+// src/bitsqz_llm.cu:164-184: without a pass of its own over two matrices).
+enum : int { kWriteNone = 0, kWriteDeq = 1, kWriteError = 2 };
+template <bool DQ, int WRITE>
 __global__ void __launch_bounds__(kThreads)
     encode_flat_kernel(const float *x, uint64_t n, bool vec, const float *__restrict__ absmax_in,
                        const unsigned *__restrict__ gmax_bits, float *__restrict__ scales_f32,
                        uint8_t *__restrict__ scale_codes, float *__restrict__ dq_out, uint8_t *__restrict__ data,
-                       float *deq_out) {   // deq_out may alias x (in-place write-back)
+                       float *deq_out, unsigned *flag) {   // deq_out may alias x (in-place write-back)
+    bool any = false;
     const int lane = threadIdx.x & 31;
     const uint64_t warp = (uint64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     const uint64_t nwarps = (uint64_t)gridDim.x * (kThreads / 32);
@@ -159,11 +164,18 @@ __global__ void __launch_bounds__(kThreads)
 #pragma unroll
                 for (int q = 0; q < 8; ++q) c[q] = nf4_code_scan(__fmul_rn(sanitize(r[it].v[q]), invb));
             }
-            if (WRITE_DEQ) {
+            if (WRITE != kWriteNone) {
                 const float sb = __shfl_sync(kFullMask, scale, j);
                 float d[8];
 #pragma unroll
                 for (int q = 0; q < 8; ++q) d[q] = __fmul_rn(sb, lut.decode(c[q]));
+                if (WRITE == kWriteError) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        d[q] = __fsub_rn(r[it].v[q], d[q]);
+                        any |= e + q < n && fabsf(d[q]) > 1.1920928955078125e-07f;
+                    }
+                }
                 if (vec && e + 8 <= n) {
                     reinterpret_cast<float4 *>(deq_out + e)[0] = make_float4(d[0], d[1], d[2], d[3]);
                     reinterpret_cast<float4 *>(deq_out + e)[1] = make_float4(d[4], d[5], d[6], d[7]);
@@ -193,6 +205,7 @@ __global__ void __launch_bounds__(kThreads)
             }
         }
     }
+    if (WRITE == kWriteError && __any_sync(kFullMask, any) && lane == 0) atomicOr(flag, 1u);
 }
 
 // ---- decode ----------------------------------------------------------------------------------
@@ -291,22 +304,25 @@ inline int grid_for(uint64_t n, int sm_count) {
 }  // namespace
 
 cudaError_t nf4_quantize(const float *d_x, uint64_t n, float *d_scales, uint8_t *d_data, float *d_deq_out, int sm_count,
-                         cudaStream_t stream) {
+                         cudaStream_t stream, unsigned *d_error_flag) {
     const bool vec = aligned(d_x, 16) && aligned(d_data, 4) && (!d_deq_out || aligned(d_deq_out, 16));
     const int grid = grid_for(n, sm_count);
-    if (d_deq_out)
-        encode_flat_kernel<false, true><<<grid, kThreads, 0, stream>>>(d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
-                                                                         nullptr, d_data, d_deq_out);
+    if (d_deq_out && d_error_flag)
+        encode_flat_kernel<false, kWriteError><<<grid, kThreads, 0, stream>>>(d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
+                                                                         nullptr, d_data, d_deq_out, d_error_flag);
+    else if (d_deq_out)
+        encode_flat_kernel<false, kWriteDeq><<<grid, kThreads, 0, stream>>>(d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
+                                                                         nullptr, d_data, d_deq_out, nullptr);
     else
-        encode_flat_kernel<false, false><<<grid, kThreads, 0, stream>>>(d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
-                                                                          nullptr, d_data, nullptr);
+        encode_flat_kernel<false, kWriteNone><<<grid, kThreads, 0, stream>>>(d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
+                                                                          nullptr, d_data, nullptr, nullptr);
     return cudaGetLastError();
 }
 
 size_t nf4dq_scratch_bytes(uint64_t n) { return (size_t)((n + 63) / 64) * sizeof(float) + 16; }
 
 cudaError_t nf4dq_quantize(const float *d_x, uint64_t n, float *d_dq, uint8_t *d_scale_codes, uint8_t *d_data,
-                           float *d_deq_out, void *d_scratch, int sm_count, cudaStream_t stream) {
+                           float *d_deq_out, void *d_scratch, int sm_count, cudaStream_t stream, unsigned *d_error_flag) {
     // scratch layout: [0,16) global-max word (+ padding), then one float per block
     unsigned *gmax = static_cast<unsigned *>(d_scratch);
     float *absmax = reinterpret_cast<float *>(static_cast<uint8_t *>(d_scratch) + 16);
@@ -315,12 +331,15 @@ cudaError_t nf4dq_quantize(const float *d_x, uint64_t n, float *d_dq, uint8_t *d
     cudaError_t err = cudaMemsetAsync(gmax, 0, 16, stream);
     if (err != cudaSuccess) return err;
     absmax_flat_kernel<<<grid, kThreads, 0, stream>>>(d_x, n, vec, absmax, gmax);
-    if (d_deq_out)
-        encode_flat_kernel<true, true><<<grid, kThreads, 0, stream>>>(d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
-                                                                        d_dq, d_data, d_deq_out);
+    if (d_deq_out && d_error_flag)
+        encode_flat_kernel<true, kWriteError><<<grid, kThreads, 0, stream>>>(d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
+                                                                        d_dq, d_data, d_deq_out, d_error_flag);
+    else if (d_deq_out)
+        encode_flat_kernel<true, kWriteDeq><<<grid, kThreads, 0, stream>>>(d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
+                                                                        d_dq, d_data, d_deq_out, nullptr);
     else
-        encode_flat_kernel<true, false><<<grid, kThreads, 0, stream>>>(d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
-                                                                         d_dq, d_data, nullptr);
+        encode_flat_kernel<true, kWriteNone><<<grid, kThreads, 0, stream>>>(d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
+                                                                         d_dq, d_data, nullptr, nullptr);
     return cudaGetLastError();
 }
 
