@@ -285,6 +285,17 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
         }
         const size_t image_room = with_image ? gemm_tc_image_bytes(N, t.n_tile, K) : 0;
         if (with_image) workspace_bytes = (workspace_bytes - image_room) & ~(size_t)127;
+        // Few row tiles and a short K (a panel times a k x k factor, a Gram matrix of a short panel): narrower tiles until
+        // three quarters of the SMs have one.  A CTA's time is the chain of its chunks of K whatever its width, but
+        // splitting its piece of B is most of a chunk; below 64 columns, or with more CTAs than that, every tile splits A
+        // once more and the time goes up again.  8192 x 256 x 256: 22.8 -> 19.0 us, 4096 x 256 x 256: 22.8 -> 16.7 us, the
+        // Gram matrix of 4096 x 256 with its reduction 26.9 -> 20.8 us, 8192 x 128 x 128: 12.5 -> 11.0 us; tiles for twice
+        // the SMs measured 37.3 us (14336 x 256 x 256, 24.7 with one 256-column tile per row tile).
+        if (!with_image && !kscale && !minuend && N <= 256) {
+            const int most_splits = workspace ? max(1, K / 256) : 1;
+            while (t.n_tile >= 128 && ((M + 127) / 128) * ((N + t.n_tile - 1) / t.n_tile) * most_splits * 4 < sm_count * 3)
+                t.n_tile = (t.n_tile / 2 + 15) / 16 * 16;
+        }
         const int tiles_tc = ((M + 127) / 128) * ((N + t.n_tile - 1) / t.n_tile);
         int splits_tc = 1;
         if (with_image) {
