@@ -988,13 +988,19 @@ bool locate_topk(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, const
            cudaMemcpyAsync(bufs.val.p, src + cnt * 2, cnt * 4, cudaMemcpyDefault, rt.stream) == cudaSuccess;
 }
 
-bool apply_topk_section(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, const bitsqz_section_t &s, const TopkHeader &h,
-                        TopkBufs &bufs, float *d_dst) {
-    if ((size_t)h.num_rows * h.num_topk_columns == 0) return true;
-    const uint16_t *idx = nullptr;
-    const float *val = nullptr;
-    if (!locate_topk(rt, c, on_device, s, h, bufs, &idx, &val)) return false;
-    return topk_apply(idx, val, h.num_rows, h.num_columns, h.num_topk_columns, d_dst, rt.status.as<unsigned>(), rt.stream) == cudaSuccess;
+// The object's lists onto the decoded matrix: error first, outliers second (src/bitsqz_llm.cu:1372-1387).
+bool apply_lists(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, const SectionHeads &heads, bool has_err, bool has_out, float *d_dst) {
+    const uint16_t *idx[2] = {};
+    const float *val[2] = {};
+    const uint32_t ke = has_err ? heads.err.num_topk_columns : 0, ko = has_out ? heads.outlier.num_topk_columns : 0;
+    if (ke && !locate_topk(rt, c, on_device, c->section_error_topk, heads.err, rt.err, &idx[0], &val[0])) return false;
+    if (ko && !locate_topk(rt, c, on_device, c->section_outlier_topk, heads.outlier, rt.outlier, &idx[1], &val[1])) return false;
+    unsigned *status = rt.status.as<unsigned>();
+    cudaError_t err = cudaSuccess;
+    if (ke && ko) err = topk_apply_two(idx[0], val[0], ke, idx[1], val[1], ko, c->num_rows, c->num_columns, d_dst, status, rt.stream);
+    else if (ke) err = topk_apply(idx[0], val[0], c->num_rows, c->num_columns, ke, d_dst, status, rt.stream);
+    else if (ko) err = topk_apply(idx[1], val[1], c->num_rows, c->num_columns, ko, d_dst, status, rt.stream);
+    return err == cudaSuccess;
 }
 
 // Enqueue one decompress call (src/bitsqz_llm.cu:1304-1393).  `c` is the 200-byte header in host memory; its payload
@@ -1052,11 +1058,7 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
     } else {
         if (!decode_section(rt, c, payload_on_device, c->section_direct, heads.direct, c->quantization_only_format, c->num_elements, &rt.q_direct, d_dst)) return fail();
     }
-    if (!lists_done) {
-        // error first, outliers second (src/bitsqz_llm.cu:1372-1387)
-        if (has_err && !apply_topk_section(rt, c, payload_on_device, c->section_error_topk, heads.err, rt.err, d_dst)) return fail();
-        if (has_out && !apply_topk_section(rt, c, payload_on_device, c->section_outlier_topk, heads.outlier, rt.outlier, d_dst)) return fail();
-    }
+    if (!lists_done && !apply_lists(rt, c, payload_on_device, heads, has_err, has_out, d_dst)) return fail();
     if (cudaMemcpyAsync(rt.h_status, rt.status.p, 64, cudaMemcpyDeviceToHost, st) != cudaSuccess) return fail();
     rt.decompress_active = true;
     return 0;
