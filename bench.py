@@ -49,7 +49,7 @@ WORKLOAD = ("configs[4]: 32 independent 4096x14336 FP32 matrices, outlier_topk=0
             "U/V NF4, S FP32, error_correction_topk=0.01, compress+decompress, matrix i on rank i % N")
 # kernels this library launches per matrix in this configuration, counted from an ncu launch list of
 # `python bench.py --single C5A` (all launches of the run, minus the decompress calls', divided by the compress calls)
-LAUNCHES_PER_COMPRESS = 59
+LAUNCHES_PER_COMPRESS = 67
 LAUNCHES_PER_DECOMPRESS = 9
 # DRAM bytes of one 4096x14336x256 product launch of gemm_tc_tma_kernel (ncu, read + write): 239.8-242.7 MB for W X (matrix
 # read along M), 250.0-251.9 MB for W^T X (read along K); the matrix itself is 234.9 MB, so it is read once.

@@ -21,6 +21,7 @@
 // the k x k core.  Everything that touches an M- or N-sized array is a kernel of this library.
 // Omega comes from cuRAND's XORWOW generator like the reference's (svd_lowrank_cuda.cu:143,289-291),
 // seeded per call, column-major N x k.
+#include "bsq_cholesky.cuh"
 #include "bsq_device.cuh"
 #include "bsq_gemm.hpp"
 #include "bsq_internal.hpp"
@@ -46,6 +47,7 @@ struct SvdWorkspace {
     float *w = nullptr;                 // k eigenvalues
     float *t = nullptr, *tinv1 = nullptr, *tinv2 = nullptr, *core = nullptr;   // k x k
     float *uc = nullptr, *vc = nullptr; // k x k outputs of the core SVD
+    float *rfac = nullptr, *dinv = nullptr;    // k x k factor that nobody asked for; 1 / its diagonal
     float *gemm_ws = nullptr;
     size_t gemm_ws_bytes = 0;
     float *solver_work = nullptr;
@@ -233,265 +235,6 @@ __global__ void __launch_bounds__(1024) cholesky_inverse_smem_kernel(const float
     for (int e = tid; e < k * k; e += nt) {
         const int i = e / k, c = e % k;
         if (c >= i) T[e] = P[row_off(i) + c];
-    }
-}
-
-// The same again for k <= kCholeskyBlockedMaxK, by 32 x 32 blocks, which takes the number of CTA-wide barriers from
-// four per column to a handful per block column.  The block-upper-triangular matrix lives in shared memory
-// (block (I, J), I <= J, at blk_id(I, J)); k is padded to a multiple of 32 with an identity.
-//   factorisation, per block column J: warp 0 factors the diagonal block in registers (one column per lane, the
-//       pivot row travels by shuffles); every thread then solves one column of the block row against it
-//       (R_JJ^T Y = G_JC, forward substitution), and all threads apply the rank-32 update to the trailing blocks;
-//       every sum runs in the order of the unblocked algorithm (the pivots use a reciprocal square root, so R agrees
-//       with it to rounding, not bit for bit);
-//   inverse: the diagonal blocks are inverted by one warp each, all at once; block column J of T = R^-1 is then
-//       T_IJ = -(sum_{L=I..J-1} T_IL R_LJ) T_JJ, two rounds of 32 x 32 block products per column.
-constexpr int kCholeskyBlockedMaxK = 256;
-constexpr int kCB = 32;
-__host__ __device__ constexpr int chol_blocks(int k) { return (k + kCB - 1) / kCB; }
-__host__ __device__ constexpr size_t cholesky_blocked_smem_bytes(int k) {
-    // packed blocks + inverted diagonal blocks + one temporary block column + 1 / diagonal + scalars
-    return ((size_t)(chol_blocks(k) * (chol_blocks(k) + 1) / 2 + 2 * chol_blocks(k)) * kCB * kCB + (size_t)chol_blocks(k) * kCB + 64) *
-           sizeof(float);
-}
-__device__ __forceinline__ int blk_id(int I, int J, int nb) { return I * nb - (I * (I - 1)) / 2 + (J - I); }
-
-// Sixteen 32 x 32 block products at a time: 64 threads per product, 4 x 4 outputs per thread (rows 4 ti .. + 3,
-// columns 4 tc .. + 3), operands read as float4: 2 shared-memory loads per 16 multiply-adds (with 2 x 2 outputs
-// per thread the loads, not the arithmetic, filled the issue slots of the one SM this kernel runs on).
-//   out -= A^T B  (AT = true:  A, B hold the contraction index in rows)
-//   out += A B    (AT = false: A holds it in columns)
-template <bool AT>
-__device__ __forceinline__ void block_mac(float (&acc)[4][4], const float *__restrict__ A, const float *__restrict__ B, int ti, int tc) {
-    if (AT) {
-#pragma unroll 4
-        for (int l = 0; l < kCB; ++l) {
-            const float4 a = *reinterpret_cast<const float4 *>(A + l * kCB + 4 * ti);
-            const float4 b = *reinterpret_cast<const float4 *>(B + l * kCB + 4 * tc);
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) acc[r][q] = fmaf(-av[r], bv[q], acc[r][q]);
-        }
-    } else {
-#pragma unroll 2
-        for (int l0 = 0; l0 < kCB; l0 += 4) {
-            float4 a[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4 *>(A + (4 * ti + r) * kCB + l0);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float4 b = *reinterpret_cast<const float4 *>(B + (l0 + u) * kCB + 4 * tc);
-                const float bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const float ar = u == 0 ? a[r].x : (u == 1 ? a[r].y : (u == 2 ? a[r].z : a[r].w));
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) acc[r][q] += ar * bv[q];
-                }
-            }
-        }
-    }
-}
-// a thread's 4 x 4 tile of a block, as four float4
-__device__ __forceinline__ void tile_load(float (&acc)[4][4], const float *O, int ti, int tc) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const float4 v = *reinterpret_cast<const float4 *>(O + (4 * ti + r) * kCB + 4 * tc);
-        acc[r][0] = v.x; acc[r][1] = v.y; acc[r][2] = v.z; acc[r][3] = v.w;
-    }
-}
-__device__ __forceinline__ void tile_store(const float (&acc)[4][4], float *O, int ti, int tc, float sign) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-        *reinterpret_cast<float4 *>(O + (4 * ti + r) * kCB + 4 * tc) =
-            make_float4(sign * acc[r][0], sign * acc[r][1], sign * acc[r][2], sign * acc[r][3]);
-}
-
-__global__ void __launch_bounds__(1024) cholesky_inverse_blocked_kernel(const float *__restrict__ G, int k, float *__restrict__ T,
-                                                                        float *__restrict__ Rcpy) {
-    extern __shared__ __align__(16) float sm[];
-    const int nb = chol_blocks(k), nbt = nb * (nb + 1) / 2;
-    float *blocks = sm;                                    // nbt blocks of 32 x 32, row-major
-    float *tinv = blocks + (size_t)nbt * kCB * kCB;        // nb inverted diagonal blocks
-    float *tmp = tinv + (size_t)nb * kCB * kCB;            // nb blocks: one block column of partial products
-    float *dinv = tmp + (size_t)nb * kCB * kCB;            // 1 / R(i, i)
-    float *red = dinv + nb * kCB;                          // 32 + 1
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-    const int bi = tid >> 5, bc = tid & 31;               // this thread's element of a block when the CTA walks blocks
-    const int part = tid >> 6, ti = (tid & 63) >> 3, tc = tid & 7;         // ... and its 4 x 4 tile of its sixteenth's block
-    // load block by block (row bi, column bc of each), padded with an identity; what lies below the diagonal of a
-    // diagonal block is never read.  Four blocks per trip, so that four global loads are in flight per thread.
-    float md = 0.0f;
-    for (int b0 = 0; b0 < nbt; b0 += 4) {
-        float v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int b = b0 + u;
-            v[u] = 0.0f;
-            if (b < nbt) {
-                int I = 0, rem = b;
-                while (rem >= nb - I) { rem -= nb - I; ++I; }      // block (I, I + rem)
-                const int i = I * kCB + bi, c = (I + rem) * kCB + bc;
-                v[u] = (i == c) ? 1.0f : 0.0f;
-                if (i < k && c < k) v[u] = G[(size_t)i * k + c];
-                if (i == c && i < k) md = fmaxf(md, v[u]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (b0 + u < nbt) blocks[(size_t)(b0 + u) * kCB * kCB + tid] = v[u];
-    }
-    for (int d = 16; d > 0; d >>= 1) md = fmaxf(md, __shfl_xor_sync(0xffffffffu, md, d));
-    if (lane == 0) red[warp] = md;
-    __syncthreads();
-    if (tid == 0) {
-        float m = 0.0f;
-        for (int w = 0; w < nwarps; ++w) m = fmaxf(m, red[w]);
-        red[32] = m > 0.0f ? m * 1.0e-5f : 0.0f;
-    }
-    __syncthreads();
-    const float shift = red[32];
-    for (int i = tid; i < k; i += nt) blocks[(size_t)blk_id(i / kCB, i / kCB, nb) * kCB * kCB + (i % kCB) * (kCB + 1)] += shift;
-    __syncthreads();
-
-    for (int J = 0; J < nb; ++J) {
-        float *D = blocks + (size_t)blk_id(J, J, nb) * kCB * kCB;
-        if (warp == 0) {                                    // diagonal block: lane c keeps column c
-            float a[kCB];
-#pragma unroll
-            for (int i = 0; i < kCB; ++i) a[i] = D[i * kCB + lane];
-            float my_inv = 0.0f;
-#pragma unroll
-            for (int j = 0; j < kCB; ++j) {
-                float d = __shfl_sync(0xffffffffu, a[j], j);
-                if (!(d > 0.5f * shift)) d = 0.5f * shift;
-                // the 32 pivots of a block are one dependent chain: reciprocal square root from the special-function
-                // unit plus one Newton step (a relative error of ~1e-7 in R(j, j) and 1 / R(j, j) alike) instead of
-                // an IEEE square root followed by an IEEE division
-                float inv = 0.0f;
-                if (d > 0.0f) {
-                    inv = rsqrtf(d);
-                    inv = inv * (1.5f - 0.5f * d * inv * inv);
-                }
-                const float r = d * inv;
-                a[j] = (lane == j) ? r : a[j] * inv;
-                if (lane == j) my_inv = inv;
-#pragma unroll
-                for (int i = j + 1; i < kCB; ++i) {
-                    const float rji = __shfl_sync(0xffffffffu, a[j], i);
-                    a[i] -= rji * a[j];
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < kCB; ++i) D[i * kCB + lane] = (i <= lane) ? a[i] : 0.0f;
-            dinv[J * kCB + lane] = my_inv;
-        }
-        __syncthreads();
-        // block row J: one thread per column, forward substitution with R_JJ^T
-        for (int col = tid; col < (nb - J - 1) * kCB; col += nt) {
-            float *X = blocks + (size_t)blk_id(J, J + 1 + col / kCB, nb) * kCB * kCB + col % kCB;
-            float y[kCB];
-#pragma unroll
-            for (int i = 0; i < kCB; ++i) {
-                float acc = X[i * kCB];
-#pragma unroll
-                for (int l = 0; l < i; ++l) acc -= D[l * kCB + i] * y[l];
-                y[i] = acc * dinv[J * kCB + i];
-            }
-#pragma unroll
-            for (int i = 0; i < kCB; ++i) X[i * kCB] = y[i];
-        }
-        __syncthreads();
-        // trailing blocks (A, B), J < A <= B: G_AB -= R_JA^T R_JB, sixteen blocks per trip
-        {
-            const int rest = nb - J - 1, pairs = rest * (rest + 1) / 2;
-            for (int pr0 = 0; pr0 < pairs; pr0 += 16) {
-                const int pr = pr0 + part;
-                if (pr < pairs) {
-                    int A = 0, rem = pr;
-                    while (rem >= rest - A) { rem -= rest - A; ++A; }
-                    const int B = A + rem;
-                    const float *RA = blocks + (size_t)blk_id(J, J + 1 + A, nb) * kCB * kCB;
-                    const float *RB = blocks + (size_t)blk_id(J, J + 1 + B, nb) * kCB * kCB;
-                    float *O = blocks + (size_t)blk_id(J + 1 + A, J + 1 + B, nb) * kCB * kCB;
-                    float acc[4][4];
-                    tile_load(acc, O, ti, tc);
-                    block_mac<true>(acc, RA, RB, ti, tc);
-                    tile_store(acc, O, ti, tc, 1.0f);
-                }
-            }
-        }
-        __syncthreads();
-    }
-    // R out and the zeros below the diagonal of R and T, block by block; the diagonal blocks' inverses, one warp each
-    for (int I = 0; I < nb; ++I) {
-        for (int Jb = 0; Jb < nb; ++Jb) {
-            const int i = I * kCB + bi, c = Jb * kCB + bc;
-            if (i < k && c < k) {
-                const size_t e = (size_t)i * k + c;
-                if (c < i) {
-                    if (T) T[e] = 0.0f;
-                    if (Rcpy) Rcpy[e] = 0.0f;
-                } else if (Rcpy) {
-                    Rcpy[e] = blocks[(size_t)blk_id(I, Jb, nb) * kCB * kCB + tid];
-                }
-            }
-        }
-    }
-    if (!T) return;                                         // only the factor was wanted (uniform over the CTA)
-    if (warp < nb) {
-        const float *D = blocks + (size_t)blk_id(warp, warp, nb) * kCB * kCB;
-        float a[kCB], t[kCB];
-#pragma unroll
-        for (int i = 0; i < kCB; ++i) { a[i] = D[i * kCB + lane]; t[i] = 0.0f; }
-        const float my_inv = dinv[warp * kCB + lane];
-#pragma unroll
-        for (int i = kCB - 1; i >= 0; --i) {
-            float acc = (lane == i) ? 1.0f : 0.0f;
-#pragma unroll
-            for (int l = i + 1; l < kCB; ++l) acc -= __shfl_sync(0xffffffffu, a[i], l) * t[l];
-            const float inv = __shfl_sync(0xffffffffu, my_inv, i);
-            t[i] = (lane >= i) ? acc * inv : 0.0f;
-        }
-#pragma unroll
-        for (int i = 0; i < kCB; ++i) tinv[(size_t)warp * kCB * kCB + i * kCB + lane] = t[i];
-    }
-    __syncthreads();
-    // block column J of T, from the left: needs T_IL for L < J (already in place) and R_LJ (still in place)
-    for (int J = 1; J < nb; ++J) {
-        for (int I0 = 0; I0 < J; I0 += 16) {
-            const int I = I0 + part;
-            if (I < J) {
-                float acc[4][4] = {};
-                for (int L = I; L < J; ++L) {
-                    const float *TL = (L == I) ? tinv + (size_t)I * kCB * kCB : blocks + (size_t)blk_id(I, L, nb) * kCB * kCB;
-                    block_mac<false>(acc, TL, blocks + (size_t)blk_id(L, J, nb) * kCB * kCB, ti, tc);
-                }
-                tile_store(acc, tmp + (size_t)I * kCB * kCB, ti, tc, 1.0f);
-            }
-        }
-        __syncthreads();
-        const float *TJ = tinv + (size_t)J * kCB * kCB;
-        for (int I0 = 0; I0 < J; I0 += 16) {
-            const int I = I0 + part;
-            if (I < J) {
-                float acc[4][4] = {};
-                block_mac<false>(acc, tmp + (size_t)I * kCB * kCB, TJ, ti, tc);
-                tile_store(acc, blocks + (size_t)blk_id(I, J, nb) * kCB * kCB, ti, tc, -1.0f);
-            }
-        }
-        __syncthreads();
-    }
-    for (int I = 0; I < nb; ++I) {
-        for (int Jb = I; Jb < nb; ++Jb) {
-            const int i = I * kCB + bi, c = Jb * kCB + bc;
-            if (i < k && c < k && c >= i) {
-                const float *src = (I == Jb) ? tinv + (size_t)I * kCB * kCB : blocks + (size_t)blk_id(I, Jb, nb) * kCB * kCB;
-                T[(size_t)i * k + c] = src[tid];
-            }
-        }
     }
 }
 
@@ -972,9 +715,14 @@ cudaError_t orthonormalise(SvdWorkspace *ws, float *Y, float *tmp, int rows, int
         // a row-sharded panel: its Gram matrix is the sum of the shards' (the one exchange per QR pass);
         // every rank then factors the same k x k matrix and gets bit-identical R
         if (sharded_rows && ws->allreduce && (err = timed_allreduce(ws, ws->g, (size_t)k * k, st)) != cudaSuccess) return err;
-        if (k <= kCholeskyBlockedMaxK) {
-            cholesky_inverse_blocked_kernel<<<1, 1024, cholesky_blocked_smem_bytes(k), st>>>(ws->g, k, factor_only ? nullptr : ws->t,
-                                                                                                pass == 0 ? r_a : r_b);
+        if (k <= kCholeskySmallMaxK) {
+            cholesky_small_kernel<<<1, 1024, cholesky_small_smem_bytes(k), st>>>(ws->g, k, factor_only ? nullptr : ws->t, pass == 0 ? r_a : r_b);
+        } else if (k <= kCholeskyBlockedMaxK) {
+            float *r_out = pass == 0 ? r_a : r_b;
+            if (!r_out) r_out = ws->rfac;
+            cholesky_factor_kernel<<<1, kCholThreads, cholesky_factor_smem_bytes(k), st>>>(ws->g, k, r_out, ws->dinv);
+            if (!factor_only)
+                cholesky_inverse_blocked_kernel<<<chol_blocks(k), kCholInvThreads, cholesky_inverse_smem_bytes(k), st>>>(r_out, ws->dinv, k, ws->t);
         } else if (k <= kCholeskySmemMaxK) {
             cholesky_inverse_smem_kernel<<<1, 1024, cholesky_smem_bytes(k), st>>>(ws->g, k, ws->t, pass == 0 ? r_a : r_b);
         } else {
@@ -1039,7 +787,8 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
               alloc_f(&ws->y2, (size_t)ws->M * ws->k) && alloc_f(&ws->z, (size_t)ws->N * ws->k) &&
               alloc_f(&ws->z2, (size_t)ws->N * ws->k) && alloc_f(&ws->g, kk) && alloc_f(&ws->w, ws->k) &&
               alloc_f(&ws->t, kk) && alloc_f(&ws->tinv1, kk) && alloc_f(&ws->tinv2, kk) && alloc_f(&ws->core, kk) &&
-              alloc_f(&ws->uc, kk) && alloc_f(&ws->vc, kk);
+              alloc_f(&ws->uc, kk) && alloc_f(&ws->vc, kk) && alloc_f(&ws->rfac, kk) &&
+              alloc_f(&ws->dinv, (size_t)chol_blocks(ws->k) * kCB);
     // split-K partials: up to 2 * SMs tiles' worth of the largest skinny product, and of the Gram matrix
     // K-split partials, and behind them room for the images of a product's second operand split beforehand
     ws->gemm_ws_bytes = std::max((size_t)ws->M * ws->k * 8, kk * 2 * (size_t)sm_count) * sizeof(float) +
@@ -1099,9 +848,14 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
             }
         }
     }
-    if (ok && ws->k <= kCholeskyBlockedMaxK)
-        ok = cudaFuncSetAttribute(cholesky_inverse_blocked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)cholesky_blocked_smem_bytes(ws->k)) == cudaSuccess;
+    if (ok && ws->k <= kCholeskySmallMaxK)
+        ok = cudaFuncSetAttribute(cholesky_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)cholesky_small_smem_bytes(ws->k)) == cudaSuccess;
+    else if (ok && ws->k <= kCholeskyBlockedMaxK)
+        ok = cudaFuncSetAttribute(cholesky_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)cholesky_factor_smem_bytes(ws->k)) == cudaSuccess &&
+             cudaFuncSetAttribute(cholesky_inverse_blocked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)cholesky_inverse_smem_bytes(ws->k)) == cudaSuccess;
     else if (ok && ws->k <= kCholeskySmemMaxK)
         ok = cudaFuncSetAttribute(cholesky_inverse_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)cholesky_smem_bytes(ws->k)) == cudaSuccess;
@@ -1116,7 +870,7 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
 void svd_workspace_destroy(SvdWorkspace *ws) {
     if (!ws) return;
     float *bufs[] = {ws->omega, ws->y, ws->y2, ws->z, ws->z2, ws->g, ws->w, ws->t, ws->tinv1, ws->tinv2,
-                     ws->core, ws->uc, ws->vc, ws->gemm_ws, ws->solver_work};
+                     ws->core, ws->uc, ws->vc, ws->rfac, ws->dinv, ws->gemm_ws, ws->solver_work};
     for (float *p : bufs)
         if (p) cudaFree(p);
     if (ws->dev_info) cudaFree(ws->dev_info);

@@ -1,0 +1,56 @@
+"""The k x k kernels of the randomized SVD (Cholesky factor and inverse by 32 x 32 blocks, block Jacobi on 1 to 8 CTAs) at the edges
+of their blocks, clusters and paddings, through bsq_svd_lowrank, against FP64 numpy.
+
+Bounds.  Each QR pass factors G + 1e-5 max(diag G) I, so columns are orthonormal to a few 1e-5, up to 2e-4 for the weakest
+direction of a wide sketch (the bounds of test_gpu_svd.py).  With orthonormal Q the residual of Q Q^T A has the squared norm
+|A|^2 - sum S^2: both sides are compared to 1e-3 of |A|^2 (twice the orthonormality bound for the two factors, and FP32 sums)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def svd_gpu(lib, a, k, niter=2):
+    m, n = a.shape
+    d_a = torch.from_numpy(a).cuda()
+    u, s, v = torch.zeros(m, k, device="cuda"), torch.zeros(k, device="cuda"), torch.zeros(n, k, device="cuda")
+    torch.cuda.synchronize()
+    assert lib.bsq_svd_lowrank(d_a.data_ptr(), m, n, k, niter, 1241, u.data_ptr(), s.data_ptr(), v.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    return u.cpu().numpy().astype(np.float64), s.cpu().numpy().astype(np.float64), v.cpu().numpy().astype(np.float64)
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 15, 16, 17, 31, 32, 33, 48, 63, 64, 65, 96, 97, 127, 128, 129, 160, 192, 224, 255, 256])
+@pytest.mark.parametrize("kind", ["noise", "small", "large"])
+def test_core_edges(lib, k, kind):
+    m, n = 640, 528
+    rng = np.random.default_rng(k)
+    a = rng.standard_normal((m, n)) @ np.diag(1.0 / np.arange(1, n + 1)) + 0.02 * rng.standard_normal((m, n))
+    a = (a * {"noise": 1.0, "small": 1e-9, "large": 1e9}[kind]).astype(np.float32)
+    u, s, v = svd_gpu(lib, a, k)
+    exact = np.linalg.svd(a.astype(np.float64), compute_uv=False)
+    norm2 = float((a.astype(np.float64) ** 2).sum())
+    assert np.all(np.diff(s) <= 1e-6 * s[0]) and np.all(s >= 0)
+    assert np.all(s <= exact[:k] * (1 + 2e-4))
+    tol = 1e-4 if k <= 128 else 2e-4
+    assert np.abs(u.T @ u - np.eye(k)).max() <= tol and np.abs(v.T @ v - np.eye(k)).max() <= tol
+    res2 = float(((a - (u * s) @ v.T) ** 2).sum())
+    assert abs(res2 - (norm2 - float((s ** 2).sum()))) <= 1e-3 * norm2
+    u2, s2, v2 = svd_gpu(lib, a, k)                          # the same input gives the same bits
+    assert np.array_equal(u, u2) and np.array_equal(s, s2) and np.array_equal(v, v2)
+
+
+@pytest.mark.parametrize("k", [5, 32, 40, 64, 100, 200, 256])
+def test_core_of_deficient_and_zero_matrices(lib, k):
+    m, n, r = 512, 448, 3
+    rng = np.random.default_rng(k)
+    a = (rng.standard_normal((m, r)) @ rng.standard_normal((r, n))).astype(np.float32)
+    u, s, v = svd_gpu(lib, a, k)
+    exact = np.linalg.svd(a.astype(np.float64), compute_uv=False)[:r]
+    assert np.isfinite(u).all() and np.isfinite(s).all() and np.isfinite(v).all()
+    assert np.max(np.abs(s[:r] - exact) / exact) <= 1e-4     # well-separated values: the contract's bound
+    assert np.all(s[r:] <= 1e-3 * s[0])
+    assert np.linalg.norm(a - (u * s) @ v.T) <= 1e-4 * np.linalg.norm(a)
+    u, s, v = svd_gpu(lib, np.zeros((m, n), np.float32), k)
+    assert np.isfinite(u).all() and np.isfinite(v).all() and not s.any()
