@@ -339,7 +339,8 @@ bool setup_runtime(Runtime &rt, bool compress, uint16_t rows, uint16_t cols, flo
         if (compress) {
             if (uv != quantization_NONE && (!rt.q_u.alloc((uint64_t)rows * r) || !rt.q_v.alloc((uint64_t)cols * r))) return false;
             if (s != quantization_NONE && !rt.q_s.alloc(r)) return false;
-            rt.svd = svd_workspace_create(rows, cols, rt.rank, svd_niters, rt.sm_count);
+            rt.svd = svd_workspace_create(rows, cols, rt.rank, svd_niters, rt.sm_count,
+                                      uv != quantization_NONE || s != quantization_NONE || ke > 0);
             if (!rt.svd) return false;
         }
     } else if (compress && q != quantization_NONE) {

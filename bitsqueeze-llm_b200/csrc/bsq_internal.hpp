@@ -135,9 +135,11 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
 struct SvdWorkspace;
 // sums `count` floats at `buf` over all ranks, enqueued on `stream`
 typedef cudaError_t (*SvdAllReduce)(void *ctx, float *buf, size_t count, cudaStream_t stream);
-SvdWorkspace *svd_workspace_create(int m, int n, int k, int niter, int sm_count);
+// coded_factors: U, S, V are quantised afterwards or an error list is made from them, so that the order of rotations in the
+// core's SVD shows in an object's bytes (bsq_svd.cu)
+SvdWorkspace *svd_workspace_create(int m, int n, int k, int niter, int sm_count, bool coded_factors = false);
 SvdWorkspace *svd_workspace_create_sharded(int m_local, int n, int k, int niter, int sm_count, SvdAllReduce allreduce,
-                                           void *allreduce_ctx, int m_total);
+                                           void *allreduce_ctx, int m_total, bool coded_factors = false);
 void svd_workspace_destroy(SvdWorkspace *ws);
 // A row-major m x n -> U (m x k row-major), S (k, descending), V (n x k row-major).
 // The random matrix is the first N x k normals of cuRAND's XORWOW sequence of `seed`, starting `offset` values in.

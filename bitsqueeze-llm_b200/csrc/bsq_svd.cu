@@ -16,8 +16,8 @@
 //     shorter than unit length instead of dividing by zero;
 //   * the small SVD works on a k x k core: B^T = Q2 C with C = R2 R1 the product of the two
 //     triangular factors, C = Uc S Vc^T, V_hat = Q2 Uc, U = Q Vc.
-// The SVD of the k x k core is a one-sided Jacobi kernel of this library up to 256 columns (one CTA up to 64, a
-// thread-block cluster above); larger cores, and devices that cannot place the cluster, go to cuSOLVER's gesvdj on
+// The SVD of the k x k core is a one-sided Jacobi kernel of this library up to 256 columns (bsq_jacobi.cuh; where the factors
+// are coded afterwards one CTA up to 64, a thread-block cluster above); larger cores, and devices that cannot place the cluster, go to cuSOLVER's gesvdj on
 // the k x k core.  Everything that touches an M- or N-sized array is a kernel of this library.
 // Omega comes from cuRAND's XORWOW generator like the reference's (svd_lowrank_cuda.cu:143,289-291),
 // seeded per call, column-major N x k.
@@ -25,6 +25,7 @@
 #include "bsq_device.cuh"
 #include "bsq_gemm.hpp"
 #include "bsq_internal.hpp"
+#include "bsq_jacobi.cuh"
 
 #include <cooperative_groups.h>
 #include <curand.h>
@@ -35,6 +36,10 @@
 #include <new>
 
 namespace bsq {
+
+// Up to this rank the block Jacobi kernel accumulates the right factor of the core, which keeps V orthonormal for singular
+// values down to rounding; above, V comes from the panel (what the accumulation would cost grows with the rank).
+constexpr int kCoreWithVMaxK = 64;
 
 struct SvdWorkspace {
     int m = 0, n = 0, k = 0, niter = 0, sm_count = 148;
@@ -66,6 +71,7 @@ struct SvdWorkspace {
     const unsigned *a_absmax_use = nullptr;
     int jc_lanes = 4;                   // lanes per column pair of the cluster Jacobi kernel for this k
     bool jc_with_v = false;             // ... and whether it accumulates the right factor (else that comes from the panel)
+    bool block_core = false;            // the core goes to block_jacobi_kernel
     bool own_core_svd = false;          // k small enough for jacobi_svd_kernel (else cuSOLVER's gesvdj on the core)
     bool seeded = false;                // omega holds the draw for `seed`
     unsigned long long seed = 0, offset = 0;
@@ -238,6 +244,11 @@ __global__ void __launch_bounds__(1024) cholesky_inverse_smem_kernel(const float
     }
 }
 
+// The two kernels below serve cores whose factors are coded afterwards (NF4 / NF4_DQ sections, error lists made from them):
+// the codes of a singular pair depend on its sign and, in a flat spectrum, on how the last bits turn neighbouring vectors
+// into one another, so another order of rotations than theirs changes most objects in most bytes (measured: 6 to 8 % of the
+// reconstructed matrix, as large a change as a library solver makes).  Objects keep their bytes; factors that stay in FP32
+// take the block kernel of bsq_jacobi.cuh.
 // SVD of the k x k core for k <= kJacobiMaxK: one-sided (Hestenes) Jacobi in one CTA, everything in shared memory.
 // The reference runs cusolverDnSgesvd on the k x n matrix B (svd_lowrank_cuda.cu:399-440); here only the k x k
 // triangular factor is left to decompose.
@@ -250,12 +261,6 @@ __global__ void __launch_bounds__(1024) cholesky_inverse_smem_kernel(const float
 // U(:, j) = column j / S(j) (zero for S(j) = 0), and a rank by counting puts S in descending order.
 constexpr int kJacobiMaxK = 128;              // what the one-CTA kernel can hold
 constexpr int kJacobiSingleMaxK = 64;         // what it is used for: above, the cluster kernel is faster
-constexpr int kJacobiMaxSweeps = 30;
-// A sweep in which no visited pair had |cos(m_p, m_q)| above this is the last one: Jacobi converges quadratically,
-// so what such a sweep's rotations leave between the columns is of the order of the square of what it met
-// (<= 1e-8, below tol), and the sweep that would only confirm it (a full sweep's time for no rotation) is not run.
-// Pairs between tol and this bound are still rotated when they are met.
-constexpr float kJacobiLastSweepCos = 1.0e-4f;
 __host__ __device__ constexpr int jacobi_len(int k) { return k <= 64 ? 64 : 128; }
 __host__ __device__ constexpr size_t jacobi_smem_bytes(int k) {
     return ((size_t)2 * ((k + 1) & ~1) * jacobi_len(k) + 2 * (size_t)((k + 1) & ~1) + 64) * sizeof(float);
@@ -764,14 +769,14 @@ cudaError_t times_w(SvdWorkspace *ws, const float *A, bool w_transposed_product,
 
 }  // namespace
 
-SvdWorkspace *svd_workspace_create(int m, int n, int k, int niter, int sm_count) {
-    return svd_workspace_create_sharded(m, n, k, niter, sm_count, nullptr, nullptr, 0);
+SvdWorkspace *svd_workspace_create(int m, int n, int k, int niter, int sm_count, bool coded_factors) {
+    return svd_workspace_create_sharded(m, n, k, niter, sm_count, nullptr, nullptr, 0, coded_factors);
 }
 
 // Row-sharded: this rank holds m of the m_total rows (all n columns); the working matrix is never the
 // transpose, so that the sharded dimension is the tall one that only GEMMs touch.
 SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int sm_count, SvdAllReduce allreduce,
-                                           void *allreduce_ctx, int m_total) {
+                                           void *allreduce_ctx, int m_total, bool coded_factors) {
     if (m <= 0 || n <= 0 || k <= 0 || niter < 0) return nullptr;
     SvdWorkspace *ws = new (std::nothrow) SvdWorkspace();
     if (!ws) return nullptr;
@@ -823,10 +828,25 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
         const char *e = getenv("BSQ_CORE_SVD");              // "cusolver": keep the library solver (A/B comparisons)
         ws->own_core_svd = ws->k <= kJacobiClusterMaxK && !(e && e[0] == 'c');
     }
+    if (ok && ws->own_core_svd && !coded_factors) {
+        const char *v = getenv("BSQ_JACOBI_V");
+        ws->jc_with_v = v ? v[0] == '1' : ws->k <= kCoreWithVMaxK;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        block_jacobi_config(&cfg, attr, ws->k, ws->jc_with_v, nullptr);
+        const BlockJacobiFn fn = block_jacobi_fn(ws->k, ws->jc_with_v);
+        int clusters = 0;
+        ws->block_core = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) == cudaSuccess &&
+                         cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters >= 1;
+        if (!ws->block_core) {                               // a device (or partition of one) that cannot place the cluster
+            cudaGetLastError();
+            ws->jc_with_v = false;
+        }
+    }
     if (ok && ws->own_core_svd && ws->k <= kJacobiSingleMaxK)
         ok = cudaFuncSetAttribute(jacobi_svd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)jacobi_smem_bytes(ws->k)) == cudaSuccess;
-    if (ok && ws->own_core_svd && ws->k > kJacobiSingleMaxK) {
+    if (ok && ws->own_core_svd && !ws->block_core && ws->k > kJacobiSingleMaxK) {
         const char *e = getenv("BSQ_JACOBI_LPP");
         ws->jc_lanes = ws->k <= 128 || (e && atoi(e) == 4) ? 4 : 2;
         {
@@ -963,9 +983,9 @@ cudaError_t svd_lowrank(SvdWorkspace *ws, const float *d_A, float *d_U, float *d
             cudaSuccess)
             return err;
     }
-    // B^T = W^T Q = Q2 C with C = R2 R1.  With the cluster Jacobi kernel the right factor comes from the panel B^T
+    // B^T = W^T Q = Q2 C with C = R2 R1.  Where the Jacobi kernel does not accumulate the right factor, that comes from the panel B^T
     // itself (B^T v_j / S(j)), so Q2 is never formed: the second pass only has to deliver R2.
-    const bool from_panel = ws->own_core_svd && k > kJacobiSingleMaxK && !ws->jc_with_v;
+    const bool from_panel = ws->own_core_svd && (k > kJacobiSingleMaxK || ws->block_core) && !ws->jc_with_v;
     if ((err = times_w(ws, d_A, true, q, false, ws->z, st)) != cudaSuccess) return err;
     if ((err = orthonormalise(ws, ws->z, ws->z2, ws->N, 2, ws->tinv1, ws->tinv2, &qz, false, st, from_panel)) != cudaSuccess) return err;
     if (from_panel) qz = ws->z;
@@ -973,7 +993,14 @@ cudaError_t svd_lowrank(SvdWorkspace *ws, const float *d_A, float *d_U, float *d
                     ws->sm_count, st)) != cudaSuccess)
         return err;
     // The row-major C read as column-major is C^T = Vc S Uc^T: the solver's "U" is Vc, its "V" is Uc.
-    if (ws->own_core_svd && k > kJacobiSingleMaxK) {
+    if (ws->block_core) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        block_jacobi_config(&cfg, attr, k, ws->jc_with_v, st);
+        const float *core = ws->core;
+        float *vc = ws->vc, *uc = ws->uc;
+        if ((err = cudaLaunchKernelEx(&cfg, block_jacobi_fn(k, ws->jc_with_v), core, k, d_S, vc, uc)) != cudaSuccess) return err;
+    } else if (ws->own_core_svd && k > kJacobiSingleMaxK) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
         jacobi_cluster_config(&cfg, attr, k, ws->jc_lanes, st);
