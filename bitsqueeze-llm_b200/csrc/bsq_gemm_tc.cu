@@ -514,15 +514,27 @@ __global__ void __launch_bounds__(256) presplit_a_kernel(const float *__restrict
 // longer matters: the product is NaN or Inf then, as it is for the reference.
 __global__ void __launch_bounds__(256) absmax_bits_kernel(const float *__restrict__ x, long ld, int rows, int cols, unsigned *out,
                                                           const float *__restrict__ colscale = nullptr) {
-    const int c4 = cols / 4;
+    const unsigned c4 = cols / 4;
     unsigned m = 0;
-    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < (long)rows * c4; e += (long)gridDim.x * blockDim.x) {
-        float4 v = *reinterpret_cast<const float4 *>(x + (e / c4) * ld + (e % c4) * 4);
-        if (colscale) {
-            const int c = (int)(e % c4) * 4;
-            v.x *= colscale[c]; v.y *= colscale[c + 1]; v.z *= colscale[c + 2]; v.w *= colscale[c + 3];
-        }
+    auto take = [&](float4 v, unsigned c) {
+        if (colscale) { v.x *= colscale[4 * c]; v.y *= colscale[4 * c + 1]; v.z *= colscale[4 * c + 2]; v.w *= colscale[4 * c + 3]; }
         m = max(max(m, __float_as_uint(v.x) & 0x7fffffffu), max(__float_as_uint(v.y) & 0x7fffffffu, max(__float_as_uint(v.z) & 0x7fffffffu, __float_as_uint(v.w) & 0x7fffffffu)));
+    };
+    if (ld == cols) {
+        // rows without gaps are one array: no row and column to work out (64-bit divisions, most of the time before), four
+        // loads in flight per thread.  14336 x 256: 10.7 -> 7.2 us.
+        const size_t total = (size_t)rows * c4, stride = (size_t)gridDim.x * blockDim.x;
+        const float4 *x4 = reinterpret_cast<const float4 *>(x);
+        for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += 4 * stride) {
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = e + u * stride < total ? x4[e + u * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) take(v[u], colscale && e + u * stride < total ? (unsigned)((e + u * stride) % c4) : 0u);
+        }
+    } else {
+        for (int r = blockIdx.x; r < rows; r += gridDim.x)
+            for (unsigned c = threadIdx.x; c < c4; c += blockDim.x) take(reinterpret_cast<const float4 *>(x + (size_t)r * ld)[c], c);
     }
     m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
@@ -783,7 +795,7 @@ cudaError_t launch_image(const GemmArgs &g, bool b_kmajor, unsigned *status, cud
         if (!(g.b_scale_fixed > 0.0f)) {
             if ((err = cudaMemsetAsync(bmax, 0, sizeof(unsigned), stream)) != cudaSuccess) return err;
             const int b_rows = b_kmajor ? g.N : g.K, b_cols = b_kmajor ? g.K : g.N;
-            absmax_bits_kernel<<<296, 256, 0, stream>>>(g.B, g.ldb, b_rows, b_cols, bmax);
+            absmax_bits_kernel<<<592, 256, 0, stream>>>(g.B, g.ldb, b_rows, b_cols, bmax);
         }
         uint4 *image16 = reinterpret_cast<uint4 *>(image);
         const float lo_scale = g.lo_unscaled ? 1.0f : kSplit16LoScale;
@@ -797,7 +809,7 @@ cudaError_t launch_image(const GemmArgs &g, bool b_kmajor, unsigned *status, cud
         // the largest |A kscale| for the scale, then the two FP16 matrices
         unsigned *amax = const_cast<unsigned *>(g.a_absmax_bits);
         if ((err = cudaMemsetAsync(amax, 0, sizeof(unsigned), stream)) != cudaSuccess) return err;
-        absmax_bits_kernel<<<296, 256, 0, stream>>>(g.A, g.lda, g.M, g.K, amax, g.kscale);
+        absmax_bits_kernel<<<592, 256, 0, stream>>>(g.A, g.lda, g.M, g.K, amax, g.kscale);
         const long units = (long)g.a_image_rows * (g.K / 8);
         presplit_a16_kernel<<<(unsigned)((units + 255) / 256), 256, 0, stream>>>(g.A, g.lda, g.M, g.K, g.kscale, reinterpret_cast<uint4 *>(g.a_image),
                                                                                   g.a_image_rows, amax, g.lo_unscaled ? 1.0f : kSplit16LoScale);
