@@ -1010,7 +1010,9 @@ cudaError_t svd_lowrank(SvdWorkspace *ws, const float *d_A, float *d_U, float *d
         err = cudaLaunchKernelEx(&cfg, jacobi_cluster_fn(k, ws->jc_lanes, ws->jc_with_v), core, k, d_S, vc, uc, status);
         if (err != cudaSuccess) return err;
     } else if (ws->own_core_svd) {
-        jacobi_svd_kernel<<<1, 512, jacobi_smem_bytes(k), st>>>(ws->core, k, d_S, ws->vc, ws->uc);
+        // eight lanes per pair and no more: warps without a pair only make a round's barrier longer (k = 64: 301 -> 290 us)
+        const int threads = std::max(1, ((k + 1) / 2 * 8 + 31) / 32) * 32;
+        jacobi_svd_kernel<<<1, threads, jacobi_smem_bytes(k), st>>>(ws->core, k, d_S, ws->vc, ws->uc);
         if ((err = cudaGetLastError()) != cudaSuccess) return err;
     } else if (cusolverDnSgesvdj(ws->solver, CUSOLVER_EIG_MODE_VECTOR, 0, k, k, ws->core, k, d_S, ws->vc, k, ws->uc, k,
                                  ws->solver_work, ws->lwork, ws->dev_info, ws->svdj) != CUSOLVER_STATUS_SUCCESS) {
