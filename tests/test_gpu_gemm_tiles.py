@@ -1,0 +1,53 @@
+"""Products whose tile width or reduction is chosen by size: 256-, 128- and 64-column tiles with ragged last tiles, K in one piece
+and split, reductions of one and of four elements per thread, the scale pass over arrays with and without gaps between rows.
+
+Bound: three tensor-core products of split operands leave at most a few 1e-7 of sum |a||b| (FP32 accumulation of up to 4096
+terms in the tensor core's order); 4e-6 is allowed."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def check(lib, a_km, b_km, M, N, K, pad, workspace):
+    g = torch.Generator(device="cuda").manual_seed(M + 3 * N + 7 * K)
+    a_rows, a_cols = (M, K) if a_km else (K, M)
+    b_rows, b_cols = (N, K) if b_km else (K, N)
+    A = torch.randn(a_rows, a_cols + pad, device="cuda", generator=g)
+    B = torch.randn(b_rows, b_cols + pad, device="cuda", generator=g)
+    C = torch.full((M, N + pad), 3.0, device="cuda")
+    ws = torch.empty(64 << 20, dtype=torch.uint8, device="cuda")
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert lib.bsq_gemm(int(a_km), int(b_km), A.data_ptr(), A.shape[1], B.data_ptr(), B.shape[1], C.data_ptr(), C.shape[1], M, N, K,
+                        ws.data_ptr() if workspace else None, ws.numel() if workspace else 0, 1, status.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    a = A[:, :a_cols].double() if a_km else A[:, :a_cols].double().T
+    b = B[:, :b_cols].double().T if b_km else B[:, :b_cols].double()
+    want, scale = a @ b, a.abs() @ b.abs()
+    assert int(status[0]) == 0
+    assert bool(((C[:, :N].double() - want).abs() <= 4e-6 * scale).all())
+    if pad:
+        assert bool((C[:, N:] == 3.0).all())
+
+
+@pytest.mark.parametrize("N", [16, 64, 112, 128, 144, 208, 240, 256])
+@pytest.mark.parametrize("M", [128, 129, 777, 4096])
+def test_panel_products(lib, M, N):
+    check(lib, True, False, M, N, N if N >= 64 else 64, 0, True)
+    check(lib, True, True, M, N, 256, 4, False)
+
+
+@pytest.mark.parametrize("N", [128, 144, 208, 256])
+@pytest.mark.parametrize("K", [512, 1031, 4096])
+def test_gram_shaped_products(lib, N, K):
+    check(lib, False, False, N, N, K, 0, True)
+    check(lib, False, False, N, N, K, 4, True)
+
+
+@pytest.mark.parametrize("shape", [(1024, 64, 2048), (4096, 48, 1536), (777, 33, 1031)])
+def test_split_products(lib, shape):
+    M, N, K = shape
+    check(lib, True, False, M, N, K, 0, True)
+    check(lib, True, False, M, N, K, 3, True)
