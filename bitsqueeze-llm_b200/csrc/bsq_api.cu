@@ -913,9 +913,19 @@ struct QuantSource {
 };
 bool aligned_to(const void *p, size_t a) { return reinterpret_cast<uintptr_t>(p) % a == 0; }
 
-// Checks of one quantised section against its 48-byte header (quantization_cuda.cu:691-734,809-876).  A device-resident
-// section whose pieces are 4-byte aligned is read where it lies; others go into the runtime's aligned buffers first.
-bool locate_quant(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, const bitsqz_section_t &s, const QuantHeader &h, int method,
+// How the sections of a payload are read.
+struct PayloadAccess {
+    bool on_device = false;               // by kernels
+    bool in_place = false;                // ... where they lie: nothing that the call writes lies over them
+};
+bool ranges_overlap(const void *a, uint64_t a_bytes, const void *b, uint64_t b_bytes) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + b_bytes && y < x + a_bytes;
+}
+
+// Checks of one quantised section against its 48-byte header (quantization_cuda.cu:691-734,809-876).  A section that may be
+// read in place and whose pieces are 4-byte aligned is; others go into the runtime's aligned buffers first.
+bool locate_quant(Runtime &rt, const bitsqz_llm_array_t *c, PayloadAccess how, const bitsqz_section_t &s, const QuantHeader &h, int method,
                   uint64_t expected_count, QuantBufs *q, QuantSource *where) {
     if (s.storage != BITSQZ_SECTION_QUANT || method == quantization_NONE || !q || q->cap < expected_count) return false;
     q->n = expected_count;
@@ -927,7 +937,7 @@ bool locate_quant(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, cons
     const uint8_t *src = static_cast<const uint8_t *>(c->payload) + s.offset;
     const uint8_t *scales = src + sizeof(QuantHeader), *dq = src + offsetof(QuantHeader, dq_scale);
     const uint64_t scale_bytes = method == NF4 ? nb * 4 : nb, data_bytes = (expected_count + 1) / 2;
-    if (on_device && aligned_to(src, 4) && aligned_to(scales + scale_bytes, 4)) {
+    if (how.in_place && aligned_to(src, 4) && aligned_to(scales + scale_bytes, 4)) {
         if (method == NF4) {
             where->scales_f32 = reinterpret_cast<const float *>(scales);
         } else {
@@ -950,14 +960,14 @@ bool locate_quant(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, cons
     }
     seg[count++] = CopySegment{q->data.p, scales + scale_bytes, data_bytes};
     where->data = q->data.as<uint8_t>();
-    if (on_device) return copy_segments(seg, count, rt.stream) == cudaSuccess;
+    if (how.on_device) return copy_segments(seg, count, rt.stream) == cudaSuccess;
     for (int i = 0; i < count; ++i)
         if (cudaMemcpyAsync(seg[i].dst, seg[i].src, seg[i].bytes, cudaMemcpyDefault, rt.stream) != cudaSuccess) return false;
     return true;
 }
 
 // One section -> `d_out` (expected_count floats).  FP32: plain copy.  QUANT: the dequantise kernel.
-bool decode_section(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, const bitsqz_section_t &s, const QuantHeader &h, int method,
+bool decode_section(Runtime &rt, const bitsqz_llm_array_t *c, PayloadAccess how, const bitsqz_section_t &s, const QuantHeader &h, int method,
                     uint64_t expected_count, QuantBufs *q, float *d_out) {
     const uint8_t *src = static_cast<const uint8_t *>(c->payload) + s.offset;
     if (s.storage == BITSQZ_SECTION_FP32) {
@@ -965,17 +975,17 @@ bool decode_section(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, co
         return cudaMemcpyAsync(d_out, src, s.size, cudaMemcpyDefault, rt.stream) == cudaSuccess;
     }
     QuantSource from;
-    if (!locate_quant(rt, c, on_device, s, h, method, expected_count, q, &from)) return false;
+    if (!locate_quant(rt, c, how, s, h, method, expected_count, q, &from)) return false;
     if (method == NF4) return nf4_dequantize(from.scales_f32, from.data, expected_count, d_out, rt.sm_count, rt.stream) == cudaSuccess;
     return nf4dq_dequantize(from.dq, from.scale_codes, from.data, expected_count, d_out, rt.sm_count, rt.stream) == cudaSuccess;
 }
 
-// The two arrays of a top-k section: where they lie (device-resident and aligned) or copied into `bufs`.
-bool locate_topk(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, const bitsqz_section_t &s, const TopkHeader &h, TopkBufs &bufs,
+// The two arrays of a top-k section: where they lie (if they may be read there and are aligned) or copied into `bufs`.
+bool locate_topk(Runtime &rt, const bitsqz_llm_array_t *c, PayloadAccess how, const bitsqz_section_t &s, const TopkHeader &h, TopkBufs &bufs,
                  const uint16_t **idx, const float **val) {
     const uint8_t *src = static_cast<const uint8_t *>(c->payload) + s.offset + sizeof(TopkHeader);
     const size_t cnt = (size_t)h.num_rows * h.num_topk_columns;
-    if (on_device && aligned_to(src, 2) && aligned_to(src + cnt * 2, 4)) {
+    if (how.in_place && aligned_to(src, 2) && aligned_to(src + cnt * 2, 4)) {
         *idx = reinterpret_cast<const uint16_t *>(src);
         *val = reinterpret_cast<const float *>(src + cnt * 2);
         return true;
@@ -984,23 +994,31 @@ bool locate_topk(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, const
     *val = bufs.val.as<float>();
     if (cnt == 0) return true;
     const CopySegment seg[2] = {{bufs.idx.p, src, cnt * 2}, {bufs.val.p, src + cnt * 2, cnt * 4}};
-    if (on_device) return copy_segments(seg, 2, rt.stream) == cudaSuccess;
+    if (how.on_device) return copy_segments(seg, 2, rt.stream) == cudaSuccess;
     return cudaMemcpyAsync(bufs.idx.p, src, cnt * 2, cudaMemcpyDefault, rt.stream) == cudaSuccess &&
            cudaMemcpyAsync(bufs.val.p, src + cnt * 2, cnt * 4, cudaMemcpyDefault, rt.stream) == cudaSuccess;
 }
 
-// The object's lists onto the decoded matrix: error first, outliers second (src/bitsqz_llm.cu:1372-1387).
-bool apply_lists(Runtime &rt, const bitsqz_llm_array_t *c, bool on_device, const SectionHeads &heads, bool has_err, bool has_out, float *d_dst) {
+// The object's lists, located before anything is written to the result (which may lie over the object) ...
+struct Lists {
     const uint16_t *idx[2] = {};
     const float *val[2] = {};
-    const uint32_t ke = has_err ? heads.err.num_topk_columns : 0, ko = has_out ? heads.outlier.num_topk_columns : 0;
-    if (ke && !locate_topk(rt, c, on_device, c->section_error_topk, heads.err, rt.err, &idx[0], &val[0])) return false;
-    if (ko && !locate_topk(rt, c, on_device, c->section_outlier_topk, heads.outlier, rt.outlier, &idx[1], &val[1])) return false;
+    uint32_t k[2] = {};                   // error, outliers; 0: none
+};
+bool locate_lists(Runtime &rt, const bitsqz_llm_array_t *c, PayloadAccess how, const SectionHeads &heads, bool has_err, bool has_out, Lists *l) {
+    l->k[0] = has_err ? heads.err.num_topk_columns : 0;
+    l->k[1] = has_out ? heads.outlier.num_topk_columns : 0;
+    return (!l->k[0] || locate_topk(rt, c, how, c->section_error_topk, heads.err, rt.err, &l->idx[0], &l->val[0])) &&
+           (!l->k[1] || locate_topk(rt, c, how, c->section_outlier_topk, heads.outlier, rt.outlier, &l->idx[1], &l->val[1]));
+}
+// ... and added to the decoded matrix: error first, outliers second (src/bitsqz_llm.cu:1372-1387).
+bool apply_lists(Runtime &rt, const bitsqz_llm_array_t *c, const Lists &l, float *d_dst) {
     unsigned *status = rt.status.as<unsigned>();
     cudaError_t err = cudaSuccess;
-    if (ke && ko) err = topk_apply_two(idx[0], val[0], ke, idx[1], val[1], ko, c->num_rows, c->num_columns, d_dst, status, rt.stream);
-    else if (ke) err = topk_apply(idx[0], val[0], c->num_rows, c->num_columns, ke, d_dst, status, rt.stream);
-    else if (ko) err = topk_apply(idx[1], val[1], c->num_rows, c->num_columns, ko, d_dst, status, rt.stream);
+    if (l.k[0] && l.k[1])
+        err = topk_apply_two(l.idx[0], l.val[0], l.k[0], l.idx[1], l.val[1], l.k[1], c->num_rows, c->num_columns, d_dst, status, rt.stream);
+    else if (l.k[0] || l.k[1])
+        err = topk_apply(l.idx[l.k[0] ? 0 : 1], l.val[l.k[0] ? 0 : 1], c->num_rows, c->num_columns, l.k[0] + l.k[1], d_dst, status, rt.stream);
     return err == cudaSuccess;
 }
 
@@ -1027,39 +1045,36 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
         if (cudaMemcpyAsync(rt.status.p, rt.h_status + 8, 4, cudaMemcpyHostToDevice, st) != cudaSuccess) return fail();
     }
     unsigned *d_status = rt.status.as<unsigned>();
-    bool lists_done = false;
+    // A result that lies over the object (an arena with the object at its end) would be written while other CTAs still
+    // read codes, scales or lists there: the sections are copied first, as those that are not aligned are.
+    PayloadAccess how;
+    how.on_device = payload_on_device;
+    how.in_place = payload_on_device && !ranges_overlap(d_dst, (uint64_t)c->num_elements * 4, c->payload,
+                                                        bitsqz_llm_get_packed_size(c) - sizeof(bitsqz_llm_array_t));
+    Lists lists;
+    if (!locate_lists(rt, c, how, heads, has_err, has_out, &lists)) return fail();
     if (c->flags & kFlagSvd) {
         const uint32_t rank = (uint16_t)c->effective_rank;
-        if (!decode_section(rt, c, payload_on_device, c->section_u, heads.u, c->svd_uv_format, (uint64_t)c->num_rows * rank, &rt.q_direct, rt.u.as<float>())) return fail();
-        if (!decode_section(rt, c, payload_on_device, c->section_s, heads.s, c->svd_s_format, rank, &rt.q_direct, rt.s.as<float>())) return fail();
-        if (!decode_section(rt, c, payload_on_device, c->section_v, heads.v, c->svd_uv_format, (uint64_t)c->num_columns * rank, &rt.q_direct, rt.v.as<float>())) return fail();
+        if (!decode_section(rt, c, how, c->section_u, heads.u, c->svd_uv_format, (uint64_t)c->num_rows * rank, &rt.q_direct, rt.u.as<float>())) return fail();
+        if (!decode_section(rt, c, how, c->section_s, heads.s, c->svd_s_format, rank, &rt.q_direct, rt.s.as<float>())) return fail();
+        if (!decode_section(rt, c, how, c->section_v, heads.v, c->svd_uv_format, (uint64_t)c->num_columns * rank, &rt.q_direct, rt.v.as<float>())) return fail();
         if (reconstruct_lowrank(rt.u.as<float>(), rt.s.as<float>(), rt.v.as<float>(), c->num_rows, c->num_columns, (int)rank,
                                 nullptr, d_dst, nullptr, d_status, rt.recon_ws.as<float>(), rt.recon_ws_bytes, rt.sm_count, st) != cudaSuccess)
             return fail();
-    } else if (c->section_direct.storage == BITSQZ_SECTION_QUANT && (has_out != has_err)) {
+    } else if (c->section_direct.storage == BITSQZ_SECTION_QUANT && (lists.k[0] != 0) != (lists.k[1] != 0)) {
         // quantised matrix with exactly one list: dequantise and add the list in one pass over the output
         // (with one list the reference's order "error list first, outliers second" has nothing to order)
-        const TopkHeader &th = has_out ? heads.outlier : heads.err;
-        TopkBufs &tb = has_out ? rt.outlier : rt.err;
-        const bitsqz_section_t &ts = has_out ? c->section_outlier_topk : c->section_error_topk;
-        const int method = c->quantization_only_format;
-        if ((size_t)th.num_rows * th.num_topk_columns == 0) {
-            if (!decode_section(rt, c, payload_on_device, c->section_direct, heads.direct, method, c->num_elements, &rt.q_direct, d_dst)) return fail();
-        } else {
-            QuantSource q;
-            const uint16_t *idx = nullptr;
-            const float *val = nullptr;
-            if (!locate_quant(rt, c, payload_on_device, c->section_direct, heads.direct, method, c->num_elements, &rt.q_direct, &q)) return fail();
-            if (!locate_topk(rt, c, payload_on_device, ts, th, tb, &idx, &val)) return fail();
-            if (nf4_dequantize_add_topk(q.scales_f32, q.dq, q.scale_codes, q.data, c->num_rows, c->num_columns, idx, val,
-                                        th.num_topk_columns, d_dst, d_status, rt.sm_count, st) != cudaSuccess)
-                return fail();
-        }
-        lists_done = true;
+        QuantSource q;
+        if (!locate_quant(rt, c, how, c->section_direct, heads.direct, c->quantization_only_format, c->num_elements, &rt.q_direct, &q)) return fail();
+        const int i = lists.k[0] ? 0 : 1;
+        if (nf4_dequantize_add_topk(q.scales_f32, q.dq, q.scale_codes, q.data, c->num_rows, c->num_columns, lists.idx[i], lists.val[i],
+                                    lists.k[i], d_dst, d_status, rt.sm_count, st) != cudaSuccess)
+            return fail();
+        lists.k[i] = 0;
     } else {
-        if (!decode_section(rt, c, payload_on_device, c->section_direct, heads.direct, c->quantization_only_format, c->num_elements, &rt.q_direct, d_dst)) return fail();
+        if (!decode_section(rt, c, how, c->section_direct, heads.direct, c->quantization_only_format, c->num_elements, &rt.q_direct, d_dst)) return fail();
     }
-    if (!lists_done && !apply_lists(rt, c, payload_on_device, heads, has_err, has_out, d_dst)) return fail();
+    if (!apply_lists(rt, c, lists, d_dst)) return fail();
     if (cudaMemcpyAsync(rt.h_status, rt.status.p, 64, cudaMemcpyDeviceToHost, st) != cudaSuccess) return fail();
     rt.decompress_active = true;
     return 0;

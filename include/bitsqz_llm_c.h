@@ -216,6 +216,8 @@ int bsq_lane_compress_begin(bsq_lane_t *lane, const float *matrix, int input_loc
 /* host object: *out (must be NULL on entry) receives it, release with bsq_free; device object: device_header (nullable) */
 int bsq_lane_compress_end(bsq_lane_t *lane, struct bitsqz_llm_array **out, struct bitsqz_llm_array *device_header,
                           uint64_t *packed_size);
+/* d_dst may lie over a device-resident object (an arena with the object inside it): its sections are then copied before
+ * anything is written.  Only an FP32 direct section must not overlap d_dst. */
 int bsq_lane_decompress_begin(bsq_lane_t *lane, const struct bitsqz_llm_array *header, int payload_on_device, float *d_dst,
                               uint64_t dst_num_elements);
 int bsq_lane_decompress_end(bsq_lane_t *lane);

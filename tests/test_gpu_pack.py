@@ -88,3 +88,55 @@ def test_damaged_device_object_is_refused(pkg, lib):
         assert lib.bsq_lane_decompress_end(lane) == 0
     finally:
         lib.bsq_lane_destroy(lane)
+
+
+# quantised matrices with no, one and two lists, low-rank objects with lists, sections that are read in place and ones that are not
+OVERLAP_CASES = [
+    (64, 512, 0.0, 0.0, -1, -1, -1, 11),
+    (192, 1024, 0.02, 0.0, -1, -1, -1, 10),
+    (192, 1024, 0.0, 0.02, -1, -1, -1, 11),
+    (256, 768, 0.01, 0.02, -1, -1, -1, 10),
+    (33, 77, 0.04, 0.04, -1, -1, -1, 11),
+    (512, 640, 0.01, 0.01, 32, 11, -1, -1),
+    (512, 640, 0.01, 0.0, 16, -1, -1, -1),
+]
+
+
+@pytest.mark.parametrize("case", OVERLAP_CASES)
+def test_result_may_lie_over_the_object(pkg, lib, case):
+    """One buffer holds the object and receives the matrix: the object at the end, in the middle and at the front of it, and
+    ending just inside and just outside.  Same bits as into a buffer of its own."""
+    rows, cols, outlier, error, rank, uv, s, q = case
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    x = torch.randn(rows, cols, device="cuda", generator=g)
+    lane = lib.bsq_lane_create(rows, cols, outlier, error, rank, 2, uv, s, q)
+    assert lane
+    try:
+        cap = int(lib.bsq_lane_packed_capacity(lane))
+        obj = torch.empty(cap, dtype=torch.uint8, device="cuda")
+        hdr, size = pkg.Array(), C.c_uint64(0)
+        torch.cuda.synchronize()
+        assert lib.bsq_lane_compress_begin(lane, x.data_ptr(), 1, obj.data_ptr(), cap) == 0
+        assert lib.bsq_lane_compress_end(lane, None, C.byref(hdr), C.byref(size)) == 0
+        n = int(size.value)
+        want = torch.empty_like(x)
+        torch.cuda.synchronize()
+        assert lib.bsq_lane_decompress_begin(lane, C.byref(hdr), 1, want.data_ptr(), rows * cols) == 0
+        assert lib.bsq_lane_decompress_end(lane) == 0
+        out_bytes, front = rows * cols * 4, (cap + 255) // 256 * 256
+        # where the object starts, counted from the start of the matrix
+        last = (out_bytes - n) // 16 * 16
+        for at in (last, last // 2 // 4 * 4, 0, -200 + 4 * 64, 64 - n // 64 * 64, -((n + 63) // 64 * 64), out_bytes, last + 2):
+            arena = torch.zeros(front + out_bytes + cap, dtype=torch.uint8, device="cuda")
+            where = arena.data_ptr() + front + at
+            arena[front + at: front + at + n] = obj[:n]
+            moved = pkg.Array.from_buffer_copy(hdr)
+            moved.payload = where + 200
+            torch.cuda.synchronize()
+            assert lib.bsq_lane_decompress_begin(lane, C.byref(moved), 1, arena.data_ptr() + front, rows * cols) == 0, at
+            assert lib.bsq_lane_decompress_end(lane) == 0, at
+            torch.cuda.synchronize()
+            got = arena[front: front + out_bytes].view(torch.int32)
+            assert torch.equal(got, want.view(torch.int32).reshape(-1)), at
+    finally:
+        lib.bsq_lane_destroy(lane)
