@@ -201,6 +201,7 @@ struct SectionPlan {
 struct CompressJob {
     bool active = false;
     bool to_device = false;               // packed object goes to a device buffer instead of a pinned host block
+    bool by_kernel = false;               // ... which a kernel of this device can write
     uint8_t *block = nullptr;             // host: header + payload (pool block or malloc); device: the caller's buffer
     bool pooled = false;
     uint64_t total = 0;                   // header + payload bytes if every planned section is present
@@ -447,12 +448,20 @@ namespace {
 
 // Where the bytes of a packed object go: into a pinned host block (device-produced bytes copied there by the stream,
 // host-known bytes written directly) or into a device buffer (both noted in the runtime's DevicePack, whose kernel
-// runs after the last stage).  put_small: `d_patch` (nullable) is a device word that replaces the four bytes at `patch_at`.
+// runs after the last stage; copied by the stream where kernels cannot reach the buffer).  put_small: `d_patch` (nullable) is a device word that replaces the four bytes at `patch_at`.
 bool put_small(Runtime &rt, const CompressJob &job, uint8_t *dst, const void *src, size_t bytes, const void *d_patch = nullptr,
                size_t patch_at = 0) {
     if (!job.to_device) {
         std::memcpy(dst, src, bytes);
         return !d_patch || cudaMemcpyAsync(dst + patch_at, d_patch, 4, cudaMemcpyDefault, rt.stream) == cudaSuccess;
+    }
+    if (!job.by_kernel) {
+        if (rt.pack.head_bytes + bytes > kStageBytes) return false;
+        uint8_t *stage = rt.h_stage + rt.pack.head_bytes;
+        rt.pack.head_bytes += (int)((bytes + 15) & ~(size_t)15);
+        std::memcpy(stage, src, bytes);
+        return cudaMemcpyAsync(dst, stage, bytes, cudaMemcpyDefault, rt.stream) == cudaSuccess &&
+               (!d_patch || cudaMemcpyAsync(dst + patch_at, d_patch, 4, cudaMemcpyDefault, rt.stream) == cudaSuccess);
     }
     PackHeaders &h = rt.pack.heads;
     if (h.pieces >= kMaxHeads || rt.pack.head_bytes + bytes > sizeof(h.bytes)) return false;
@@ -462,7 +471,7 @@ bool put_small(Runtime &rt, const CompressJob &job, uint8_t *dst, const void *sr
     return true;
 }
 bool put_device(Runtime &rt, const CompressJob &job, uint8_t *dst, const void *d_src, size_t bytes) {
-    if (!job.to_device) return cudaMemcpyAsync(dst, d_src, bytes, cudaMemcpyDefault, rt.stream) == cudaSuccess;
+    if (!job.by_kernel) return cudaMemcpyAsync(dst, d_src, bytes, cudaMemcpyDefault, rt.stream) == cudaSuccess;
     if (rt.pack.segments >= kMaxCopySegments) return false;
     rt.pack.seg[rt.pack.segments++] = CopySegment{dst, d_src, bytes};
     return true;
@@ -606,6 +615,9 @@ int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_p
     job.to_device = d_packed != nullptr;
     if (job.to_device) {
         if (capacity < job.total) return 1;
+        const Reach reach = memory_reach(d_packed, job.total);
+        if (reach == Reach::kNone) return 1;
+        job.by_kernel = reach == Reach::kKernels;
         job.block = d_packed;
     } else {
         job.pooled = true;
@@ -719,7 +731,7 @@ int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_p
     }
     if (ko > 0) ok = ok && emit_topk_section(rt, job, rt.outlier, payload + job.sec_out.offset);
     if (error_path) ok = ok && emit_topk_section(rt, job, rt.err, payload + job.sec_err.offset);
-    if (job.to_device) {
+    if (job.by_kernel) {
         PackHeaders &h = rt.pack.heads;
         const bitsqz_llm_array_t hdr = object_header(rt, job, error_path);
         static_assert(sizeof(hdr) == sizeof(h.object), "the object's header");
@@ -753,7 +765,14 @@ int compress_end(Runtime &rt, bitsqz_llm_array_t **out, bitsqz_llm_array_t *head
     const bool has_error_topk = job.error_path && rt.h_status[1] != 0;      // src/bitsqz_llm.cu:1160-1178
     const bitsqz_llm_array_t hdr = object_header(rt, job, has_error_topk);
     if (job.to_device) {
-        if (header_out) *header_out = hdr;                    // (the device copy was written with the sections)
+        if (!job.by_kernel) {                                 // (otherwise written with the sections)
+            std::memcpy(rt.h_stage, &hdr, sizeof(hdr));
+            if (cudaMemcpyAsync(job.block, rt.h_stage, sizeof(hdr), cudaMemcpyDefault, st) != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) {
+                abandon_job(rt);
+                return 1;
+            }
+        }
+        if (header_out) *header_out = hdr;
     } else {
         std::memcpy(job.block, &hdr, sizeof(hdr));
         if (out) *out = reinterpret_cast<bitsqz_llm_array_t *>(job.block);
@@ -817,13 +836,14 @@ bool section_method_ok(const bitsqz_section_t &s, int method) {                 
 }
 
 // The small headers that sit inside the payload, fetched before anything is decided from them: straight reads for a
-// host payload, one small kernel (and one wait) for a device-resident payload, which also clears the status words.
+// host payload, one small kernel (and one wait) for a device-resident payload, which also clears the status words, copies
+// (and one wait) for one that kernels cannot reach.
 struct SectionHeads {
     QuantHeader u, s, v, direct;
     TopkHeader outlier, err;
 };
 
-bool fetch_heads(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_device, SectionHeads *heads) {
+bool fetch_heads(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_device, Reach reach, SectionHeads *heads) {
     std::memset(heads, 0, sizeof(*heads));
     const uint8_t *payload = static_cast<const uint8_t *>(c->payload);
     struct Want { const bitsqz_section_t *sec; void *dst; size_t bytes; uint8_t storage; };
@@ -849,7 +869,13 @@ bool fetch_heads(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_devic
         into[list.count++] = w.dst;
     }
     if (payload_on_device) {
-        if (fetch_heads(list, rt.h_stage, rt.status.as<unsigned>(), rt.stream) != cudaSuccess) return false;
+        if (reach == Reach::kKernels) {
+            if (fetch_heads(list, rt.h_stage, rt.status.as<unsigned>(), rt.stream) != cudaSuccess) return false;
+        } else {
+            if (reach == Reach::kNone && list.count > 0) return false;
+            for (int i = 0; i < list.count; ++i)
+                if (cudaMemcpyAsync(rt.h_stage + 64 * i, list.src[i], list.length[i], cudaMemcpyDefault, rt.stream) != cudaSuccess) return false;
+        }
         if (list.count > 0 && cudaStreamSynchronize(rt.stream) != cudaSuccess) return false;
         for (int i = 0; i < list.count; ++i) std::memcpy(into[i], rt.h_stage + 64 * i, list.length[i]);
     }
@@ -1034,11 +1060,13 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
         return 1;
     };
     SectionHeads heads;
-    if (!fetch_heads(rt, c, payload_on_device, &heads)) return fail();
+    const uint64_t payload_bytes = bitsqz_llm_get_packed_size(c) - sizeof(bitsqz_llm_array_t);
+    const Reach reach = payload_on_device ? memory_reach(c->payload, payload_bytes) : Reach::kCopies;
+    if (!fetch_heads(rt, c, payload_on_device, reach, &heads)) return fail();
     const bool has_out = c->flags & kFlagOutlier, has_err = c->flags & kFlagError;
     if (has_out && !topk_section_ok(rt.outlier, c, c->section_outlier_topk, heads.outlier)) return 1;
     if (has_err && !topk_section_ok(rt.err, c, c->section_error_topk, heads.err)) return 1;
-    if (!payload_on_device && cudaMemsetAsync(rt.status.p, 0, 64, st) != cudaSuccess) return fail();
+    if (reach != Reach::kKernels && cudaMemsetAsync(rt.status.p, 0, 64, st) != cudaSuccess) return fail();
     if (rt.inject_status) {
         rt.h_status[8] = rt.inject_status;
         rt.inject_status = 0;
@@ -1048,9 +1076,8 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
     // A result that lies over the object (an arena with the object at its end) would be written while other CTAs still
     // read codes, scales or lists there: the sections are copied first, as those that are not aligned are.
     PayloadAccess how;
-    how.on_device = payload_on_device;
-    how.in_place = payload_on_device && !ranges_overlap(d_dst, (uint64_t)c->num_elements * 4, c->payload,
-                                                        bitsqz_llm_get_packed_size(c) - sizeof(bitsqz_llm_array_t));
+    how.on_device = reach == Reach::kKernels;
+    how.in_place = how.on_device && !ranges_overlap(d_dst, (uint64_t)c->num_elements * 4, c->payload, payload_bytes);
     Lists lists;
     if (!locate_lists(rt, c, how, heads, has_err, has_out, &lists)) return fail();
     if (c->flags & kFlagSvd) {

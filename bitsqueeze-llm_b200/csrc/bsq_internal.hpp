@@ -98,6 +98,14 @@ struct HeadList {
     int length[kMaxHeads];                                   // at most 64
     int count;
 };
+// How [p, p + bytes) may be reached from the current device.  Kernels fault where a stream copy works (another GPU's memory) or
+// returns an error (memory that CUDA does not know), so the caller's pointer is looked at before one is launched on it.
+enum class Reach {
+    kNone,                                                   // some of it is not CUDA memory
+    kCopies,                                                 // stream copies only: another device's memory, page-locked, managed
+    kKernels                                                 // this device's memory from one end to the other
+};
+Reach memory_reach(const void *p, uint64_t bytes);
 // Copies up to kMaxCopySegments pieces of device memory, of any alignment, in one launch.
 cudaError_t copy_segments(const CopySegment *segments, int count, cudaStream_t stream);
 // The same together with the headers and, into page-locked `mirror`, the status words.

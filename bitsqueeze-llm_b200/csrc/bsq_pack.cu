@@ -15,8 +15,28 @@
 #include "bsq_device.cuh"
 #include "bsq_internal.hpp"
 
+#include <cuda.h>
+
+#include <mutex>
+
 namespace bsq {
 namespace {
+
+// cuPointerGetAttributes from the driver, looked up once (the library links the runtime only).
+typedef CUresult (*PointerAttributesFn)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+PointerAttributesFn pointer_attributes() {
+    static PointerAttributesFn fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<PointerAttributesFn>(p);
+        else
+            cudaGetLastError();
+    });
+    return fn;
+}
 
 constexpr int kCopyThreads = 256;
 constexpr unsigned kCopyUnits = 2048;                        // 16-byte units per CTA: 32 KB, eight per thread
@@ -125,6 +145,30 @@ unsigned fill(CopyArgs &c, const CopySegment *segments, int count) {
 }
 
 }  // namespace
+
+// A buffer may consist of several mappings (an allocator's expandable segments): each of them is asked for.
+Reach memory_reach(const void *p, uint64_t bytes) {
+    const PointerAttributesFn ask = pointer_attributes();
+    int device = 0;
+    if (!ask || cudaGetDevice(&device) != cudaSuccess) return Reach::kCopies;
+    bool kernels = true;
+    const CUdeviceptr end = reinterpret_cast<CUdeviceptr>(p) + bytes;
+    CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+    do {
+        unsigned type = 0, managed = 0;
+        int ordinal = -1;
+        CUdeviceptr start = 0;
+        size_t size = 0;
+        CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                       CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+        void *into[5] = {&type, &managed, &ordinal, &start, &size};
+        if (ask(5, what, into, at) != CUDA_SUCCESS || type == 0) return Reach::kNone;
+        if (type != CU_MEMORYTYPE_DEVICE || managed || ordinal != device) kernels = false;
+        if (start > at || start + size <= at) return Reach::kCopies;     // no range to go by: the copies check it themselves
+        at = start + size;
+    } while (at < end);
+    return kernels ? Reach::kKernels : Reach::kCopies;
+}
 
 cudaError_t copy_segments(const CopySegment *segments, int count, cudaStream_t stream) {
     if (count < 0 || count > kMaxCopySegments) return cudaErrorInvalidValue;

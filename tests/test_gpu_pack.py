@@ -140,3 +140,50 @@ def test_result_may_lie_over_the_object(pkg, lib, case):
             assert torch.equal(got, want.view(torch.int32).reshape(-1)), at
     finally:
         lib.bsq_lane_destroy(lane)
+
+
+@pytest.mark.parametrize("case", [(33, 77, 0.04, 0.04, -1, -1, -1, 11), (256, 1024, 0.01, 0.0, -1, -1, -1, 10), (129, 203, 0.02, 0.02, 13, 10, 11, -1),
+                                  (515, 1001, 0.0, 0.0, -1, -1, -1, -1)])
+def test_objects_in_memory_that_kernels_do_not_reach(pkg, lib, case):
+    """Page-locked host memory handed over as the object's buffer stands for all memory that is not this device's own (another
+    GPU's): stream copies move it, with the same bytes as ever.  Memory that CUDA does not know is refused on the host, both
+    ways, before anything is launched on it, and the lane goes on working."""
+    rows, cols, outlier, error, rank, uv, s, q = case
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    x = torch.randn(rows, cols, device="cuda", generator=g)
+    lane = lib.bsq_lane_create(rows, cols, outlier, error, rank, 2, uv, s, q)
+    assert lane
+    try:
+        cap = int(lib.bsq_lane_packed_capacity(lane))
+        pinned = torch.full((cap,), 0xA5, dtype=torch.uint8).pin_memory()
+        pageable = np.zeros(cap, np.uint8)
+        hdr, size, out = pkg.Array(), C.c_uint64(0), C.c_void_p(None)
+        torch.cuda.synchronize()
+        assert lib.bsq_lane_compress_begin(lane, x.data_ptr(), 1, pageable.ctypes.data, cap) == 1
+        assert not pageable.any()
+        assert lib.bsq_lane_compress_begin(lane, x.data_ptr(), 1, pinned.data_ptr(), cap) == 0
+        assert lib.bsq_lane_compress_end(lane, None, C.byref(hdr), C.byref(size)) == 0
+        assert lib.bsq_lane_compress_begin(lane, x.data_ptr(), 1, None, 0) == 0
+        assert lib.bsq_lane_compress_end(lane, C.byref(out), None, None) == 0
+        n = int(size.value)
+        host = np.frombuffer(C.string_at(out.value, n), np.uint8).copy()
+        got = pinned.numpy()[:n].copy()
+        assert int(lib.bsq_get_packed_size(out)) == n and hdr.payload == pinned.data_ptr() + 200
+        host[192:200] = got[192:200]
+        assert np.array_equal(got, host)
+        y_host, y = torch.empty_like(x), torch.empty_like(x)
+        torch.cuda.synchronize()
+        assert lib.bsq_lane_decompress_begin(lane, out, 0, y_host.data_ptr(), rows * cols) == 0
+        assert lib.bsq_lane_decompress_end(lane) == 0
+        if q != pkg.NONE or rank > 0:                         # an object without inner headers was never looked into
+            pageable[:n] = got
+            bad = pkg.Array.from_buffer_copy(hdr)
+            bad.payload = pageable.ctypes.data + 200
+            assert lib.bsq_lane_decompress_begin(lane, C.byref(bad), 1, y.data_ptr(), rows * cols) == 1
+        assert lib.bsq_lane_decompress_begin(lane, C.byref(hdr), 1, y.data_ptr(), rows * cols) == 0
+        assert lib.bsq_lane_decompress_end(lane) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(y.view(torch.int32), y_host.view(torch.int32))
+        lib.bsq_free(out)
+    finally:
+        lib.bsq_lane_destroy(lane)
