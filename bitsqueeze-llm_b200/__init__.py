@@ -113,6 +113,7 @@ SIGNATURES = {
     "bsq_batch_compress": (_i, [_vp, C.POINTER(_vp), _i, _i, C.POINTER(_vp), _u64, C.POINTER(_vp), _vp, C.POINTER(_u64)]),
     "bsq_batch_decompress": (_i, [_vp, C.POINTER(_vp), _i, _i, C.POINTER(_vp), _u64]),
     "bsq_test_inject_status": (None, [_i, _u32]),
+    "bsq_test_inject_lane_status": (None, [_vp, _i, _u32]),
     "bsq_build_info": (C.c_char_p, []),
 }
 

@@ -758,7 +758,12 @@ int compress_end(Runtime &rt, bitsqz_llm_array_t **out, bitsqz_llm_array_t *head
     CompressJob &job = rt.job;
     if (!job.active) return 1;
     cudaStream_t st = rt.stream;
-    if (cudaStreamSynchronize(st) != cudaSuccess || rt.h_status[0] != 0) {
+    const bool done = cudaStreamSynchronize(st) == cudaSuccess;
+    if (!done || rt.h_status[0] != 0) {
+        if (done && job.to_device && !job.by_kernel) {            // as the pack kernel does; abandon_job waits for it
+            std::memset(rt.h_stage, 0, sizeof(bitsqz_llm_array_t));
+            cudaMemcpyAsync(job.block, rt.h_stage, sizeof(bitsqz_llm_array_t), cudaMemcpyDefault, st);
+        }
         abandon_job(rt);
         return 1;
     }
@@ -1320,6 +1325,11 @@ void bsq_test_inject_status(int which, uint32_t bits) {
     if (!slot) return;
     std::lock_guard<std::mutex> g(slot->mu);
     (which ? slot->decompress : slot->compress).inject_status = bits;
+}
+
+// The same for the next call of a lane.
+void bsq_test_inject_lane_status(bsq_lane *lane, int which, uint32_t bits) {
+    if (lane) (which ? lane->decompress : lane->compress).inject_status = bits;
 }
 
 }  // extern "C"

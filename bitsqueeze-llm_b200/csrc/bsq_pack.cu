@@ -7,7 +7,8 @@
 //   * the device pieces go through 16-byte stores; where source and destination are not aligned alike, 16 bytes are put
 //     together from five aligned words (the pieces are 2- or 1-byte aligned only for ragged shapes);
 //   * the section headers and the object's header travel in the kernel's parameters; the error section's entry and flag
-//     are dropped on the device when the error flag says so;
+//     are dropped on the device when the error flag says so, and the whole header is zeroed when a kernel of the call has
+//     reported an error (the call fails then, and nothing that could pass for an object is left in the buffer);
 //   * the status words go to the caller's page-locked mirror.
 // Bound by launch latency up to a few MB, by memory above (9.7 MB of a 4096 x 4096 NF4_DQ object: 6.7 us).  Measured with
 // the calls around it: compress 256 x 1024 NF4_DQ 71 -> 40 us, 4096 x 4096 114 -> 75 us; decompress 4096 x 4096, which also
@@ -110,9 +111,9 @@ __global__ void __launch_bounds__(kCopyThreads) pack_object_kernel(const __grid_
             q.dst[i] = b;
         }
     }
-    const bool no_error = status[1] == 0;
+    const bool failed = status[0] != 0, no_error = status[1] == 0;
     for (int i = threadIdx.x; i < (int)sizeof(h.object); i += kCopyThreads) {
-        uint8_t b = h.object[i];
+        uint8_t b = failed ? 0 : h.object[i];
         if (no_error) {
             if (i >= h.error_entry_at && i < h.error_entry_at + h.error_entry_length) b = 0;
             if (i == h.flags_at) b &= (uint8_t)~h.error_flag;

@@ -202,7 +202,8 @@ int bsq_shard_svd_profile_read(bsq_shard_svd_t *handle, float *ms, int *kinds, i
  * same layout (200-byte header, then the payload): copying packed_size bytes from it to the host gives a buffer that
  * load_bitsqz_llm_from_buffer accepts.  For such a device-resident object bsq_lane_compress_end fills *device_header,
  * a host copy of the header whose `payload` member is the DEVICE address of the payload; pass that header to
- * bsq_lane_decompress_begin with payload_on_device = 1. */
+ * bsq_lane_decompress_begin with payload_on_device = 1.  A call that fails in bsq_lane_compress_end because one of its
+ * kernels reported an error leaves 200 zero bytes in place of the header. */
 typedef struct bsq_lane bsq_lane_t;
 bsq_lane_t *bsq_lane_create(uint16_t num_rows, uint16_t num_columns, float outlier_topk_ratio, float error_correction_topk_ratio,
                             int svd_ranks, int svd_niters, int svd_uv_format, int svd_s_format, int quantization_only_format);
@@ -248,6 +249,8 @@ int bsq_batch_decompress(bsq_batch_t *batch, const struct bitsqz_llm_array *cons
  * current device starts with `bits` set in its device status word, as if a kernel had reported them; that call must
  * return 1.  Lets the error path be tested without making a kernel fail. */
 void bsq_test_inject_status(int which, uint32_t bits);
+/* The same for the next compress (which = 0) or decompress (which = 1) call begun on a lane. */
+void bsq_test_inject_lane_status(bsq_lane_t *lane, int which, uint32_t bits);
 
 /* library build tag: "sm_100a" plus the compile date */
 const char *bsq_build_info(void);

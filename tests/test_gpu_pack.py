@@ -187,3 +187,42 @@ def test_objects_in_memory_that_kernels_do_not_reach(pkg, lib, case):
         lib.bsq_free(out)
     finally:
         lib.bsq_lane_destroy(lane)
+
+
+@pytest.mark.parametrize("where", ["device", "pinned"])
+@pytest.mark.parametrize("case", [(256, 1024, 0.01, 0.0, -1, -1, -1, 10), (129, 203, 0.02, 0.02, 13, 10, 11, -1)])
+def test_failed_compress_leaves_no_object(pkg, lib, case, where):
+    """A call whose status word is set (from the host, no kernel fails) returns 1 and leaves a zeroed header, also in a buffer
+    that held a good object before; the lane's next call is a good one again."""
+    rows, cols, outlier, error, rank, uv, s, q = case
+    x = torch.randn(rows, cols, device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows))
+    lane = lib.bsq_lane_create(rows, cols, outlier, error, rank, 2, uv, s, q)
+    assert lane
+    try:
+        cap = int(lib.bsq_lane_packed_capacity(lane))
+        buf = torch.zeros(cap, dtype=torch.uint8, device="cuda") if where == "device" else torch.zeros(cap, dtype=torch.uint8).pin_memory()
+        hdr, size = pkg.Array(), C.c_uint64(0)
+
+        def compress():
+            torch.cuda.synchronize()
+            assert lib.bsq_lane_compress_begin(lane, x.data_ptr(), 1, buf.data_ptr(), cap) == 0
+            return lib.bsq_lane_compress_end(lane, None, C.byref(hdr), C.byref(size))
+        assert compress() == 0
+        good = buf.cpu().numpy().copy()
+        lib.bsq_test_inject_lane_status(lane, 0, 1)           # "a bounded wait ran out"
+        assert compress() == 1
+        left = buf.cpu().numpy().copy()
+        assert not left[:200].any()
+        y = torch.empty_like(x)
+        obj = lib.bsq_load_from_buffer(left.ctypes.data, left.size)
+        if obj:
+            assert lib.bsq_lane_decompress_begin(lane, obj, 0, y.data_ptr(), rows * cols) == 1
+            lib.bsq_free(obj)
+        assert compress() == 0
+        assert np.array_equal(buf.cpu().numpy(), good)
+        lib.bsq_test_inject_lane_status(lane, 1, 1)
+        for want in (1, 0):
+            assert lib.bsq_lane_decompress_begin(lane, C.byref(hdr), 1, y.data_ptr(), rows * cols) == 0
+            assert lib.bsq_lane_decompress_end(lane) == want
+    finally:
+        lib.bsq_lane_destroy(lane)
