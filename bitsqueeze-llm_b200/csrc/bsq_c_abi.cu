@@ -123,25 +123,27 @@ int bsq_residual_error(const float *d_a, const float *d_b, uint64_t n, float *d_
     return rc(residual_error(d_a, d_b, n, d_e, d_flag, device_sm_count(), as_stream(stream)));
 }
 
-int bsq_svd_lowrank(const float *d_A, int m, int n, int k, int niter, unsigned long long seed, float *d_U, float *d_S,
-                    float *d_V, void *stream) {
+static int svd_once(const float *d_A, int m, int n, int k, int niter, unsigned long long seed, unsigned long long offset, bool coded_factors,
+                    float *d_U, float *d_S, float *d_V, void *stream) {
     if (!d_A || !d_U || !d_S || !d_V || m <= 0 || n <= 0 || k <= 0 || niter < 0) return 1;
-    SvdWorkspace *ws = svd_workspace_create(m, n, k, niter, device_sm_count());
+    SvdWorkspace *ws = svd_workspace_create(m, n, k, niter, device_sm_count(), coded_factors);
     if (!ws) return 1;
-    const cudaError_t e = svd_lowrank(ws, d_A, d_U, d_S, d_V, seed, nullptr, as_stream(stream));
+    const cudaError_t e = svd_lowrank(ws, d_A, d_U, d_S, d_V, seed, nullptr, as_stream(stream), offset);
     const cudaError_t s = svd_workspace_finish(ws, as_stream(stream));  // the workspace dies with this call
     svd_workspace_destroy(ws);
     return rc(e) | rc(s);
 }
+int bsq_svd_lowrank(const float *d_A, int m, int n, int k, int niter, unsigned long long seed, float *d_U, float *d_S,
+                    float *d_V, void *stream) {
+    return svd_once(d_A, m, n, k, niter, seed, 0, false, d_U, d_S, d_V, stream);
+}
 int bsq_svd_lowrank_at(const float *d_A, int m, int n, int k, int niter, unsigned long long seed, unsigned long long offset,
                        float *d_U, float *d_S, float *d_V, void *stream) {
-    if (!d_A || !d_U || !d_S || !d_V || m <= 0 || n <= 0 || k <= 0 || niter < 0) return 1;
-    SvdWorkspace *ws = svd_workspace_create(m, n, k, niter, device_sm_count());
-    if (!ws) return 1;
-    const cudaError_t e = svd_lowrank(ws, d_A, d_U, d_S, d_V, seed, nullptr, as_stream(stream), offset);
-    const cudaError_t s = svd_workspace_finish(ws, as_stream(stream));
-    svd_workspace_destroy(ws);
-    return rc(e) | rc(s);
+    return svd_once(d_A, m, n, k, niter, seed, offset, false, d_U, d_S, d_V, stream);
+}
+int bsq_svd_lowrank_coded(const float *d_A, int m, int n, int k, int niter, unsigned long long seed, float *d_U, float *d_S,
+                          float *d_V, void *stream) {
+    return svd_once(d_A, m, n, k, niter, seed, 0, true, d_U, d_S, d_V, stream);
 }
 int bsq_gemm(int a_kmajor, int b_kmajor, const float *d_A, long lda, const float *d_B, long ldb, float *d_C, long ldc, int M,
              int N, int K, float *d_workspace, size_t workspace_bytes, int allow_tensor_cores, uint32_t *d_status, void *stream) {

@@ -131,6 +131,10 @@ int bsq_svd_lowrank(const float *d_A, int m, int n, int k, int niter, unsigned l
  * offset 0): the range finder's random matrix is the N_work x k block of XORWOW normals that starts there. */
 int bsq_svd_lowrank_at(const float *d_A, int m, int n, int k, int niter, unsigned long long seed, unsigned long long offset,
                        float *d_U, float *d_S, float *d_V, void *stream);
+/* The same with the order of rotations in the core's SVD that compress uses where U, S and V are coded afterwards (NF4, NF4_DQ)
+ * or an error list is made from them: other kernels up to 256 columns, results that differ by rounding. */
+int bsq_svd_lowrank_coded(const float *d_A, int m, int n, int k, int niter, unsigned long long seed, float *d_U, float *d_S,
+                          float *d_V, void *stream);
 /* reconstruct_lowrank_cuda (reconstruct_lowrank_cuda.cuh:73-78): d_out = (U diag(S)) V^T.
  * d_minuend non-NULL: d_out = d_minuend - (U diag(S)) V^T and *d_flag |= any(|d_out| > FLT_EPSILON).
  * d_status (nullable) receives bit 0 if a bounded wait inside the product kernel gave up (d_out is then incomplete). */

@@ -1,11 +1,14 @@
 """The k x k kernels of the randomized SVD (Cholesky factor and inverse by 32 x 32 blocks, block Jacobi on 1 to 8 CTAs) at the edges
-of their blocks, clusters and paddings, through bsq_svd_lowrank, against FP64 numpy.
+of their blocks, clusters and paddings, through bsq_svd_lowrank, against FP64 numpy; and the kernels that take the core's SVD where factors are
+coded (one CTA up to 64 columns, rows dealt over a cluster above) by the same checks and those of test_gpu_svd.py, through bsq_svd_lowrank_coded.
 
 Bounds.  Each QR pass factors G + 1e-5 max(diag G) I, so columns are orthonormal to a few 1e-5, up to 2e-4 for the weakest
 direction of a wide sketch (the bounds of test_gpu_svd.py).  With orthonormal Q the residual of Q Q^T A has the squared norm
 |A|^2 - sum S^2: both sides are compared to 1e-3 of |A|^2 (twice the orthonormality bound for the two factors, and FP32 sums)."""
 import numpy as np
 import pytest
+
+import test_gpu_svd
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
@@ -54,3 +57,31 @@ def test_core_of_deficient_and_zero_matrices(lib, k):
     assert np.linalg.norm(a - (u * s) @ v.T) <= 1e-4 * np.linalg.norm(a)
     u, s, v = svd_gpu(lib, np.zeros((m, n), np.float32), k)
     assert np.isfinite(u).all() and np.isfinite(v).all() and not s.any()
+
+
+class CodedFactors:
+    """The library with bsq_svd_lowrank standing for the kernels of coded factors."""
+
+    def __init__(self, lib):
+        self.bsq_svd_lowrank = lib.bsq_svd_lowrank_coded
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 8, 15, 16, 17, 31, 32, 33, 48, 63, 64, 65, 96, 127, 128, 129, 131, 160, 200, 255, 256])
+@pytest.mark.parametrize("kind", ["noise", "large"])
+def test_core_edges_of_coded_factors(lib, k, kind):
+    test_core_edges(CodedFactors(lib), k, kind)
+
+
+@pytest.mark.parametrize("k", [5, 32, 40, 64, 65, 100, 200, 256])
+def test_coded_core_of_deficient_and_zero_matrices(lib, k):
+    test_core_of_deficient_and_zero_matrices(CodedFactors(lib), k)
+
+
+@pytest.mark.parametrize("case", [(1024, 512, 64, 2), (512, 2048, 32, 2), (2048, 1024, 128, 1), (300, 180, 20, 3), (1024, 768, 96, 2),
+                                  (700, 900, 131, 2), (1024, 1024, 160, 2), (1536, 1024, 256, 2)])
+def test_coded_factors_accuracy_against_exact(lib, case):
+    test_gpu_svd.test_svd_accuracy_against_exact(CodedFactors(lib), case)
+
+
+def test_coded_factors_of_rank_deficient_and_zero_inputs(lib):
+    test_gpu_svd.test_svd_rank_deficient_and_zero_inputs(CodedFactors(lib))

@@ -63,8 +63,8 @@ def test_reconstruct_matches_fp64(lib, oracle, shape):
 
 
 @pytest.mark.parametrize("case", [(1024, 512, 64, 2), (512, 2048, 32, 2), (2048, 1024, 128, 1), (300, 180, 20, 3),
-                                  # cores for the cluster Jacobi kernel: below and at its 128 columns, odd, between 128
-                                  # and 256 and at 256 (where the products take the kernel with B split beforehand)
+                                  # wider cores: clusters of 3, 5 and 8 CTAs (8 at every width where factors are coded),
+                                  # odd, and at 256 the products take the kernel with B split beforehand
                                   (1024, 768, 96, 2), (700, 900, 131, 2), (1024, 1024, 160, 2), (1536, 1024, 256, 2)])
 def test_svd_accuracy_against_exact(lib, case):
     m, n, k, niter = case
