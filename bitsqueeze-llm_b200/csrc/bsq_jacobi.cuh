@@ -7,8 +7,9 @@
 //   out: M = U diag(S) V^T with S descending; U column-major k x k; Vcol column-major k x k: V itself (kWithV), or
 //        column j of M V divided by S(j)^2 -- the matrix that turns the panel the core came from into its singular
 //        vectors (B^T v_j / S(j) with v_j = (M V)(:, j) / S(j)), for which nothing has to accumulate the rotations.
-// Column pairs (p, q) are rotated until all columns of M V are orthogonal to tol (LAPACK's sgesvj criterion,
-// |m_p . m_q| <= tol |m_p| |m_q|, tol = sqrt(len) eps).
+// Column pairs (p, q) are rotated until all columns of M V are orthogonal to tol, |m_p . m_q| <= tol |m_p| |m_q| with
+// tol = sqrt(len) eps / 4: a quarter of LAPACK's sgesvj criterion, which costs no sweep (the last one is recognised by
+// kJacobiLastSweepCos) and leaves the vectors that much closer to orthogonal.
 //
 // What bounds it is one dependent chain -- dot product, angle, rotation -- per round of disjoint pairs, k - 1 rounds per
 // sweep and 7 to 9 sweeps whatever the split.  So the columns, not the rows, are dealt over the CTAs: CTA c of a cluster
@@ -19,8 +20,11 @@
 // out side by side in the halves of the warp: half as many trips through shared memory and CTA barriers per round, which
 // otherwise cost as much as the rotations (16 lanes per pair and a trip per round: 0.46 us per round at 256 columns).
 // A sweep: the pairs inside the blocks (a tournament of 8 column pairs), then 2 x CTAs - 1 steps of a tournament of the blocks.
-//   Measured: k = 256 1734 -> 802 us, k = 128 568 -> 313 us against the kernel that deals rows over the CTAs; singular values
-//   and factors as close to 64 bits as its, and closer where the matrix is scaled by 1e-9 (the core is scaled to FP32's range).
+//   Measured against the kernels that deal rows over the CTAs (above 64 columns) or keep the core in one CTA, on 50 cores per
+//   rank (flat, 1/i, geometric, rank-3 and 1e-9-scaled spectra), time and distance from 64 bits of the singular values:
+//     k = 256 1323 -> 800 us, 2.3e-5 -> 5.4e-8; k = 128 461 -> 287 us, 1.3e-5 -> 5.7e-8; k = 64 222 -> 129 us, 5.3e-6 -> 5.5e-8;
+//     k = 32 91 -> 62 us, 2.3e-6 -> 5.7e-8
+//   and of U diag(S) V^T 3.5e-5 -> 1.0e-6, 1.6e-5 -> 5.0e-7, 7.7e-7 -> 9.5e-8, 7.7e-7 -> 4.8e-8.
 #pragma once
 
 #include "bsq_device.cuh"
@@ -99,13 +103,16 @@ __device__ __forceinline__ float column_dot(const float2 (&x)[kPairs], const flo
     }
     return (s0.x + s1.x) + (s0.y + s1.y);
 }
+// x' = c x - s y, y' = s x + c y as corrections, x - s (y + h x) and y + s (x - h y) with h = s / (1 + c), the tangent of half
+// the angle (Rutishauser's form): what is rounded besides x' and y' themselves is a multiple of s, where a rounded cosine
+// lengthens or shortens both columns in every rotation.
 template <int kPairs>
-__device__ __forceinline__ void column_rotate(float2 (&x)[kPairs], float2 (&y)[kPairs], float c, float s) {
-    const float2 c2 = make_float2(c, c), s2 = make_float2(s, s), n2 = make_float2(-s, -s);
+__device__ __forceinline__ void column_rotate(float2 (&x)[kPairs], float2 (&y)[kPairs], float h, float s) {
+    const float2 h2 = make_float2(h, h), m2 = make_float2(-h, -h), s2 = make_float2(s, s), n2 = make_float2(-s, -s);
 #pragma unroll
     for (int u = 0; u < kPairs; ++u) {
-        const float2 p = fma2(c2, x[u], mul2(n2, y[u]));
-        y[u] = fma2(s2, x[u], mul2(c2, y[u]));
+        const float2 p = fma2(n2, fma2(h2, x[u], y[u]), x[u]);
+        y[u] = fma2(s2, fma2(m2, y[u], x[u]), y[u]);
         x[u] = p;
     }
 }
@@ -136,7 +143,7 @@ struct Quad {
 
 // Makes p0 orthogonal to q0 and p1 to q1 (squared norms np., nq., updated): two rotations at once.  Returns whether one of
 // the pairs was above the bound of the last sweep (this half's pair).  The core is scaled so that nothing here leaves FP32's
-// range; pairs of columns below 1e-18 of the largest entry are left as they are.
+// range; pairs whose product is below 1e-19 (both columns below about 4e-17 of the largest entry) are left as they are.
 template <int kPairs, bool kWithV>
 __device__ __forceinline__ bool rotate_two(float2 (&p0)[kPairs], float2 (&q0)[kPairs], float2 (&p1)[kPairs], float2 (&q1)[kPairs],
                                            float2 (&vp0)[kPairs], float2 (&vq0)[kPairs], float2 (&vp1)[kPairs], float2 (&vq1)[kPairs],
@@ -145,21 +152,25 @@ __device__ __forceinline__ bool rotate_two(float2 (&p0)[kPairs], float2 (&q0)[kP
     const float alpha = upper ? np1 : np0, beta = upper ? nq1 : nq0;
     const float ab = alpha * beta, gg = g * g;
     const bool turn = gg > fmaxf(tol2 * ab, 1.2e-38f);
-    // tan = 2 g / (d + sign(d) sqrt(d^2 + 4 g^2)), d = beta - alpha: to a few units in the last place, far below the
-    // tolerance in what it leaves of the pair's product
-    const float d = beta - alpha, r = fmaf(d, d, 4.0f * gg);
-    float t = copysignf(2.0f, d) * g * rcp_ftz(fabsf(d) + r * rsqrt_ftz(r));
-    if (!turn) t = 0.0f;
-    const float c = rsqrt_ftz(fmaf(t, t, 1.0f)), s = c * t, tg = t * g;
-    const float oc = __shfl_xor_sync(0xffffffffu, c, 16), os = __shfl_xor_sync(0xffffffffu, s, 16), otg = __shfl_xor_sync(0xffffffffu, tg, 16);
+    // the angle from that of twice its size, whose cosine and sine are |d| / r and 2 g / r with d = beta - alpha,
+    // r^2 = d^2 + 4 g^2: with q = 1 + |d| / r and e = 1 / sqrt(2 q), sin = 2 g / r e, 1 + cos = 1 + q e, tan = 2 (2 g / r) e^2,
+    // and h = sin / (1 + cos).  All to a few units in the last place, far below the tolerance in what that leaves of the pair's product.
+    // The rotation is as orthogonal as s = 2 h / (1 + h^2) is true for the h that is used, whatever that is: s gets a correction
+    // that makes it so to the last place.  (IEEE divisions and roots throughout give the same distances from 64 bits and take half
+    // as long again.)
+    const float d = beta - alpha, ir = turn ? rsqrt_ftz(fmaf(d, d, 4.0f * gg)) : 0.0f;
+    const float sin2 = copysignf(2.0f, d) * g * ir, q = fmaf(fabsf(d), ir, 1.0f), e = rsqrt_ftz(q + q);
+    const float sin0 = sin2 * e, cos1 = fmaf(q, e, 1.0f), h = sin0 * rcp_ftz(cos1);
+    const float s = fmaf(fmaf(-sin0, fmaf(h, h, 1.0f), h + h), 0.5f * cos1, sin0), tg = 2.0f * sin2 * e * e * g;
+    const float oh = __shfl_xor_sync(0xffffffffu, h, 16), os = __shfl_xor_sync(0xffffffffu, s, 16), otg = __shfl_xor_sync(0xffffffffu, tg, 16);
     const float s0 = upper ? os : s, s1 = upper ? s : os;
     if (s0 != 0.0f || s1 != 0.0f) {                           // (uniform over the warp)
-        const float c0 = upper ? oc : c, c1 = upper ? c : oc, tg0 = upper ? otg : tg, tg1 = upper ? tg : otg;
-        column_rotate<kPairs>(p0, q0, c0, s0);
-        column_rotate<kPairs>(p1, q1, c1, s1);
+        const float h0 = upper ? oh : h, h1 = upper ? h : oh, tg0 = upper ? otg : tg, tg1 = upper ? tg : otg;
+        column_rotate<kPairs>(p0, q0, h0, s0);
+        column_rotate<kPairs>(p1, q1, h1, s1);
         if (kWithV) {
-            column_rotate<kPairs>(vp0, vq0, c0, s0);
-            column_rotate<kPairs>(vp1, vq1, c1, s1);
+            column_rotate<kPairs>(vp0, vq0, h0, s0);
+            column_rotate<kPairs>(vp1, vq1, h1, s1);
         }
         np0 = fmaxf(np0 - tg0, 0.0f);
         nq0 += tg0;
@@ -228,7 +239,7 @@ __global__ void __launch_bounds__(kJbThreads, 1) block_jacobi_kernel(const float
     const int shift = (mx > 0.0f && mx < INFINITY) ? min(100, max(-104, 23 - ilogbf(mx))) : 0;
     const float scale = exp2f((float)shift);
 
-    const float tol = sqrtf((float)kLen) * 5.9604645e-08f, tol2 = tol * tol;
+    const float tol = sqrtf((float)kLen) * (0.25f * 5.9604645e-08f), tol2 = tol * tol;
     Quad<kPairs, kWithV> c4;
     auto straight = [&]() {                                   // (a0, b0) and (a1, b1)
         return rotate_two<kPairs, kWithV>(c4.a[0], c4.b[0], c4.a[1], c4.b[1], c4.av[0], c4.bv[0], c4.av[1], c4.bv[1], c4.na[0], c4.nb[0],

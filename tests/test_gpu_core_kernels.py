@@ -59,6 +59,23 @@ def test_core_of_deficient_and_zero_matrices(lib, k):
     assert np.isfinite(u).all() and np.isfinite(v).all() and not s.any()
 
 
+@pytest.mark.parametrize("k", [8, 16, 17, 33, 48, 64, 65, 100, 128, 200, 256])
+@pytest.mark.parametrize("kind", ["1/i", "flat"])
+def test_rotations_of_fp32_factors_keep_lengths(lib, k, kind):
+    """A matrix of k columns at rank k: its row space is captured whole, so S are its singular values but for rounding.  2e-6 of
+    |S|: a sweep rotates a column k times and there are 8 or 9, and where each rotation rounds an element once, without a bias,
+    that is sqrt(9 * 256) * 2^-25 = 1.4e-6 at 256 columns, with half as much again for the sums of the panel products.  (A rounded
+    cosine in every rotation is a bias: 3e-5 to 6e-5 at 256 columns.)"""
+    rng = np.random.default_rng(k)
+    m = 2 * k + 64
+    q1, q2 = np.linalg.qr(rng.standard_normal((m, k)))[0], np.linalg.qr(rng.standard_normal((k, k)))[0]
+    sv = 1.0 / np.arange(1, k + 1) + 0.05 if kind == "1/i" else 1.0 + 0.1 * rng.random(k)
+    a = ((q1 * sv) @ q2.T).astype(np.float32)
+    exact = np.linalg.svd(a.astype(np.float64), compute_uv=False)
+    s = svd_gpu(lib, a, k)[1]
+    assert np.linalg.norm(s - exact) <= 2e-6 * np.linalg.norm(exact)
+
+
 class CodedFactors:
     """The library with bsq_svd_lowrank standing for the kernels of coded factors."""
 
