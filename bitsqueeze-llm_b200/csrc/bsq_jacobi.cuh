@@ -23,8 +23,9 @@
 //   Measured against the kernels that deal rows over the CTAs (above 64 columns) or keep the core in one CTA, on 50 cores per
 //   rank (flat, 1/i, geometric, rank-3 and 1e-9-scaled spectra), time and distance from 64 bits of the singular values:
 //     k = 256 1323 -> 800 us, 2.3e-5 -> 5.4e-8; k = 128 461 -> 287 us, 1.3e-5 -> 5.7e-8; k = 64 222 -> 129 us, 5.3e-6 -> 5.5e-8;
-//     k = 32 91 -> 62 us, 2.3e-6 -> 5.7e-8
-//   and of U diag(S) V^T 3.5e-5 -> 1.0e-6, 1.6e-5 -> 5.0e-7, 7.7e-7 -> 9.5e-8, 7.7e-7 -> 4.8e-8.
+//     k = 32 91 -> 62 us, 2.3e-6 -> 5.7e-8; k = 16 42 -> 32 us, 6.7e-7 -> 5.4e-8
+//   and of U diag(S) V^T 3.5e-5 -> 1.0e-6, 1.6e-5 -> 5.0e-7, 7.7e-7 -> 9.5e-8, 7.7e-7 -> 4.8e-8, 5.0e-7 -> 4.8e-8.  (Below 12 and
+//   from 17 to 20 columns the other kernel is 3 to 9 us faster, and as much further off.)
 #pragma once
 
 #include "bsq_device.cuh"
@@ -270,6 +271,7 @@ __global__ void __launch_bounds__(kJbThreads, 1) block_jacobi_kernel(const float
         if (l < 2) norm[l] = l ? n[1] : n[0];
     };
     int cur = 0;
+    const int steps = k > kJbCols ? 2 * kCtas - 1 : 0;        // up to 16 columns there is one block and nothing to pair it with
     // where a CTA's blocks go after a step: block 0 ("top") of CTA 0 stays, the others move one place around the ring
     //   top of CTA 1, 2, .. , last, bottom of the last, .. , 1, 0, top of CTA 1
     const int top_cta = (cr == 0 || cr == kCtas - 1) ? cr : cr + 1, top_blk = (cr == 0 || cr != kCtas - 1) ? 0 : 1;
@@ -327,7 +329,7 @@ __global__ void __launch_bounds__(kJbThreads, 1) block_jacobi_kernel(const float
             }
         }
         // ---- block against block ----
-        for (int step = 0; step < 2 * kCtas - 1; ++step) {
+        for (int step = 0; step < steps; ++step) {
             X = cols + (size_t)cur * 2 * kBlock;
             Y = X + kBlock;
             nx = nrm + cur * 2 * kJbCols;
@@ -351,7 +353,7 @@ __global__ void __launch_bounds__(kJbThreads, 1) block_jacobi_kernel(const float
                          cluster.map_shared_rank(nrm, top_cta) + (nxt * 2 + top_blk) * kJbCols + 2 * w);
                 }
             }
-            if (step == 2 * kCtas - 2) {
+            if (step == steps - 1) {
                 const unsigned mine = __syncthreads_or(big) ? 1u : 0u;
                 if (tid < kCtas) cluster.map_shared_rank(votes, tid)[((sweep + 1) & 1) * 8 + cr] = mine;
             }
@@ -359,6 +361,11 @@ __global__ void __launch_bounds__(kJbThreads, 1) block_jacobi_kernel(const float
             // next of these barriers, which this CTA reaches when it has read it.
             cluster.sync();
             cur = nxt;
+        }
+        if (steps == 0) {                                     // (one CTA)
+            const unsigned mine = __syncthreads_or(big) ? 1u : 0u;
+            if (tid == 0) votes[((sweep + 1) & 1) * 8] = mine;
+            __syncthreads();
         }
     }
 
