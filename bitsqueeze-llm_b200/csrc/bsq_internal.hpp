@@ -50,7 +50,7 @@ cudaError_t topk_rows(const float *d_in, float *d_residual, uint32_t rows, uint3
 cudaError_t topk_apply(const uint16_t *d_idx, const float *d_val, uint32_t rows, uint32_t cols, uint32_t k,
                        float *d_dense, unsigned *d_status, cudaStream_t stream);
 
-// Two lists, the first before the second where they name the same element, in one launch.
+// Two lists, the first before the second where they name the same element, in one launch or two.
 cudaError_t topk_apply_two(const uint16_t *d_idx0, const float *d_val0, uint32_t k0, const uint16_t *d_idx1, const float *d_val1,
                            uint32_t k1, uint32_t rows, uint32_t cols, float *d_dense, unsigned *d_status, cudaStream_t stream);
 

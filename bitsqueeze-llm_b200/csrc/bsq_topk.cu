@@ -215,8 +215,9 @@ __global__ void topk_apply_kernel(const uint16_t *__restrict__ idx, const float 
 
 // Two lists of the same rows, the first added before the second (the reference applies its error list, then its outliers,
 // src/bitsqz_llm.cu:1372-1387): one warp per row, so that the order holds without a launch between the lists and the row's
-// sectors are fetched while everything about both lists is.  Four entries of each list in flight per lane.
-// 4096 x 14336 with 143 and 72 entries per row: see the decompress figures (221 us a call, 225 us with a launch per list).
+// sectors are fetched while everything about both lists is.  Four entries of each list in flight per lane; a trip of a warp
+// (128 entries of a list) is a chain of two loads and a store, 1 us, which is what bounds it while the device has rows to
+// spare for few warps.  topk_apply_two says where it stands in for two launches.
 __device__ __forceinline__ void apply_row(const uint16_t *idx, const float *val, unsigned cols, unsigned k, float *row, unsigned lane,
                                           unsigned *status) {
     for (unsigned j0 = lane; j0 < k; j0 += 128) {
@@ -398,6 +399,20 @@ cudaError_t topk_apply_two(const uint16_t *d_idx0, const float *d_val0, uint32_t
                            uint32_t k1, uint32_t rows, uint32_t cols, float *d_dense, unsigned *d_status, cudaStream_t stream) {
     if (!d_dense || rows == 0 || cols == 0) return cudaErrorInvalidValue;
     if ((k0 && (!d_idx0 || !d_val0)) || (k1 && (!d_idx1 || !d_val1))) return cudaErrorInvalidValue;
+    // One launch saves the gap between two (about 3 us), as long as a warp's trips take no longer than that and the entries
+    // are too few for the two launches' larger grids to matter; and lists that name most of a row find it in the L1 cache when one
+    // warp walks it.  us in one / two launches: 256 x 1024 with 10 + 5 entries a row 8.2 / 11.3, 512 x 14336 with
+    // 143 + 287 10.5 / 13.3, 4096 x 14336 with 143 + 72 34.8 / 37.9, 2048 x 4096 with 4096 + 4096 160 / 521; on the other
+    // side 64 x 14336 with 717 + 717 18.6 / 11.3, all 14336 twice 238 / 62, 4096 x 14336 with 717 + 717 190 / 144, 8192 x 4096
+    // with 250 + 100 65 / 60.
+    const uint64_t entries = (uint64_t)rows * ((uint64_t)k0 + k1);
+    const uint32_t trips = (k0 + 127) / 128 + (k1 + 127) / 128;
+    const bool short_lists = entries <= 1400000 && (trips <= 3 || (rows >= 512 && trips <= 5));
+    const bool dense_lists = rows >= 1024 && 5 * ((uint64_t)k0 + k1) >= 2 * (uint64_t)cols;
+    if (!short_lists && !dense_lists) {
+        const cudaError_t err = topk_apply(d_idx0, d_val0, rows, cols, k0, d_dense, d_status, stream);
+        return err != cudaSuccess ? err : topk_apply(d_idx1, d_val1, rows, cols, k1, d_dense, d_status, stream);
+    }
     topk_apply_two_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(d_idx0, d_val0, k0, d_idx1, d_val1, k1, rows, cols, d_dense, d_status);
     return cudaGetLastError();
 }
