@@ -247,8 +247,10 @@ __global__ void __launch_bounds__(1024) cholesky_inverse_smem_kernel(const float
 // The two kernels below serve cores whose factors are coded afterwards (NF4 / NF4_DQ sections, error lists made from them):
 // the codes of a singular pair depend on its sign and, in a flat spectrum, on how the last bits turn neighbouring vectors
 // into one another, so another order of rotations than theirs changes most objects in most bytes (measured: 6 to 8 % of the
-// reconstructed matrix, as large a change as a library solver makes).  Objects keep their bytes; factors that stay in FP32
-// take the block kernel of bsq_jacobi.cuh.
+// reconstructed matrix, as large a change as a library solver makes).  An error list is whole numbers too: which elements of
+// the residual are the largest and in which order changes with the last bits of factors that are themselves FP32.  Objects
+// that hold codes or such a list keep their bytes; where all that can change is the rounding of FP32 values, the factors come
+// from the block kernel of bsq_jacobi.cuh.
 // SVD of the k x k core for k <= kJacobiMaxK: one-sided (Hestenes) Jacobi in one CTA, everything in shared memory.
 // The reference runs cusolverDnSgesvd on the k x n matrix B (svd_lowrank_cuda.cu:399-440); here only the k x k
 // triangular factor is left to decompose.
