@@ -597,7 +597,9 @@ bitsqz_llm_array_t object_header(const Runtime &rt, const CompressJob &job, bool
 // Enqueue one compress call on the runtime's stream: staging of a host input, every stage, and the copies of the
 // results into their final place.  d_packed == nullptr: the object goes to a pinned host block; otherwise into the
 // caller's device buffer of `capacity` bytes.  Returns without waiting; compress_end finishes the call.
-int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_packed, uint64_t capacity, bool want_profile) {
+// in_flight: how many calls of this configuration the caller keeps going side by side (a hint: results do not depend on it).
+int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_packed, uint64_t capacity, bool want_profile,
+                   int in_flight = 1) {
     if (rt.job.active || rt.decompress_active) return 1;
     CompressJob &job = rt.job;
     job = CompressJob{};
@@ -680,6 +682,11 @@ int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_p
         // can count on.  Every call here uses block 1: same singular values as that first reference call to ~5e-5
         // relative, and the same object for the same input on every call.
         const unsigned long long omega_offset = (unsigned long long)std::min(rows, cols) * rank;
+        // Three matrices or more with 150 million elements between them keep the SMs busy: SM time is what counts then, not the
+        // length of one call's chain of kernels.  Wide against narrow tiles of the panel products, same box: 4 x 4096 x 4096
+        // rank 256 4.53 / 4.43 ms, 4 x 8192 x 4096 4.98 / 4.94, 3 x 4096 x 14336 5.32 / 5.32, 6 x 8192 x 4096 5.92 / 5.96 (rank 128
+        // 4.45 / 4.53), 6 x 4096 x 14336 8.05 / 8.14, 8 x 4096 x 14336 10.11 / 10.30.
+        svd_workspace_device_full(rt.svd, in_flight >= 3 && (uint64_t)in_flight * n >= 150000000ull);
         if (svd_lowrank(rt.svd, d_src, rt.u.as<float>(), rt.s.as<float>(), rt.v.as<float>(), 1234ULL, d_status, st, omega_offset,
                         residual_bound ? d_status + 8 : nullptr) != cudaSuccess)
             return fail();
@@ -1222,6 +1229,16 @@ bool lane_setup(bsq_lane *lane, uint16_t rows, uint16_t cols, float outlier, flo
                          BITSQZ_LLM_INPUT_DEVICE);
 }
 
+int lane_compress_begin(bsq_lane *lane, const float *matrix, int input_location, void *d_packed, uint64_t capacity, int in_flight) {
+    try {
+        if (!lane || !matrix) return 1;
+        if (input_location != BITSQZ_LLM_INPUT_HOST && input_location != BITSQZ_LLM_INPUT_DEVICE) return 1;
+        return compress_begin(lane->compress, matrix, input_location, static_cast<uint8_t *>(d_packed), capacity, false, in_flight);
+    } catch (...) {
+        return 1;
+    }
+}
+
 }  // namespace
 
 extern "C" {
@@ -1266,13 +1283,7 @@ void *bsq_lane_stream(bsq_lane *lane, int decompress_side) {
 }
 
 int bsq_lane_compress_begin(bsq_lane *lane, const float *matrix, int input_location, void *d_packed, uint64_t capacity) {
-    try {
-        if (!lane || !matrix) return 1;
-        if (input_location != BITSQZ_LLM_INPUT_HOST && input_location != BITSQZ_LLM_INPUT_DEVICE) return 1;
-        return compress_begin(lane->compress, matrix, input_location, static_cast<uint8_t *>(d_packed), capacity, false);
-    } catch (...) {
-        return 1;
-    }
+    return lane_compress_begin(lane, matrix, input_location, d_packed, capacity, 1);
 }
 
 int bsq_lane_compress_end(bsq_lane *lane, struct bitsqz_llm_array **out, struct bitsqz_llm_array *device_header, uint64_t *packed_size) {
@@ -1392,7 +1403,8 @@ int bsq_batch_compress(bsq_batch *b, const float *const *matrices, int count, in
     for (int i = 0; i < count && rc == 0; ++i) {
         if (i >= L) rc |= finish(i - L);
         if (rc == 0) {
-            rc |= bsq_lane_compress_begin(b->lanes[i % L], matrices[i], input_location, to_device ? d_packed[i] : nullptr, capacity);
+            rc |= lane_compress_begin(b->lanes[i % L], matrices[i], input_location, to_device ? d_packed[i] : nullptr, capacity,
+                                      std::min(L, count));
             if (rc == 0) begun = i + 1;
         }
     }

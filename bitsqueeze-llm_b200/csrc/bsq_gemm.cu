@@ -268,15 +268,16 @@ size_t gemm_workspace_bytes(int M, int N, int max_splits) { return (size_t)M * N
 // Picks the K split so that about two CTAs per SM are busy; partials go to `workspace` (may be null: no split).
 cudaError_t gemm(bool a_kmajor, bool b_kmajor, const float *A, long lda, const float *B, long ldb, float *C, long ldc, int M,
                  int N, int K, const float *kscale, const float *minuend, long ldm, unsigned *flag, unsigned *status,
-                 float *workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream, const unsigned *a_absmax_bits, float b_bound) {
+                 float *workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream, const unsigned *a_absmax_bits, float b_bound,
+                 bool device_full) {
     return gemm_select(tensor_cores_enabled(), a_kmajor, b_kmajor, A, lda, B, ldb, C, ldc, M, N, K, kscale, minuend, ldm, flag,
-                       status, workspace, workspace_bytes, sm_count, stream, a_absmax_bits, b_bound);
+                       status, workspace, workspace_bytes, sm_count, stream, a_absmax_bits, b_bound, device_full);
 }
 
 cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, const float *A, long lda, const float *B, long ldb,
                         float *C, long ldc, int M, int N, int K, const float *kscale, const float *minuend, long ldm,
                         unsigned *flag, unsigned *status, float *workspace, size_t workspace_bytes, int sm_count,
-                        cudaStream_t stream, const unsigned *a_absmax_bits, float b_bound) {
+                        cudaStream_t stream, const unsigned *a_absmax_bits, float b_bound, bool device_full) {
     if (M <= 0 || N <= 0 || K <= 0) return cudaErrorInvalidValue;
     if (allow_tensor_cores) {
         // tensor-core path: one 128-row tile per CTA, two CTAs per SM up to N = 128; K is split so that the tiles fill
@@ -311,8 +312,11 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
         // splitting its piece of B is most of a chunk; below 64 columns, or with more CTAs than that, every tile splits A
         // once more and the time goes up again.  8192 x 256 x 256: 22.8 -> 19.0 us, 4096 x 256 x 256: 22.8 -> 16.7 us, the
         // Gram matrix of 4096 x 256 with its reduction 26.9 -> 20.8 us, 8192 x 128 x 128: 12.5 -> 11.0 us; tiles for twice
-        // the SMs measured 37.3 us (14336 x 256 x 256, 24.7 with one 256-column tile per row tile).
-        if (!with_image && !kscale && !minuend && N <= 256) {
+        // the SMs measured 37.3 us (14336 x 256 x 256, 24.7 with one 256-column tile per row tile).  Narrow tiles take more SM
+        // time in all (4096 x 256 x 256: 32 CTAs for 22.8 us, 128 for 16.7), so not where other matrices fill the device
+        // (`device_full`: eight compress calls of 4096 x 14336, rank 256, side by side: 10.30 ms with narrow tiles, 10.11 with wide ones).
+        // Every width splits K alike (as often as K / 256 allows), so results are the same bits.
+        if (!device_full && !with_image && !kscale && !minuend && N <= 256) {
             const int most_splits = workspace ? max(1, K / 256) : 1;
             while (t.n_tile >= 128 && ((M + 127) / 128) * ((N + t.n_tile - 1) / t.n_tile) * most_splits * 4 < sm_count * 3)
                 t.n_tile = (t.n_tile / 2 + 15) / 16 * 16;

@@ -131,12 +131,12 @@ void *host_block_take(size_t bytes);
 cudaError_t gemm(bool a_kmajor, bool b_kmajor, const float *A, long lda, const float *B, long ldb, float *C, long ldc, int M,
                  int N, int K, const float *kscale, const float *minuend, long ldm, unsigned *flag, unsigned *status,
                  float *workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream, const unsigned *a_absmax_bits = nullptr,
-                 float b_bound = 0.0f);
+                 float b_bound = 0.0f, bool device_full = false);
 // The same with the kernel choice explicit: allow_tensor_cores = false keeps the product on the FP32 pipes.
 cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, const float *A, long lda, const float *B, long ldb,
                         float *C, long ldc, int M, int N, int K, const float *kscale, const float *minuend, long ldm,
                         unsigned *flag, unsigned *status, float *workspace, size_t workspace_bytes, int sm_count,
-                        cudaStream_t stream, const unsigned *a_absmax_bits = nullptr, float b_bound = 0.0f);
+                        cudaStream_t stream, const unsigned *a_absmax_bits = nullptr, float b_bound = 0.0f, bool device_full = false);
 // (a_absmax_bits: device word with the bits of an upper bound of |A|, b_bound: an upper bound of |B| known on the host,
 // 0 = none -- with a bound on |A| the 256-column products split their operands into FP16 halves, bsq_gemm_tc.cuh)
 
@@ -149,6 +149,8 @@ SvdWorkspace *svd_workspace_create(int m, int n, int k, int niter, int sm_count,
 SvdWorkspace *svd_workspace_create_sharded(int m_local, int n, int k, int niter, int sm_count, SvdAllReduce allreduce,
                                            void *allreduce_ctx, int m_total, bool coded_factors = false);
 void svd_workspace_destroy(SvdWorkspace *ws);
+// whether other work fills the device beside the calls that follow (chooses tile widths, not results; no until set)
+void svd_workspace_device_full(SvdWorkspace *ws, bool full);
 // A row-major m x n -> U (m x k row-major), S (k, descending), V (n x k row-major).
 // The random matrix is the first N x k normals of cuRAND's XORWOW sequence of `seed`, starting `offset` values in.
 cudaError_t svd_lowrank(SvdWorkspace *ws, const float *d_A, float *d_U, float *d_S, float *d_V,

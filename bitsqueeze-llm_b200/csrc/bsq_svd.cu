@@ -71,6 +71,7 @@ struct SvdWorkspace {
     const unsigned *a_absmax_use = nullptr;
     int jc_lanes = 4;                   // lanes per column pair of the cluster Jacobi kernel for this k
     bool jc_with_v = false;             // ... and whether it accumulates the right factor (else that comes from the panel)
+    bool device_full = false;           // other work fills the device beside this (chooses tile widths, not results)
     bool block_core = false;            // the core goes to block_jacobi_kernel
     bool own_core_svd = false;          // k small enough for jacobi_svd_kernel (else cuSOLVER's gesvdj on the core)
     bool seeded = false;                // omega holds the draw for `seed`
@@ -717,7 +718,7 @@ cudaError_t orthonormalise(SvdWorkspace *ws, float *Y, float *tmp, int rows, int
         const bool factor_only = last_factor_only && pass + 1 == passes;
         // G = src^T src
         cudaError_t err = gemm(false, false, src, k, src, k, ws->g, k, k, k, rows, nullptr, nullptr, 0, nullptr, ws->status, ws->gemm_ws,
-                               ws->gemm_ws_bytes, ws->sm_count, st);
+                               ws->gemm_ws_bytes, ws->sm_count, st, nullptr, 0.0f, ws->device_full);
         if (err != cudaSuccess) return err;
         // a row-sharded panel: its Gram matrix is the sum of the shards' (the one exchange per QR pass);
         // every rank then factors the same k x k matrix and gets bit-identical R
@@ -740,7 +741,7 @@ cudaError_t orthonormalise(SvdWorkspace *ws, float *Y, float *tmp, int rows, int
         if (factor_only) break;
         // dst = src T
         err = gemm(true, false, src, k, ws->t, k, dst, k, rows, k, k, nullptr, nullptr, 0, nullptr, ws->status, ws->gemm_ws,
-                   ws->gemm_ws_bytes, ws->sm_count, st);
+                   ws->gemm_ws_bytes, ws->sm_count, st, nullptr, 0.0f, ws->device_full);
         if (err != cudaSuccess) return err;
         std::swap(src, dst);
     }
@@ -762,7 +763,7 @@ cudaError_t times_w(SvdWorkspace *ws, const float *A, bool w_transposed_product,
                            nullptr, 0, nullptr, ws->status, ws->gemm_ws, ws->gemm_ws_bytes, ws->sm_count, st, ws->a_absmax_valid ? ws->a_absmax_use : nullptr,
                            // what X can hold: standard normal draws from 32-bit uniforms stay below 6.7, the columns of an
                            // orthonormalised panel have norm 1 (a loose bound costs FP16 range, not precision)
-                           x_colmajor ? 16.0f : 1024.0f);
+                           x_colmajor ? 16.0f : 1024.0f, ws->device_full);
     span_end(ws, sp, st);
     // row-sharded W: W^T X contracts over the sharded rows, so the shards' partial products are summed
     if (err == cudaSuccess && w_transposed_product && ws->allreduce) err = timed_allreduce(ws, C, (size_t)rows_out * ws->k, st);
@@ -889,6 +890,8 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
     return ws;
 }
 
+void svd_workspace_device_full(SvdWorkspace *ws, bool full) { ws->device_full = full; }
+
 void svd_workspace_destroy(SvdWorkspace *ws) {
     if (!ws) return;
     float *bufs[] = {ws->omega, ws->y, ws->y2, ws->z, ws->z2, ws->g, ws->w, ws->t, ws->tinv1, ws->tinv2,
@@ -992,7 +995,7 @@ cudaError_t svd_lowrank(SvdWorkspace *ws, const float *d_A, float *d_U, float *d
     if ((err = orthonormalise(ws, ws->z, ws->z2, ws->N, 2, ws->tinv1, ws->tinv2, &qz, false, st, from_panel)) != cudaSuccess) return err;
     if (from_panel) qz = ws->z;
     if ((err = gemm(true, false, ws->tinv2, k, ws->tinv1, k, ws->core, k, k, k, k, nullptr, nullptr, 0, nullptr, ws->status, nullptr, 0,
-                    ws->sm_count, st)) != cudaSuccess)
+                    ws->sm_count, st, nullptr, 0.0f, ws->device_full)) != cudaSuccess)
         return err;
     // The row-major C read as column-major is C^T = Vc S Uc^T: the solver's "U" is Vc, its "V" is Uc.
     if (ws->block_core) {
@@ -1025,10 +1028,10 @@ cudaError_t svd_lowrank(SvdWorkspace *ws, const float *d_A, float *d_U, float *d
     float *d_left = ws->transposed ? d_V : d_U;            // M x k factor
     float *d_right = ws->transposed ? d_U : d_V;           // N x k factor
     if ((err = gemm(true, true, q, k, ws->vc, k, d_left, k, ws->M, k, k, nullptr, nullptr, 0, nullptr, ws->status, ws->gemm_ws, ws->gemm_ws_bytes,
-                    ws->sm_count, st)) != cudaSuccess)
+                    ws->sm_count, st, nullptr, 0.0f, ws->device_full)) != cudaSuccess)
         return err;
     return gemm(true, true, qz, k, ws->uc, k, d_right, k, ws->N, k, k, nullptr, nullptr, 0, nullptr, ws->status, ws->gemm_ws, ws->gemm_ws_bytes,
-                ws->sm_count, st);
+                ws->sm_count, st, nullptr, 0.0f, ws->device_full);
 }
 
 size_t reconstruct_workspace_bytes(int m, int n, int k) {

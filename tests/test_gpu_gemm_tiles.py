@@ -3,6 +3,8 @@ and split, reductions of one and of four elements per thread, the scale pass ove
 
 Bound: three tensor-core products of split operands leave at most a few 1e-7 of sum |a||b| (FP32 accumulation of up to 4096
 terms in the tensor core's order); 4e-6 is allowed."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -51,3 +53,31 @@ def test_split_products(lib, shape):
     M, N, K = shape
     check(lib, True, False, M, N, K, 0, True)
     check(lib, True, False, M, N, K, 3, True)
+
+
+@pytest.mark.parametrize("shape", [(4096, 4800, 256, 11), (4800, 8000, 144, 10), (8200, 4608, 128, -1)])
+def test_objects_do_not_depend_on_the_matrices_in_flight(pkg, lib, shape):
+    """A batch whose matrices fill the device keeps the panel products' tiles wide: same bytes as one matrix at a time."""
+    rows, cols, rank, uv = shape
+    mats = [torch.randn(rows, cols, device="cuda", generator=torch.Generator(device="cuda").manual_seed(i)) for i in range(8)]
+    batch = lib.bsq_batch_create(rows, cols, 0.01, 0.0, rank, 1, uv, -1, -1, 8)
+    assert batch
+    try:
+        cap = int(lib.bsq_lane_packed_capacity(lib.bsq_batch_lane(batch, 0)))
+        want = []
+        for m in mats:
+            buf, size = torch.zeros(cap, dtype=torch.uint8, device="cuda"), C.c_uint64(0)
+            torch.cuda.synchronize()
+            assert lib.bsq_lane_compress_begin(lib.bsq_batch_lane(batch, 0), m.data_ptr(), 1, buf.data_ptr(), cap) == 0
+            assert lib.bsq_lane_compress_end(lib.bsq_batch_lane(batch, 0), None, None, C.byref(size)) == 0
+            want.append(buf[200: int(size.value)].clone())
+        for count in (2, 4, 8):
+            bufs = [torch.zeros(cap, dtype=torch.uint8, device="cuda") for _ in range(count)]
+            vp = C.c_void_p * count
+            torch.cuda.synchronize()
+            assert lib.bsq_batch_compress(batch, vp(*[m.data_ptr() for m in mats[:count]]), count, 1, vp(*[b.data_ptr() for b in bufs]), cap,
+                                          None, None, None) == 0
+            for b, w in zip(bufs, want):
+                assert torch.equal(b[200: 200 + w.numel()], w), count
+    finally:
+        lib.bsq_batch_destroy(batch)
