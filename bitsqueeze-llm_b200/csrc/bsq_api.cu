@@ -1037,15 +1037,16 @@ bool locate_topk(Runtime &rt, const bitsqz_llm_array_t *c, PayloadAccess how, co
            cudaMemcpyAsync(bufs.val.p, src + cnt * 2, cnt * 4, cudaMemcpyDefault, rt.stream) == cudaSuccess;
 }
 
-// The object's lists, located before anything is written to the result (which may lie over the object) ...
+// The object's lists ...
 struct Lists {
     const uint16_t *idx[2] = {};
     const float *val[2] = {};
     uint32_t k[2] = {};                   // error, outliers; 0: none
+    bool located = false;
 };
-bool locate_lists(Runtime &rt, const bitsqz_llm_array_t *c, PayloadAccess how, const SectionHeads &heads, bool has_err, bool has_out, Lists *l) {
-    l->k[0] = has_err ? heads.err.num_topk_columns : 0;
-    l->k[1] = has_out ? heads.outlier.num_topk_columns : 0;
+bool locate_lists(Runtime &rt, const bitsqz_llm_array_t *c, PayloadAccess how, const SectionHeads &heads, Lists *l) {
+    if (l->located) return true;
+    l->located = true;
     return (!l->k[0] || locate_topk(rt, c, how, c->section_error_topk, heads.err, rt.err, &l->idx[0], &l->val[0])) &&
            (!l->k[1] || locate_topk(rt, c, how, c->section_outlier_topk, heads.outlier, rt.outlier, &l->idx[1], &l->val[1]));
 }
@@ -1086,12 +1087,16 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
     }
     unsigned *d_status = rt.status.as<unsigned>();
     // A result that lies over the object (an arena with the object at its end) would be written while other CTAs still
-    // read codes, scales or lists there: the sections are copied first, as those that are not aligned are.
+    // read codes, scales or lists there: the sections are copied first, as those that are not aligned are.  (Elsewhere the
+    // lists come last: of a host object the largest copy is then under way while the small ones are queued.)
     PayloadAccess how;
     how.on_device = reach == Reach::kKernels;
-    how.in_place = how.on_device && !ranges_overlap(d_dst, (uint64_t)c->num_elements * 4, c->payload, payload_bytes);
+    const bool over_object = ranges_overlap(d_dst, (uint64_t)c->num_elements * 4, c->payload, payload_bytes);
+    how.in_place = how.on_device && !over_object;
     Lists lists;
-    if (!locate_lists(rt, c, how, heads, has_err, has_out, &lists)) return fail();
+    lists.k[0] = has_err ? heads.err.num_topk_columns : 0;
+    lists.k[1] = has_out ? heads.outlier.num_topk_columns : 0;
+    if (over_object && !locate_lists(rt, c, how, heads, &lists)) return fail();
     if (c->flags & kFlagSvd) {
         const uint32_t rank = (uint16_t)c->effective_rank;
         if (!decode_section(rt, c, how, c->section_u, heads.u, c->svd_uv_format, (uint64_t)c->num_rows * rank, &rt.q_direct, rt.u.as<float>())) return fail();
@@ -1105,6 +1110,7 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
         // (with one list the reference's order "error list first, outliers second" has nothing to order)
         QuantSource q;
         if (!locate_quant(rt, c, how, c->section_direct, heads.direct, c->quantization_only_format, c->num_elements, &rt.q_direct, &q)) return fail();
+        if (!locate_lists(rt, c, how, heads, &lists)) return fail();
         const int i = lists.k[0] ? 0 : 1;
         if (nf4_dequantize_add_topk(q.scales_f32, q.dq, q.scale_codes, q.data, c->num_rows, c->num_columns, lists.idx[i], lists.val[i],
                                     lists.k[i], d_dst, d_status, rt.sm_count, st) != cudaSuccess)
@@ -1113,7 +1119,7 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
     } else {
         if (!decode_section(rt, c, how, c->section_direct, heads.direct, c->quantization_only_format, c->num_elements, &rt.q_direct, d_dst)) return fail();
     }
-    if (!apply_lists(rt, c, lists, d_dst)) return fail();
+    if (!locate_lists(rt, c, how, heads, &lists) || !apply_lists(rt, c, lists, d_dst)) return fail();
     if (cudaMemcpyAsync(rt.h_status, rt.status.p, 64, cudaMemcpyDeviceToHost, st) != cudaSuccess) return fail();
     rt.decompress_active = true;
     return 0;
