@@ -1074,7 +1074,11 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
     };
     SectionHeads heads;
     const uint64_t payload_bytes = bitsqz_llm_get_packed_size(c) - sizeof(bitsqz_llm_array_t);
-    const Reach reach = payload_on_device ? memory_reach(c->payload, payload_bytes) : Reach::kCopies;
+    // FP32 sections move by stream copies; only where there are others do kernels look into the payload
+    bool kernels_read = false;
+    for (const bitsqz_section_t *s : {&c->section_u, &c->section_s, &c->section_v, &c->section_direct, &c->section_outlier_topk, &c->section_error_topk})
+        kernels_read = kernels_read || s->storage == BITSQZ_SECTION_QUANT || s->storage == BITSQZ_SECTION_TOPK;
+    const Reach reach = payload_on_device && kernels_read ? memory_reach(c->payload, payload_bytes) : Reach::kCopies;
     if (!fetch_heads(rt, c, payload_on_device, reach, &heads)) return fail();
     const bool has_out = c->flags & kFlagOutlier, has_err = c->flags & kFlagError;
     if (has_out && !topk_section_ok(rt.outlier, c, c->section_outlier_topk, heads.outlier)) return 1;
