@@ -19,7 +19,7 @@
 namespace bsq {
 namespace {
 
-// ---- rows that fit shared memory, k <= kCandCap ----------------------------------------------
+// ---- rows that fit shared memory, k <= kCandCap (ragged_rows_fit for rows off 16 bytes) --------
 // One group of G warps per row (bsq_rowgroup.cuh); a CTA holds several groups, rows are dealt out
 // round-robin over all groups of the grid.  kBulk: 16-byte aligned rows, which a bulk copy moves; other rows (cols not a
 // multiple of 4, or a matrix that starts off a 16-byte boundary) are moved by the lanes, four bytes at a time, eight loads
@@ -323,6 +323,18 @@ static GroupGeometry group_geometry(uint32_t cols) {
 static bool topk_rows_fit_smem(uint32_t cols, uint32_t k) {
     return k > 0 && k <= (uint32_t)kCandCap && cols <= 24576u && group_geometry(cols).group_bytes <= 110u * 1024u;
 }
+// Rows that no bulk copy can move: up to how many entries the group kernel is the faster one.  Its bound is the k-th largest of
+// the two largest float4 of every lane; as k comes near the number of those (two per lane, or the row's float4) more elements
+// reach it than there is room for, and the row is done once more the slow way: 2 to 3 times the generic kernel's time.
+// us, group / generic: 148 x 1001 k = 80 16 / 16, k = 128 51 / 16; 2000 x 3001 k = 96 29 / 68, k = 128 125 / 70; 8192 x 8190 k = 160
+// 139 / 563, k = 192 718 / 565; 2000 x 14335 k = 208 74 / 211, k = 240 395 / 211; 600 x 63 k = 16 10 / 12, k = 24 35 / 12.
+// With many rows the generic kernel's passes weigh more, so the line lies a little higher.
+static bool ragged_rows_fit(uint32_t rows, uint32_t cols, uint32_t k) {
+    const int G = group_geometry(cols).G;
+    if (k > (cols + 3) / 4 || (G == 8 && k > 216)) return false;
+    if (G == 8 || rows >= 1024) return G == 8 || k <= (G == 2 ? 112u : 176u);
+    return k <= (G == 2 ? 80u : 160u) && (k <= 32 || 5 * k <= cols);
+}
 // rows that a bulk copy can move: whole 16-byte pieces at 16-byte boundaries
 static bool bulk_rows(const void *d_in, const void *d_residual, uint32_t cols) {
     return cols % 4 == 0 && reinterpret_cast<uintptr_t>(d_in) % 16 == 0 && reinterpret_cast<uintptr_t>(d_residual) % 16 == 0;
@@ -360,13 +372,13 @@ cudaError_t topk_rows(const float *d_in, float *d_residual, uint32_t rows, uint3
         return cudaSuccess;
     }
     if (!d_idx || !d_val) return cudaErrorInvalidValue;
-    if (topk_rows_fit_smem(cols, k)) {
+    const bool bulk = bulk_rows(d_in, d_residual, cols);
+    if (topk_rows_fit_smem(cols, k) && (bulk || ragged_rows_fit(rows, cols, k))) {
         if (d_bound) {
             const cudaError_t e = cudaMemsetAsync(d_bound, 0, sizeof(unsigned), stream);
             if (e != cudaSuccess) return e;
             if (bound_written) *bound_written = true;
         }
-        const bool bulk = bulk_rows(d_in, d_residual, cols);
 #define BSQ_TOPK(G_)                                                                                                             \
     (bulk ? launch_group<G_, true>(d_in, d_residual, rows, cols, k, d_idx, d_val, d_status, sm_count, stream, d_bound) \
           : launch_group<G_, false>(d_in, d_residual, rows, cols, k, d_idx, d_val, d_status, sm_count, stream, d_bound))

@@ -52,6 +52,26 @@ def test_ragged_topk_matches_oracle(lib, oracle, cols, shift):
                 assert bool((buf[shift + rows * cols:] == 0).all())
 
 
+@pytest.mark.parametrize("rows,cols,k", [(1023, 63, 16), (1023, 63, 17), (1024, 65, 17), (1024, 65, 18), (7, 129, 32), (7, 129, 33), (7, 166, 33),
+                                         (1023, 1001, 80), (1023, 1001, 81), (1024, 1001, 112), (1024, 1001, 113), (40, 4099, 160),
+                                         (40, 4099, 161), (1024, 4099, 176), (1024, 4099, 177), (5, 8195, 216), (5, 8195, 217)])
+def test_ragged_topk_either_side_of_the_lines(lib, oracle, rows, cols, k):
+    """Where the kernel for short lists of ragged rows ends and the one for any shape begins (ragged_rows_fit)."""
+    x = np.random.default_rng(rows + cols + k).standard_normal((rows, cols)).astype(np.float32)
+    x[rows // 2, : cols // 2] = 0.0
+    x[rows - 1] = np.round(x[rows - 1])                       # ties
+    want_i, want_v, want_res = oracle.topk_rows(x, k, zero_selected=True)
+    d_x = torch.from_numpy(x).cuda()
+    d_i, d_v = torch.zeros(rows, k, dtype=torch.int16, device="cuda"), torch.zeros(rows, k, device="cuda")
+    res, status = torch.empty_like(d_x), torch.zeros(4, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert lib.bsq_topk_rows(d_x.data_ptr(), res.data_ptr(), rows, cols, k, d_i.data_ptr(), d_v.data_ptr(), status.data_ptr(), None) == 0
+    torch.cuda.synchronize()
+    assert int(status[0]) == 0
+    assert np.array_equal(d_i.cpu().numpy().view(np.uint16), want_i) and np.array_equal(bits(d_v.cpu().numpy()), bits(want_v))
+    assert np.array_equal(bits(res.cpu().numpy()), bits(want_res))
+
+
 @pytest.mark.parametrize("shape", [(1, 1), (1, 63), (3, 65), (17, 1003), (64, 1024), (129, 515)])
 @pytest.mark.parametrize("q", [10, 11])
 def test_error_list_of_a_quantised_matrix_matches_oracle(pkg, lib, oracle, shape, q):
