@@ -331,9 +331,11 @@ static bool topk_rows_fit_smem(uint32_t cols, uint32_t k) {
 // With many rows the generic kernel's passes weigh more, so the line lies a little higher.
 static bool ragged_rows_fit(uint32_t rows, uint32_t cols, uint32_t k) {
     const int G = group_geometry(cols).G;
-    if (k > (cols + 3) / 4 || (G == 8 && k > 216)) return false;
-    if (G == 8 || rows >= 1024) return G == 8 || k <= (G == 2 ? 112u : 176u);
-    return k <= (G == 2 ? 80u : 160u) && (k <= 32 || 5 * k <= cols);
+    if (k > (cols + 3) / 4) return false;
+    if (G == 8) return k <= 216;
+    const uint32_t most = G == 2 ? (rows >= 2000 ? 112 : rows >= 1024 ? 108 : rows >= 700 ? 100 : 80)
+                                 : (rows >= 2000 ? 176 : rows >= 1024 ? 168 : 160);
+    return k <= most && (rows >= 1024 || k <= 32 || 5 * k <= cols);
 }
 // rows that a bulk copy can move: whole 16-byte pieces at 16-byte boundaries
 static bool bulk_rows(const void *d_in, const void *d_residual, uint32_t cols) {

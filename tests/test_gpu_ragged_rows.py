@@ -53,8 +53,9 @@ def test_ragged_topk_matches_oracle(lib, oracle, cols, shift):
 
 
 @pytest.mark.parametrize("rows,cols,k", [(1023, 63, 16), (1023, 63, 17), (1024, 65, 17), (1024, 65, 18), (7, 129, 32), (7, 129, 33), (7, 166, 33),
-                                         (1023, 1001, 80), (1023, 1001, 81), (1024, 1001, 112), (1024, 1001, 113), (40, 4099, 160),
-                                         (40, 4099, 161), (1024, 4099, 176), (1024, 4099, 177), (5, 8195, 216), (5, 8195, 217)])
+                                         (699, 1001, 80), (699, 1001, 81), (1023, 1001, 100), (1023, 1001, 101), (1024, 1001, 108),
+                                         (1024, 1001, 109), (2000, 515, 112), (2000, 515, 113), (40, 4099, 160), (40, 4099, 161),
+                                         (1024, 4099, 168), (1024, 4099, 169), (2000, 4099, 176), (2000, 4099, 177), (5, 8195, 216), (5, 8195, 217)])
 def test_ragged_topk_either_side_of_the_lines(lib, oracle, rows, cols, k):
     """Where the kernel for short lists of ragged rows ends and the one for any shape begins (ragged_rows_fit)."""
     x = np.random.default_rng(rows + cols + k).standard_normal((rows, cols)).astype(np.float32)
