@@ -413,17 +413,19 @@ cudaError_t topk_apply_two(const uint16_t *d_idx0, const float *d_val0, uint32_t
                            uint32_t k1, uint32_t rows, uint32_t cols, float *d_dense, unsigned *d_status, cudaStream_t stream) {
     if (!d_dense || rows == 0 || cols == 0) return cudaErrorInvalidValue;
     if ((k0 && (!d_idx0 || !d_val0)) || (k1 && (!d_idx1 || !d_val1))) return cudaErrorInvalidValue;
-    // One launch saves the gap between two (about 3 us), as long as a warp's trips take no longer than that and the entries
-    // are too few for the two launches' larger grids to matter; and lists that name most of a row find it in the L1 cache when one
-    // warp walks it.  us in one / two launches: 256 x 1024 with 10 + 5 entries a row 8.2 / 11.3, 512 x 14336 with
-    // 143 + 287 10.5 / 13.3, 4096 x 14336 with 143 + 72 34.8 / 37.9, 2048 x 4096 with 4096 + 4096 160 / 521; on the other
-    // side 64 x 14336 with 717 + 717 18.6 / 11.3, all 14336 twice 238 / 62, 4096 x 14336 with 717 + 717 190 / 144, 8192 x 4096
-    // with 250 + 100 65 / 60.
-    const uint64_t entries = (uint64_t)rows * ((uint64_t)k0 + k1);
+    // A decompress call is 2 to 6 us shorter with one launch than with two, until a warp's trips take longer than that (few
+    // rows), or a matrix beyond the L2 wants the two launches' larger grids; and lists that name a good part of a row find it in
+    // the L1 cache when one warp walks it.  us a call, one / two launches, calls of either taken in turn: 300 x 4096
+    // with 41 + 20 entries a row 38 / 41, 64 x 8192 with 82 + 164 39 / 41; 4001 x 4096 with 41 + 82 56 / 59; 2048 x 4096 with
+    // 41 + 819 55 / 67, 1000 x 8192 with 3277 + 3277 112 / 189; on the other side 8 x 14336 with 5734 + 5734 125 / 39, 64 x 14336 with
+    // 717 + 717 43 / 41, 4001 x 14336 with 717 + 717 267 / 225, 6144 x 8192 with 82 + 1638 352 / 281.
+    const uint64_t listed = (uint64_t)k0 + k1, entries = rows * listed, elements = (uint64_t)rows * cols;
     const uint32_t trips = (k0 + 127) / 128 + (k1 + 127) / 128;
-    const bool short_lists = entries <= 1400000 && (trips <= 3 || (rows >= 512 && trips <= 5));
-    const bool dense_lists = rows >= 1024 && 5 * ((uint64_t)k0 + k1) >= 2 * (uint64_t)cols;
-    if (!short_lists && !dense_lists) {
+    bool one_launch;
+    if (rows >= 512 && 5 * listed >= cols) one_launch = elements <= (32u << 20) || 2 * listed >= cols;
+    else if (entries > 1400000) one_launch = trips <= 3;
+    else one_launch = trips <= (rows >= 512 ? 8u : 5u);
+    if (!one_launch) {
         const cudaError_t err = topk_apply(d_idx0, d_val0, rows, cols, k0, d_dense, d_status, stream);
         return err != cudaSuccess ? err : topk_apply(d_idx1, d_val1, rows, cols, k1, d_dense, d_status, stream);
     }

@@ -12,11 +12,11 @@ torch = pytest.importorskip("torch")
 
 # rows, cols, error entries, outlier entries per row
 SHAPES = [
-    (2, 70, 1, 1), (3, 300, 1, 128), (9, 700, 127, 256),                   # up to three trips of 128 entries: one launch
-    (9, 700, 129, 129), (64, 1024, 700, 700),                             # more, few rows: two
-    (511, 1024, 300, 200), (512, 1024, 300, 200), (512, 1024, 300, 257),   # five trips from 512 rows on, six
-    (4100, 1024, 170, 171), (4108, 1024, 170, 171),        # 1.398 and 1.401 million entries
-    (1023, 1000, 200, 200), (1024, 1000, 200, 200), (1024, 1000, 900, 700), (1023, 1000, 1000, 700), (1024, 2000, 399, 400),     # dense lists
+    (2, 70, 1, 1), (3, 300, 1, 128), (9, 700, 127, 256), (9, 1000, 300, 200),       # up to five trips of 128 entries: one launch
+    (9, 1000, 300, 300), (64, 1024, 700, 700),                             # more, few rows: two
+    (511, 6000, 500, 400), (512, 6000, 500, 400), (512, 6000, 500, 600),   # eight trips from 512 rows on, nine
+    (4100, 2048, 170, 171), (4108, 2048, 170, 171), (4100, 2048, 1, 370),         # 1.398 and 1.401 million entries, in four trips and three
+    (511, 1000, 100, 100), (512, 1000, 100, 100), (512, 1000, 900, 700), (511, 1000, 1000, 700), (600, 2000, 399, 400),      # dense lists
 ]
 
 
