@@ -12,8 +12,8 @@
 //   cholesky_inverse_blocked_kernel  one CTA per block row of R^-1, which needs nothing from the other rows:
 //       T_IJ = -(sum_{L=I..J-1} T_IL R_LJ) T_JJ from left to right.
 // Every value is the same sum in the same order as in the one-CTA kernel that did both before, so results are too, bit for
-// bit.  That one (cholesky_small_kernel) stays for k <= 64.  Measured, both kernels against it: k = 256 74 + 25 against
-// 134 us, k = 192 49 + 19 against 80 us, k = 128 29 + 13 against 43 us, k = 100 29 + 13 against 42 us.
+// bit.  That one (cholesky_small_kernel) stays for k <= 64.  In launch lists of whole calls, both kernels against it: k = 256
+// 78 + 26 against 138 us, k = 128 30 + 12 against 49 us.
 #pragma once
 
 #include "bsq_device.cuh"
