@@ -683,7 +683,7 @@ int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_p
         // relative, and the same object for the same input on every call.
         const unsigned long long omega_offset = (unsigned long long)std::min(rows, cols) * rank;
         // Three matrices or more with 150 million elements between them keep the SMs busy: SM time is what counts then, not the
-        // length of one call's chain of kernels.  Wide against narrow tiles of the panel products, same box: 4 x 4096 x 4096
+        // length of one call's chain of kernels.  Wide against narrow tiles of the panel products, runs of either in turn: 4 x 4096 x 4096
         // rank 256 4.53 / 4.43 ms, 4 x 8192 x 4096 4.98 / 4.94, 3 x 4096 x 14336 5.32 / 5.32, 6 x 8192 x 4096 5.92 / 5.96 (rank 128
         // 4.45 / 4.53), 6 x 4096 x 14336 8.05 / 8.14, 8 x 4096 x 14336 10.11 / 10.30.
         svd_workspace_device_full(rt.svd, in_flight >= 3 && (uint64_t)in_flight * n >= 150000000ull);
