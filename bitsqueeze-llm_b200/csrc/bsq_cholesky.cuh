@@ -5,15 +5,19 @@
 // s / 2 under every pivot keep a rank-deficient panel from dividing by zero or taking the root of a negative number:
 // deficient directions just come out shorter than unit length (an all-zero panel gives R = R^-1 = 0).
 //
-// Work by 32 x 32 blocks, k padded to a multiple of 32 with an identity, in two kernels:
-//   cholesky_factor_kernel   one CTA.  What bounds it is the chain of k pivots: while one warp factors the diagonal block of
-//       step J, the other warps apply step J - 1 to the rest of the matrix; only the block that the next pivots need is
-//       updated first.
-//   cholesky_inverse_blocked_kernel  one CTA per block row of R^-1, which needs nothing from the other rows:
-//       T_IJ = -(sum_{L=I..J-1} T_IL R_LJ) T_JJ from left to right.
-// Every value is the same sum in the same order as in the one-CTA kernel that did both before, so results are too, bit for
-// bit.  That one (cholesky_small_kernel) stays for k <= 64.  In launch lists of whole calls, both kernels against it: k = 256
-// 78 + 26 against 138 us, k = 128 30 + 12 against 49 us.
+// Work by 32 x 32 blocks in shared memory, k padded to a multiple of 32 with an identity.  What bounds it is the chain of k pivots:
+// root, shuffle and multiply-add of about 70 clocks each; everything else is arranged around the warp that walks it.
+//   * That warp has a scheduler (almost) to itself.  It takes the next pivot's row by shuffle and the rows below through shared memory,
+//     behind its own shuffles: 105 clocks per pivot (a round trip through shared memory on the chain, roots that scale for
+//     subnormal arguments and stores to global memory in between: 230).
+//   * The block row is a forward substitution right behind the pivots, eight at a time (named barriers), the block of the next
+//     pivots is updated right behind that, and all other updates run beside the chain.  From about 200 columns on those are
+//     what an SM's multiply-adds take: 53 us at 256 columns for 8 blocks, 17 us at 128 for 4.
+//   * R and the inverses of its diagonal blocks go out block row by block row, and other CTAs make the rows of the inverse
+//     from them while the factor goes on: T_IJ = -(sum_{L=I..J-1} T_IL R_LJ) T_JJ from left to right.
+// Every value is the same sum in the same order whatever the number of CTAs or launches.  Back to back, factor and inverse, against the
+// two kernels (one CTA; one per block row) and, up to 64 columns, the single CTA that did this before: k = 256 64 against 99 us,
+// 192 41 / 67, 128 25 / 41, 64 14.6 / 18.7, 32 6.5 / 10.5; the factor alone 53 / 79 us at 256, 17 / 30 us at 128.
 #pragma once
 
 #include "bsq_device.cuh"
@@ -26,547 +30,582 @@ constexpr int kCB = 32;
 constexpr int kCBB = kCB * kCB;
 constexpr int kCTs = kCB + 4;
 __host__ __device__ constexpr int chol_blocks(int k) { return (k + kCB - 1) / kCB; }
-__host__ __device__ constexpr size_t cholesky_factor_smem_bytes(int k) {
-    return ((size_t)(chol_blocks(k) * (chol_blocks(k) + 1) / 2 + chol_blocks(k)) * kCBB + kCBB + 3 * kCB + 64) * sizeof(float);
-}
 __device__ __forceinline__ int blk_id(int I, int J, int nb) { return I * nb - (I * (I - 1)) / 2 + (J - I); }
-// Block products, 64 threads each, 4 x 4 outputs per thread (rows 4 ti .. + 3, columns 4 tc .. + 3): acc -= A^T B, both
-// operands with the contraction index in rows (lda, ldb apart), which is the form in which a warp's reads of either are one
-// conflict-free float4 per 16 multiply-adds.
+// 16 bytes of shared memory; volatile, so that the loads of a step stay in front of the work that is meant to hide them
+__device__ __forceinline__ float4 lds4(unsigned at) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
+}
+// Two FP32 multiply-adds per instruction; each half rounds as the scalar instruction does.
+__device__ __forceinline__ float2 chol_fma2(float2 a, float2 b, float2 c) {
+    float2 r;
+    asm volatile("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<unsigned long long &>(r))
+                 : "l"(reinterpret_cast<unsigned long long &>(a)), "l"(reinterpret_cast<unsigned long long &>(b)),
+                 "l"(reinterpret_cast<unsigned long long &>(c)));
+    return r;
+}
+// Block products, acc -= A^T B: both operands with the contraction index in rows (lda, ldb apart).  A 16-byte load of shared memory
+// takes four clocks of the SM however many lanes read the same, so what bounds these is loads per multiply-add: 16 threads take
+// a block, 8 x 8 outputs each (rows 8 ti .. + 7, columns 8 tc .. + 7), four loads per 64 multiply-adds.  The next row is on its
+// way while one is multiplied.
+struct MacRow {
+    float4 a0, a1, b0, b1;
+};
+__device__ __forceinline__ void mac_fetch(MacRow &m, unsigned A, unsigned B) {
+    m.a0 = lds4(A);
+    m.a1 = lds4(A + 16);
+    m.b0 = lds4(B);
+    m.b1 = lds4(B + 16);
+}
+__device__ __forceinline__ void mac_row(float2 (&acc)[8][4], const MacRow &m) {
+    const float av[8] = {m.a0.x, m.a0.y, m.a0.z, m.a0.w, m.a1.x, m.a1.y, m.a1.z, m.a1.w};
+    const float2 bv[4] = {make_float2(m.b0.x, m.b0.y), make_float2(m.b0.z, m.b0.w), make_float2(m.b1.x, m.b1.y), make_float2(m.b1.z, m.b1.w)};
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[r][q] = chol_fma2(make_float2(-av[r], -av[r]), bv[q], acc[r][q]);
+}
 template <int lda, int ldb>
-__device__ __forceinline__ void block_mac(float (&acc)[4][4], const float *__restrict__ A, const float *__restrict__ B, int ti, int tc) {
-#pragma unroll 8
-    for (int l = 0; l < kCB; ++l) {
-        const float4 a = *reinterpret_cast<const float4 *>(A + l * lda + 4 * ti);
-        const float4 b = *reinterpret_cast<const float4 *>(B + l * ldb + 4 * tc);
-        const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[r][q] = fmaf(-av[r], bv[q], acc[r][q]);
+__device__ __forceinline__ void block_mac(float2 (&acc)[8][4], const float *A_, const float *B_, int ti, int tc) {
+    unsigned A = smem_u32(A_ + 8 * ti), B = smem_u32(B_ + 8 * tc);
+    MacRow m0, m1;
+    mac_fetch(m0, A, B);
+#pragma unroll 2
+    for (int l = 0; l < kCB; l += 2) {
+        mac_fetch(m1, A + 4 * lda, B + 4 * ldb);
+        mac_row(acc, m0);
+        if (l + 2 < kCB) {
+            A += 8 * lda;
+            B += 8 * ldb;
+        }
+        mac_fetch(m0, A, B);                                // (the last trip reads a row again)
+        mac_row(acc, m1);
     }
 }
-// a thread's 4 x 4 tile of a block, as four float4
-__device__ __forceinline__ void tile_load(float (&acc)[4][4], const float *O, int ti, int tc) {
+// a thread's 8 x 8 tile of a block
+__device__ __forceinline__ void tile_load(float2 (&acc)[8][4], const float *O, int ti, int tc) {
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; q += 2) {
+            const float4 v = *reinterpret_cast<const float4 *>(O + (8 * ti + r) * kCB + 8 * tc + 2 * q);
+            acc[r][q] = make_float2(v.x, v.y);
+            acc[r][q + 1] = make_float2(v.z, v.w);
+        }
+}
+__device__ __forceinline__ void tile_store(const float2 (&acc)[8][4], float *O, int ti, int tc) {
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int q = 0; q < 4; q += 2)
+            *reinterpret_cast<float4 *>(O + (8 * ti + r) * kCB + 8 * tc + 2 * q) = make_float4(acc[r][q].x, acc[r][q].y, acc[r][q + 1].x, acc[r][q + 1].y);
+}
+// The same by 64 threads, 4 x 4 outputs each, where there are more warps than blocks: a third of the time for twice the loads.
+// kRows rows of the product.
+template <int lda, int ldb, int kRows>
+__device__ __forceinline__ void block_mac_wide(float2 (&acc)[4][2], const float *A_, const float *B_, int t) {
+    const unsigned A = smem_u32(A_ + 4 * (t >> 3)), B = smem_u32(B_ + 4 * (t & 7));
+    constexpr int kG = 8;
+#pragma unroll
+    for (int l0 = 0; l0 < kRows; l0 += kG) {
+        float4 x[kG], y[kG];
+#pragma unroll
+        for (int l = 0; l < kG; ++l) {
+            x[l] = lds4(A + (l0 + l) * lda * 4);
+            y[l] = lds4(B + (l0 + l) * ldb * 4);
+        }
+#pragma unroll
+        for (int l = 0; l < kG; ++l) {
+            const float av[4] = {x[l].x, x[l].y, x[l].z, x[l].w};
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const float2 n = make_float2(-av[r], -av[r]);
+                acc[r][0] = chol_fma2(n, make_float2(y[l].x, y[l].y), acc[r][0]);
+                acc[r][1] = chol_fma2(n, make_float2(y[l].z, y[l].w), acc[r][1]);
+            }
+        }
+    }
+}
+__device__ __forceinline__ void tile_load_wide(float2 (&acc)[4][2], const float *O, int t) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-        const float4 v = *reinterpret_cast<const float4 *>(O + (4 * ti + r) * kCB + 4 * tc);
-        acc[r][0] = v.x; acc[r][1] = v.y; acc[r][2] = v.z; acc[r][3] = v.w;
+        const float4 v = *reinterpret_cast<const float4 *>(O + (4 * (t >> 3) + r) * kCB + 4 * (t & 7));
+        acc[r][0] = make_float2(v.x, v.y);
+        acc[r][1] = make_float2(v.z, v.w);
     }
 }
-__device__ __forceinline__ void tile_store(const float (&acc)[4][4], float *O, int ti, int tc) {
+__device__ __forceinline__ void tile_store_wide(const float2 (&acc)[4][2], float *O, int t) {
 #pragma unroll
     for (int r = 0; r < 4; ++r)
-        *reinterpret_cast<float4 *>(O + (4 * ti + r) * kCB + 4 * tc) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+        *reinterpret_cast<float4 *>(O + (4 * (t >> 3) + r) * kCB + 4 * (t & 7)) = make_float4(acc[r][0].x, acc[r][0].y, acc[r][1].x, acc[r][1].y);
 }
 
-// R (row-major k x k, upper triangular, zeros below the diagonal) from G (only read); Dinv: 1 / its diagonal, as the pivots
-// were worked out.
-constexpr int kCholStep = 8;                              // pivots per trip of the diagonal block's loop
-constexpr int kCholThreads = 512;
-__global__ void __launch_bounds__(kCholThreads) cholesky_factor_kernel(const float *__restrict__ G, int k, float *__restrict__ R,
-                                                               float *__restrict__ Dinv) {
+// Named CTA barriers: `threads` threads in all, whole warps.
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void copy16_async(void *dst_smem, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src) : "memory");
+}
+
+// The dynamic shared memory of the kernel below: functions that are not inlined take offsets into it, so that their accesses are
+// known to be to shared memory.
+__device__ __forceinline__ float *chol_smem() {
     extern __shared__ __align__(16) float sm[];
-    const int nb = chol_blocks(k), nbt = nb * (nb + 1) / 2;
-    float *blocks = sm;                                    // nbt blocks of 32 x 32, row-major
-    float *row = blocks + (size_t)nbt * kCBB;              // block row J of R: block C at C
-    float *dia = row + (size_t)nb * kCBB;                  // the diagonal block of R
-    float *dinv = dia + kCBB;                              // 1 / its diagonal
-    float *piv = dinv + kCB;                         // pivot rows of the diagonal block, two in turn
-    float *red = piv + 2 * kCB;                            // 32 + 1
-    constexpr int kParts = kCholThreads / 64;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int part = tid >> 6, ti = (tid & 63) >> 3, tc = tid & 7;         // this thread's 4 x 4 tile of its part's block
-    // load block by block (four elements of a row per thread), padded with an identity; what lies below the diagonal of
-    // a diagonal block is never read.  Four loads in flight per thread.
-    float md = 0.0f;
-    for (int b0 = 0; b0 < nbt; b0 += 8) {
-        float4 v[4];
+    return sm;
+}
+
+constexpr int kCholStep = 8;                              // pivots per trip of the loops below
+constexpr int kCholThreads = 384;
+constexpr int kCholWarps = kCholThreads / 32;
+constexpr int kCholWorkers = kCholWarps / 4 * 3, kCholPanel = 4, kCholTrail = kCholWorkers - kCholPanel;       // warps beside the pivots' scheduler: for the block row, for updates that can wait
+// What the CTAs of one launch share in global memory; all zero between launches (the last CTA to leave clears it).
+struct CholeskySync {
+    unsigned ticket;                                       // roles are taken in the order in which CTAs start
+    unsigned rows;                                         // block rows of R that are out
+    unsigned done;
+};
+__host__ __device__ constexpr size_t cholesky_blocked_smem_bytes(int k) {
+    // the factor's blocks (the inverse: a row of blocks, sums, two blocks), the diagonal block and 1 / diagonal twice, scalars
+    return ((size_t)(chol_blocks(k) * (chol_blocks(k) + 1) / 2 > 2 * chol_blocks(k) + 2 ? chol_blocks(k) * (chol_blocks(k) + 1) / 2 : 2 * chol_blocks(k) + 2) * kCBB +
+            2 * (kCBB + 3 * kCB) + kCB * kCTs + 2 * kCB + 64) *
+           sizeof(float);
+}
+
+// A step of the elimination for the 32 rows that a lane keeps of its column (pairs of rows): every row i > j loses row[i] v.
+// row: the step's row of the diagonal block of R, fetched before what is to hide the way.
+struct StepRow {
+    float4 q[kCB / 4];
+};
+__device__ __forceinline__ void step_fetch(StepRow &s, unsigned row, int j) {
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int b = b0 + 2 * u + (tid >> 8);
-            float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if (b < nbt) {
-                int I = 0, rem = b;
-                while (rem >= nb - I) { rem -= nb - I; ++I; }      // block (I, I + rem)
-                const int i = I * kCB + ((tid & 255) >> 3), c = (I + rem) * kCB + 4 * (tid & 7);
-                if ((k & 3) == 0 && i < k && c < k) {
-                    const float4 g = *reinterpret_cast<const float4 *>(G + (size_t)i * k + c);
-                    x[0] = g.x; x[1] = g.y; x[2] = g.z; x[3] = g.w;
-                } else {
+    for (int i4 = (j + 1) / 4; i4 < kCB / 4; ++i4) s.q[i4] = lds4(row + 16 * i4);
+}
+__device__ __forceinline__ void eliminate(float2 (&y)[kCB / 2], const StepRow &s, int j, float v) {
+    const float2 v2 = make_float2(-v, -v);
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) x[q] = (i < k && c + q < k) ? G[(size_t)i * k + c + q] : (i == c + q ? 1.0f : 0.0f);
-                }
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (i == c + q && i < k) md = fmaxf(md, x[q]);
-            }
-            v[u] = make_float4(x[0], x[1], x[2], x[3]);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int b = b0 + 2 * u + (tid >> 8);
-            if (b < nbt) reinterpret_cast<float4 *>(blocks + (size_t)b * kCBB)[tid & 255] = v[u];
-        }
+    for (int i4 = (j + 1) / 4 * 4; i4 < kCB; i4 += 4) {
+        const float4 p = s.q[i4 / 4];
+        if (i4 > j) y[i4 / 2] = chol_fma2(make_float2(p.x, p.y), v2, y[i4 / 2]);
+        else if (i4 + 1 > j) y[i4 / 2].y = fmaf(p.y, -v, y[i4 / 2].y);
+        if (i4 + 2 > j) y[i4 / 2 + 1] = chol_fma2(make_float2(p.z, p.w), v2, y[i4 / 2 + 1]);
+        else if (i4 + 3 > j) y[i4 / 2 + 1].y = fmaf(p.w, -v, y[i4 / 2 + 1].y);
     }
-    for (int d = 16; d > 0; d >>= 1) md = fmaxf(md, __shfl_xor_sync(0xffffffffu, md, d));
-    if (lane == 0) red[warp] = md;
-    __syncthreads();
-    if (tid == 0) {
-        float m = 0.0f;
-        for (int w = 0; w < kCholThreads / 32; ++w) m = fmaxf(m, red[w]);
-        red[32] = m > 0.0f ? m * 1.0e-5f : 0.0f;
-    }
-    // zeros below R's diagonal blocks
-    for (int i = kCB + warp; i < k; i += kCholThreads / 32)
-        for (int c = lane; c < i / kCB * kCB; c += 32) R[(size_t)i * k + c] = 0.0f;
-    __syncthreads();
-    const float shift = red[32];
-    for (int i = tid; i < k; i += kCholThreads) blocks[(size_t)blk_id(i / kCB, i / kCB, nb) * kCBB + (i % kCB) * (kCB + 1)] += shift;
-    __syncthreads();
-    for (int J = 0; J < nb; ++J) {
-        const int rest = nb - J - 1;                        // blocks to the right of the diagonal block
-        if (warp == 0) {
-            const float *D = blocks + (size_t)blk_id(J, J, nb) * kCBB;
-            // lane c keeps column c; the scaled pivot row goes through shared memory, four of its values per load; rows move up
-            // after every eight pivots, so that the loop's code is short enough to stay in the instruction cache
-            float a[kCB];
+}
+__device__ __forceinline__ float row_of(const float2 (&y)[kCB / 2], int j) { return j & 1 ? y[j / 2].y : y[j / 2].x; }
+__device__ __forceinline__ void rows_up(float2 (&y)[kCB / 2]) {
 #pragma unroll
-            for (int i = 0; i < kCB; ++i) a[i] = D[i * kCB + lane];
-            float my_inv = 0.0f;
+    for (int i = 0; i + kCholStep / 2 < kCB / 2; ++i) y[i] = y[i + kCholStep / 2];
+}
+__device__ __forceinline__ float chol_rsqrt_ftz(float x) {
+    float r;
+    asm volatile("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// The pivots of a diagonal block, one warp: lane c keeps column c.  Row j of R goes to dia, 1 / R(j, j) to dinv; every kCholStep rows the
+// warps of the block row (panel threads with this one) are let on.  The row in front of dia is zero.
+// kNormal: the floor under the pivots is a normal number, so every pivot is, and its root needs no scaling.
+// Rows move up after every kCholStep pivots, in a lane and in what is read of dia.
+template <bool kNormal>
+__device__ __forceinline__ void factor_diagonal(int at_d, int at_dia, int at_dinv, float half, int panel) {
+    const float *D = chol_smem() + at_d;
+    float *dia = chol_smem() + at_dia, *dinv = chol_smem() + at_dinv;
+    const int lane = threadIdx.x & 31;
+    float2 a[kCB / 2];
+#pragma unroll
+    for (int i = 0; i < kCB / 2; ++i) a[i] = make_float2(D[2 * i * kCB + lane], D[(2 * i + 1) * kCB + lane]);
+    float d = a[0].x, v = 0.0f;                             // the next pivot before its root, valid in its lane
+    const unsigned dia_at = smem_u32(dia);
 #pragma unroll 1
-            for (int j0 = 0; j0 < kCB; j0 += kCholStep) {
+    for (int j0 = 0; j0 < kCB; j0 += kCholStep) {
 #pragma unroll
-                for (int j = 0; j < kCholStep; ++j) {
-                    float d = a[j];                         // valid in lane j0 + j
-                    if (!(d > 0.5f * shift)) d = 0.5f * shift;
-                    float inv = 0.0f;
-                    if (d > 0.0f) {
-                        inv = rsqrtf(d);
-                        inv = inv * (1.5f - 0.5f * d * inv * inv);
-                    }
-                    const float r = d * inv;
-                    const bool mine = lane == j0 + j;
-                    if (mine) my_inv = inv;
-                    inv = __shfl_sync(0xffffffffu, inv, j0 + j);
-                    a[j] = mine ? r : a[j] * inv;
-                    float *pj = piv + (j & 1) * kCB;        // the scaled pivot row from column j0 on
-                    pj[(lane - j0) & 31] = a[j];
-                    dia[(j0 + j) * kCB + lane] = (j0 + j <= lane) ? a[j] : 0.0f;
-                    __syncwarp();
-#pragma unroll
-                    for (int i4 = (j + 1) / 4 * 4; i4 < kCB; i4 += 4) {
-                        const float4 p = *reinterpret_cast<const float4 *>(pj + i4);
-                        const float pv[4] = {p.x, p.y, p.z, p.w};
-#pragma unroll
-                        for (int q = 0; q < 4; ++q)
-                            if (i4 + q > j) a[i4 + q] -= pv[q] * a[j];
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i + kCholStep < kCB; ++i) a[i] = a[i + kCholStep];
-            }
-            dinv[lane] = my_inv;
-            Dinv[J * kCB + lane] = my_inv;
-        } else if (J > 0 && part > 0) {
-            // the rest of step J - 1: G_AB -= R_{J-1,A}^T R_{J-1,B} for J <= A <= B except the diagonal block (J, J)
-            const int r1 = rest + 1, pairs = r1 * (r1 + 1) / 2;
-            for (int pr = part; pr < pairs; pr += kParts - 1) {
-                int A = 0, rem = pr;
-                while (rem >= r1 - A) { rem -= r1 - A; ++A; }
-                float *O = blocks + (size_t)blk_id(J + A, J + A + rem, nb) * kCBB;
-                float acc[4][4];
-                tile_load(acc, O, ti, tc);
-                block_mac<kCB, kCB>(acc, row + (size_t)(J + A) * kCBB, row + (size_t)(J + A + rem) * kCBB, ti, tc);
-                tile_store(acc, O, ti, tc);
-            }
+        for (int j = 0; j < kCholStep; ++j) {
+            d = fmaxf(d, half);                             // (a NaN as well)
+            float inv = kNormal ? chol_rsqrt_ftz(d) : rsqrtf(d);
+            // row j of the other columns takes what the pivot before takes from it by shuffle, the rows below by way of shared memory
+            // behind this pivot's own shuffle: neither waits for more than it needs
+            const float p = __shfl_sync(kFullMask, v, j0 + j);
+            StepRow before;
+            step_fetch(before, dia_at + ((j0 + j - 1) * kCB + j0) * 4, j);
+            if (j & 1) a[j / 2].y = fmaf(p, -v, a[j / 2].y);
+            else a[j / 2].x = fmaf(p, -v, a[j / 2].x);
+            const bool mine = lane == j0 + j;
+            const float aj = mine ? d : row_of(a, j);
+            inv = inv * (1.5f - 0.5f * d * inv * inv);
+            if (!kNormal) inv = d > 0.0f ? inv : 0.0f;
+            const float inv_all = __shfl_sync(kFullMask, inv, j0 + j);
+            eliminate(a, before, j, v);
+            v = aj * inv_all;
+            d = fmaf(-v, v, row_of(a, j + 1));              // the next pivot, in its lane
+            dia[(j0 + j) * kCB + lane] = v;
+            if (mine) dinv[j0 + j] = inv;
+            __syncwarp();
         }
-        __syncthreads();
-        {   // diagonal block out
-            for (int e = tid; e < kCBB; e += kCholThreads) {
-                const int i = J * kCB + e / kCB, c = J * kCB + e % kCB;
-                if (i < k && c < k) R[(size_t)i * k + c] = dia[e];
-            }
-        }
-        if (rest == 0) break;
-        // block row J, one thread per column: forward substitution with R_JJ^T, every value into the rows below as soon as it is known
-        for (int col = tid; col < rest * kCB; col += kCholThreads) {
-            const float *X = blocks + (size_t)blk_id(J, J + 1 + col / kCB, nb) * kCBB + col % kCB;
-            float *Yr = row + (size_t)(J + 1 + col / kCB) * kCBB + col % kCB;
-            const int c = (J + 1) * kCB + col;
-            float *out = R + (size_t)J * kCB * k + c;
-            float y[kCB];
-#pragma unroll
-            for (int i = 0; i < kCB; ++i) y[i] = X[i * kCB];
-#pragma unroll
-            for (int l = 0; l < kCB; ++l) {
-                const float v = y[l] * dinv[l];
-                Yr[l * kCB] = v;
-                if (c < k && J * kCB + l < k) out[(size_t)l * k] = v;
-#pragma unroll
-                for (int i4 = (l + 1) / 4 * 4; i4 < kCB; i4 += 4) {
-                    const float4 p = *reinterpret_cast<const float4 *>(dia + l * kCB + i4);
-                    const float pv[4] = {p.x, p.y, p.z, p.w};
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (i4 + q > l) y[i4 + q] -= pv[q] * v;
-                }
-            }
-        }
-        __syncthreads();
-        // the block of the next pivots first, two elements per thread
-        {
-            const float *RA = row + (size_t)(J + 1) * kCBB;
-            float *O = blocks + (size_t)blk_id(J + 1, J + 1, nb) * kCBB;
-            float s0 = O[warp * kCB + lane], s1 = O[(warp + 16) * kCB + lane];
-#pragma unroll
-            for (int l = 0; l < kCB; ++l) {
-                const float x = RA[l * kCB + lane];
-                s0 = fmaf(-RA[l * kCB + warp], x, s0);
-                s1 = fmaf(-RA[l * kCB + warp + 16], x, s1);
-            }
-            O[warp * kCB + lane] = s0;
-            O[(warp + 16) * kCB + lane] = s1;
-        }
-        __syncthreads();
+        if (panel > 32) bar_arrive(1 + j0 / kCholStep, panel);
+        rows_up(a);
     }
 }
 
-// T = R^-1 (row-major k x k, zeros below the diagonal); CTA I makes block row I.  Everything it needs of R comes in at once.
-// The transposes of T_IL and of the sums are what is kept, so that every product has the form A^T B of block_mac:
-//   T_IJ^T = -(T_JJ)^T S_J^T with S_J = sum_L T_IL R_LJ, and S_C^T += (R_JC)^T T_IJ^T for the columns C still to come.
-constexpr int kCholInvThreads = 512;
-__host__ __device__ constexpr size_t cholesky_inverse_smem_bytes(int k) {
-    return (size_t)(chol_blocks(k) * (chol_blocks(k) + 1) / 2 + 2 * chol_blocks(k)) * kCBB * sizeof(float) + kCB * kCTs * sizeof(float);
+// kCols columns of a block row per thread (in blocks beside one another): forward substitution with R_JJ^T, behind the pivots.  X: the
+// columns, in place.
+template <int kCols>
+__device__ __forceinline__ void block_row(int at_x, int at_dia, int at_dinv, int panel, bool first) {
+    float *X = chol_smem() + at_x;
+    const unsigned dia_at = smem_u32(chol_smem() + at_dia), dinv_at = smem_u32(chol_smem() + at_dinv);
+    float2 y[kCols][kCB / 2];
+#pragma unroll
+    for (int u = 0; u < kCols; ++u)
+#pragma unroll
+        for (int i = 0; i < kCB / 2; ++i) y[u][i] = make_float2(X[u * kCBB + 2 * i * kCB], X[u * kCBB + (2 * i + 1) * kCB]);
+#pragma unroll 1
+    for (int j0 = 0; j0 < kCB; j0 += kCholStep) {
+        bar_sync(1 + j0 / kCholStep, panel);
+        const float4 d0 = lds4(dinv_at + 4 * j0), d1 = lds4(dinv_at + 4 * j0 + 16);
+        const float dv[kCholStep] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+#pragma unroll
+        for (int j = 0; j < kCholStep; ++j) {
+            StepRow now;
+            step_fetch(now, dia_at + ((j0 + j) * kCB + j0) * 4, j);
+#pragma unroll
+            for (int u = 0; u < kCols; ++u) {
+                const float v = row_of(y[u], j) * dv[j];
+                X[u * kCBB + (j0 + j) * kCB] = v;
+                eliminate(y[u], now, j, v);
+            }
+        }
+        if (first) bar_arrive(6 + j0 / kCholStep, 32 + 64);
+#pragma unroll
+        for (int u = 0; u < kCols; ++u) rows_up(y[u]);
+    }
 }
-__global__ void __launch_bounds__(kCholInvThreads, 1) cholesky_inverse_blocked_kernel(const float *__restrict__ R, const float *__restrict__ Dinv, int k, float *__restrict__ T) {
-    extern __shared__ __align__(16) float sm[];
-    const int nb = chol_blocks(k), I = blockIdx.x, n = nb - I;           // blocks I .. nb - 1 of rows and columns
-    float *rb = sm;                                        // block (L, C) of R, L, C counted from I: at blk_id(L, C, n)
-    float *tj = rb + (size_t)(n * (n + 1) / 2) * kCBB;     // T_JJ, J counted from I
-    float *sum = tj + (size_t)n * kCBB;                    // -S_C^T
-    float *tij = sum + (size_t)n * kCBB;                   // T_IJ^T, rows kCTs apart
-    const int tid = threadIdx.x, part = tid >> 6, ti = (tid & 63) >> 3, tc = tid & 7;
-#pragma unroll 4
-    for (int b = tid >> 8; b < n * (n + 1) / 2; b += kCholInvThreads / 256) {
-        int L = 0, rem = b;
-        while (rem >= n - L) { rem -= n - L; ++L; }
-        const int i = (I + L) * kCB + ((tid & 255) >> 3), c = (I + L + rem) * kCB + 4 * (tid & 7);
-        float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+
+// The inverse of a diagonal block of R, one warp: lane c keeps column c, rows from the bottom up.  A row's sum begins with what the row
+// below has just given, so all 496 multiply-adds are one chain; a row of R and its reciprocal are fetched while the row below is summed.
+__device__ __forceinline__ void invert_diagonal(const float *D, float my_inv, float (&t)[kCB], int lane) {
+    const unsigned at = smem_u32(D);
+    StepRow row, next;
+    float inv = __shfl_sync(kFullMask, my_inv, kCB - 1), next_inv = 0.0f;
+#pragma unroll
+    for (int i = kCB - 1; i >= 0; --i) {
+        if (i > 0) {
+            step_fetch(next, at + (i - 1) * kCB * 4, i - 1);
+            next_inv = __shfl_sync(kFullMask, my_inv, i - 1);
+        }
+        float acc = (lane == i) ? 1.0f : 0.0f;
+#pragma unroll
+        for (int l4 = (i + 1) / 4 * 4; l4 < kCB; l4 += 4) {
+            const float4 p = row.q[l4 / 4];
+            if (l4 > i) acc -= p.x * t[l4];
+            if (l4 + 1 > i) acc -= p.y * t[l4 + 1];
+            if (l4 + 2 > i) acc -= p.z * t[l4 + 2];
+            if (l4 + 3 > i) acc -= p.w * t[l4 + 3];
+        }
+        t[i] = (lane >= i) ? acc * inv : 0.0f;
+        row = next;
+        inv = next_inv;
+    }
+}
+
+// Block (A, B) loses R_LA^T R_LB; a lane of 16.
+__device__ __noinline__ void chol_update(int nb, int A, int B, int L) {
+    float *blocks = chol_smem(), *O = blocks + blk_id(A, B, nb) * kCBB;
+    const int ti = (threadIdx.x & 15) >> 2, tc = threadIdx.x & 3;
+    float2 acc[8][4];
+    tile_load(acc, O, ti, tc);
+    block_mac<kCB, kCB>(acc, blocks + blk_id(L, A, nb) * kCBB, blocks + blk_id(L, B, nb) * kCBB, ti, tc);
+    tile_store(acc, O, ti, tc);
+}
+// ... thread t of 64
+__device__ __noinline__ void chol_update_wide(int nb, int A, int B, int L, int t) {
+    float *blocks = chol_smem(), *O = blocks + blk_id(A, B, nb) * kCBB;
+    float2 acc[4][2];
+    tile_load_wide(acc, O, t);
+    block_mac_wide<kCB, kCB, kCB>(acc, blocks + blk_id(L, A, nb) * kCBB, blocks + blk_id(L, B, nb) * kCBB, t);
+    tile_store_wide(acc, O, t);
+}
+
+// R (row-major k x k, upper triangular, zeros below the diagonal) from G, and the diagonal blocks of T = R^-1 if T is given.
+// sync (may be null): told which block rows are out.
+__device__ __forceinline__ void cholesky_factor(const float *__restrict__ G, int k, float *R, float *T, CholeskySync *sync) {
+    float *sm = chol_smem();
+    const int nb = chol_blocks(k), nbt = nb * (nb + 1) / 2;
+    float *blocks = sm;                                    // nbt blocks of 32 x 32, row-major; those above the diagonal end as R's
+    float *dia = blocks + (size_t)nbt * kCBB + kCB;        // the diagonal block of R (what lies below its diagonal is never used), behind a row of zeros
+    float *dinv = dia + kCBB + kCB;                        // 1 / its diagonal (reads of dia run on for up to 23 floats)
+    constexpr int kDia = kCBB + 3 * kCB;                   // two of each in turn, from step to step
+    float *red = dinv + kDia + kCB;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // load block by block (four elements of a row per thread), padded with an identity; what lies below the diagonal of
+    // a diagonal block is never used
+    for (int e = tid; e < nbt * (kCBB / 4); e += kCholThreads) {
+        int I = 0, rem = e / (kCBB / 4);
+        while (rem >= nb - I) { rem -= nb - I; ++I; }      // block (I, I + rem)
+        const int at = e % (kCBB / 4), i = I * kCB + (at >> 3), c = (I + rem) * kCB + 4 * (at & 7);
+        float *dst = blocks + (size_t)4 * e;
         if ((k & 3) == 0 && i < k && c < k) {
-            const float4 g = *reinterpret_cast<const float4 *>(R + (size_t)i * k + c);
-            x[0] = g.x; x[1] = g.y; x[2] = g.z; x[3] = g.w;
+            copy16_async(dst, G + (size_t)i * k + c);
         } else {
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (i < k && c + q < k) x[q] = R[(size_t)i * k + c + q];
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (i == c + q && i >= k) x[q] = 1.0f;          // padding: an identity
+            for (int q = 0; q < 4; ++q) dst[q] = (i < k && c + q < k) ? G[(size_t)i * k + c + q] : (i == c + q ? 1.0f : 0.0f);
         }
-        reinterpret_cast<float4 *>(rb + (size_t)b * kCBB)[tid & 255] = make_float4(x[0], x[1], x[2], x[3]);
     }
-    for (int i = tid >> 5; i < kCB; i += kCholInvThreads / 32)           // zeros left of the diagonal block
-        for (int c = tid & 31; c < I * kCB; c += 32)
-            if (I * kCB + i < k) T[(size_t)(I * kCB + i) * k + c] = 0.0f;
+    if (tid < 2 * kCB) dia[(tid >> 5) * kDia + lane - kCB] = 0.0f;
+    float md = tid < k ? fmaxf(G[(size_t)tid * k + tid], 0.0f) : 0.0f;
+    for (int d = 16; d > 0; d >>= 1) md = fmaxf(md, __shfl_xor_sync(0xffffffffu, md, d));
+    if (lane == 0) red[warp] = md;
+    // zeros below R's diagonal blocks
+    for (int i = kCB + warp; i < k; i += kCholWarps)
+        for (int c = lane; c < i / kCB * kCB; c += 32) R[(size_t)i * k + c] = 0.0f;
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
-    // the diagonal blocks' inverses, one warp each: lane c keeps column c, rows from the bottom up
-    if ((tid >> 5) < n) {
-        const int b = tid >> 5, lane = tid & 31;
-        const float *D = rb + (size_t)blk_id(b, b, n) * kCBB;
-        float t[kCB];
-        const float my_inv = Dinv[(I + b) * kCB + lane];
+    float m = 0.0f;
 #pragma unroll
-        for (int i = kCB - 1; i >= 0; --i) {
-            float acc = (lane == i) ? 1.0f : 0.0f;
-#pragma unroll
-            for (int l4 = (i + 1) / 4 * 4; l4 < kCB; l4 += 4) {
-                const float4 p = *reinterpret_cast<const float4 *>(D + i * kCB + l4);
-                const float pv[4] = {p.x, p.y, p.z, p.w};
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (l4 + q > i) acc -= pv[q] * t[l4 + q];
-            }
-            const float inv = __shfl_sync(0xffffffffu, my_inv, i);
-            t[i] = (lane >= i) ? acc * inv : 0.0f;
-        }
-#pragma unroll
-        for (int i = 0; i < kCB; ++i) tj[(size_t)b * kCBB + i * kCB + lane] = t[i];
-    }
+    for (int w = 0; w < kCholeskyBlockedMaxK / 32; ++w) m = fmaxf(m, red[w]);
+    const float shift = m > 0.0f ? m * 1.0e-5f : 0.0f, half = 0.5f * shift;
+    if (tid < k) blocks[(size_t)blk_id(tid / kCB, tid / kCB, nb) * kCBB + (tid % kCB) * (kCB + 1)] += shift;
     __syncthreads();
-    for (int J = 0; J < n; ++J) {
-        // T_IJ^T = (T_JJ)^T (-S_J^T), two elements per thread
-        {
-            const int i = tid & 31, c0 = tid >> 5;          // elements (c0, i) and (c0 + 16, i) of the transposed block
-            float o0 = 0.0f, o1 = 0.0f;
-            if (J == 0) {
-                o0 = tj[i * kCB + c0];
-                o1 = tj[i * kCB + c0 + 16];
-            } else {
-                const float *A = tj + (size_t)J * kCBB, *B = sum + (size_t)J * kCBB;
-#pragma unroll 8
-                for (int l = 0; l < kCB; ++l) {
-                    const float b = B[l * kCB + i];
-                    o0 = fmaf(A[l * kCB + c0], b, o0);
-                    o1 = fmaf(A[l * kCB + c0 + 16], b, o1);
+    // Warp 0 has a scheduler to itself but for the two warps that finish rows.  Of the warps on the other three, the first four take
+    // the block row, the others the updates that are not urgent and the block of the next pivots.
+    const int wi = (warp & 3) ? (warp >> 2) * 3 + (warp & 3) - 1 : -1;
+    const int half_warp = 2 * wi + (lane >> 4);
+    // Two warps finish a block row while the next one is made: one writes it out -- on another scheduler than warp 0's where a small
+    // matrix leaves a worker free --, the other inverts its diagonal block, which is the diagonal block of the inverse.  (A store per
+    // pivot, behind the comparisons that a ragged edge needs, cost the pivots' warp 60 of 185 clocks each.)
+    const int writer = nb <= kCholPanel ? kCholWarps - 1 : 4, inverter = 8;
+    auto finish_row = [&](int J) {
+        const float *d = dia + (J & 1) * kDia;
+        const int row0 = J * kCB, col = row0 + lane;
+        const bool whole = row0 + kCB <= k;
+        if (warp == writer) {
+            for (int b = 0; b < nb - J; ++b) {
+                const float *src = b == 0 ? d + lane : blocks + (size_t)blk_id(J, J + b, nb) * kCBB + lane;
+                float *out = R + (size_t)row0 * k + col + b * kCB;
+                const bool in = col + b * kCB < k;
+#pragma unroll 1
+                for (int l0 = 0; l0 < kCB; l0 += 8) {
+                    float v[8];
+#pragma unroll
+                    for (int l = 0; l < 8; ++l) {
+                        v[l] = src[(l0 + l) * kCB];
+                        if (b == 0 && lane < l0 + l) v[l] = 0.0f;
+                    }
+                    if (in) {
+#pragma unroll
+                        for (int l = 0; l < 8; ++l)
+                            if (whole || row0 + l0 + l < k) out[(size_t)(l0 + l) * k] = v[l];
+                    }
                 }
             }
-            tij[c0 * kCTs + i] = o0;
-            tij[(c0 + 16) * kCTs + i] = o1;
+        } else if (T != nullptr) {
+            float t[kCB];
+            invert_diagonal(d, dinv[(J & 1) * kDia + lane], t, lane);
+            float *out = T + (size_t)row0 * k + col;
+            if (col < k) {
+#pragma unroll
+                for (int i = 0; i < kCB; ++i)
+                    if (whole || row0 + i < k) out[(size_t)i * k] = t[i];
+            }
+        }
+        if (sync) {
+            bar_sync(11, 64);
+            if (warp == writer && lane == 0) {
+                __threadfence();
+                asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(&sync->rows), "r"(J + 1) : "memory");
+            }
+        }
+    };
+    for (int J = 0; J < nb; ++J) {
+        const int at_dia = (int)(dia - sm) + (J & 1) * kDia, at_dinv = at_dia + kCBB + kCB;
+        const int rest = nb - J - 1;                        // blocks to the right of the diagonal block
+        const int panel_warps = rest ? 1 + rest / 2 : 0;    // one for the next pivots' columns, two blocks for each of the others
+        const int panel = 32 * (1 + panel_warps);           // threads of the barriers between the pivots and the block row
+        if (warp == 0) {
+            if (half >= 1.17549435e-38f) factor_diagonal<true>(blk_id(J, J, nb) * kCBB, at_dia, at_dinv, half, panel);
+            else factor_diagonal<false>(blk_id(J, J, nb) * kCBB, at_dia, at_dinv, half, panel);
+        } else if (warp == writer || warp == inverter) {
+            if (J > 0) {
+                if (warp == kCholWarps - 1) bar_arrive(5, 32 * kCholWorkers);
+                finish_row(J - 1);
+            }
+        } else if (wi >= 0) {
+            // ---- G_AB -= R_{J-1,A}^T R_{J-1,B}: row J first, for the block row that follows ----
+            if (J > 0) {
+                if (rest <= kCholWorkers / 2) {
+                    if (wi / 2 < rest) chol_update_wide(nb, J, J + 1 + wi / 2, J - 1, (wi & 1) * 32 + lane);
+                } else if (half_warp < rest) {
+                    chol_update(nb, J, J + 1 + half_warp, J - 1);
+                }
+                __syncwarp();
+                if (wi < panel_warps) bar_sync(5, 32 * kCholWorkers);
+                else bar_arrive(5, 32 * kCholWorkers);
+            }
+            if (wi < panel_warps) {
+                const int b = wi == 0 ? 1 : 2 * wi;         // first block, counted from the diagonal
+                const int at_x = blk_id(J, J + b, nb) * kCBB + lane;
+                if (wi > 0 && b < rest) block_row<2>(at_x, at_dia, at_dinv, panel, false);
+                else block_row<1>(at_x, at_dia, at_dinv, panel, wi == 0);
+            } else if (wi >= kCholPanel && rest) {
+                // ---- then the blocks below, that of the next pivots before all others ----
+                constexpr int kTasks = 2 * kCholTrail;      // at a time
+                const int h = half_warp - 2 * kCholPanel;
+                if (J > 0) {
+                    if (rest <= 2) {                        // at most three blocks, for two pairs of warps
+                        for (int t = h >> 2; h < kTasks / 4 * 4 && t < rest * (rest + 1) / 2; t += kTasks / 4)
+                            chol_update_wide(nb, J + 1 + t / 2, J + 1 + (t + 1) / 2, J - 1, ((wi - kCholPanel) & 1) * 32 + lane);
+                    } else {
+                        for (int t = h; t < rest * (rest + 1) / 2; t = t < kTasks ? 2 * kTasks - 1 - h : t + kTasks) {
+                            int A = 0, rem = t;
+                            while (rem >= rest - A) { rem -= rest - A; ++A; }
+                            chol_update(nb, J + 1 + A, J + 1 + A + rem, J - 1);
+                        }
+                    }
+                    __syncwarp();
+                }
+                if (wi < kCholPanel + 2) {
+                    // ---- the block of the next pivots, 4 x 4 outputs per thread of two warps, behind its block row ----
+                    if (J > 0) bar_sync(10, 64);
+                    const float *RA = blocks + (size_t)blk_id(J, J + 1, nb) * kCBB;
+                    float *O = blocks + (size_t)blk_id(J + 1, J + 1, nb) * kCBB;
+                    const int t = (wi - kCholPanel) * 32 + lane;
+                    float2 acc[4][2];
+                    tile_load_wide(acc, O, t);
+#pragma unroll 1
+                    for (int j0 = 0; j0 < kCB; j0 += kCholStep) {
+                        bar_sync(6 + j0 / kCholStep, 32 + 64);
+                        block_mac_wide<kCB, kCB, kCholStep>(acc, RA + j0 * kCB, RA + j0 * kCB, t);
+                    }
+                    tile_store_wide(acc, O, t);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (warp == writer || warp == inverter) finish_row(nb - 1);
+}
+
+// Block row I of T = R^-1 (row-major k x k, zeros below the diagonal) right of its diagonal block, from left to right, behind the
+// factor's block rows and the diagonal blocks of T.  The transposes of T_IL and of the sums are what is kept, so that every product
+// has the form A^T B of block_mac:
+//   T_IJ^T = -(T_JJ)^T S_J^T with S_J = sum_L T_IL R_LJ, and S_C^T += (R_JC)^T T_IJ^T for the columns C still to come.
+// sync: waited on for the block rows (null: they are there).  Gives up if they do not come.
+__device__ __forceinline__ void cholesky_inverse_row(int I, int k, const float *R, float *T, CholeskySync *sync, unsigned *status) {
+    const int nb = chol_blocks(k);
+    float *rb = chol_smem();                               // block row J of R right of its diagonal block
+    float *sum = rb + (size_t)nb * kCBB;                   // -S_C^T, at C
+    float *tj = sum + (size_t)nb * kCBB;                   // T_JJ
+    float *tij = tj + kCBB;                                // T_IJ^T, rows kCTs apart
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, half_warp = tid >> 4, ti = (tid & 15) >> 2, tc = tid & 3;
+    for (int row = I; row < (I == nb - 2 ? nb : I + 1); ++row)           // zeros left of the diagonal block; the last row's as well
+        for (int i = warp; i < kCB; i += kCholWarps)
+            for (int c = lane; c < row * kCB; c += 32)
+                if (row * kCB + i < k) T[(size_t)(row * kCB + i) * k + c] = 0.0f;
+    for (int J = I; J < nb; ++J) {
+        bool here = true;
+        if (sync && tid == 0) {
+            unsigned rows = 0;
+            for (unsigned i = 0; i < kMbarSpinLimit; ++i) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(rows) : "l"(&sync->rows) : "memory");
+                if (rows > (unsigned)J) break;
+                __nanosleep(32);
+            }
+            here = rows > (unsigned)J;
+            if (!here && status) atomicOr(status, kStatusBarrierTimeout);
+        }
+        if (!__syncthreads_and(here)) return;
+        // T_JJ and the blocks of R (past the first-level cache, which may hold older rows' lines)
+        for (int e = tid; e < (nb - J) * (kCBB / 4); e += kCholThreads) {
+            const int b = e / (kCBB / 4), at = e % (kCBB / 4), i = J * kCB + (at >> 3), c = (J + b) * kCB + 4 * (at & 7);
+            const float *src = (b == 0 ? T : R) + (size_t)i * k + c;
+            float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if ((k & 3) == 0 && i < k && c < k) {
+                const float4 g = __ldcg(reinterpret_cast<const float4 *>(src));
+                x[0] = g.x; x[1] = g.y; x[2] = g.z; x[3] = g.w;
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (i < k && c + q < k) x[q] = __ldcg(src + q);
+            }
+            reinterpret_cast<float4 *>(b == 0 ? tj : rb + (size_t)(b - 1) * kCBB)[at] = make_float4(x[0], x[1], x[2], x[3]);
+        }
+        __syncthreads();
+        // T_IJ^T = (T_JJ)^T (-S_J^T), four elements of a column per thread of eight warps
+        if (warp < 8) {
+            const int c0 = 4 * warp;                        // elements (c0 .. + 3, lane) of the transposed block
+            float o[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if (J == I) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) o[q] = tj[lane * kCB + c0 + q];
+            } else {
+                const float *B = sum + (size_t)J * kCBB + lane;
+                const unsigned at_t = smem_u32(tj + c0);
+#pragma unroll
+                for (int l = 0; l < kCB; ++l) {
+                    const float4 t = lds4(at_t + l * kCB * 4);
+                    const float b = B[l * kCB];
+                    o[0] = fmaf(t.x, b, o[0]);
+                    o[1] = fmaf(t.y, b, o[1]);
+                    o[2] = fmaf(t.z, b, o[2]);
+                    o[3] = fmaf(t.w, b, o[3]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tij[(c0 + q) * kCTs + lane] = o[q];
         }
         __syncthreads();
         // out, a row of T at a time (its column index is the row index of the transposed block)
-        for (int r = tid >> 5; r < kCB; r += kCholInvThreads / 32) {
-            const int i = I * kCB + r, c = (I + J) * kCB + (tid & 31);
-            if (i < k && c < k) T[(size_t)i * k + c] = tij[(tid & 31) * kCTs + r];
-        }
-        for (int C = J + 1 + part; C < n; C += kCholInvThreads / 64) {
-            float acc[4][4] = {};
+        if (J > I)
+            for (int r = warp; r < kCB; r += kCholWarps) {
+                const int i = I * kCB + r, c = J * kCB + lane;
+                if (i < k && c < k) T[(size_t)i * k + c] = tij[lane * kCTs + r];
+            }
+        if (nb - J - 1 <= kCholWarps / 2) {
+            if (J + 1 + warp / 2 < nb) {
+                const int C = J + 1 + warp / 2, t = (warp & 1) * 32 + lane;
+                float2 acc[4][2] = {};
+                float *S = sum + (size_t)C * kCBB;
+                if (J > I) tile_load_wide(acc, S, t);
+                block_mac_wide<kCB, kCTs, kCB>(acc, rb + (size_t)(C - J - 1) * kCBB, tij, t);
+                tile_store_wide(acc, S, t);
+            }
+        } else if (J + 1 + half_warp < nb) {
+            const int C = J + 1 + half_warp;
+            float2 acc[8][4] = {};
             float *S = sum + (size_t)C * kCBB;
-            if (J > 0) tile_load(acc, S, ti, tc);
-            block_mac<kCB, kCTs>(acc, rb + (size_t)blk_id(J, C, n) * kCBB, tij, ti, tc);
+            if (J > I) tile_load(acc, S, ti, tc);
+            block_mac<kCB, kCTs>(acc, rb + (size_t)(C - J - 1) * kCBB, tij, ti, tc);
             tile_store(acc, S, ti, tc);
         }
-        __syncthreads();                                   // the sums of the next column are whole, tij may be overwritten
+        __syncthreads();                                   // the sums of the next column are whole, rb, tj and tij may be overwritten
     }
 }
 
-// Sixteen 32 x 32 block products at a time: 64 threads per product, 4 x 4 outputs per thread (rows 4 ti .. + 3,
-// columns 4 tc .. + 3), operands read as float4: 2 shared-memory loads per 16 multiply-adds (with 2 x 2 outputs
-// per thread the loads, not the arithmetic, filled the issue slots of the one SM this kernel runs on).
-//   out -= A^T B  (AT = true:  A, B hold the contraction index in rows)
-//   out += A B    (AT = false: A holds it in columns)
-template <bool AT>
-__device__ __forceinline__ void block_mac_any(float (&acc)[4][4], const float *__restrict__ A, const float *__restrict__ B, int ti, int tc) {
-    if (AT) {
-#pragma unroll 4
-        for (int l = 0; l < kCB; ++l) {
-            const float4 a = *reinterpret_cast<const float4 *>(A + l * kCB + 4 * ti);
-            const float4 b = *reinterpret_cast<const float4 *>(B + l * kCB + 4 * tc);
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) acc[r][q] = fmaf(-av[r], bv[q], acc[r][q]);
-        }
-    } else {
-#pragma unroll 2
-        for (int l0 = 0; l0 < kCB; l0 += 4) {
-            float4 a[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4 *>(A + (4 * ti + r) * kCB + l0);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float4 b = *reinterpret_cast<const float4 *>(B + (l0 + u) * kCB + 4 * tc);
-                const float bv[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const float ar = u == 0 ? a[r].x : (u == 1 ? a[r].y : (u == 2 ? a[r].z : a[r].w));
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) acc[r][q] += ar * bv[q];
-                }
-            }
-        }
-    }
+// What a launch does.  kCholBoth: the CTA that starts first factors, the others follow with the rows of the inverse: the shortest
+// time for one matrix.  kCholFactor (and the diagonal blocks of T if T is given), then kCholInverse: nobody waits for anybody, which is
+// less time of all SMs together where other work wants them (k = 256: 64 us on 8 SMs against 54 us on 1 and 28 us on 7; eight compress and
+// decompress calls of 4096 x 14336 side by side 11.88 ms in two launches, 12.05 ms in one).
+enum CholeskyPart { kCholBoth, kCholFactor, kCholInverse };
+__host__ __device__ constexpr int cholesky_grid(int k, CholeskyPart part) {
+    return part == kCholFactor || chol_blocks(k) == 1 ? 1 : chol_blocks(k) - (part == kCholInverse ? 1 : 0);
 }
-__device__ __forceinline__ void tile_store_signed(const float (&acc)[4][4], float *O, int ti, int tc, float sign) {
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-        *reinterpret_cast<float4 *>(O + (4 * ti + r) * kCB + 4 * tc) =
-            make_float4(sign * acc[r][0], sign * acc[r][1], sign * acc[r][2], sign * acc[r][3]);
-}
-
-// Up to kCholeskySmallMaxK columns, where a second launch costs more than it spreads (k = 64: 19 us here, 15 + 8 in the two
-// kernels above; k = 32: 11 against 6.5 + 6.5), one CTA factors and inverts: forward substitutions per block row, then the
-// inverse block column by block column.
-constexpr int kCholeskySmallMaxK = 64;
-__host__ __device__ constexpr size_t cholesky_small_smem_bytes(int k) {
-    // packed blocks + inverted diagonal blocks + one temporary block column + 1 / diagonal + scalars
-    return ((size_t)(chol_blocks(k) * (chol_blocks(k) + 1) / 2 + 2 * chol_blocks(k)) * kCB * kCB + (size_t)chol_blocks(k) * kCB + 64) *
-           sizeof(float);
-}
-__global__ void __launch_bounds__(1024) cholesky_small_kernel(const float *__restrict__ G, int k, float *__restrict__ T,
-                                                                        float *__restrict__ Rcpy) {
-    extern __shared__ __align__(16) float sm[];
-    const int nb = chol_blocks(k), nbt = nb * (nb + 1) / 2;
-    float *blocks = sm;                                    // nbt blocks of 32 x 32, row-major
-    float *tinv = blocks + (size_t)nbt * kCB * kCB;        // nb inverted diagonal blocks
-    float *tmp = tinv + (size_t)nb * kCB * kCB;            // nb blocks: one block column of partial products
-    float *dinv = tmp + (size_t)nb * kCB * kCB;            // 1 / R(i, i)
-    float *red = dinv + nb * kCB;                          // 32 + 1
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarps = nt >> 5;
-    const int bi = tid >> 5, bc = tid & 31;               // this thread's element of a block when the CTA walks blocks
-    const int part = tid >> 6, ti = (tid & 63) >> 3, tc = tid & 7;         // ... and its 4 x 4 tile of its sixteenth's block
-    // load block by block (row bi, column bc of each), padded with an identity; what lies below the diagonal of a
-    // diagonal block is never read.  Four blocks per trip, so that four global loads are in flight per thread.
-    float md = 0.0f;
-    for (int b0 = 0; b0 < nbt; b0 += 4) {
-        float v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int b = b0 + u;
-            v[u] = 0.0f;
-            if (b < nbt) {
-                int I = 0, rem = b;
-                while (rem >= nb - I) { rem -= nb - I; ++I; }      // block (I, I + rem)
-                const int i = I * kCB + bi, c = (I + rem) * kCB + bc;
-                v[u] = (i == c) ? 1.0f : 0.0f;
-                if (i < k && c < k) v[u] = G[(size_t)i * k + c];
-                if (i == c && i < k) md = fmaxf(md, v[u]);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-            if (b0 + u < nbt) blocks[(size_t)(b0 + u) * kCB * kCB + tid] = v[u];
-    }
-    for (int d = 16; d > 0; d >>= 1) md = fmaxf(md, __shfl_xor_sync(0xffffffffu, md, d));
-    if (lane == 0) red[warp] = md;
-    __syncthreads();
-    if (tid == 0) {
-        float m = 0.0f;
-        for (int w = 0; w < nwarps; ++w) m = fmaxf(m, red[w]);
-        red[32] = m > 0.0f ? m * 1.0e-5f : 0.0f;
-    }
-    __syncthreads();
-    const float shift = red[32];
-    for (int i = tid; i < k; i += nt) blocks[(size_t)blk_id(i / kCB, i / kCB, nb) * kCB * kCB + (i % kCB) * (kCB + 1)] += shift;
-    __syncthreads();
-
-    for (int J = 0; J < nb; ++J) {
-        float *D = blocks + (size_t)blk_id(J, J, nb) * kCB * kCB;
-        if (warp == 0) {                                    // diagonal block: lane c keeps column c
-            float a[kCB];
-#pragma unroll
-            for (int i = 0; i < kCB; ++i) a[i] = D[i * kCB + lane];
-            float my_inv = 0.0f;
-#pragma unroll
-            for (int j = 0; j < kCB; ++j) {
-                float d = __shfl_sync(0xffffffffu, a[j], j);
-                if (!(d > 0.5f * shift)) d = 0.5f * shift;
-                // the 32 pivots of a block are one dependent chain: reciprocal square root from the special-function
-                // unit plus one Newton step (a relative error of ~1e-7 in R(j, j) and 1 / R(j, j) alike) instead of
-                // an IEEE square root followed by an IEEE division
-                float inv = 0.0f;
-                if (d > 0.0f) {
-                    inv = rsqrtf(d);
-                    inv = inv * (1.5f - 0.5f * d * inv * inv);
-                }
-                const float r = d * inv;
-                a[j] = (lane == j) ? r : a[j] * inv;
-                if (lane == j) my_inv = inv;
-#pragma unroll
-                for (int i = j + 1; i < kCB; ++i) {
-                    const float rji = __shfl_sync(0xffffffffu, a[j], i);
-                    a[i] -= rji * a[j];
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < kCB; ++i) D[i * kCB + lane] = (i <= lane) ? a[i] : 0.0f;
-            dinv[J * kCB + lane] = my_inv;
-        }
+__global__ void __launch_bounds__(kCholThreads, 1) cholesky_kernel(const float *__restrict__ G, int k, float *R, float *T, CholeskySync *sync,
+                                                                   unsigned *status, CholeskyPart part) {
+    __shared__ unsigned s_role;
+    int role = part == kCholInverse ? (int)blockIdx.x + 1 : 0;
+    const bool together = part == kCholBoth && gridDim.x > 1;
+    if (together) {
+        if (threadIdx.x == 0) s_role = atomicAdd(&sync->ticket, 1u);
         __syncthreads();
-        // block row J: one thread per column, forward substitution with R_JJ^T
-        for (int col = tid; col < (nb - J - 1) * kCB; col += nt) {
-            float *X = blocks + (size_t)blk_id(J, J + 1 + col / kCB, nb) * kCB * kCB + col % kCB;
-            float y[kCB];
-#pragma unroll
-            for (int i = 0; i < kCB; ++i) {
-                float acc = X[i * kCB];
-#pragma unroll
-                for (int l = 0; l < i; ++l) acc -= D[l * kCB + i] * y[l];
-                y[i] = acc * dinv[J * kCB + i];
-            }
-#pragma unroll
-            for (int i = 0; i < kCB; ++i) X[i * kCB] = y[i];
-        }
-        __syncthreads();
-        // trailing blocks (A, B), J < A <= B: G_AB -= R_JA^T R_JB, sixteen blocks per trip
-        {
-            const int rest = nb - J - 1, pairs = rest * (rest + 1) / 2;
-            for (int pr0 = 0; pr0 < pairs; pr0 += 16) {
-                const int pr = pr0 + part;
-                if (pr < pairs) {
-                    int A = 0, rem = pr;
-                    while (rem >= rest - A) { rem -= rest - A; ++A; }
-                    const int B = A + rem;
-                    const float *RA = blocks + (size_t)blk_id(J, J + 1 + A, nb) * kCB * kCB;
-                    const float *RB = blocks + (size_t)blk_id(J, J + 1 + B, nb) * kCB * kCB;
-                    float *O = blocks + (size_t)blk_id(J + 1 + A, J + 1 + B, nb) * kCB * kCB;
-                    float acc[4][4];
-                    tile_load(acc, O, ti, tc);
-                    block_mac_any<true>(acc, RA, RB, ti, tc);
-                    tile_store_signed(acc, O, ti, tc, 1.0f);
-                }
-            }
-        }
-        __syncthreads();
+        role = (int)s_role;
     }
-    // R out and the zeros below the diagonal of R and T, block by block; the diagonal blocks' inverses, one warp each
-    for (int I = 0; I < nb; ++I) {
-        for (int Jb = 0; Jb < nb; ++Jb) {
-            const int i = I * kCB + bi, c = Jb * kCB + bc;
-            if (i < k && c < k) {
-                const size_t e = (size_t)i * k + c;
-                if (c < i) {
-                    if (T) T[e] = 0.0f;
-                    if (Rcpy) Rcpy[e] = 0.0f;
-                } else if (Rcpy) {
-                    Rcpy[e] = blocks[(size_t)blk_id(I, Jb, nb) * kCB * kCB + tid];
-                }
-            }
-        }
-    }
-    if (!T) return;                                         // only the factor was wanted (uniform over the CTA)
-    if (warp < nb) {
-        const float *D = blocks + (size_t)blk_id(warp, warp, nb) * kCB * kCB;
-        float a[kCB], t[kCB];
-#pragma unroll
-        for (int i = 0; i < kCB; ++i) { a[i] = D[i * kCB + lane]; t[i] = 0.0f; }
-        const float my_inv = dinv[warp * kCB + lane];
-#pragma unroll
-        for (int i = kCB - 1; i >= 0; --i) {
-            float acc = (lane == i) ? 1.0f : 0.0f;
-#pragma unroll
-            for (int l = i + 1; l < kCB; ++l) acc -= __shfl_sync(0xffffffffu, a[i], l) * t[l];
-            const float inv = __shfl_sync(0xffffffffu, my_inv, i);
-            t[i] = (lane >= i) ? acc * inv : 0.0f;
-        }
-#pragma unroll
-        for (int i = 0; i < kCB; ++i) tinv[(size_t)warp * kCB * kCB + i * kCB + lane] = t[i];
-    }
-    __syncthreads();
-    // block column J of T, from the left: needs T_IL for L < J (already in place) and R_LJ (still in place)
-    for (int J = 1; J < nb; ++J) {
-        for (int I0 = 0; I0 < J; I0 += 16) {
-            const int I = I0 + part;
-            if (I < J) {
-                float acc[4][4] = {};
-                for (int L = I; L < J; ++L) {
-                    const float *TL = (L == I) ? tinv + (size_t)I * kCB * kCB : blocks + (size_t)blk_id(I, L, nb) * kCB * kCB;
-                    block_mac_any<false>(acc, TL, blocks + (size_t)blk_id(L, J, nb) * kCB * kCB, ti, tc);
-                }
-                tile_store_signed(acc, tmp + (size_t)I * kCB * kCB, ti, tc, 1.0f);
-            }
-        }
-        __syncthreads();
-        const float *TJ = tinv + (size_t)J * kCB * kCB;
-        for (int I0 = 0; I0 < J; I0 += 16) {
-            const int I = I0 + part;
-            if (I < J) {
-                float acc[4][4] = {};
-                block_mac_any<false>(acc, tmp + (size_t)I * kCB * kCB, TJ, ti, tc);
-                tile_store_signed(acc, blocks + (size_t)blk_id(I, J, nb) * kCB * kCB, ti, tc, -1.0f);
-            }
-        }
-        __syncthreads();
-    }
-    for (int I = 0; I < nb; ++I) {
-        for (int Jb = I; Jb < nb; ++Jb) {
-            const int i = I * kCB + bi, c = Jb * kCB + bc;
-            if (i < k && c < k && c >= i) {
-                const float *src = (I == Jb) ? tinv + (size_t)I * kCB * kCB : blocks + (size_t)blk_id(I, Jb, nb) * kCB * kCB;
-                T[(size_t)i * k + c] = src[tid];
-            }
+    if (role == 0) cholesky_factor(G, k, R, T, together ? sync : nullptr);
+    else cholesky_inverse_row(role - 1, k, R, T, together ? sync : nullptr, status);
+    if (together && threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&sync->done, 1u) + 1 == gridDim.x) {               // everybody has read what is cleared here
+            sync->ticket = 0;
+            sync->rows = 0;
+            sync->done = 0;
         }
     }
 }

@@ -52,7 +52,8 @@ struct SvdWorkspace {
     float *w = nullptr;                 // k eigenvalues
     float *t = nullptr, *tinv1 = nullptr, *tinv2 = nullptr, *core = nullptr;   // k x k
     float *uc = nullptr, *vc = nullptr; // k x k outputs of the core SVD
-    float *rfac = nullptr, *dinv = nullptr;    // k x k factor that nobody asked for; 1 / its diagonal
+    float *rfac = nullptr;              // k x k factor that nobody asked for
+    CholeskySync *chol_sync = nullptr;  // zero between launches
     float *gemm_ws = nullptr;
     size_t gemm_ws_bytes = 0;
     float *solver_work = nullptr;
@@ -723,14 +724,19 @@ cudaError_t orthonormalise(SvdWorkspace *ws, float *Y, float *tmp, int rows, int
         // a row-sharded panel: its Gram matrix is the sum of the shards' (the one exchange per QR pass);
         // every rank then factors the same k x k matrix and gets bit-identical R
         if (sharded_rows && ws->allreduce && (err = timed_allreduce(ws, ws->g, (size_t)k * k, st)) != cudaSuccess) return err;
-        if (k <= kCholeskySmallMaxK) {
-            cholesky_small_kernel<<<1, 1024, cholesky_small_smem_bytes(k), st>>>(ws->g, k, factor_only ? nullptr : ws->t, pass == 0 ? r_a : r_b);
-        } else if (k <= kCholeskyBlockedMaxK) {
+        if (k <= kCholeskyBlockedMaxK) {
             float *r_out = pass == 0 ? r_a : r_b;
             if (!r_out) r_out = ws->rfac;
-            cholesky_factor_kernel<<<1, kCholThreads, cholesky_factor_smem_bytes(k), st>>>(ws->g, k, r_out, ws->dinv);
-            if (!factor_only)
-                cholesky_inverse_blocked_kernel<<<chol_blocks(k), kCholInvThreads, cholesky_inverse_smem_bytes(k), st>>>(r_out, ws->dinv, k, ws->t);
+            const auto launch = [&](CholeskyPart part) {
+                cholesky_kernel<<<cholesky_grid(k, part), kCholThreads, cholesky_blocked_smem_bytes(k), st>>>(
+                    ws->g, k, r_out, factor_only ? nullptr : ws->t, ws->chol_sync, ws->status, part);
+            };
+            if (factor_only || ws->device_full) {
+                launch(kCholFactor);
+                if (!factor_only && chol_blocks(k) > 1) launch(kCholInverse);
+            } else {
+                launch(kCholBoth);
+            }
         } else if (k <= kCholeskySmemMaxK) {
             cholesky_inverse_smem_kernel<<<1, 1024, cholesky_smem_bytes(k), st>>>(ws->g, k, ws->t, pass == 0 ? r_a : r_b);
         } else {
@@ -795,14 +801,15 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
               alloc_f(&ws->y2, (size_t)ws->M * ws->k) && alloc_f(&ws->z, (size_t)ws->N * ws->k) &&
               alloc_f(&ws->z2, (size_t)ws->N * ws->k) && alloc_f(&ws->g, kk) && alloc_f(&ws->w, ws->k) &&
               alloc_f(&ws->t, kk) && alloc_f(&ws->tinv1, kk) && alloc_f(&ws->tinv2, kk) && alloc_f(&ws->core, kk) &&
-              alloc_f(&ws->uc, kk) && alloc_f(&ws->vc, kk) && alloc_f(&ws->rfac, kk) &&
-              alloc_f(&ws->dinv, (size_t)chol_blocks(ws->k) * kCB);
+              alloc_f(&ws->uc, kk) && alloc_f(&ws->vc, kk) && alloc_f(&ws->rfac, kk);
     // split-K partials: up to 2 * SMs tiles' worth of the largest skinny product, and of the Gram matrix
     // K-split partials, and behind them room for the images of a product's second operand split beforehand
     ws->gemm_ws_bytes = std::max((size_t)ws->M * ws->k * 8, kk * 2 * (size_t)sm_count) * sizeof(float) +
                         gemm_tc_image_bytes(ws->k, ws->k <= 256 ? ws->k : 128, std::max(ws->M, ws->N)) + 256;
     ok = ok && alloc_f(&ws->gemm_ws, ws->gemm_ws_bytes / sizeof(float));
     ok = ok && cudaMalloc(reinterpret_cast<void **>(&ws->dev_info), sizeof(int)) == cudaSuccess;
+    ok = ok && cudaMalloc(reinterpret_cast<void **>(&ws->chol_sync), sizeof(CholeskySync)) == cudaSuccess &&
+         cudaMemset(ws->chol_sync, 0, sizeof(CholeskySync)) == cudaSuccess && cudaStreamSynchronize(nullptr) == cudaSuccess;
     ok = ok && cudaMalloc(reinterpret_cast<void **>(&ws->own_status), sizeof(unsigned)) == cudaSuccess;
     ok = ok && cudaMalloc(reinterpret_cast<void **>(&ws->a_absmax), sizeof(unsigned)) == cudaSuccess;
     ok = ok && curandCreateGenerator(&ws->rng, CURAND_RNG_PSEUDO_DEFAULT) == CURAND_STATUS_SUCCESS;
@@ -871,14 +878,9 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
             }
         }
     }
-    if (ok && ws->k <= kCholeskySmallMaxK)
-        ok = cudaFuncSetAttribute(cholesky_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)cholesky_small_smem_bytes(ws->k)) == cudaSuccess;
-    else if (ok && ws->k <= kCholeskyBlockedMaxK)
-        ok = cudaFuncSetAttribute(cholesky_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)cholesky_factor_smem_bytes(ws->k)) == cudaSuccess &&
-             cudaFuncSetAttribute(cholesky_inverse_blocked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)cholesky_inverse_smem_bytes(ws->k)) == cudaSuccess;
+    if (ok && ws->k <= kCholeskyBlockedMaxK)
+        ok = cudaFuncSetAttribute(cholesky_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)cholesky_blocked_smem_bytes(ws->k)) == cudaSuccess;
     else if (ok && ws->k <= kCholeskySmemMaxK)
         ok = cudaFuncSetAttribute(cholesky_inverse_smem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)cholesky_smem_bytes(ws->k)) == cudaSuccess;
@@ -895,10 +897,11 @@ void svd_workspace_device_full(SvdWorkspace *ws, bool full) { ws->device_full = 
 void svd_workspace_destroy(SvdWorkspace *ws) {
     if (!ws) return;
     float *bufs[] = {ws->omega, ws->y, ws->y2, ws->z, ws->z2, ws->g, ws->w, ws->t, ws->tinv1, ws->tinv2,
-                     ws->core, ws->uc, ws->vc, ws->rfac, ws->dinv, ws->gemm_ws, ws->solver_work};
+                     ws->core, ws->uc, ws->vc, ws->rfac, ws->gemm_ws, ws->solver_work};
     for (float *p : bufs)
         if (p) cudaFree(p);
     if (ws->dev_info) cudaFree(ws->dev_info);
+    if (ws->chol_sync) cudaFree(ws->chol_sync);
     if (ws->own_status) cudaFree(ws->own_status);
     if (ws->a_absmax) cudaFree(ws->a_absmax);
     for (cudaEvent_t e : ws->span_ev)
