@@ -17,8 +17,8 @@
 // "minuend - C" with an any(|.| > FLT_EPSILON) flag (the reference's subtract_kernel + has_nonzero_kernel,
 // src/bitsqz_llm.cu:164-184).
 //
-// This version computes on the FP32 pipes (128 x 128 x 16 tiles, 8 x 8 per thread, double-buffered
-// shared memory).
+// This version computes on the FP32 pipes (tiles of 128 x 128, 128 x 64 or 64 x 64 outputs, pieces of 16 of K by asynchronous copies).
+#include "bsq_device.cuh"
 #include "bsq_gemm.hpp"
 #include "bsq_internal.hpp"
 
@@ -27,140 +27,168 @@
 namespace bsq {
 namespace {
 
-constexpr int BM = 128, BN = 128, BK = 16, GT = 256;
-constexpr int PAD = 4;
+constexpr int BM = 128, BN = 128, BK = 16, GT = 256;         // (what K is split by; the tiles themselves are TM x TN)
 
-template <bool KMAJOR>
-__device__ __forceinline__ void load_tile(const float *__restrict__ P, long ld, int rows_total, int k_total, int row0, int k0,
-                                          int k_end, float (*S)[BM + PAD], bool vec_ok, const float *kscale) {
-    // fills S[kk][r] = op(row0 + r, k0 + kk) for r < 128, kk < 16 (zero outside the matrix / split)
-    const int t = threadIdx.x;
-    if (KMAJOR) {
+// One operand's piece of a step: kRows rows or columns of the output tile by BK of K, as it lies in memory: contiguous along K
+// (kKMajor: row r at r (BK + 4)) or along the rows (k at k (kRows + 4)).
+template <bool kKMajor, int kRows>
+struct Piece {
+    static constexpr int kLd = kKMajor ? BK + 4 : kRows + 4;
+    static constexpr int kFloats = kKMajor ? kRows * kLd : BK * kLd;
+
+    // Starts the copies of rows row0 .. and k0 .. (zero outside the matrix and the split).  kVec: rows are 16-byte aligned.
+    template <bool kVec>
+    static __device__ __forceinline__ void fetch(float *S, const float *__restrict__ P, long ld, int rows_total, int row0, int k0, int k_end) {
+        constexpr int kW = kVec ? 4 : 1;                     // floats per copy
+        constexpr int kInner = (kKMajor ? BK : kRows) / kW, kCopies = kRows * BK / kW;
+        static_assert(kCopies % GT == 0, "whole copies per thread");
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int r = (t >> 2) + h * 64, kk = (t & 3) * 4;
-            const int gr = row0 + r, gk = k0 + kk;
-            float v[4] = {0.f, 0.f, 0.f, 0.f};
-            if (gr < rows_total) {
-                const float *src = P + (long)gr * ld + gk;
-                if (vec_ok && gk + 3 < k_end) {
-                    const float4 q = *reinterpret_cast<const float4 *>(src);
-                    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (gk + j < k_end) v[j] = src[j];
-                }
-                if (kscale) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (gk + j < k_end) v[j] = __fmul_rn(v[j], kscale[gk + j]);
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) S[kk + j][r] = v[j];
-        }
-    } else {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int kk = (t >> 5) + h * 8, r = (t & 31) * 4;
-            const int gk = k0 + kk, gr = row0 + r;
-            float v[4] = {0.f, 0.f, 0.f, 0.f};
-            if (gk < k_end) {
-                const float *src = P + (long)gk * ld + gr;
-                if (vec_ok && gr + 3 < rows_total) {
-                    const float4 q = *reinterpret_cast<const float4 *>(src);
-                    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (gr + j < rows_total) v[j] = src[j];
-                }
-                if (kscale) {
-                    const float s = kscale[gk];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) v[j] = __fmul_rn(v[j], s);
-                }
-            }
-            *reinterpret_cast<float4 *>(&S[kk][r]) = make_float4(v[0], v[1], v[2], v[3]);
+        for (int u = 0; u < kCopies / GT; ++u) {
+            const int e = threadIdx.x + u * GT, outer = e / kInner, inner = e % kInner * kW;
+            const int r = row0 + (kKMajor ? outer : inner), k = k0 + (kKMajor ? inner : outer);
+            // what of the copy lies inside, in bytes
+            const int left = kKMajor ? (r < rows_total ? k_end - k : 0) : (k < k_end ? rows_total - r : 0);
+            const int bytes = min(max(left, 0), kW) * 4;
+            const float *src = bytes ? P + (kKMajor ? (long)r * ld + k : (long)k * ld + r) : P;
+            const unsigned dst = smem_u32(S + outer * kLd + inner);
+            if (kVec) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+            else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
         }
     }
-    (void)k_total;
-}
+};
 
-template <bool A_KMAJOR, bool B_KMAJOR>
-__global__ void __launch_bounds__(GT) gemm_kernel(GemmArgs g) {
-    __shared__ __align__(16) float As[2][BK][BM + PAD];
-    __shared__ __align__(16) float Bs[2][BK][BN + PAD];
+// TM x TN outputs per CTA, TM / 16 x TN / 16 per thread; thread (ty, tx) has rows ty + 16 i of an operand that lies along K
+// (neighbouring rows then start 20 floats apart: no bank twice in eight lanes) and 4 ty .. + 3 of every 64 of one that lies along
+// the rows.  Pieces come in by asynchronous copies kStages - 1 steps ahead.  Each output is one chain of multiply-adds over its split's
+// K, whatever the tile.
+template <bool A_KMAJOR, bool B_KMAJOR, int TM, int TN, int kStages, bool kVecA, bool kVecB>
+__global__ void __launch_bounds__(GT, A_KMAJOR && B_KMAJOR && TM * TN == 128 * 128 ? 1 : 2) gemm_kernel(GemmArgs g) {
+    using PA = Piece<A_KMAJOR, TM>;
+    using PB = Piece<B_KMAJOR, TN>;
+    constexpr int MI = TM / 16, NI = TN / 16;
+    __shared__ __align__(16) float As[kStages][PA::kFloats];
+    __shared__ __align__(16) float Bs[kStages][PB::kFloats];
     const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
     const int k_begin = blockIdx.z * g.k_per_split;
     const int k_end = min(g.K, k_begin + g.k_per_split);
-    const bool a_vec = (reinterpret_cast<uintptr_t>(g.A) % 16 == 0) && (g.lda % 4 == 0);
-    const bool b_vec = (reinterpret_cast<uintptr_t>(g.B) % 16 == 0) && (g.ldb % 4 == 0);
-    float acc[8][8];
+    const int steps = k_end > k_begin ? (k_end - k_begin + BK - 1) / BK : 0;
+    float acc[MI][NI];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < MI; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-
-    int buf = 0;
-    if (k_begin < k_end) {
-        load_tile<A_KMAJOR>(g.A, g.lda, g.M, g.K, m0, k_begin, k_end, As[0], a_vec, g.kscale);
-        load_tile<B_KMAJOR>(g.B, g.ldb, g.N, g.K, n0, k_begin, k_end, Bs[0], b_vec, nullptr);
-    }
-    __syncthreads();
-    for (int k0 = k_begin; k0 < k_end; k0 += BK) {
-        if (k0 + BK < k_end) {
-            load_tile<A_KMAJOR>(g.A, g.lda, g.M, g.K, m0, k0 + BK, k_end, As[buf ^ 1], a_vec, g.kscale);
-            load_tile<B_KMAJOR>(g.B, g.ldb, g.N, g.K, n0, k0 + BK, k_end, Bs[buf ^ 1], b_vec, nullptr);
+        for (int j = 0; j < NI; ++j) acc[i][j] = 0.0f;
+    auto fetch = [&](int step) {
+        if (step < steps) {
+            const int k0 = k_begin + step * BK, s = step % kStages;
+            PA::template fetch<kVecA>(As[s], g.A, g.lda, g.M, m0, k0, k_end);
+            PB::template fetch<kVecB>(Bs[s], g.B, g.ldb, g.N, n0, k0, k_end);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            const float4 a0 = *reinterpret_cast<const float4 *>(&As[buf][kk][ty * 4]);
-            const float4 a1 = *reinterpret_cast<const float4 *>(&As[buf][kk][64 + ty * 4]);
-            const float4 b0 = *reinterpret_cast<const float4 *>(&Bs[buf][kk][tx * 4]);
-            const float4 b1 = *reinterpret_cast<const float4 *>(&Bs[buf][kk][64 + tx * 4]);
-            const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+    for (int s = 0; s < kStages - 1; ++s) fetch(s);
+    for (int step = 0; step < steps; ++step) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+        __syncthreads();                                     // this step's pieces are here, and nobody reads the ones before
+        fetch(step + kStages - 1);
+        const float *A = As[step % kStages], *B = Bs[step % kStages];
+        const int k0 = k_begin + step * BK;
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
+        for (int k4 = 0; k4 < BK; k4 += 4) {
+            float4 aq[A_KMAJOR ? MI : 1], bq[B_KMAJOR ? NI : 1];         // four of K of an operand that lies along it
+            if (A_KMAJOR) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int i = 0; i < MI; ++i) aq[i] = *reinterpret_cast<const float4 *>(A + (ty + 16 * i) * PA::kLd + k4);
+            }
+            if (B_KMAJOR) {
+#pragma unroll
+                for (int j = 0; j < NI; ++j) bq[j] = *reinterpret_cast<const float4 *>(B + (tx + 16 * j) * PB::kLd + k4);
+            }
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+                float a[MI], b[NI];
+#pragma unroll
+                for (int i = 0; i < MI; i += A_KMAJOR ? 1 : 4) {
+                    if (A_KMAJOR) {
+                        a[i] = kk == 0 ? aq[i].x : (kk == 1 ? aq[i].y : (kk == 2 ? aq[i].z : aq[i].w));
+                    } else {
+                        const float4 q = *reinterpret_cast<const float4 *>(A + (k4 + kk) * PA::kLd + 16 * i + 4 * ty);
+                        a[i] = q.x; a[i + 1] = q.y; a[i + 2] = q.z; a[i + 3] = q.w;
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < NI; j += B_KMAJOR ? 1 : 4) {
+                    if (B_KMAJOR) {
+                        b[j] = kk == 0 ? bq[j].x : (kk == 1 ? bq[j].y : (kk == 2 ? bq[j].z : bq[j].w));
+                    } else {
+                        const float4 q = *reinterpret_cast<const float4 *>(B + (k4 + kk) * PB::kLd + 16 * j + 4 * tx);
+                        b[j] = q.x; b[j + 1] = q.y; b[j + 2] = q.z; b[j + 3] = q.w;
+                    }
+                }
+                if (g.kscale) {
+                    const float ks = k0 + k4 + kk < k_end ? g.kscale[k0 + k4 + kk] : 0.0f;
+#pragma unroll
+                    for (int i = 0; i < MI; ++i) a[i] = __fmul_rn(a[i], ks);
+                }
+#pragma unroll
+                for (int i = 0; i < MI; ++i)
+#pragma unroll
+                    for (int j = 0; j < NI; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+            }
         }
-        __syncthreads();
-        buf ^= 1;
     }
 
     float *C = g.C + (long)blockIdx.z * g.split_stride;
     bool any = false;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int gm = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
+    for (int i = 0; i < MI; ++i) {
+        const int gm = m0 + (A_KMAJOR ? ty + 16 * i : 64 * (i / 4) + 4 * ty + i % 4);
         if (gm >= g.M) continue;
+        float *row = C + (long)gm * g.ldc;
 #pragma unroll
-        for (int jh = 0; jh < 2; ++jh) {
-            const int gn = n0 + jh * 64 + tx * 4;
-            float v[4] = {acc[i][jh * 4 + 0], acc[i][jh * 4 + 1], acc[i][jh * 4 + 2], acc[i][jh * 4 + 3]};
+        for (int j0 = 0; j0 < NI; j0 += 4) {
+            // four columns: neighbours, or 16 apart
+            const int step = B_KMAJOR ? 16 : 1, gn = n0 + (B_KMAJOR ? tx + 16 * j0 : 16 * j0 + 4 * tx);
+            float v[4] = {acc[i][j0], acc[i][j0 + 1], acc[i][j0 + 2], acc[i][j0 + 3]};
             if (g.minuend) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (gn + j < g.N) {
-                        v[j] = __fsub_rn(g.minuend[(long)gm * g.ldm + gn + j], v[j]);
+                    if (gn + j * step < g.N) {
+                        v[j] = __fsub_rn(g.minuend[(long)gm * g.ldm + gn + j * step], v[j]);
                         any |= fabsf(v[j]) > 1.1920928955078125e-07f;
                     }
             }
-            float *dst = C + (long)gm * g.ldc + gn;
-            if (gn + 3 < g.N && (reinterpret_cast<uintptr_t>(dst) % 16 == 0)) {
-                *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+            if (!B_KMAJOR && gn + 3 < g.N && (reinterpret_cast<uintptr_t>(row + gn) % 16 == 0)) {
+                *reinterpret_cast<float4 *>(row + gn) = make_float4(v[0], v[1], v[2], v[3]);
             } else {
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (gn + j < g.N) dst[j] = v[j];
+                    if (gn + j * step < g.N) row[gn + j * step] = v[j];
             }
         }
     }
     if (g.flag && __any_sync(0xffffffffu, any) && (t & 31) == 0) atomicOr(g.flag, 1u);
+}
+
+template <bool A_KMAJOR, bool B_KMAJOR, int TM, int TN, int kStages>
+void launch_fp32(const GemmArgs &g, cudaStream_t stream) {
+    const bool va = reinterpret_cast<uintptr_t>(g.A) % 16 == 0 && g.lda % 4 == 0, vb = reinterpret_cast<uintptr_t>(g.B) % 16 == 0 && g.ldb % 4 == 0;
+    const dim3 grid((g.N + TN - 1) / TN, (g.M + TM - 1) / TM, g.splits);
+    if (va && vb) gemm_kernel<A_KMAJOR, B_KMAJOR, TM, TN, kStages, true, true><<<grid, GT, 0, stream>>>(g);
+    else if (va) gemm_kernel<A_KMAJOR, B_KMAJOR, TM, TN, kStages, true, false><<<grid, GT, 0, stream>>>(g);
+    else if (vb) gemm_kernel<A_KMAJOR, B_KMAJOR, TM, TN, kStages, false, true><<<grid, GT, 0, stream>>>(g);
+    else gemm_kernel<A_KMAJOR, B_KMAJOR, TM, TN, kStages, false, false><<<grid, GT, 0, stream>>>(g);
+}
+// Tiles: 128 columns unless there are at most 64; 64 rows where there are no more, or where 128 leave the device idle.  What bounds a
+// small product is the way of its few steps from memory: copies that are waited for one by one and 128 x 128 tiles for everything took
+// 14 to 18 us for each product of 777 x 1031 at rank 48, whole compress and decompress calls of that shape 0.79 ms, now 0.64;
+// 2048 x 5120 at rank 64, whose Gram matrices run here, 1.14 and 1.08 ms.
+template <bool A_KMAJOR, bool B_KMAJOR>
+void launch_fp32(const GemmArgs &g, int sm_count, cudaStream_t stream) {
+    if (g.N > 64) launch_fp32<A_KMAJOR, B_KMAJOR, 128, 128, 2>(g, stream);
+    else if (g.M <= 64 || (long)((g.M + 127) / 128) * g.splits < sm_count) launch_fp32<A_KMAJOR, B_KMAJOR, 64, 64, 4>(g, stream);
+    else launch_fp32<A_KMAJOR, B_KMAJOR, 128, 64, 3>(g, stream);
 }
 
 // C = sum over splits of the partial results, in split order (the order fixes the result bit for bit).  VEC = 4: four
@@ -417,11 +445,10 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
     } else {
         g.C = C; g.ldc = ldc; g.split_stride = 0;
     }
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, splits);
-    if (a_kmajor && b_kmajor) gemm_kernel<true, true><<<grid, GT, 0, stream>>>(g);
-    else if (a_kmajor) gemm_kernel<true, false><<<grid, GT, 0, stream>>>(g);
-    else if (b_kmajor) gemm_kernel<false, true><<<grid, GT, 0, stream>>>(g);
-    else gemm_kernel<false, false><<<grid, GT, 0, stream>>>(g);
+    if (a_kmajor && b_kmajor) launch_fp32<true, true>(g, sm_count, stream);
+    else if (a_kmajor) launch_fp32<true, false>(g, sm_count, stream);
+    else if (b_kmajor) launch_fp32<false, true>(g, sm_count, stream);
+    else launch_fp32<false, false>(g, sm_count, stream);
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess || splits == 1) return err;
     return launch_reduce(workspace, C, M, N, ldc, splits, sm_count, stream);

@@ -81,3 +81,36 @@ def test_objects_do_not_depend_on_the_matrices_in_flight(pkg, lib, shape):
                 assert torch.equal(b[200: 200 + w.numel()], w), count
     finally:
         lib.bsq_batch_destroy(batch)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (63, 64, 15), (64, 63, 16), (65, 64, 17), (64, 65, 63), (127, 48, 65), (128, 128, 64), (129, 129, 100), (300, 64, 48),
+                                   (2000, 40, 4096), (777, 100, 1031), (40, 40, 2050)])
+@pytest.mark.parametrize("a_km,b_km", [(1, 0), (1, 1), (0, 0), (0, 1)])
+@pytest.mark.parametrize("off,pad", [(0, 0), (1, 0), (0, 1), (3, 4)])
+def test_fp32_tiles(lib, shape, a_km, b_km, off, pad):
+    """The FP32-pipe kernel at the edges of its tiles (64 and 128 rows and columns, 16 of K, K split and whole), operands on and off 16-byte
+    boundaries.  A chain of up to 4096 multiply-adds per split and their sums: 4e-6 of sum |a||b| as above (about 64 2^-24 expected)."""
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + 3 * N + 7 * K)
+
+    def operand(rows, cols):
+        flat = torch.randn(off + rows * (cols + pad), device="cuda", generator=g)
+        return flat[off:].view(rows, cols + pad)
+    A = operand(*((M, K) if a_km else (K, M)))
+    B = operand(*((N, K) if b_km else (K, N)))
+    a = A[:, :K].double() if a_km else A[:, :M].double().T
+    b = B[:, :K].double().T if b_km else B[:, :N].double()
+    want, scale = a @ b, a.abs() @ b.abs()
+    ws = torch.empty(64 << 20, dtype=torch.uint8, device="cuda")
+    out = []
+    for workspace in (True, False, True):
+        C = torch.full((M, N + pad), 3.0, device="cuda")
+        status = torch.zeros(4, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        assert lib.bsq_gemm(a_km, b_km, A.data_ptr(), A.shape[1], B.data_ptr(), B.shape[1], C.data_ptr(), C.shape[1], M, N, K,
+                            ws.data_ptr() if workspace else None, ws.numel() if workspace else 0, 0, status.data_ptr(), None) == 0
+        torch.cuda.synchronize()
+        assert bool(((C[:, :N].double() - want).abs() <= 4e-6 * scale).all())
+        assert bool((C[:, N:] == 3.0).all())
+        out.append(C)
+    assert torch.equal(out[0], out[2])
