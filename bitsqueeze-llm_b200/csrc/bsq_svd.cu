@@ -17,7 +17,7 @@
 //   * the small SVD works on a k x k core: B^T = Q2 C with C = R2 R1 the product of the two
 //     triangular factors, C = Uc S Vc^T, V_hat = Q2 Uc, U = Q Vc.
 // The SVD of the k x k core is a one-sided Jacobi kernel of this library up to 256 columns (bsq_jacobi.cuh; where the factors
-// are coded afterwards one CTA up to 64, a thread-block cluster above); larger cores, and devices that cannot place the cluster, go to cuSOLVER's gesvdj on
+// are coded afterwards bsq_ring_jacobi.cuh, below 48 columns the one-CTA kernel here); larger cores, and devices that cannot place the cluster, go to cuSOLVER's gesvdj on
 // the k x k core.  Everything that touches an M- or N-sized array is a kernel of this library.
 // Omega comes from cuRAND's XORWOW generator like the reference's (svd_lowrank_cuda.cu:143,289-291),
 // seeded per call, column-major N x k.
@@ -26,6 +26,7 @@
 #include "bsq_gemm.hpp"
 #include "bsq_internal.hpp"
 #include "bsq_jacobi.cuh"
+#include "bsq_ring_jacobi.cuh"
 
 #include <cooperative_groups.h>
 #include <curand.h>
@@ -70,7 +71,7 @@ struct SvdWorkspace {
     unsigned *a_absmax = nullptr;       // bits of the largest |A| of the current call (scale of the FP16 split of the big products)
     bool a_absmax_valid = false;
     const unsigned *a_absmax_use = nullptr;
-    int jc_lanes = 4;                   // lanes per column pair of the cluster Jacobi kernel for this k
+    RingLaunch ring = {};               // the core's kernel for coded factors above kRingMinK columns
     bool jc_with_v = false;             // ... and whether it accumulates the right factor (else that comes from the panel)
     bool device_full = false;           // other work fills the device beside this (chooses tile widths, not results)
     bool block_core = false;            // the core goes to block_jacobi_kernel
@@ -246,14 +247,14 @@ __global__ void __launch_bounds__(1024) cholesky_inverse_smem_kernel(const float
     }
 }
 
-// The two kernels below serve cores whose factors are coded afterwards (NF4 / NF4_DQ sections, error lists made from them):
+// The kernel below and that of bsq_ring_jacobi.cuh serve cores whose factors are coded afterwards (NF4 / NF4_DQ sections, error lists made from them):
 // the codes of a singular pair depend on its sign and, in a flat spectrum, on how the last bits turn neighbouring vectors
 // into one another, so another order of rotations than theirs changes most objects in most bytes (measured: 6 to 8 % of the
 // reconstructed matrix, as large a change as a library solver makes).  An error list is whole numbers too: which elements of
 // the residual are the largest and in which order changes with the last bits of factors that are themselves FP32.  Objects
 // that hold codes or such a list keep their bytes; where all that can change is the rounding of FP32 values, the factors come
 // from the block kernel of bsq_jacobi.cuh.
-// SVD of the k x k core for k <= kJacobiMaxK: one-sided (Hestenes) Jacobi in one CTA, everything in shared memory.
+// SVD of the k x k core for k <= kRingMinK: one-sided (Hestenes) Jacobi in one CTA, everything in shared memory.
 // The reference runs cusolverDnSgesvd on the k x n matrix B (svd_lowrank_cuda.cu:399-440); here only the k x k
 // triangular factor is left to decompose.
 //   in : C, row-major k x k; read as the column-major matrix M = C^T (column j = row j of C)
@@ -263,22 +264,24 @@ __global__ void __launch_bounds__(1024) cholesky_inverse_smem_kernel(const float
 // schedule), 8 lanes serve a pair, a CTA barrier separates the rounds.  Squared column norms are carried along
 // through the rotations and recomputed exactly at the start of every sweep.  At the end S(j) = |column j|,
 // U(:, j) = column j / S(j) (zero for S(j) = 0), and a rank by counting puts S in descending order.
-constexpr int kJacobiMaxK = 128;              // what the one-CTA kernel can hold
-constexpr int kJacobiSingleMaxK = 64;         // what it is used for: above, the cluster kernel is faster
-__host__ __device__ constexpr int jacobi_len(int k) { return k <= 64 ? 64 : 128; }
+constexpr int kJacobiSingleMaxK = 64;         // cores whose right factor is accumulated
+constexpr int kJacobiClusterMaxK = 256;       // larger ones go to the library solver
+constexpr int kJacobiLen = 64;                // padded column length
 __host__ __device__ constexpr size_t jacobi_smem_bytes(int k) {
-    return ((size_t)2 * ((k + 1) & ~1) * jacobi_len(k) + 2 * (size_t)((k + 1) & ~1) + 64) * sizeof(float);
+    return ((size_t)2 * ((k + 1) & ~1) * kJacobiLen + 2 * (size_t)((k + 1) & ~1) + 64) * sizeof(float);
 }
 
-__global__ void __launch_bounds__(512) jacobi_svd_kernel(const float *__restrict__ C, int k, float *__restrict__ S,
+// (One CTA per SM told to the compiler: without that it schedules as if other warps hid a chain's latencies; k = 48 163 -> 158 us.)
+__global__ void __launch_bounds__(256, 1) jacobi_svd_kernel(const float *__restrict__ C, int k, float *__restrict__ S,
                                                          float *__restrict__ Ucol, float *__restrict__ Vcol) {
     extern __shared__ __align__(16) float sm[];
-    const int LEN = jacobi_len(k), kp = (k + 1) & ~1, npairs = kp / 2;
+    constexpr int LEN = kJacobiLen;
+    const int kp = (k + 1) & ~1, npairs = kp / 2;
     float *M = sm, *V = M + (size_t)kp * LEN, *nrm = V + (size_t)kp * LEN;
     int *rank_of = reinterpret_cast<int *>(nrm + kp);
     const int tid = threadIdx.x, nt = blockDim.x;
     const int slot = tid >> 3, l = tid & 7;                   // 8 lanes per pair, 64 pair slots
-    const int F4 = LEN / 32;                                  // float4 per lane and column: 2 or 4
+    constexpr int F4 = LEN / 32;                              // float4 per lane and column
     for (int e0 = tid; e0 < kp * LEN; e0 += 4 * nt) {        // four global loads in flight per thread
         float v[4];
 #pragma unroll
@@ -329,15 +332,13 @@ __global__ void __launch_bounds__(512) jacobi_svd_kernel(const float *__restrict
                 else { p = (r + slot) % (kp - 1); q = (r + kp - 1 - slot) % (kp - 1); }
             }
             float4 *mp = reinterpret_cast<float4 *>(M + (size_t)p * LEN), *mq = reinterpret_cast<float4 *>(M + (size_t)q * LEN);
-            float4 ap[4], aq[4];
+            float4 ap[F4], aq[F4];
             float g = 0.0f;
 #pragma unroll
-            for (int f = 0; f < 4; ++f) {
-                if (f < F4) {
-                    ap[f] = mp[f * 8 + l];
-                    aq[f] = mq[f * 8 + l];
-                    g += ap[f].x * aq[f].x + ap[f].y * aq[f].y + ap[f].z * aq[f].z + ap[f].w * aq[f].w;
-                }
+            for (int f = 0; f < F4; ++f) {
+                ap[f] = mp[f * 8 + l];
+                aq[f] = mq[f * 8 + l];
+                g += ap[f].x * aq[f].x + ap[f].y * aq[f].y + ap[f].z * aq[f].z + ap[f].w * aq[f].w;
             }
             g = sum8(g);
             const float alpha = nrm[p], beta = nrm[q];
@@ -349,15 +350,13 @@ __global__ void __launch_bounds__(512) jacobi_svd_kernel(const float *__restrict
                 const float c = rsqrtf(1.0f + t * t), sn = c * t;
                 float4 *vp = reinterpret_cast<float4 *>(V + (size_t)p * LEN), *vq = reinterpret_cast<float4 *>(V + (size_t)q * LEN);
 #pragma unroll
-                for (int f = 0; f < 4; ++f) {
-                    if (f < F4) {
-                        const float4 x = ap[f], y = aq[f];
-                        mp[f * 8 + l] = make_float4(c * x.x - sn * y.x, c * x.y - sn * y.y, c * x.z - sn * y.z, c * x.w - sn * y.w);
-                        mq[f * 8 + l] = make_float4(sn * x.x + c * y.x, sn * x.y + c * y.y, sn * x.z + c * y.z, sn * x.w + c * y.w);
-                        const float4 u = vp[f * 8 + l], w = vq[f * 8 + l];
-                        vp[f * 8 + l] = make_float4(c * u.x - sn * w.x, c * u.y - sn * w.y, c * u.z - sn * w.z, c * u.w - sn * w.w);
-                        vq[f * 8 + l] = make_float4(sn * u.x + c * w.x, sn * u.y + c * w.y, sn * u.z + c * w.z, sn * u.w + c * w.w);
-                    }
+                for (int f = 0; f < F4; ++f) {
+                    const float4 x = ap[f], y = aq[f];
+                    mp[f * 8 + l] = make_float4(c * x.x - sn * y.x, c * x.y - sn * y.y, c * x.z - sn * y.z, c * x.w - sn * y.w);
+                    mq[f * 8 + l] = make_float4(sn * x.x + c * y.x, sn * x.y + c * y.y, sn * x.z + c * y.z, sn * x.w + c * y.w);
+                    const float4 u = vp[f * 8 + l], w = vq[f * 8 + l];
+                    vp[f * 8 + l] = make_float4(c * u.x - sn * w.x, c * u.y - sn * w.y, c * u.z - sn * w.z, c * u.w - sn * w.w);
+                    vq[f * 8 + l] = make_float4(sn * u.x + c * w.x, sn * u.y + c * w.y, sn * u.z + c * w.z, sn * u.w + c * w.w);
                 }
                 if (l == 0) {
                     nrm[p] = fmaxf(alpha - t * g, 0.0f);
@@ -393,289 +392,6 @@ __global__ void __launch_bounds__(512) jacobi_svd_kernel(const float *__restrict
         Ucol[o] = sj > 0.0f ? M[(size_t)j * LEN + i] / sj : 0.0f;
         Vcol[o] = V[(size_t)j * LEN + i];
     }
-}
-
-// The same Jacobi iteration for larger cores, up to kJacobiClusterMaxK (two 256 x 256 matrices do not fit one SM's
-// shared memory, and already at 128 x 128 one SM's shared-memory bandwidth is the limit): a thread-block cluster of
-// 8 CTAs, each holding a slice of LEN / 8 rows of every column of M and V.  A column
-// pair's dot product is the sum of the eight slices' partial products: every CTA stores its partials into the
-// shared memory of all eight (distributed shared memory), one cluster barrier later every CTA adds them in the
-// same order, so all of them see bit-identical values, take identical decisions and rotate their own slices with
-// identical angles.  Control flow is the same in all CTAs by construction (same data, same arithmetic), which is
-// what the hardware cluster barrier needs; the sweep count is bounded.
-constexpr int kJacobiClusterMaxK = 256;
-constexpr int kJcCtas = 8;                                   // 16 measured slower: the partial products take longer to arrive
-__host__ __device__ constexpr int jacobi_cluster_len(int k) { return k <= 128 ? 128 : 256; }     // padded column length
-__host__ __device__ constexpr size_t jacobi_cluster_smem_bytes(int k) {
-    // M and V slices, norms, two rounds of CTAs x LEN / 2 partial products, CTAs x LEN partial norms, ranks, votes, mbarriers
-    return ((size_t)2 * ((k + 1) & ~1) * (jacobi_cluster_len(k) / kJcCtas) + ((k + 1) & ~1) + kJcCtas * jacobi_cluster_len(k) +
-            kJcCtas * jacobi_cluster_len(k) + jacobi_cluster_len(k) + 64) *
-           sizeof(float);
-}
-
-// The shared::cluster address of `smem_addr` (a shared::cta address of this CTA) in CTA `rank` of the cluster.
-__device__ __forceinline__ unsigned cluster_addr(unsigned smem_addr, unsigned rank) {
-    unsigned r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-    return r;
-}
-// 16-byte store into another CTA's shared memory that counts itself off on that CTA's mbarrier when it has landed:
-// the receiver waits for the bytes, no fence and no cluster-wide barrier on the sender's side.
-__device__ __forceinline__ void st_async_f4(unsigned dst, const float4 &v, unsigned mbar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "f"(v.x),
-                 "f"(v.y), "f"(v.z), "f"(v.w), "r"(mbar)
-                 : "memory");
-}
-
-// kWithV = false leaves the right factor out: nothing accumulates the rotations (half the shared-memory traffic of a
-// round), and Vcol receives column j of M divided by S(j)^2 instead -- the k x k matrix that turns the panel the core
-// came from into its singular vectors (B^T v_j / S(j) with v_j = M(:, j) / S(j)).
-template <int kJcLen, int kLpp, bool kWithV>
-__global__ void __launch_bounds__(kJcLen / 2 * kLpp, 1) jacobi_svd_cluster_kernel(const float *__restrict__ C, int k, float *__restrict__ S,
-                                                                        float *__restrict__ Ucol, float *__restrict__ Vcol,
-                                                                        unsigned *__restrict__ status) {
-    constexpr int kJcRows = kJcLen / kJcCtas, kJcF4 = kJcRows / (4 * kLpp);      // rows per CTA; float4 per lane and column
-    static_assert(kLpp == 2 || kLpp == 4, "lanes per column pair");
-    static_assert(kJcF4 == 1 || kJcF4 == 2 || kJcF4 == 4, "float4 per lane and column");
-    constexpr int kSlots = kJcLen / 2;                                   // pair slots = partial products per CTA and round
-    constexpr unsigned kRoundBytes = kJcCtas * kSlots * sizeof(float);   // what one CTA receives per round
-    namespace cg = cooperative_groups;
-    cg::cluster_group cluster = cg::this_cluster();
-    const unsigned cr = cluster.block_rank();                 // this CTA holds rows cr * kJcRows .. + kJcRows - 1
-    extern __shared__ __align__(16) float sm[];
-    const int kp = (k + 1) & ~1, npairs = kp / 2;
-    float *M = sm, *V = M + (size_t)kp * kJcRows, *nrm = V + (size_t)kp * kJcRows;
-    float *part = nrm + ((kp + 3) & ~3);                      // [2][kJcCtas][kSlots], 16-byte aligned
-    float *npart = part + 2 * kJcCtas * kSlots;               // [kJcCtas][kJcLen]
-    int *rank_of = reinterpret_cast<int *>(npart + kJcCtas * kJcLen);
-    int *votes = rank_of + kJcLen;                            // [kJcCtas]
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(votes + kJcCtas);      // [2], one per parity of the round counter
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
-    const int slot = tid / kLpp, l = tid % kLpp;              // kLpp lanes per pair, kSlots pair slots, kJcF4 float4 per lane and column
-    // A warp holds 32 / kLpp pair slots, that many partial products per round, in groups of four: the warp is cut
-    // into as many parts as it has groups, and in each part lane d (d < 8) sends the part's group as one 16-byte
-    // store to CTA d.
-    static_assert(kJcCtas == 8, "one sending lane per destination CTA and group");
-    constexpr int kPartLanes = 4 * kLpp;                      // lanes that own one group of four slots
-    const int part_lane0 = lane / kPartLanes * kPartLanes;
-    const bool sender = lane - part_lane0 < kJcCtas;
-    const unsigned part_to = cluster_addr(smem_u32(part + cr * kSlots + (tid >> 5) * (32 / kLpp) + part_lane0 / kLpp), lane & 7);
-    const unsigned mbar_to = cluster_addr(smem_u32(mbar), lane & 7);
-    // A column slice of more than one float4 per lane starts at a multiple of 128 bytes, the same banks for every
-    // slot: slot s takes its float4 in the order f ^ (s mod kJcF4), so neighbouring slots spread over all banks.
-    const int fsw = slot & (kJcF4 - 1);
-    const int row0 = cr * kJcRows;
-    if (tid == 0) {
-        mbar_init(&mbar[0], 1);
-        mbar_init(&mbar[1], 1);
-        mbar_fence_init();
-    }
-    for (int e0 = tid; e0 < kp * kJcRows; e0 += 4 * nt) {
-        float v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int e = e0 + u * nt, j = e / kJcRows, i = row0 + e % kJcRows;
-            v[u] = (e < kp * kJcRows && j < k && i < k) ? C[(size_t)j * k + i] : 0.0f;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int e = e0 + u * nt, j = e / kJcRows, i = row0 + e % kJcRows;
-            if (e < kp * kJcRows) {
-                M[e] = v[u];
-                if (kWithV) V[e] = (i == j && j < k) ? 1.0f : 0.0f;
-            }
-        }
-    }
-    __syncthreads();
-    const float tol = sqrtf((float)kJcLen) * 5.9604645e-08f, tol2 = tol * tol;
-    auto sum4 = [&](float x) {                                // over the lanes of a pair
-        if (kLpp == 4) x += __shfl_xor_sync(0xffffffffu, x, 2, 4);
-        x += __shfl_xor_sync(0xffffffffu, x, 1, kLpp);
-        return x;
-    };
-    // Exact squared norms of all columns (partial over this CTA's rows, exchanged, added in CTA order) and, on the
-    // same cluster barrier, the CTAs' votes: bit 0 = "met a pair above kJacobiLastSweepCos in the last sweep", bit 1 = "a wait ran out".
-    // Every CTA reads the same eight votes, so all of them leave the sweep loop in the same sweep whatever happened.
-    // (The first of these barriers also makes the mbarriers' initialisation known to the whole cluster.)
-    auto norms_and_votes = [&](int my_vote) {
-        for (int j0 = 0; j0 < kp; j0 += nt / kLpp) {          // uniform trip count: shuffles inside
-            const int j = j0 + slot;
-            float acc = 0.0f;
-            if (j < kp) {
-#pragma unroll
-                for (int f = 0; f < kJcF4; ++f) {
-                    const float4 a = reinterpret_cast<const float4 *>(M + (size_t)j * kJcRows)[f * kLpp + l];
-                    acc += a.x * a.x + a.y * a.y + a.z * a.z + a.w * a.w;
-                }
-            }
-            acc = sum4(acc);
-            if (l == 0 && j < kp) {
-#pragma unroll
-                for (int d = 0; d < kJcCtas; ++d) cluster.map_shared_rank(npart, d)[cr * kJcLen + j] = acc;
-            }
-        }
-        if (tid < kJcCtas) cluster.map_shared_rank(votes, tid)[cr] = my_vote;
-        cluster.sync();
-        for (int j = tid; j < kp; j += nt) {
-            float a = 0.0f;
-#pragma unroll
-            for (int d = 0; d < kJcCtas; ++d) a += npart[d * kJcLen + j];
-            nrm[j] = a;
-        }
-        int all = 0;
-#pragma unroll
-        for (int d = 0; d < kJcCtas; ++d) all |= votes[d];
-        __syncthreads();
-        return all;
-    };
-    // The rotation of V's columns is not needed before the next round's end (nothing reads V to take a decision),
-    // so it is kept back and done while the next round's partial products are in flight.
-    // Columns p, q of one round belong to one pair slot; the barrier at the end of every round orders this slot's
-    // late rotation before the rotation that the columns' next owners keep back in their turn.
-    int dv_p = 0, dv_q = 0;
-    float dv_c = 1.0f, dv_sn = 0.0f;
-    bool dv_pending = false;
-    auto apply_to_v = [&]() {
-        if (!kWithV || !dv_pending) return;
-        float4 *vp = reinterpret_cast<float4 *>(V + (size_t)dv_p * kJcRows), *vq = reinterpret_cast<float4 *>(V + (size_t)dv_q * kJcRows);
-        const float c = dv_c, sn = dv_sn;
-#pragma unroll
-        for (int f = 0; f < kJcF4; ++f) {
-            const int i4 = (f ^ fsw) * kLpp + l;
-            const float4 u = vp[i4], w = vq[i4];
-            vp[i4] = make_float4(c * u.x - sn * w.x, c * u.y - sn * w.y, c * u.z - sn * w.z, c * u.w - sn * w.w);
-            vq[i4] = make_float4(sn * u.x + c * w.x, sn * u.y + c * w.y, sn * u.z + c * w.z, sn * u.w + c * w.w);
-        }
-        dv_pending = false;
-    };
-    // One round's exchange: every CTA sends its kSlots partial products to all eight (itself included) with stores
-    // that count off on the receiver's mbarrier of the round's parity; a receiver's phase ends when all
-    // kRoundBytes are there.  Two buffers and two mbarriers are enough: a CTA sends round i + 2 only after it has
-    // round i + 1 from everybody, and everybody sent round i + 1 after the CTA barrier that ends its round i, so
-    // nobody still reads or waits for round i then.
-    int vote = 1;
-    bool failed = false;                                      // a wait ran out: stop sending and waiting, finish quickly
-    unsigned it = 0;                                          // rounds so far
-    for (int sweep = 0;; ++sweep) {
-        const int all = norms_and_votes(vote);
-        if (!(all & 1) || (all & 2) || sweep == kJacobiMaxSweeps) break;
-        bool rotated = false;
-        for (int r = 0; r < kp - 1; ++r, ++it) {
-            const unsigned par = it & 1, phase = (it >> 1) & 1;
-            if (tid == 0) mbar_expect_tx(&mbar[par], kRoundBytes);
-            const bool active = slot < npairs;
-            int p = 0, q = 0;
-            if (active) {
-                if (slot == 0) { p = kp - 1; q = r; }
-                else {                                        // (r + slot) mod (kp - 1) and (r - slot) mod (kp - 1)
-                    p = r + slot;
-                    q = r + kp - 1 - slot;
-                    p -= p >= kp - 1 ? kp - 1 : 0;
-                    q -= q >= kp - 1 ? kp - 1 : 0;
-                }
-            }
-            float4 *mp = reinterpret_cast<float4 *>(M + (size_t)p * kJcRows), *mq = reinterpret_cast<float4 *>(M + (size_t)q * kJcRows);
-            float4 ap[kJcF4], aq[kJcF4];
-            float g = 0.0f;
-#pragma unroll
-            for (int f = 0; f < kJcF4; ++f) {
-                ap[f] = mp[(f ^ fsw) * kLpp + l];
-                aq[f] = mq[(f ^ fsw) * kLpp + l];
-                g += ap[f].x * aq[f].x + ap[f].y * aq[f].y + ap[f].z * aq[f].z + ap[f].w * aq[f].w;
-            }
-            const float alpha = nrm[p], beta = nrm[q];
-            g = sum4(g);
-            {
-                float4 g4;
-                g4.x = __shfl_sync(0xffffffffu, g, part_lane0);
-                g4.y = __shfl_sync(0xffffffffu, g, part_lane0 + kLpp);
-                g4.z = __shfl_sync(0xffffffffu, g, part_lane0 + 2 * kLpp);
-                g4.w = __shfl_sync(0xffffffffu, g, part_lane0 + 3 * kLpp);
-                if (sender && !failed)
-                    st_async_f4(part_to + par * (unsigned)(kJcCtas * kSlots * sizeof(float)), g4, mbar_to + par * (unsigned)sizeof(uint64_t));
-            }
-            apply_to_v();                                     // the previous round's rotation of V, while the stores travel
-            // one lane per warp polls the barrier (256 polling threads get in the way of the stores that are arriving in
-            // this CTA's shared memory); the warp's other lanes take its word
-            {
-                int got = 1;
-                if (lane == 0 && !failed) got = mbar_wait_bounded(&mbar[par], phase, status) ? 1 : 0;
-                got = __shfl_sync(0xffffffffu, got, 0);
-                if (!got) failed = true;
-            }
-            const float *pp = part + par * kJcCtas * kSlots + slot;
-            g = ((pp[0] + pp[kSlots]) + (pp[2 * kSlots] + pp[3 * kSlots])) + ((pp[4 * kSlots] + pp[5 * kSlots]) + (pp[6 * kSlots] + pp[7 * kSlots]));
-            if (active && alpha > 0.0f && beta > 0.0f && g * g > tol2 * alpha * beta) {
-                // tangent, cosine and sine to a few units in the last place: what they leave of the pair's
-                // product is far below the tolerance, and every CTA gets the same bits from the same inputs
-                const float zeta = __fdividef(beta - alpha, 2.0f * g);
-                const float w = fmaf(zeta, zeta, 1.0f);
-                const float t = fabsf(zeta) > 1.0e8f ? __fdividef(0.5f, zeta) : __fdividef(copysignf(1.0f, zeta), fabsf(zeta) + w * rsqrtf(w));
-                const float c = rsqrtf(fmaf(t, t, 1.0f)), sn = c * t;
-#pragma unroll
-                for (int f = 0; f < kJcF4; ++f) {
-                    const float4 x = ap[f], y = aq[f];
-                    mp[(f ^ fsw) * kLpp + l] = make_float4(c * x.x - sn * y.x, c * x.y - sn * y.y, c * x.z - sn * y.z, c * x.w - sn * y.w);
-                    mq[(f ^ fsw) * kLpp + l] = make_float4(sn * x.x + c * y.x, sn * x.y + c * y.y, sn * x.z + c * y.z, sn * x.w + c * y.w);
-                }
-                dv_p = p; dv_q = q; dv_c = c; dv_sn = sn; dv_pending = true;
-                if (l == 0) {
-                    nrm[p] = fmaxf(alpha - t * g, 0.0f);
-                    nrm[q] = beta + t * g;
-                }
-                rotated = rotated || g * g > kJacobiLastSweepCos * kJacobiLastSweepCos * alpha * beta;
-            }
-            __syncthreads();                                  // this CTA's slices are rotated before the next round reads them
-        }
-        vote = (__syncthreads_or(rotated) ? 1 : 0) | (__syncthreads_or(failed) ? 2 : 0);
-    }
-    apply_to_v();                                             // the last rotation kept back
-    for (int j = tid; j < kp; j += nt) nrm[j] = sqrtf(nrm[j]);           // singular values: the norms are fresh, nothing rotated since
-    __syncthreads();
-    for (int j = tid; j < k; j += nt) {
-        const float sj = nrm[j];
-        int rk = 0;
-        for (int i = 0; i < k; ++i) {
-            const float si = nrm[i];
-            rk += (si > sj || (si == sj && i < j)) ? 1 : 0;
-        }
-        rank_of[j] = rk;
-        if (cr == 0) S[rk] = sj;
-    }
-    __syncthreads();
-    for (int e = tid; e < k * kJcRows; e += nt) {
-        const int j = e / kJcRows, i = row0 + e % kJcRows;
-        if (i < k) {
-            const float sj = nrm[j];
-            const size_t o = (size_t)rank_of[j] * k + i;
-            Ucol[o] = sj > 0.0f ? M[e] / sj : 0.0f;
-            Vcol[o] = kWithV ? V[e] : (sj > 0.0f ? M[e] / (sj * sj) : 0.0f);
-        }
-    }
-    cluster.sync();                                           // nobody leaves while a neighbour could still store into it
-}
-
-// The instance of the cluster kernel for a core of k columns: `lanes` threads per pair slot, with or without the
-// accumulated right factor.
-typedef void (*JacobiClusterFn)(const float *, int, float *, float *, float *, unsigned *);
-JacobiClusterFn jacobi_cluster_fn(int k, int lanes, bool with_v) {
-    if (k <= 128) return with_v ? jacobi_svd_cluster_kernel<128, 4, true> : jacobi_svd_cluster_kernel<128, 4, false>;
-    if (lanes == 4) return with_v ? jacobi_svd_cluster_kernel<256, 4, true> : jacobi_svd_cluster_kernel<256, 4, false>;
-    return with_v ? jacobi_svd_cluster_kernel<256, 2, true> : jacobi_svd_cluster_kernel<256, 2, false>;
-}
-
-// Launch configuration of the cluster kernel: one cluster of kJcCtas CTAs, `lanes` threads per pair slot.
-void jacobi_cluster_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, int k, int lanes, cudaStream_t st) {
-    cfg->gridDim = dim3(kJcCtas, 1, 1);
-    cfg->blockDim = dim3(jacobi_cluster_len(k) / 2 * lanes, 1, 1);
-    cfg->dynamicSmemBytes = jacobi_cluster_smem_bytes(k);
-    cfg->stream = st;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kJcCtas;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg->attrs = attr;
-    cfg->numAttrs = 1;
 }
 
 // A timed span of the current call (no-ops unless the workspace's profiling is on).
@@ -853,25 +569,23 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
             ws->jc_with_v = false;
         }
     }
-    if (ok && ws->own_core_svd && ws->k <= kJacobiSingleMaxK)
+    if (ok && ws->own_core_svd && !ws->block_core && ws->k <= kRingMinK)
         ok = cudaFuncSetAttribute(jacobi_svd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)jacobi_smem_bytes(ws->k)) == cudaSuccess;
-    if (ok && ws->own_core_svd && !ws->block_core && ws->k > kJacobiSingleMaxK) {
-        const char *e = getenv("BSQ_JACOBI_LPP");
-        ws->jc_lanes = ws->k <= 128 || (e && atoi(e) == 4) ? 4 : 2;
-        {
+    if (ok && ws->own_core_svd && !ws->block_core && ws->k > kRingMinK) {
+        if (ws->k > kJacobiSingleMaxK) {
             const char *v = getenv("BSQ_JACOBI_V");           // 1 / 0: with / without the accumulated right factor (A/B comparisons)
             ws->jc_with_v = v ? v[0] == '1' : false;
         }
-        ok = cudaFuncSetAttribute(jacobi_cluster_fn(ws->k, ws->jc_lanes, ws->jc_with_v), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)jacobi_cluster_smem_bytes(ws->k)) == cudaSuccess;
-        if (ok) {
-            // a device (or partition of one) that cannot place a cluster of 8 such CTAs keeps the library solver
+        ws->ring = ring_jacobi_launch(ws->k, ws->jc_with_v);
+        ok = cudaFuncSetAttribute(ws->ring.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ws->ring.smem) == cudaSuccess;
+        if (ok && ws->ring.ctas > 1) {
+            // a device (or partition of one) that cannot place the cluster keeps the library solver
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute attr[1];
-            jacobi_cluster_config(&cfg, attr, ws->k, ws->jc_lanes, nullptr);
+            ring_jacobi_config(&cfg, attr, ws->ring, nullptr);
             int clusters = 0;
-            const cudaError_t q = cudaOccupancyMaxActiveClusters(&clusters, jacobi_cluster_fn(ws->k, ws->jc_lanes, ws->jc_with_v), &cfg);
+            const cudaError_t q = cudaOccupancyMaxActiveClusters(&clusters, ws->ring.fn, &cfg);
             if (q != cudaSuccess || clusters < 1) {
                 cudaGetLastError();
                 ws->own_core_svd = false;
@@ -1008,15 +722,14 @@ cudaError_t svd_lowrank(SvdWorkspace *ws, const float *d_A, float *d_U, float *d
         const float *core = ws->core;
         float *vc = ws->vc, *uc = ws->uc;
         if ((err = cudaLaunchKernelEx(&cfg, block_jacobi_fn(k, ws->jc_with_v), core, k, d_S, vc, uc)) != cudaSuccess) return err;
-    } else if (ws->own_core_svd && k > kJacobiSingleMaxK) {
+    } else if (ws->own_core_svd && k > kRingMinK) {
         cudaLaunchConfig_t cfg = {};
         cudaLaunchAttribute attr[1];
-        jacobi_cluster_config(&cfg, attr, k, ws->jc_lanes, st);
+        ring_jacobi_config(&cfg, attr, ws->ring, st);
         const float *core = ws->core;
         float *vc = ws->vc, *uc = ws->uc;
         unsigned *status = ws->status;
-        err = cudaLaunchKernelEx(&cfg, jacobi_cluster_fn(k, ws->jc_lanes, ws->jc_with_v), core, k, d_S, vc, uc, status);
-        if (err != cudaSuccess) return err;
+        if ((err = cudaLaunchKernelEx(&cfg, ws->ring.fn, core, k, d_S, vc, uc, status)) != cudaSuccess) return err;
     } else if (ws->own_core_svd) {
         // eight lanes per pair and no more: warps without a pair only make a round's barrier longer (k = 64: 301 -> 290 us)
         const int threads = std::max(1, ((k + 1) / 2 * 8 + 31) / 32) * 32;
