@@ -591,6 +591,7 @@ __host__ __device__ constexpr int cholesky_grid(int k, CholeskyPart part) {
 __global__ void __launch_bounds__(kCholThreads, 1) cholesky_kernel(const float *__restrict__ G, int k, float *R, float *T, CholeskySync *sync,
                                                                    unsigned *status, CholeskyPart part) {
     __shared__ unsigned s_role;
+    chain_begin();
     int role = part == kCholInverse ? (int)blockIdx.x + 1 : 0;
     const bool together = part == kCholBoth && gridDim.x > 1;
     if (together) {

@@ -165,6 +165,30 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity
     return false;
 }
 
+// First statement of a kernel that may be launched while the one before it still runs (launch_chained): waits until that one is done and
+// its stores are visible, then lets the next one's CTAs come.  A no-op in kernels launched the ordinary way.
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+// Launches a kernel that begins with chain_begin(): its CTAs may take their places while the kernel before it in the stream runs, which
+// hides the launch: compress and decompress of 777 x 1031 at rank 48 (75 kernels) 0.642 -> 0.545 ms, 2048 x 5120 at rank 64 1.044 -> 0.969 ms,
+// 8192 x 4096 at rank 256 2.979 -> 2.905 ms.  chained: false keeps the ordinary order (where other streams want the SMs that waiting CTAs would hold).
+template <class... P, class... A>
+cudaError_t launch_chained(bool chained, void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
+}
+
 // CTA-wide wait for a bulk copy: only warp 0 polls the barrier (a polling warp burns issue slots
 // whether 1 or 32 of its lanes spin), everybody else parks at the CTA barrier.  Returns false, for
 // all threads alike, if the wait gave up.

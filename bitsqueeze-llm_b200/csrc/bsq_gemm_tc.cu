@@ -210,6 +210,7 @@ __device__ __forceinline__ void tile_epilogue(const GemmArgs &g, unsigned tmem_d
 
 template <bool A_KMAJOR, bool B_KMAJOR, int NMAX>
 __global__ void __launch_bounds__(NT) gemm_tc_kernel(GemmArgs g, unsigned *status) {
+    chain_begin();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar_free[STAGES];
     __shared__ __align__(8) uint64_t bar_done;
@@ -456,6 +457,7 @@ struct HalfSlot {
 template <bool B_KMAJOR>
 __global__ void __launch_bounds__(256) presplit_b_kernel(const float *__restrict__ B, long ldb, int N, int K, int n_tile, int chunks,
                                                          float4 *__restrict__ image) {
+    chain_begin();
     const int n0 = blockIdx.y * n_tile;
     const int Nt = min(n_tile, N - n0);
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -496,6 +498,7 @@ __global__ void __launch_bounds__(256) presplit_b_kernel(const float *__restrict
 // rows past M are zeros.  The values are those the product kernel's transform warps would make of the same A.
 __global__ void __launch_bounds__(256) presplit_a_kernel(const float *__restrict__ A, long lda, int M, int K, const float *__restrict__ kscale,
                                                          float *__restrict__ image, int rows_pad) {
+    chain_begin();
     const int k4 = K / 4;
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long)rows_pad * k4) return;
@@ -514,6 +517,7 @@ __global__ void __launch_bounds__(256) presplit_a_kernel(const float *__restrict
 // longer matters: the product is NaN or Inf then, as it is for the reference.
 __global__ void __launch_bounds__(256) absmax_bits_kernel(const float *__restrict__ x, long ld, int rows, int cols, unsigned *out,
                                                           const float *__restrict__ colscale = nullptr) {
+    chain_begin();
     const unsigned c4 = cols / 4;
     unsigned m = 0;
     auto take = [&](float4 v, unsigned c) {
@@ -547,6 +551,7 @@ template <bool B_KMAJOR>
 __global__ void __launch_bounds__(256) presplit_b16_kernel(const float *__restrict__ B, long ldb, int N, int K, int n_tile, int chunks,
                                                            uint4 *__restrict__ image, const unsigned *__restrict__ absmax_bits, float fixed_scale,
                                                            float lo_scale) {
+    chain_begin();
     const int n0 = blockIdx.y * n_tile;
     const int Nt = min(n_tile, N - n0);
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -588,6 +593,7 @@ __global__ void __launch_bounds__(256) presplit_b16_kernel(const float *__restri
 __global__ void __launch_bounds__(256) presplit_a16_kernel(const float *__restrict__ A, long lda, int M, int K, const float *__restrict__ kscale,
                                                            uint4 *__restrict__ image, int rows_pad, const unsigned *__restrict__ absmax_bits,
                                                            float lo_scale) {
+    chain_begin();
     const int k8 = K / 8;
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long)rows_pad * k8) return;
@@ -607,6 +613,7 @@ __global__ void __launch_bounds__(256) presplit_a16_kernel(const float *__restri
 
 template <bool A_KMAJOR, int NMAX>
 __global__ void __launch_bounds__(NT2, NMAX <= 128 ? 2 : 1) gemm_tc_image_kernel(GemmArgs g, unsigned *status) {
+    chain_begin();
     // chunks of A in flight in registers per thread: what is in flight per SM is what bounds these products (the
     // pieces of A are small and far apart in HBM), so as many as the registers of 2 CTAs (N <= 128) or 1 CTA hold
     constexpr int DEPTH = NMAX <= 128 ? IMG_DEPTH_2CTA : IMG_DEPTH_1CTA;
@@ -759,8 +766,7 @@ cudaError_t launch(const GemmArgs &g, unsigned *status, cudaStream_t stream) {
     cudaError_t err = cudaFuncSetAttribute(gemm_tc_kernel<AK, BK, NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     dim3 grid((g.M + TM - 1) / TM, (g.N + g.n_tile - 1) / g.n_tile, g.splits);
-    gemm_tc_kernel<AK, BK, NMAX><<<grid, NT, smem, stream>>>(g, status);
-    return cudaGetLastError();
+    return launch_chained(g.chained, gemm_tc_kernel<AK, BK, NMAX>, grid, NT, smem, stream, g, status);
 }
 
 // Ring lengths of the image kernel for a tile of N columns: two stages of A and four images of B (two chunks of head
@@ -799,10 +805,10 @@ cudaError_t launch_image(const GemmArgs &g, bool b_kmajor, unsigned *status, cud
         }
         uint4 *image16 = reinterpret_cast<uint4 *>(image);
         const float lo_scale = g.lo_unscaled ? 1.0f : kSplit16LoScale;
-        if (b_kmajor) presplit_b16_kernel<true><<<pgrid, 256, 0, stream>>>(g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image16, bmax, g.b_scale_fixed, lo_scale);
-        else presplit_b16_kernel<false><<<pgrid, 256, 0, stream>>>(g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image16, bmax, g.b_scale_fixed, lo_scale);
-    } else if (b_kmajor) presplit_b_kernel<true><<<pgrid, 256, 0, stream>>>(g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image);
-    else presplit_b_kernel<false><<<pgrid, 256, 0, stream>>>(g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image);
+        if (b_kmajor) launch_chained(g.chained, presplit_b16_kernel<true>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image16, bmax, g.b_scale_fixed, lo_scale);
+        else launch_chained(g.chained, presplit_b16_kernel<false>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image16, bmax, g.b_scale_fixed, lo_scale);
+    } else if (b_kmajor) launch_chained(g.chained, presplit_b_kernel<true>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image);
+    else launch_chained(g.chained, presplit_b_kernel<false>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     if (g.use_tma && g.a_image && g.f16) {
@@ -824,8 +830,7 @@ cudaError_t launch_image(const GemmArgs &g, bool b_kmajor, unsigned *status, cud
     err = cudaFuncSetAttribute(gemm_tc_image_kernel<AK, NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     dim3 grid((g.M + TM - 1) / TM, n_tiles, g.splits);
-    gemm_tc_image_kernel<AK, NMAX><<<grid, NT2, smem, stream>>>(g, status);
-    return cudaGetLastError();
+    return launch_chained(g.chained, gemm_tc_image_kernel<AK, NMAX>, grid, NT2, smem, stream, g, status);
 }
 
 }  // namespace

@@ -129,6 +129,7 @@ struct TileWalk {
 // the 16-bit images cannot be made in place.
 template <bool A_KMAJOR, int NMAX, bool F16 = false>
 __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_constant__ CUtensorMap tmap_a, GemmArgs g, unsigned *status) {
+    chain_begin();
     extern __shared__ unsigned char smem_dyn[];
     unsigned char *base = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);      // the swizzle wants 1024-byte aligned slots
     constexpr int KS = F16 ? 64 : bsq::KS;                 // K per slot of A
@@ -607,8 +608,7 @@ template <bool AK, int NMAX, bool F16 = false>
 cudaError_t launch_tma(const CUtensorMap &map, const GemmArgs &g, dim3 grid, size_t smem, unsigned *status, cudaStream_t stream) {
     cudaError_t err = cudaFuncSetAttribute(gemm_tc_tma_kernel<AK, NMAX, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
-    gemm_tc_tma_kernel<AK, NMAX, F16><<<grid, NTH, smem, stream>>>(map, g, status);
-    return cudaGetLastError();
+    return launch_chained(g.chained, gemm_tc_tma_kernel<AK, NMAX, F16>, grid, NTH, smem, stream, map, g, status);
 }
 
 }  // namespace

@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(kJbThreads, 1) block_jacobi_kernel(const float
     int *rank_of = reinterpret_cast<int *>(maxes + 8);        // [block][column]
     const int tid = threadIdx.x, w = tid >> 5, l = tid & 31;
     const bool upper = l >= 16;
+    chain_begin();
     cluster.sync();                                           // every CTA runs before anybody stores into its shared memory
 
     // ---- the two blocks of this CTA, zero-padded; V = identity ----

@@ -96,6 +96,7 @@ __global__ void __launch_bounds__(ring_max_threads(kLen), 1) ring_jacobi_kernel(
     cg::cluster_group cluster = cg::this_cluster();
     const int cr = kCluster ? (int)cluster.block_rank() : 0, ctas = kCluster ? (int)cluster.num_blocks() : 1;
     extern __shared__ __align__(16) float sm[];
+    chain_begin();
     const int tid = threadIdx.x, lane = tid & 31, w = __shfl_sync(kFullMask, tid >> 5, 0), wpc = blockDim.x >> 5;
     const int spc = wpc * kS;                                 // slots of a CTA
     float *boxes = sm;                                        // [parity][warp][0: from above (p), 1: from below (q)][kCol]

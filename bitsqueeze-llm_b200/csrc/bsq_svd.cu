@@ -275,6 +275,7 @@ __host__ __device__ constexpr size_t jacobi_smem_bytes(int k) {
 __global__ void __launch_bounds__(256, 1) jacobi_svd_kernel(const float *__restrict__ C, int k, float *__restrict__ S,
                                                          float *__restrict__ Ucol, float *__restrict__ Vcol) {
     extern __shared__ __align__(16) float sm[];
+    chain_begin();
     constexpr int LEN = kJacobiLen;
     const int kp = (k + 1) & ~1, npairs = kp / 2;
     float *M = sm, *V = M + (size_t)kp * LEN, *nrm = V + (size_t)kp * LEN;
@@ -444,8 +445,8 @@ cudaError_t orthonormalise(SvdWorkspace *ws, float *Y, float *tmp, int rows, int
             float *r_out = pass == 0 ? r_a : r_b;
             if (!r_out) r_out = ws->rfac;
             const auto launch = [&](CholeskyPart part) {
-                cholesky_kernel<<<cholesky_grid(k, part), kCholThreads, cholesky_blocked_smem_bytes(k), st>>>(
-                    ws->g, k, r_out, factor_only ? nullptr : ws->t, ws->chol_sync, ws->status, part);
+                launch_chained(!ws->device_full, cholesky_kernel, cholesky_grid(k, part), kCholThreads, cholesky_blocked_smem_bytes(k), st,
+                               ws->g, k, r_out, factor_only ? nullptr : ws->t, ws->chol_sync, ws->status, part);
             };
             if (factor_only || ws->device_full) {
                 launch(kCholFactor);
@@ -733,8 +734,8 @@ cudaError_t svd_lowrank(SvdWorkspace *ws, const float *d_A, float *d_U, float *d
     } else if (ws->own_core_svd) {
         // eight lanes per pair and no more: warps without a pair only make a round's barrier longer (k = 64: 301 -> 290 us)
         const int threads = std::max(1, ((k + 1) / 2 * 8 + 31) / 32) * 32;
-        jacobi_svd_kernel<<<1, threads, jacobi_smem_bytes(k), st>>>(ws->core, k, d_S, ws->vc, ws->uc);
-        if ((err = cudaGetLastError()) != cudaSuccess) return err;
+        if ((err = launch_chained(!ws->device_full, jacobi_svd_kernel, 1, threads, jacobi_smem_bytes(k), st, ws->core, k, d_S, ws->vc, ws->uc)) != cudaSuccess)
+            return err;
     } else if (cusolverDnSgesvdj(ws->solver, CUSOLVER_EIG_MODE_VECTOR, 0, k, k, ws->core, k, d_S, ws->vc, k, ws->uc, k,
                                  ws->solver_work, ws->lwork, ws->dev_info, ws->svdj) != CUSOLVER_STATUS_SUCCESS) {
         return cudaErrorUnknown;
