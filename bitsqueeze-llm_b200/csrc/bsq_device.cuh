@@ -172,7 +172,7 @@ __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 // Launches a kernel that begins with chain_begin(): its CTAs may take their places while the kernel before it in the stream runs, which
-// hides the launch: compress and decompress of 777 x 1031 at rank 48 (75 kernels) 0.642 -> 0.545 ms, 2048 x 5120 at rank 64 1.044 -> 0.969 ms,
+// hides the launch: compress and decompress of 777 x 1031 at rank 48 (54 kernels) 0.642 -> 0.545 ms, 2048 x 5120 at rank 64 1.044 -> 0.969 ms,
 // 8192 x 4096 at rank 256 2.979 -> 2.905 ms.  chained: false keeps the ordinary order (where other streams want the SMs that waiting CTAs would hold).
 template <class... P, class... A>
 cudaError_t launch_chained(bool chained, void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
