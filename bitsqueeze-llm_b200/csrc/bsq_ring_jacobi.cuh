@@ -490,7 +490,7 @@ RingLaunch ring_jacobi_launch(int k, bool with_v) {
     if (k <= 64) return {ring_jacobi_kernel<64, true, false>, 1, all, ring_smem_bytes<64, true>(all)};
     RingLaunch r;
     r.ctas = (all + kRingWarps - 1) / kRingWarps;
-    r.warps = kRingWarps;
+    r.warps = (all + r.ctas - 1) / r.ctas;
     if (k <= 128) {
         r.fn = with_v ? ring_jacobi_kernel<128, true, true> : ring_jacobi_kernel<128, false, true>;
         r.smem = with_v ? ring_smem_bytes<128, true>(r.warps) : ring_smem_bytes<128, false>(r.warps);
