@@ -307,7 +307,7 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
                         unsigned *flag, unsigned *status, float *workspace, size_t workspace_bytes, int sm_count,
                         cudaStream_t stream, const unsigned *a_absmax_bits, float b_bound, bool device_full) {
     if (M <= 0 || N <= 0 || K <= 0) return cudaErrorInvalidValue;
-    const bool chained = !device_full && !kscale && !minuend;        // (the products of the range finder)
+    const bool chained = !device_full;
     if (allow_tensor_cores) {
         // tensor-core path: one 128-row tile per CTA, two CTAs per SM up to N = 128; K is split so that the tiles fill
         // the SMs once
