@@ -1,6 +1,6 @@
 """The k x k kernels of the randomized SVD (Cholesky factor and inverse by 32 x 32 blocks, block Jacobi on 1 to 8 CTAs) at the edges
 of their blocks, clusters and paddings, through bsq_svd_lowrank, against FP64 numpy; and the kernels that take the core's SVD where factors are
-coded (one CTA up to 64 columns, rows dealt over a cluster above) by the same checks and those of test_gpu_svd.py, through bsq_svd_lowrank_coded.
+coded (one CTA up to 48 columns, columns on a ring of warps above, over a cluster above 64) by the same checks and those of test_gpu_svd.py, through bsq_svd_lowrank_coded.
 
 Bounds.  Each QR pass factors G + 1e-5 max(diag G) I, so columns are orthonormal to a few 1e-5, up to 2e-4 for the weakest
 direction of a wide sketch (the bounds of test_gpu_svd.py).  With orthonormal Q the residual of Q Q^T A has the squared norm
