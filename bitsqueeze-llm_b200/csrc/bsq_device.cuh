@@ -165,7 +165,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity
     return false;
 }
 
-// First statement of a kernel that may be launched while the one before it still runs (launch_chained): waits until that one is done and
+// First statement (outside every branch: nothing may be read or written before it) of a kernel that may be launched while the one before it still runs (launch_chained): waits until that one is done and
 // its stores are visible, then lets the next one's CTAs come.  A no-op in kernels launched the ordinary way.
 __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");

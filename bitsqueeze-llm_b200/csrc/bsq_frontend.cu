@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(256, 4)
     frontend_select_kernel(const float *__restrict__ in, unsigned rows, unsigned cols, unsigned k,
                            uint16_t *__restrict__ out_idx, float *__restrict__ out_val, float *__restrict__ absmax_scratch,
                            unsigned *gmax_bits, unsigned *row_counter, unsigned *hint_word) {
+    chain_begin();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const RowGroup<G> g;
     const StreamLayout lay = stream_layout(cols, 0);
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(256, 4)
                            const uint16_t *__restrict__ idx, const float *__restrict__ absmax_scratch,
                            const unsigned *__restrict__ gmax_bits, float *__restrict__ dq_out,
                            uint8_t *__restrict__ scale_codes, uint8_t *__restrict__ data, unsigned *row_counter) {
+    chain_begin();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const RowGroup<G> g;
     const StreamLayout lay = stream_layout(cols, 2);
@@ -294,10 +296,10 @@ cudaError_t launch_front(int method, const float *d_in, uint32_t rows, uint32_t 
     if (events) cudaEventRecord(events[1], stream);
     err = persistent_grid(frontend_encode_kernel<G>, f2.threads, f2.smem, sm_count, rows, f2.groups, &grid);
     if (err != cudaSuccess) return err;
-    frontend_encode_kernel<G><<<grid, f2.threads, f2.smem, stream>>>(d_in, rows, cols, k, d_idx, absmax, gmax, d_dq,
-                                                                      d_scale_codes, d_data, gmax + 2);
+    err = launch_chained(true, frontend_encode_kernel<G>, grid, f2.threads, f2.smem, stream, d_in, rows, cols, k, d_idx, absmax, gmax, d_dq,
+                         d_scale_codes, d_data, gmax + 2);
     if (events) cudaEventRecord(events[2], stream);
-    return cudaGetLastError();
+    return err;
 }
 
 }  // namespace

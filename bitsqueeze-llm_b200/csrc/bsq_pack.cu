@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(kCopyThreads) copy_segments_kernel(const __gri
 
 __global__ void __launch_bounds__(kCopyThreads) pack_object_kernel(const __grid_constant__ CopyArgs c, const __grid_constant__ PackHeaders h,
                                                                    const unsigned *status, unsigned *mirror) {
+    chain_begin();
     copy_all(c);
     if (blockIdx.x != gridDim.x - 1) return;
     // the last CTA: headers and status (its share of the pieces is the smallest)
@@ -185,8 +186,7 @@ cudaError_t pack_object(const CopySegment *segments, int count, const PackHeader
     if (count < 0 || count > kMaxCopySegments) return cudaErrorInvalidValue;
     CopyArgs c;
     const unsigned ctas = fill(c, segments, count);
-    pack_object_kernel<<<ctas + 1, kCopyThreads, 0, stream>>>(c, headers, d_status, mirror);
-    return cudaGetLastError();
+    return launch_chained(true, pack_object_kernel, ctas + 1, kCopyThreads, 0, stream, c, headers, d_status, mirror);
 }
 
 cudaError_t fetch_heads(const HeadList &heads, uint8_t *host, unsigned *d_status, cudaStream_t stream) {

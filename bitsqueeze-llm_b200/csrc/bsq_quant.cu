@@ -76,6 +76,7 @@ __device__ __forceinline__ float gather_block_value(const float (&am)[4], int la
 __global__ void __launch_bounds__(kThreads) absmax_flat_kernel(const float *__restrict__ x, uint64_t n, bool vec,
                                                                float *__restrict__ absmax_out,
                                                                unsigned *__restrict__ gmax_bits) {
+    chain_begin();
     const int lane = threadIdx.x & 31;
     const uint64_t warp = (uint64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     const uint64_t nwarps = (uint64_t)gridDim.x * (kThreads / 32);
@@ -111,6 +112,7 @@ __global__ void __launch_bounds__(kThreads)
                        const unsigned *__restrict__ gmax_bits, float *__restrict__ scales_f32,
                        uint8_t *__restrict__ scale_codes, float *__restrict__ dq_out, uint8_t *__restrict__ data,
                        float *deq_out, unsigned *flag) {   // deq_out may alias x (in-place write-back)
+    chain_begin();
     bool any = false;
     const int lane = threadIdx.x & 31;
     const uint64_t warp = (uint64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
@@ -308,15 +310,14 @@ cudaError_t nf4_quantize(const float *d_x, uint64_t n, float *d_scales, uint8_t 
     const bool vec = aligned(d_x, 16) && aligned(d_data, 4) && (!d_deq_out || aligned(d_deq_out, 16));
     const int grid = grid_for(n, sm_count);
     if (d_deq_out && d_error_flag)
-        encode_flat_kernel<false, kWriteError><<<grid, kThreads, 0, stream>>>(d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
+        return launch_chained(true, encode_flat_kernel<false, kWriteError>, grid, kThreads, 0, stream, d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
                                                                          nullptr, d_data, d_deq_out, d_error_flag);
     else if (d_deq_out)
-        encode_flat_kernel<false, kWriteDeq><<<grid, kThreads, 0, stream>>>(d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
+        return launch_chained(true, encode_flat_kernel<false, kWriteDeq>, grid, kThreads, 0, stream, d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
                                                                          nullptr, d_data, d_deq_out, nullptr);
     else
-        encode_flat_kernel<false, kWriteNone><<<grid, kThreads, 0, stream>>>(d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
+        return launch_chained(true, encode_flat_kernel<false, kWriteNone>, grid, kThreads, 0, stream, d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
                                                                           nullptr, d_data, nullptr, nullptr);
-    return cudaGetLastError();
 }
 
 size_t nf4dq_scratch_bytes(uint64_t n) { return (size_t)((n + 63) / 64) * sizeof(float) + 16; }
@@ -331,16 +332,16 @@ cudaError_t nf4dq_quantize(const float *d_x, uint64_t n, float *d_dq, uint8_t *d
     cudaError_t err = cudaMemsetAsync(gmax, 0, 16, stream);
     if (err != cudaSuccess) return err;
     absmax_flat_kernel<<<grid, kThreads, 0, stream>>>(d_x, n, vec, absmax, gmax);
+    if ((err = cudaGetLastError()) != cudaSuccess) return err;
     if (d_deq_out && d_error_flag)
-        encode_flat_kernel<true, kWriteError><<<grid, kThreads, 0, stream>>>(d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
+        return launch_chained(true, encode_flat_kernel<true, kWriteError>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
                                                                         d_dq, d_data, d_deq_out, d_error_flag);
     else if (d_deq_out)
-        encode_flat_kernel<true, kWriteDeq><<<grid, kThreads, 0, stream>>>(d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
+        return launch_chained(true, encode_flat_kernel<true, kWriteDeq>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
                                                                         d_dq, d_data, d_deq_out, nullptr);
     else
-        encode_flat_kernel<true, kWriteNone><<<grid, kThreads, 0, stream>>>(d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
+        return launch_chained(true, encode_flat_kernel<true, kWriteNone>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
                                                                          d_dq, d_data, nullptr, nullptr);
-    return cudaGetLastError();
 }
 
 uint64_t nf4dq_static_max_elements() { return kStaticMaxElems; }

@@ -29,6 +29,7 @@ __global__ void __launch_bounds__(512)
     topk_rows_group_kernel(const float *__restrict__ in, float *residual, unsigned rows, unsigned cols, unsigned k,
                            uint16_t *__restrict__ out_idx, float *__restrict__ out_val, unsigned *status, unsigned group_bytes,
                            unsigned ctl_off, unsigned *bound) {
+    chain_begin();
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const RowGroup<G> g;
     unsigned char *base = smem_raw + (size_t)g.gid * group_bytes;
@@ -359,9 +360,8 @@ static cudaError_t launch_group(const float *d_in, float *d_residual, uint32_t r
     unsigned grid = (unsigned)sm_count * (unsigned)per_sm;
     const unsigned needed = (rows + f.groups - 1) / f.groups;
     if (grid > needed) grid = needed;
-    topk_rows_group_kernel<G, kBulk><<<grid, f.threads, smem, stream>>>(d_in, d_residual, rows, cols, k, d_idx, d_val, d_status,
-                                                                  f.group_bytes, f.ctl_off, d_bound);
-    return cudaGetLastError();
+    return launch_chained(true, topk_rows_group_kernel<G, kBulk>, grid, f.threads, smem, stream, d_in, d_residual, rows, cols, k, d_idx, d_val, d_status,
+                          f.group_bytes, f.ctl_off, d_bound);
 }
 
 cudaError_t topk_rows(const float *d_in, float *d_residual, uint32_t rows, uint32_t cols, uint32_t k, uint16_t *d_idx,
