@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(ring_max_threads(kLen), 1) ring_jacobi_kernel(
 #pragma unroll
         for (int i = 0; i < 4; ++i) mbar_expect_tx(&mbar[i], kTx);
     }
+    if (kCluster) cluster.sync();                             // every CTA runs, its mbarriers ready, before anybody stores into its shared memory
 
     // ---- this warp's columns ----
     // slot s: p = s (the last column in slot 0), q = kp - 1 - s (column 0 in slot 0)

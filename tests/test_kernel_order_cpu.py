@@ -1,0 +1,55 @@
+"""Orders that the kernels' sources have to keep because no run can be relied on to show that they are broken: a store that comes too
+early usually still lands where it should.  The sources are read as text."""
+import glob
+import os
+import re
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "bitsqueeze-llm_b200", "csrc")
+
+
+def block(text, at):
+    """The balanced {...} that opens at or behind `at`."""
+    start, depth = text.index("{", at), 0
+    for i in range(start, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[start: i + 1]
+    raise ValueError("unbalanced braces")
+
+
+def sources():
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))):
+        with open(path) as f:
+            text = f.read()
+        yield os.path.basename(path), re.sub(r"//[^\n]*", "", re.sub(r"/\*.*?\*/", "", text, flags=re.S))
+
+
+def kernels():
+    """name -> (parameters, body) of every __global__ function."""
+    found = {}
+    for _, text in sources():
+        for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s+)?(\w+)\s*\(", text):
+            end, depth = m.end(), 1
+            while depth:
+                depth += {"(": 1, ")": -1}.get(text[end], 0)
+                end += 1
+            found[m.group(1)] = (text[m.end(): end - 1], block(text, end))
+    return found
+
+
+KERNELS = kernels()
+
+
+def test_kernels_are_found():
+    assert {"ring_jacobi_kernel", "block_jacobi_kernel", "cholesky_kernel", "gemm_kernel", "topk_rows_group_kernel"} <= set(KERNELS)
+
+
+@pytest.mark.parametrize("name", sorted(n for n, (_, body) in KERNELS.items() if "this_cluster()" in body))
+def test_clusters_meet_before_they_store_into_one_another(name):
+    """CTAs of a cluster are scheduled together but need not have started together: shared memory of another CTA may be touched only
+    behind a barrier of the cluster."""
+    body = KERNELS[name][1]
+    remote = min(m.start() for m in re.finditer(r"map_shared_rank|st\w*_async\w*\(|put_remote", body))
+    assert 0 <= body.find("cluster.sync()") < remote
