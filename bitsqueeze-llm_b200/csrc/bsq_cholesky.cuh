@@ -327,7 +327,7 @@ __device__ __noinline__ void chol_update_wide(int nb, int A, int B, int L, int t
 
 // R (row-major k x k, upper triangular, zeros below the diagonal) from G, and the diagonal blocks of T = R^-1 if T is given.
 // sync (may be null): told which block rows are out.
-__device__ __forceinline__ void cholesky_factor(const float *__restrict__ G, int k, float *R, float *T, CholeskySync *sync) {
+__device__ __forceinline__ void cholesky_factor(const float *G, int k, float *R, float *T, CholeskySync *sync) {
     float *sm = chol_smem();
     const int nb = chol_blocks(k), nbt = nb * (nb + 1) / 2;
     float *blocks = sm;                                    // nbt blocks of 32 x 32, row-major; those above the diagonal end as R's
@@ -588,7 +588,7 @@ enum CholeskyPart { kCholBoth, kCholFactor, kCholInverse };
 __host__ __device__ constexpr int cholesky_grid(int k, CholeskyPart part) {
     return part == kCholFactor || chol_blocks(k) == 1 ? 1 : chol_blocks(k) - (part == kCholInverse ? 1 : 0);
 }
-__global__ void __launch_bounds__(kCholThreads, 1) cholesky_kernel(const float *__restrict__ G, int k, float *R, float *T, CholeskySync *sync,
+__global__ void __launch_bounds__(kCholThreads, 1) cholesky_kernel(const float *G, int k, float *R, float *T, CholeskySync *sync,
                                                                    unsigned *status, CholeskyPart part) {
     __shared__ unsigned s_role;
     chain_begin();

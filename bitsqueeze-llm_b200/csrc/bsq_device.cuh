@@ -165,8 +165,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity
     return false;
 }
 
-// First statement (outside every branch: nothing may be read or written before it) of a kernel that may be launched while the one before it still runs (launch_chained): waits until that one is done and
-// its stores are visible, then lets the next one's CTAs come.  A no-op in kernels launched the ordinary way.
+// For kernels that may be launched while the one before them still runs (launch_chained): waits until that one is done and its stores are
+// visible, then lets the next one's CTAs come.  A no-op in kernels launched the ordinary way.
+//   * Outside every branch, and nothing in memory is read or written before it.
+//   * What the kernel before may write comes in through plain pointers: `const` with __restrict__, or __ldg, says that nobody writes the
+//     data while the kernel runs -- which is not so while it waits -- and lets loads move in front of the wait.  (The caller's matrix in
+//     the front end is read that way: the encoder comes behind the selection, the selection behind a memset.)
 __device__ __forceinline__ void chain_begin() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -121,8 +121,8 @@ __device__ __forceinline__ void encode_and_store(const RowGroup<G> &g, GroupCtl 
 template <int G>
 __global__ void __launch_bounds__(256, 4)
     frontend_encode_kernel(const float *__restrict__ in, unsigned rows, unsigned cols, unsigned k,
-                           const uint16_t *__restrict__ idx, const float *__restrict__ absmax_scratch,
-                           const unsigned *__restrict__ gmax_bits, float *__restrict__ dq_out,
+                           const uint16_t *idx, const float *absmax_scratch,
+                           const unsigned *gmax_bits, float *__restrict__ dq_out,
                            uint8_t *__restrict__ scale_codes, uint8_t *__restrict__ data, unsigned *row_counter) {
     chain_begin();
     extern __shared__ __align__(128) unsigned char smem_raw[];

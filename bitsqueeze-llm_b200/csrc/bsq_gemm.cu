@@ -198,7 +198,7 @@ void launch_fp32(const GemmArgs &g, int sm_count, cudaStream_t stream) {
 // 48 partials of 256 x 256: 4.6 us, 4 of 4096 x 256: 7.2 us; before, with a 64-bit division per element and eight loads in
 // flight, 5.8 us in the mean over a rank-256 call's fourteen reductions, 5.3 us now.
 template <int VEC>
-__global__ void __launch_bounds__(256) reduce_splits_kernel(const float *__restrict__ part, float *__restrict__ C, unsigned total, int N, long ldc,
+__global__ void __launch_bounds__(256) reduce_splits_kernel(const float *part, float *__restrict__ C, unsigned total, int N, long ldc,
                                                             int splits, size_t split_stride) {
     constexpr int U = VEC == 4 ? 8 : 32;
     chain_begin();

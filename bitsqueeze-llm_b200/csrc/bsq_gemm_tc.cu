@@ -455,7 +455,7 @@ struct HalfSlot {
 // One thread per (chunk, k quad, column): the four values B(16 c + 4 kc .. + 3, n0 + r) split into the hi and the lo
 // unit of the chunk's image.  k past K gives zeros.
 template <bool B_KMAJOR>
-__global__ void __launch_bounds__(256) presplit_b_kernel(const float *__restrict__ B, long ldb, int N, int K, int n_tile, int chunks,
+__global__ void __launch_bounds__(256) presplit_b_kernel(const float *B, long ldb, int N, int K, int n_tile, int chunks,
                                                          float4 *__restrict__ image) {
     chain_begin();
     const int n0 = blockIdx.y * n_tile;
@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(256) presplit_b_kernel(const float *__restrict
 
 // A (contiguous along K, times kscale) split into two row-major rows_pad x K matrices, hi then lo, four k per thread;
 // rows past M are zeros.  The values are those the product kernel's transform warps would make of the same A.
-__global__ void __launch_bounds__(256) presplit_a_kernel(const float *__restrict__ A, long lda, int M, int K, const float *__restrict__ kscale,
+__global__ void __launch_bounds__(256) presplit_a_kernel(const float *A, long lda, int M, int K, const float *kscale,
                                                          float *__restrict__ image, int rows_pad) {
     chain_begin();
     const int k4 = K / 4;
@@ -515,8 +515,8 @@ __global__ void __launch_bounds__(256) presplit_a_kernel(const float *__restrict
 // The largest |x| of a rows x cols matrix (leading dimension ld) as float bits, by atomicMax into *out (cleared by the
 // caller).  Non-finite values leave bits >= 0x7f800000 there, which split16_scale answers with... a scale that no
 // longer matters: the product is NaN or Inf then, as it is for the reference.
-__global__ void __launch_bounds__(256) absmax_bits_kernel(const float *__restrict__ x, long ld, int rows, int cols, unsigned *out,
-                                                          const float *__restrict__ colscale = nullptr) {
+__global__ void __launch_bounds__(256) absmax_bits_kernel(const float *x, long ld, int rows, int cols, unsigned *out,
+                                                          const float *colscale = nullptr) {
     chain_begin();
     const unsigned c4 = cols / 4;
     unsigned m = 0;
@@ -548,8 +548,8 @@ __global__ void __launch_bounds__(256) absmax_bits_kernel(const float *__restric
 // B(32 c + 8 kc .. + 7, n0 + r), scaled, as the hi and the lo unit of the chunk's image (same unit order and image size
 // as the TF32 images, which hold 16 k per chunk).  k past K gives zeros.
 template <bool B_KMAJOR>
-__global__ void __launch_bounds__(256) presplit_b16_kernel(const float *__restrict__ B, long ldb, int N, int K, int n_tile, int chunks,
-                                                           uint4 *__restrict__ image, const unsigned *__restrict__ absmax_bits, float fixed_scale,
+__global__ void __launch_bounds__(256) presplit_b16_kernel(const float *B, long ldb, int N, int K, int n_tile, int chunks,
+                                                           uint4 *__restrict__ image, const unsigned *absmax_bits, float fixed_scale,
                                                            float lo_scale) {
     chain_begin();
     const int n0 = blockIdx.y * n_tile;
@@ -590,8 +590,8 @@ __global__ void __launch_bounds__(256) presplit_b16_kernel(const float *__restri
 
 // The FP16 form of presplit_a_kernel: two row-major rows_pad x K matrices of FP16 values, hi then lo, eight k per thread;
 // the scale comes from *absmax_bits, the largest |A(m, k) kscale(k)| (absmax_bits_kernel with the same kscale).
-__global__ void __launch_bounds__(256) presplit_a16_kernel(const float *__restrict__ A, long lda, int M, int K, const float *__restrict__ kscale,
-                                                           uint4 *__restrict__ image, int rows_pad, const unsigned *__restrict__ absmax_bits,
+__global__ void __launch_bounds__(256) presplit_a16_kernel(const float *A, long lda, int M, int K, const float *kscale,
+                                                           uint4 *__restrict__ image, int rows_pad, const unsigned *absmax_bits,
                                                            float lo_scale) {
     chain_begin();
     const int k8 = K / 8;

@@ -182,7 +182,7 @@ __device__ __forceinline__ bool rotate_two(float2 (&p0)[kPairs], float2 (&q0)[kP
 }
 
 template <int kCtas, bool kWithV>
-__global__ void __launch_bounds__(kJbThreads, 1) block_jacobi_kernel(const float *__restrict__ C, int k, float *__restrict__ S,
+__global__ void __launch_bounds__(kJbThreads, 1) block_jacobi_kernel(const float *C, int k, float *__restrict__ S,
                                                                    float *__restrict__ Ucol, float *__restrict__ Vcol) {
     constexpr int kLen = block_jacobi_len(kCtas), kCol = kLen * (kWithV ? 2 : 1);      // rows of M; floats per column (V's below M's)
     constexpr int kPairs = kLen / 64;                                    // float2 per lane and column

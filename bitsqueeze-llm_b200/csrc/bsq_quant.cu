@@ -73,7 +73,7 @@ __device__ __forceinline__ float gather_block_value(const float (&am)[4], int la
 }
 
 // ---- NF4_DQ pass 1: per-block absmax (1.0 for an all-zero block) and the global maximum ----
-__global__ void __launch_bounds__(kThreads) absmax_flat_kernel(const float *__restrict__ x, uint64_t n, bool vec,
+__global__ void __launch_bounds__(kThreads) absmax_flat_kernel(const float *x, uint64_t n, bool vec,
                                                                float *__restrict__ absmax_out,
                                                                unsigned *__restrict__ gmax_bits) {
     chain_begin();
@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(kThreads) absmax_flat_kernel(const float *__re
 enum : int { kWriteNone = 0, kWriteDeq = 1, kWriteError = 2 };
 template <bool DQ, int WRITE>
 __global__ void __launch_bounds__(kThreads)
-    encode_flat_kernel(const float *x, uint64_t n, bool vec, const float *__restrict__ absmax_in,
-                       const unsigned *__restrict__ gmax_bits, float *__restrict__ scales_f32,
+    encode_flat_kernel(const float *x, uint64_t n, bool vec, const float *absmax_in,
+                       const unsigned *gmax_bits, float *__restrict__ scales_f32,
                        uint8_t *__restrict__ scale_codes, float *__restrict__ dq_out, uint8_t *__restrict__ data,
                        float *deq_out, unsigned *flag) {   // deq_out may alias x (in-place write-back)
     chain_begin();

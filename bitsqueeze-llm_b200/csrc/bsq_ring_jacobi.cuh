@@ -85,7 +85,7 @@ __host__ __device__ constexpr size_t ring_smem_bytes(int warps) {
 }
 
 template <int kLen, bool kWithV, bool kCluster>
-__global__ void __launch_bounds__(ring_max_threads(kLen), 1) ring_jacobi_kernel(const float *__restrict__ C, int k, float *__restrict__ S,
+__global__ void __launch_bounds__(ring_max_threads(kLen), 1) ring_jacobi_kernel(const float *C, int k, float *__restrict__ S,
                                                                                 float *__restrict__ Ucol, float *__restrict__ Vcol,
                                                                                 unsigned *__restrict__ status) {
     static_assert(kLen > 64 || kWithV, "one CTA keeps V in the upper half of its warps");

@@ -272,7 +272,7 @@ __host__ __device__ constexpr size_t jacobi_smem_bytes(int k) {
 }
 
 // (One CTA per SM told to the compiler: without that it schedules as if other warps hid a chain's latencies; k = 48 163 -> 158 us.)
-__global__ void __launch_bounds__(256, 1) jacobi_svd_kernel(const float *__restrict__ C, int k, float *__restrict__ S,
+__global__ void __launch_bounds__(256, 1) jacobi_svd_kernel(const float *C, int k, float *__restrict__ S,
                                                          float *__restrict__ Ucol, float *__restrict__ Vcol) {
     extern __shared__ __align__(16) float sm[];
     chain_begin();

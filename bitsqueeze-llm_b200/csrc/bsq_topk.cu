@@ -26,7 +26,7 @@ namespace {
 // in flight per lane: 16 us against 49 us of the generic kernel's six passes over the row for 1501 x 3001, k = 30.
 template <int G, bool kBulk>
 __global__ void __launch_bounds__(512)
-    topk_rows_group_kernel(const float *__restrict__ in, float *residual, unsigned rows, unsigned cols, unsigned k,
+    topk_rows_group_kernel(const float *in, float *residual, unsigned rows, unsigned cols, unsigned k,
                            uint16_t *__restrict__ out_idx, float *__restrict__ out_val, unsigned *status, unsigned group_bytes,
                            unsigned ctl_off, unsigned *bound) {
     chain_begin();

@@ -53,3 +53,32 @@ def test_clusters_meet_before_they_store_into_one_another(name):
     body = KERNELS[name][1]
     remote = min(m.start() for m in re.finditer(r"map_shared_rank|st\w*_async\w*\(|put_remote", body))
     assert 0 <= body.find("cluster.sync()") < remote
+
+
+CHAINED = sorted(n for n, (_, body) in KERNELS.items() if "chain_begin()" in body)
+# inputs that are complete before the kernel in front of theirs has started: the caller's matrix
+COMPLETE = {"frontend_select_kernel": {"in"}, "frontend_encode_kernel": {"in"}}
+
+
+def test_kernels_launched_chained_wait():
+    launched = set()
+    for _, text in sources():
+        for m in re.finditer(r"launch_chained\(", text):
+            args = text[m.end(): m.end() + 400]
+            target = re.match(r"[^,]*(?:\([^()]*\))?[^,]*,\s*(\w+)", args)
+            if target and target.group(1) != "void":
+                launched.add(target.group(1))
+    assert len(launched) >= 12 and launched <= set(CHAINED)
+
+
+@pytest.mark.parametrize("name", CHAINED)
+def test_inputs_of_chained_kernels_are_read_behind_the_wait(name):
+    """While a chained kernel waits, the kernel before it may still write its inputs.  A `const ... *__restrict__` parameter promises that
+    nobody does, and the compiler may then read it through the read-only path and in front of the wait."""
+    params, body = KERNELS[name]
+    promised = set(re.findall(r"const\s+\w+\s*\*\s*__restrict__\s*(\w+)", params))
+    assert promised <= COMPLETE.get(name, set())
+    assert "__ldg(" not in body
+    before = body[1: body.index("chain_begin()")]
+    assert before.count("{") == before.count("}")                # not in a branch
+    assert not re.search(r"\b(?:if|for|while)\s*\(|__syncthreads|cluster\.sync\(\)", before)
