@@ -60,6 +60,14 @@ __device__ __forceinline__ void tma_load_2d(void *dst_smem, const CUtensorMap *m
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// This thread has read its share of a raw slot: the producer's next copy may overwrite it.  The copy writes through the async proxy, which
+// the arrival alone does not order behind the reads: they may still be under way when it is seen.  (Without the fence, products of two
+// matrices side by side had single rows wrong, a few units of four k, in 3 to 6 % of the calls where waiting CTAs of the next kernels shared
+// the SM.  The fence costs nothing that shows: 8192 x 256 x 4096 65.2 us either way, 4096 x 256 x 8192 63.5 -> 62.4.)
+__device__ __forceinline__ void raw_read_done(uint64_t *bar) {
+    fence_proxy_async_smem();
+    mbar_arrive(bar);
+}
 // Position in a ring of `n` stages and the parity of its current round.  Every role walks its rings with one of these:
 // a division and a remainder by the (run-time) ring length per stage were most of what the single threads that issue
 // the copies and the MMAs executed per stage.
@@ -352,7 +360,7 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
                         w[u] = box0[t * 8 + (u ^ (t & 7))];
                         w[8 + u] = box1[t * 8 + (u ^ (t & 7))];
                     }
-                    mbar_arrive(&bars.raw_empty[sr]);
+                    raw_read_done(&bars.raw_empty[sr]);
                     uint4 *hi16 = reinterpret_cast<uint4 *>(hi), *lo16 = reinterpret_cast<uint4 *>(lo);
 #pragma unroll
                     for (int c8 = 0; c8 < 8; ++c8) {
@@ -387,7 +395,7 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
                                 w[kg * 8 + q] = make_float4(e[0], e[1], e[2], e[3]);
                             }
                         }
-                        mbar_arrive(&bars.raw_empty[sr]);
+                        raw_read_done(&bars.raw_empty[sr]);
                         uint4 *hi16 = reinterpret_cast<uint4 *>(hi), *lo16 = reinterpret_cast<uint4 *>(lo);
 #pragma unroll
                         for (int c8 = 0; c8 < 8; ++c8) {
@@ -413,7 +421,7 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
                         }
                         w[q] = make_float4(e[0], e[1], e[2], e[3]);
                     }
-                    mbar_arrive(&bars.raw_empty[sr]);                    // (shared-memory reads above are complete: their values are in registers)
+                    raw_read_done(&bars.raw_empty[sr]);
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
                         const int at = t * 8 + (q ^ (t & 7));            // unit q of row t sits at position q ^ (t & 7)

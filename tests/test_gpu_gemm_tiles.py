@@ -114,3 +114,59 @@ def test_fp32_tiles(lib, shape, a_km, b_km, off, pad):
         assert bool((C[:, N:] == 3.0).all())
         out.append(C)
     assert torch.equal(out[0], out[2])
+
+
+def test_products_side_by_side_give_the_bits_of_products_alone(lib):
+    """The products of a rank-256 range finder for two matrices on two streams, kernels of both on the same SMs: every product as when it
+    ran alone, bit for bit.  Both orientations of A through the FP16 raw slots, Gram and panel products between them."""
+    m, n, k = 4096, 4800, 256
+
+    class Chain:
+        def __init__(self, seed):
+            g = torch.Generator(device="cuda").manual_seed(seed)
+            self.stream = torch.cuda.Stream()
+            self.a, self.omega = torch.randn(m, n, device="cuda", generator=g), torch.randn(k, m, device="cuda", generator=g)
+            self.qn, self.qm = torch.randn(n, k, device="cuda", generator=g) / n ** 0.5, torch.randn(m, k, device="cuda", generator=g) / m ** 0.5
+            self.t = torch.randn(k, k, device="cuda", generator=g).triu() / 16
+            self.bound = self.a.abs().max().view(torch.int32).reshape(1).clone()
+            self.ws, self.status = torch.empty(160 << 20, dtype=torch.uint8, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
+            self.out = [torch.empty(*shape, device="cuda") for shape in ((n, k), (k, k), (n, k), (m, k), (k, k), (m, k), (n, k))]
+            self.wrong = torch.zeros(len(self.out), dtype=torch.int64, device="cuda")
+
+        def product(self, a_km, b_km, A, B, C, M, N, K, bounded):
+            tail = (self.bound.data_ptr() if bounded else 1, self.status.data_ptr(), self.stream.cuda_stream)
+            call = lib.bsq_gemm_bounded if bounded else lib.bsq_gemm
+            assert call(a_km, b_km, A.data_ptr(), A.shape[1], B.data_ptr(), B.shape[1], C.data_ptr(), N, M, N, K, self.ws.data_ptr(), self.ws.numel(), *tail) == 0
+
+        def run(self):
+            y, gy, qy, z, gz, qz, w = self.out
+            self.product(0, 1, self.a, self.omega, y, n, k, m, True)
+            self.product(0, 0, y, y, gy, k, k, n, False)
+            self.product(1, 0, y, self.t, qy, n, k, k, False)
+            self.product(1, 0, self.a, self.qn, z, m, k, n, True)
+            self.product(0, 0, z, z, gz, k, k, m, False)
+            self.product(1, 0, z, self.t, qz, m, k, k, False)
+            self.product(0, 0, self.a, self.qm, w, n, k, m, True)
+
+        def check(self):
+            with torch.cuda.stream(self.stream):
+                self.wrong += torch.stack([(o != r).any() for o, r in zip(self.out, self.want)])
+                for o in self.out:
+                    o.fill_(float("nan"))
+    chains = [Chain(1), Chain(2)]
+    torch.cuda.synchronize()
+    for c in chains:
+        c.run()
+        torch.cuda.synchronize()
+        c.want = [o.clone() for o in c.out]
+        assert bool(((c.out[3].double() - c.a.double() @ c.qn.double()).abs() <= 4e-6 * (c.a.double().abs() @ c.qn.double().abs())).all())
+    for i in range(150):
+        for c in chains:
+            c.run()
+        for c in chains:
+            c.check()
+        if i % 8 == 7:
+            torch.cuda.synchronize()
+    torch.cuda.synchronize()
+    for c in chains:
+        assert c.wrong.tolist() == [0] * len(c.out) and int(c.status[0]) == 0

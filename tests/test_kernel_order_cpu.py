@@ -82,3 +82,11 @@ def test_inputs_of_chained_kernels_are_read_behind_the_wait(name):
     before = body[1: body.index("chain_begin()")]
     assert before.count("{") == before.count("}")                # not in a branch
     assert not re.search(r"\b(?:if|for|while)\s*\(|__syncthreads|cluster\.sync\(\)", before)
+
+
+def test_raw_slots_are_handed_back_behind_a_proxy_fence():
+    """A copy into shared memory is not ordered behind another thread's reads by that thread's arrival on an mbarrier alone."""
+    text = dict(sources())["bsq_gemm_tma.cu"]
+    assert not re.search(r"mbar_arrive\(&bars\.raw_empty", text) and text.count("raw_read_done(&bars.raw_empty") == 3
+    done = block(text, text.index("void raw_read_done"))
+    assert 0 <= done.find("fence_proxy_async_smem()") < done.find("mbar_arrive(")
