@@ -601,9 +601,13 @@ __global__ void __launch_bounds__(kCholThreads, 1) cholesky_kernel(const float *
     }
     if (role == 0) cholesky_factor(G, k, R, T, together ? sync : nullptr);
     else cholesky_inverse_row(role - 1, k, R, T, together ? sync : nullptr, status);
-    if (together && threadIdx.x == 0) {
+    if (!together) return;
+    // The factor's last row is still on its way out when this thread gets here: if the other CTAs have given up on it, this CTA is the last
+    // to leave, and a row announced behind the clearing would stand as the next launch's.
+    __syncthreads();
+    if (threadIdx.x == 0) {
         __threadfence();
-        if (atomicAdd(&sync->done, 1u) + 1 == gridDim.x) {               // everybody has read what is cleared here
+        if (atomicAdd(&sync->done, 1u) + 1 == gridDim.x) {               // everybody has read, and written, what is cleared here
             sync->ticket = 0;
             sync->rows = 0;
             sync->done = 0;

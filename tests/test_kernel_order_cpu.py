@@ -90,3 +90,11 @@ def test_raw_slots_are_handed_back_behind_a_proxy_fence():
     assert not re.search(r"mbar_arrive\(&bars\.raw_empty", text) and text.count("raw_read_done(&bars.raw_empty") == 3
     done = block(text, text.index("void raw_read_done"))
     assert 0 <= done.find("fence_proxy_async_smem()") < done.find("mbar_arrive(")
+
+
+def test_cholesky_announces_every_row_before_it_counts_itself_out():
+    """CholeskySync has to be zero between launches also behind a wait that ran out: the warp that announces the last row and the thread
+    that clears the words are different ones."""
+    body = KERNELS["cholesky_kernel"][1]
+    work, count = body.index("cholesky_factor("), body.index("atomicAdd(&sync->done")
+    assert re.search(r"(?m)^    __syncthreads\(\);", body[work: count])
