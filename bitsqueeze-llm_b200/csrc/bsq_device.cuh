@@ -165,19 +165,21 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity
     return false;
 }
 
-// For kernels that may be launched while the one before them still runs (launch_chained): waits until that one is done and its stores are
-// visible, then lets the next one's CTAs come.  A no-op in kernels launched the ordinary way.
+// For kernels that may be launched before the one in front of them is done (launch_chained): waits until that one is done and its stores
+// are visible.  A no-op in kernels launched the ordinary way.
 //   * Outside every branch, and nothing in memory is read or written before it.
 //   * What the kernel before may write comes in through plain pointers: `const` with __restrict__, or __ldg, says that nobody writes the
 //     data while the kernel runs -- which is not so while it waits -- and lets loads move in front of the wait.  (The caller's matrix in
 //     the front end is read that way: the encoder comes behind the selection, the selection behind a memset.)
-__device__ __forceinline__ void chain_begin() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-// Launches a kernel that begins with chain_begin(): its CTAs may take their places while the kernel before it in the stream runs, which
-// hides the launch: compress and decompress of 777 x 1031 at rank 48 (54 kernels) 0.642 -> 0.545 ms, 2048 x 5120 at rank 64 1.044 -> 0.969 ms,
-// 8192 x 4096 at rank 256 2.979 -> 2.905 ms.  chained: false keeps the ordinary order (where other streams want the SMs that waiting CTAs would hold).
+//   * No kernel lets the next one's CTAs come early (griddepcontrol.launch_dependents): they come as its own CTAs leave, into places that
+//     are free anyway.  Let in at the start they waited on their SMs for as long as the kernel ran, up to 1.1 ms of a core's SVD, and kept
+//     other streams' kernels out.  Compress calls, ms, let in at the start / when CTAs leave / ordinary launches: four of 2048 x 4096 at rank 256
+//     5.38 / 3.18 / 3.30, eight of 4096 x 4096 11.2 / 5.20 / 5.27, two of 8192 x 4096 at rank 128 1.77 / 1.60 / 1.70; one at a time: below.
+__device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Launches a kernel that begins with chain_begin(): its launch is worked out, and its CTAs take their places, while the last CTAs of the
+// kernel before leave.  One compress call, ordinary launches / CTAs let in at the start / as it is, us: 777 x 1031 at rank 48 553 / 458 / 447,
+// 2048 x 5120 at rank 64 912 / 828 / 822, 8192 x 4096 at rank 128 1323 / 1310 / 1249, at rank 256 2800 / 2745 / 2685, 1501 x 3001 with
+// lists 74 / 66 / 66.  chained: false keeps the ordinary order.
 template <class... P, class... A>
 cudaError_t launch_chained(bool chained, void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
     cudaLaunchConfig_t cfg = {};
