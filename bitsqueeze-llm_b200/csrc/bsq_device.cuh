@@ -179,9 +179,10 @@ __device__ __forceinline__ void chain_begin() { asm volatile("griddepcontrol.wai
 // Launches a kernel that begins with chain_begin(): its launch is worked out, and its CTAs take their places, while the last CTAs of the
 // kernel before leave.  One compress call, ordinary launches / CTAs let in at the start / as it is, us: 777 x 1031 at rank 48 553 / 458 / 447,
 // 2048 x 5120 at rank 64 912 / 828 / 822, 8192 x 4096 at rank 128 1323 / 1310 / 1249, at rank 256 2800 / 2745 / 2685, 1501 x 3001 with
-// lists 74 / 66 / 66.  chained: false keeps the ordinary order.
+// lists 74 / 66 / 66.  Side by side no worse in any setting, so there is no rule on when: eight calls of 4096 x 14336 at rank 256 10.0 ms with
+// ordinary launches and as it is, two of 2048 x 2048 NF4_DQ 75.6 / 67.0 us, four of 4096 x 4096 175 / 171.
 template <class... P, class... A>
-cudaError_t launch_chained(bool chained, void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
+cudaError_t launch_chained(void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     cfg.gridDim = grid;
@@ -191,7 +192,7 @@ cudaError_t launch_chained(bool chained, void (*fn)(P...), dim3 grid, dim3 block
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = chained ? 1 : 0;
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
 }
 

@@ -296,9 +296,7 @@ cudaError_t launch_front(int method, const float *d_in, uint32_t rows, uint32_t 
     if (events) cudaEventRecord(events[1], stream);
     err = persistent_grid(frontend_encode_kernel<G>, f2.threads, f2.smem, sm_count, rows, f2.groups, &grid);
     if (err != cudaSuccess) return err;
-    // chained only where its waiting CTAs leave the device to others: with a grid that fills it, two matrices of 4096 x 4096 on two
-    // lanes took 39 us each, in the ordinary order 32
-    err = launch_chained(grid <= (unsigned)sm_count, frontend_encode_kernel<G>, grid, f2.threads, f2.smem, stream, d_in, rows, cols, k, d_idx, absmax, gmax, d_dq,
+    err = launch_chained(frontend_encode_kernel<G>, grid, f2.threads, f2.smem, stream, d_in, rows, cols, k, d_idx, absmax, gmax, d_dq,
                          d_scale_codes, d_data, gmax + 2);
     if (events) cudaEventRecord(events[2], stream);
     return err;

@@ -176,10 +176,10 @@ template <bool A_KMAJOR, bool B_KMAJOR, int TM, int TN, int kStages>
 void launch_fp32(const GemmArgs &g, cudaStream_t stream) {
     const bool va = reinterpret_cast<uintptr_t>(g.A) % 16 == 0 && g.lda % 4 == 0, vb = reinterpret_cast<uintptr_t>(g.B) % 16 == 0 && g.ldb % 4 == 0;
     const dim3 grid((g.N + TN - 1) / TN, (g.M + TM - 1) / TM, g.splits);
-    if (va && vb) launch_chained(g.chained, gemm_kernel<A_KMAJOR, B_KMAJOR, TM, TN, kStages, true, true>, grid, GT, 0, stream, g);
-    else if (va) launch_chained(g.chained, gemm_kernel<A_KMAJOR, B_KMAJOR, TM, TN, kStages, true, false>, grid, GT, 0, stream, g);
-    else if (vb) launch_chained(g.chained, gemm_kernel<A_KMAJOR, B_KMAJOR, TM, TN, kStages, false, true>, grid, GT, 0, stream, g);
-    else launch_chained(g.chained, gemm_kernel<A_KMAJOR, B_KMAJOR, TM, TN, kStages, false, false>, grid, GT, 0, stream, g);
+    if (va && vb) launch_chained(gemm_kernel<A_KMAJOR, B_KMAJOR, TM, TN, kStages, true, true>, grid, GT, 0, stream, g);
+    else if (va) launch_chained(gemm_kernel<A_KMAJOR, B_KMAJOR, TM, TN, kStages, true, false>, grid, GT, 0, stream, g);
+    else if (vb) launch_chained(gemm_kernel<A_KMAJOR, B_KMAJOR, TM, TN, kStages, false, true>, grid, GT, 0, stream, g);
+    else launch_chained(gemm_kernel<A_KMAJOR, B_KMAJOR, TM, TN, kStages, false, false>, grid, GT, 0, stream, g);
 }
 // Tiles: 128 columns unless there are at most 64; 64 rows where there are no more, or where 128 leave the device idle.  What bounds a
 // small product is the way of its few steps from memory: copies that are waited for one by one and 128 x 128 tiles for everything took
@@ -234,12 +234,12 @@ __global__ void __launch_bounds__(256) reduce_splits_kernel(const float *part, f
 }
 
 cudaError_t launch_reduce(const float *workspace, float *C, int M, int N, long ldc, int splits, int sm_count,
-                          cudaStream_t stream, bool chained) {
+                          cudaStream_t stream) {
     const size_t total = (size_t)M * N;                      // (K is only split for fewer tiles than the device has slots: a few million elements)
     const bool aligned = ((reinterpret_cast<uintptr_t>(workspace) | reinterpret_cast<uintptr_t>(C)) & 15) == 0 && N % 4 == 0 && ldc % 4 == 0;
     if (aligned && total >= (size_t)sm_count * 1024)
-        return launch_chained(chained, reduce_splits_kernel<4>, (unsigned)((total / 4 + 255) / 256), 256, 0, stream, workspace, C, (unsigned)total, N, ldc, splits, total);
-    return launch_chained(chained, reduce_splits_kernel<1>, (unsigned)((total + 255) / 256), 256, 0, stream, workspace, C, (unsigned)total, N, ldc, splits, total);
+        return launch_chained(reduce_splits_kernel<4>, (unsigned)((total / 4 + 255) / 256), 256, 0, stream, workspace, C, (unsigned)total, N, ldc, splits, total);
+    return launch_chained(reduce_splits_kernel<1>, (unsigned)((total + 255) / 256), 256, 0, stream, workspace, C, (unsigned)total, N, ldc, splits, total);
 }
 
 // BSQ_GEMM_IMAGE=0 keeps the tensor-core kernel that splits B inside every CTA, =2 uses the kernel with B split
@@ -307,7 +307,6 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
                         unsigned *flag, unsigned *status, float *workspace, size_t workspace_bytes, int sm_count,
                         cudaStream_t stream, const unsigned *a_absmax_bits, float b_bound, bool device_full) {
     if (M <= 0 || N <= 0 || K <= 0) return cudaErrorInvalidValue;
-    const bool chained = !device_full;
     if (allow_tensor_cores) {
         // tensor-core path: one 128-row tile per CTA, two CTAs per SM up to N = 128; K is split so that the tiles fill
         // the SMs once
@@ -317,7 +316,6 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
         // N up to 256 is one tile; wider products (the reconstruction) are cut into 128-column tiles
         t.n_tile = N <= 256 ? N : 128;
         t.flag = minuend ? flag : nullptr;
-        t.chained = chained;
         // B split beforehand when several row tiles share it and the workspace has room for its images (at its end)
         const size_t image_bytes = gemm_tc_image_bytes(N, t.n_tile, K);
         // (measured: the products are then bound by what the CTAs draw from L2, A once and B's images once per row
@@ -425,7 +423,7 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
         if (gemm_tc_eligible(t, a_kmajor, b_kmajor)) {
             cudaError_t err = gemm_tc_launch(t, a_kmajor, b_kmajor, status, stream);
             if (err != cudaSuccess || t.splits == 1) return err;
-            return launch_reduce(workspace, C, M, N, ldc, t.splits, sm_count, stream, t.chained);
+            return launch_reduce(workspace, C, M, N, ldc, t.splits, sm_count, stream);
         }
     }
     const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
@@ -439,7 +437,6 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
     GemmArgs g{};
     g.A = A; g.B = B; g.M = M; g.N = N; g.K = K; g.lda = lda; g.ldb = ldb;
     g.kscale = kscale;
-    g.chained = chained;
     g.splits = splits;
     g.k_per_split = ((K + splits - 1) / splits + BK - 1) / BK * BK;
     g.minuend = minuend; g.ldm = ldm; g.flag = minuend ? flag : nullptr;
@@ -454,7 +451,7 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
     else launch_fp32<false, false>(g, sm_count, stream);
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess || splits == 1) return err;
-    return launch_reduce(workspace, C, M, N, ldc, splits, sm_count, stream, g.chained);
+    return launch_reduce(workspace, C, M, N, ldc, splits, sm_count, stream);
 }
 
 }  // namespace bsq

@@ -41,7 +41,6 @@ struct GemmArgs {
     bool lo_unscaled;              // the low halves are fp16(x s - hi) without the factor 2^11, so that all three products of a
                                    // term can share ONE accumulator (the persistent product's 256-column tiles); elements more
                                    // than 2^18 below the operand's largest then lose bits of their low half
-    bool chained = false;               // its kernels may come while the one before still runs
 };
 
 // Tensor-core path: true if the shape qualifies (N a multiple of 16, 16-byte aligned operands with leading

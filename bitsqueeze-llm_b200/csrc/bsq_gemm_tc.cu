@@ -766,7 +766,7 @@ cudaError_t launch(const GemmArgs &g, unsigned *status, cudaStream_t stream) {
     cudaError_t err = cudaFuncSetAttribute(gemm_tc_kernel<AK, BK, NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     dim3 grid((g.M + TM - 1) / TM, (g.N + g.n_tile - 1) / g.n_tile, g.splits);
-    return launch_chained(g.chained, gemm_tc_kernel<AK, BK, NMAX>, grid, NT, smem, stream, g, status);
+    return launch_chained(gemm_tc_kernel<AK, BK, NMAX>, grid, NT, smem, stream, g, status);
 }
 
 // Ring lengths of the image kernel for a tile of N columns: two stages of A and four images of B (two chunks of head
@@ -805,10 +805,10 @@ cudaError_t launch_image(const GemmArgs &g, bool b_kmajor, unsigned *status, cud
         }
         uint4 *image16 = reinterpret_cast<uint4 *>(image);
         const float lo_scale = g.lo_unscaled ? 1.0f : kSplit16LoScale;
-        if (b_kmajor) launch_chained(g.chained, presplit_b16_kernel<true>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image16, bmax, g.b_scale_fixed, lo_scale);
-        else launch_chained(g.chained, presplit_b16_kernel<false>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image16, bmax, g.b_scale_fixed, lo_scale);
-    } else if (b_kmajor) launch_chained(g.chained, presplit_b_kernel<true>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image);
-    else launch_chained(g.chained, presplit_b_kernel<false>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image);
+        if (b_kmajor) launch_chained(presplit_b16_kernel<true>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image16, bmax, g.b_scale_fixed, lo_scale);
+        else launch_chained(presplit_b16_kernel<false>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image16, bmax, g.b_scale_fixed, lo_scale);
+    } else if (b_kmajor) launch_chained(presplit_b_kernel<true>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image);
+    else launch_chained(presplit_b_kernel<false>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     if (g.use_tma && g.a_image && g.f16) {
@@ -830,7 +830,7 @@ cudaError_t launch_image(const GemmArgs &g, bool b_kmajor, unsigned *status, cud
     err = cudaFuncSetAttribute(gemm_tc_image_kernel<AK, NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
     dim3 grid((g.M + TM - 1) / TM, n_tiles, g.splits);
-    return launch_chained(g.chained, gemm_tc_image_kernel<AK, NMAX>, grid, NT2, smem, stream, g, status);
+    return launch_chained(gemm_tc_image_kernel<AK, NMAX>, grid, NT2, smem, stream, g, status);
 }
 
 }  // namespace

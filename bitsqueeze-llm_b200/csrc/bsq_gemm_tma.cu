@@ -616,7 +616,7 @@ template <bool AK, int NMAX, bool F16 = false>
 cudaError_t launch_tma(const CUtensorMap &map, const GemmArgs &g, dim3 grid, size_t smem, unsigned *status, cudaStream_t stream) {
     cudaError_t err = cudaFuncSetAttribute(gemm_tc_tma_kernel<AK, NMAX, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
-    return launch_chained(g.chained, gemm_tc_tma_kernel<AK, NMAX, F16>, grid, NTH, smem, stream, map, g, status);
+    return launch_chained(gemm_tc_tma_kernel<AK, NMAX, F16>, grid, NTH, smem, stream, map, g, status);
 }
 
 }  // namespace

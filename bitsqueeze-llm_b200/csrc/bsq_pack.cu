@@ -186,7 +186,7 @@ cudaError_t pack_object(const CopySegment *segments, int count, const PackHeader
     if (count < 0 || count > kMaxCopySegments) return cudaErrorInvalidValue;
     CopyArgs c;
     const unsigned ctas = fill(c, segments, count);
-    return launch_chained(true, pack_object_kernel, ctas + 1, kCopyThreads, 0, stream, c, headers, d_status, mirror);
+    return launch_chained(pack_object_kernel, ctas + 1, kCopyThreads, 0, stream, c, headers, d_status, mirror);
 }
 
 cudaError_t fetch_heads(const HeadList &heads, uint8_t *host, unsigned *d_status, cudaStream_t stream) {

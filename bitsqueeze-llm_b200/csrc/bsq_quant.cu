@@ -310,13 +310,13 @@ cudaError_t nf4_quantize(const float *d_x, uint64_t n, float *d_scales, uint8_t 
     const bool vec = aligned(d_x, 16) && aligned(d_data, 4) && (!d_deq_out || aligned(d_deq_out, 16));
     const int grid = grid_for(n, sm_count);
     if (d_deq_out && d_error_flag)
-        return launch_chained(true, encode_flat_kernel<false, kWriteError>, grid, kThreads, 0, stream, d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
+        return launch_chained(encode_flat_kernel<false, kWriteError>, grid, kThreads, 0, stream, d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
                                                                          nullptr, d_data, d_deq_out, d_error_flag);
     else if (d_deq_out)
-        return launch_chained(true, encode_flat_kernel<false, kWriteDeq>, grid, kThreads, 0, stream, d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
+        return launch_chained(encode_flat_kernel<false, kWriteDeq>, grid, kThreads, 0, stream, d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
                                                                          nullptr, d_data, d_deq_out, nullptr);
     else
-        return launch_chained(true, encode_flat_kernel<false, kWriteNone>, grid, kThreads, 0, stream, d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
+        return launch_chained(encode_flat_kernel<false, kWriteNone>, grid, kThreads, 0, stream, d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
                                                                           nullptr, d_data, nullptr, nullptr);
 }
 
@@ -334,13 +334,13 @@ cudaError_t nf4dq_quantize(const float *d_x, uint64_t n, float *d_dq, uint8_t *d
     absmax_flat_kernel<<<grid, kThreads, 0, stream>>>(d_x, n, vec, absmax, gmax);
     if ((err = cudaGetLastError()) != cudaSuccess) return err;
     if (d_deq_out && d_error_flag)
-        return launch_chained(true, encode_flat_kernel<true, kWriteError>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
+        return launch_chained(encode_flat_kernel<true, kWriteError>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
                                                                         d_dq, d_data, d_deq_out, d_error_flag);
     else if (d_deq_out)
-        return launch_chained(true, encode_flat_kernel<true, kWriteDeq>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
+        return launch_chained(encode_flat_kernel<true, kWriteDeq>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
                                                                         d_dq, d_data, d_deq_out, nullptr);
     else
-        return launch_chained(true, encode_flat_kernel<true, kWriteNone>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
+        return launch_chained(encode_flat_kernel<true, kWriteNone>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
                                                                          d_dq, d_data, nullptr, nullptr);
 }
 

@@ -445,7 +445,7 @@ cudaError_t orthonormalise(SvdWorkspace *ws, float *Y, float *tmp, int rows, int
             float *r_out = pass == 0 ? r_a : r_b;
             if (!r_out) r_out = ws->rfac;
             const auto launch = [&](CholeskyPart part) {
-                launch_chained(!ws->device_full, cholesky_kernel, cholesky_grid(k, part), kCholThreads, cholesky_blocked_smem_bytes(k), st,
+                launch_chained(cholesky_kernel, cholesky_grid(k, part), kCholThreads, cholesky_blocked_smem_bytes(k), st,
                                ws->g, k, r_out, factor_only ? nullptr : ws->t, ws->chol_sync, ws->status, part);
             };
             if (factor_only || ws->device_full) {
@@ -734,7 +734,7 @@ cudaError_t svd_lowrank(SvdWorkspace *ws, const float *d_A, float *d_U, float *d
     } else if (ws->own_core_svd) {
         // eight lanes per pair and no more: warps without a pair only make a round's barrier longer (k = 64: 301 -> 290 us)
         const int threads = std::max(1, ((k + 1) / 2 * 8 + 31) / 32) * 32;
-        if ((err = launch_chained(!ws->device_full, jacobi_svd_kernel, 1, threads, jacobi_smem_bytes(k), st, ws->core, k, d_S, ws->vc, ws->uc)) != cudaSuccess)
+        if ((err = launch_chained(jacobi_svd_kernel, 1, threads, jacobi_smem_bytes(k), st, ws->core, k, d_S, ws->vc, ws->uc)) != cudaSuccess)
             return err;
     } else if (cusolverDnSgesvdj(ws->solver, CUSOLVER_EIG_MODE_VECTOR, 0, k, k, ws->core, k, d_S, ws->vc, k, ws->uc, k,
                                  ws->solver_work, ws->lwork, ws->dev_info, ws->svdj) != CUSOLVER_STATUS_SUCCESS) {

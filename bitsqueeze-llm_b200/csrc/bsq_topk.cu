@@ -360,7 +360,7 @@ static cudaError_t launch_group(const float *d_in, float *d_residual, uint32_t r
     unsigned grid = (unsigned)sm_count * (unsigned)per_sm;
     const unsigned needed = (rows + f.groups - 1) / f.groups;
     if (grid > needed) grid = needed;
-    return launch_chained(true, topk_rows_group_kernel<G, kBulk>, grid, f.threads, smem, stream, d_in, d_residual, rows, cols, k, d_idx, d_val, d_status,
+    return launch_chained(topk_rows_group_kernel<G, kBulk>, grid, f.threads, smem, stream, d_in, d_residual, rows, cols, k, d_idx, d_val, d_status,
                           f.group_bytes, f.ctl_off, d_bound);
 }
 
