@@ -266,6 +266,7 @@ __global__ void __launch_bounds__(ring_max_threads(kLen), 1) ring_jacobi_kernel(
     unsigned it = 0;                                          // rounds so far
     int vote = 1, sp_last = 0;                                // bit 0: a pair above kJacobiLastSweepCos in the last sweep, bit 1: a wait ran out
     bool failed = false;                                      // a wait ran out: stop sending and waiting, finish quickly
+    unsigned failed_at = 0;                                   // ... in this round
     const int own_slot = w * kS + own;
     for (int sweep = 0;; ++sweep) {
         // exact squared norms (in between they are carried along through the rotations), into every CTA, with the votes
@@ -430,6 +431,7 @@ __global__ void __launch_bounds__(ring_max_threads(kLen), 1) ring_jacobi_kernel(
                         failed = __any_sync(kFullMask, !mbar_wait_bounded(&mbar[2 + par], phase, status));
                         if (lane == 0 && !failed) mbar_expect_tx(&mbar[2 + par], kTx);
                     }
+                    if (failed && failed_at == 0) failed_at = it + 1;
                 }
                 take(box_at + par * box_par, P[kS - 1]);
                 take(box_at + par * box_par + kCol * 4, Q[0]);
@@ -476,7 +478,17 @@ __global__ void __launch_bounds__(ring_max_threads(kLen), 1) ring_jacobi_kernel(
                 out(Q[j], col_of(j, 1));
             }
     }
-    if (kCluster) cluster.sync();                             // nobody leaves while a neighbour could still store into it
+    if (kCluster) {
+        // A warp that gave up: the neighbour may have sent the round that was waited for all the same, and the one behind it (not more, since
+        // it got nothing back).  These stores land, or do not come, before this CTA's shared memory goes away.
+        if (failed) {
+            for (unsigned i = failed_at - 1; i <= failed_at; ++i) {
+                if (rem_up) mbar_wait_bounded(&mbar[i & 1], (i >> 1) & 1, status);
+                if (rem_dn) mbar_wait_bounded(&mbar[2 + (i & 1)], (i >> 1) & 1, status);
+            }
+        }
+        cluster.sync();                                       // nobody leaves while a neighbour could still store into it
+    }
 }
 
 typedef void (*RingJacobiFn)(const float *, int, float *, float *, float *, unsigned *);

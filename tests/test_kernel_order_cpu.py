@@ -102,3 +102,11 @@ def test_cholesky_announces_every_row_before_it_counts_itself_out():
     body = KERNELS["cholesky_kernel"][1]
     work, count = body.index("cholesky_factor("), body.index("atomicAdd(&sync->done")
     assert re.search(r"(?m)^    __syncthreads\(\);", body[work: count])
+
+
+def test_ring_waits_for_stores_in_flight_before_it_leaves():
+    """A CTA whose wait for a neighbour's column ran out must not give its shared memory back while that column may still come."""
+    body = KERNELS["ring_jacobi_kernel"][1]
+    leave = body[body.index("float *sv = "):]
+    drain, last = leave.find("if (failed)"), leave.rfind("cluster.sync()")
+    assert 0 <= drain < last and leave[drain: last].count("mbar_wait_bounded(") == 2
