@@ -5,6 +5,11 @@ coded (one CTA up to 48 columns, columns on a ring of warps above, over a cluste
 Bounds.  Each QR pass factors G + 1e-5 max(diag G) I, so columns are orthonormal to a few 1e-5, up to 2e-4 for the weakest
 direction of a wide sketch (the bounds of test_gpu_svd.py).  With orthonormal Q the residual of Q Q^T A has the squared norm
 |A|^2 - sum S^2: both sides are compared to 1e-3 of |A|^2 (twice the orthonormality bound for the two factors, and FP32 sums)."""
+import ctypes as C
+import ctypes.util
+import glob
+import os
+
 import numpy as np
 import pytest
 
@@ -102,3 +107,95 @@ def test_coded_factors_accuracy_against_exact(lib, case):
 
 def test_coded_factors_of_rank_deficient_and_zero_inputs(lib):
     test_gpu_svd.test_svd_rank_deficient_and_zero_inputs(CodedFactors(lib))
+
+
+@pytest.mark.parametrize("k", [49, 53, 54, 57, 62, 70, 101, 150, 197])
+def test_core_of_coded_factors_with_partly_filled_warps(lib, k):
+    """Ranks that leave one, two or three of the last warp's four column pairs empty, on one CTA (49 to 64 columns) and on clusters."""
+    test_core_edges(CodedFactors(lib), k, "noise")
+    test_core_of_deficient_and_zero_matrices(CodedFactors(lib), k)
+
+
+def omega_of(n, k, seed):
+    """The range finder's random matrix, n x k: cuRAND's default sequence, column-major."""
+    found = glob.glob(os.path.join(os.path.dirname(torch.__file__), "..", "nvidia", "curand", "lib", "libcurand.so.10"))
+    rand = C.CDLL(found[0] if found else ctypes.util.find_library("curand") or "libcurand.so.10")
+    gen, count = C.c_void_p(), n * k + (n * k & 1)
+    out = np.empty(count, np.float32)
+    assert rand.curandCreateGeneratorHost(C.byref(gen), 100) == 0
+    assert rand.curandSetPseudoRandomGeneratorSeed(gen, C.c_ulonglong(seed)) == 0
+    assert rand.curandGenerateNormal(gen, C.c_void_p(out.ctypes.data), C.c_size_t(count), C.c_float(0.0), C.c_float(1.0)) == 0
+    rand.curandDestroyGenerator(gen)
+    return out[: n * k].reshape(k, n).T.astype(np.float64)
+
+
+def orthonormalised(y, passes):
+    factors = []
+    for _ in range(passes):
+        g = y.T @ y
+        r = np.linalg.cholesky(g + 1e-5 * g.diagonal().max() * np.eye(len(g))).T
+        y = y @ np.linalg.inv(r)
+        factors.append(r)
+    return y, factors
+
+
+def rotated(m, first_round=0):
+    """One-sided Jacobi of the columns of m in FP64, pairs in the order of the round-robin tournament that the kernels keep: columns, lengths
+    (descending) and how far from a tie the closest decision on a rotation's sense was."""
+    k = m.shape[1]
+    kp, length = (k + 1) & ~1, 64 if k <= 64 else 128 if k <= 128 else 256
+    m, margin = np.hstack([m, np.zeros((len(m), kp - k))]), np.inf
+    for _ in range(30):
+        norm, big = (m * m).sum(0), False
+        for i in range(kp - 1):
+            r, slot = (i + first_round) % (kp - 1), np.arange(1, kp // 2)
+            p, q = np.append(kp - 1, (r + slot) % (kp - 1)), np.append(r, (r + kp - 1 - slot) % (kp - 1))
+            a, b, g = norm[p], norm[q], (m[:, p] * m[:, q]).sum(0)
+            on = (a > 0) & (b > 0) & (g * g > length * 2.0 ** -48 * a * b)
+            p, q, a, b, g = p[on], q[on], a[on], b[on], g[on]
+            if len(p) == 0:
+                continue
+            zeta = (b - a) / (2 * g)
+            margin = min(margin, float((np.abs(b - a) / np.maximum(a, b)).min()))
+            t = np.copysign(1.0, zeta) / (np.abs(zeta) + np.sqrt(1 + zeta * zeta))
+            c = 1 / np.sqrt(1 + t * t)
+            m[:, p], m[:, q] = c * m[:, p] - c * t * m[:, q], c * t * m[:, p] + c * m[:, q]
+            norm[p], norm[q] = np.maximum(a - t * g, 0), b + t * g
+            big |= bool((g * g > 1e-8 * a * b).any())
+        if not big:
+            break
+    norm = np.sqrt((m * m).sum(0))
+    order = np.argsort(-norm, kind="stable")[:k]
+    return m[:, order] / norm[order], norm[order], margin
+
+
+def coded_case(k, seed):
+    """A matrix of rank k whose singular values are k distinct ones between 1 and 2, its SVD as the stage works it out, in FP64, and the matrix
+    whose columns the core kernel rotates."""
+    rng = np.random.default_rng(seed)
+    m, n = 2 * k + 64, k + 37
+    left, right = np.linalg.qr(rng.standard_normal((m, k)))[0], np.linalg.qr(rng.standard_normal((n, k)))[0]
+    a = ((left * (2 - np.arange(k) / k)) @ right.T).astype(np.float32)
+    w = a.astype(np.float64)
+    q, _ = orthonormalised(w @ omega_of(n, k, 1241), 1)
+    for it in range(2):
+        z, _ = orthonormalised(w.T @ q, 1)
+        q, _ = orthonormalised(w @ z, 1 + it)
+    _, (r1, r2) = orthonormalised(w.T @ q, 2)
+    return a, q, (r2 @ r1).T
+
+
+
+@pytest.mark.parametrize("k,seed", [(33, 1000), (48, 1002), (49, 1002), (53, 1003), (64, 1003), (65, 1004), (70, 70), (101, 1003)])
+def test_order_of_rotations_of_coded_factors(lib, k, seed):
+    """Codes depend on the sign that each singular pair comes out with, and that on the order of the rotations.  Every pair has the sign that
+    the restated order gives: left vectors within 0.05 of the FP64 ones (a core off by 3e-6 in every element, as FP32 products leave it, moves
+    them by 1e-4, and the seeds are such that no rotation's sense is closer to a tie than 1e-4).  Begun one round later the order gives 9 to 42
+    other signs.  Up to 101 columns: beyond, a core that far off takes other senses."""
+    a, q, core = coded_case(k, seed)
+    vec, s, margin = rotated(core.copy())
+    assert margin > 1e-4
+    assert ((vec * rotated(core.copy(), 1)[0]).sum(0) < 0).any()
+    u, s_gpu, _ = svd_gpu(CodedFactors(lib), a, k)
+    assert np.abs(s_gpu - s).max() <= 1e-4 * s[0]
+    assert (np.abs(u - q @ vec).max(axis=0) <= 0.05).all()

@@ -177,3 +177,58 @@ def test_status_word_set_by_a_stage_fails_the_call(pkg, lib):
     assert pkg.decompress_packed(good[1], d_y.data_ptr(), rows * cols) == 1
     assert pkg.decompress_packed(good[1], d_y.data_ptr(), rows * cols) == 0
     lib.bsq_decompress_release()
+
+
+@pytest.mark.parametrize("cfg", [(2048, 4096, 0.005, 0.01, 256, 2, 11, -1, -1), (1024, 2048, 0.01, 0.01, 128, 1, 10, -1, -1), (1501, 3001, 0.005, 0.01, -1, 1, -1, -1, 11),
+                                 (777, 1031, 0.005, 0.0, 48, 2, -1, -1, -1)])
+def test_objects_and_matrices_do_not_depend_on_the_other_lanes(pkg, lib, cfg):
+    """Two and four matrices in flight, on the lanes of a batch and on lanes begun one by one: object and matrix of every one as when it was
+    alone, bit for bit, each time.  Error lists on: an element of a product that is off in its last bits shows in them."""
+    rows, cols = cfg[0], cfg[1]
+    batch = lib.bsq_batch_create(*cfg, 4)
+    assert batch
+    lanes = [lib.bsq_batch_lane(batch, i) for i in range(4)]
+    cap = int(lib.bsq_lane_packed_capacity(lanes[0]))
+    mats = [torch.from_numpy(matrix_for(cfg, i)).cuda() for i in range(4)]
+    bufs = [torch.zeros(cap, dtype=torch.uint8, device="cuda") for _ in mats]
+    outs = [torch.zeros(rows, cols, device="cuda") for _ in mats]
+    headers, sizes = (pkg.Array * 4)(), (C.c_uint64 * 4)()
+    vp = C.c_void_p * 4
+    pointers = vp(*[C.addressof(h) for h in headers])
+
+    def size_of(i):
+        return C.pointer(C.c_uint64.from_buffer(sizes, 8 * i))
+
+    def compress(count, one_by_one):
+        if not one_by_one:
+            assert lib.bsq_batch_compress(batch, vp(*[m.data_ptr() for m in mats]), count, 1, vp(*[b.data_ptr() for b in bufs]), cap, None, headers, sizes) == 0
+            assert lib.bsq_batch_decompress(batch, pointers, count, 1, vp(*[o.data_ptr() for o in outs]), rows * cols) == 0
+            return
+        for i in range(count):
+            assert lib.bsq_lane_compress_begin(lanes[i], mats[i].data_ptr(), 1, bufs[i].data_ptr(), cap) == 0
+        for i in range(count):
+            assert lib.bsq_lane_compress_end(lanes[i], None, C.byref(headers[i]), size_of(i)) == 0
+        for i in range(count):
+            assert lib.bsq_lane_decompress_begin(lanes[i], C.byref(headers[i]), 1, outs[i].data_ptr(), rows * cols) == 0
+        for i in range(count):
+            assert lib.bsq_lane_decompress_end(lanes[i]) == 0
+    try:
+        torch.cuda.synchronize()
+        want = []
+        for i in range(4):
+            assert lib.bsq_lane_compress_begin(lanes[i], mats[i].data_ptr(), 1, bufs[i].data_ptr(), cap) == 0
+            assert lib.bsq_lane_compress_end(lanes[i], None, C.byref(headers[i]), size_of(i)) == 0
+            assert lib.bsq_lane_decompress_begin(lanes[i], C.byref(headers[i]), 1, outs[i].data_ptr(), rows * cols) == 0
+            assert lib.bsq_lane_decompress_end(lanes[i]) == 0
+            want.append((bufs[i][200: int(sizes[i])].clone(), outs[i].clone()))
+        for count in (2, 4):
+            for trial in range(24):
+                torch.cuda.synchronize()
+                compress(count, trial % 2 == 1)
+                for i in range(count):
+                    assert torch.equal(bufs[i][200: int(sizes[i])], want[i][0]), (count, trial, i)
+                    assert torch.equal(outs[i].view(torch.int32), want[i][1].view(torch.int32)), (count, trial, i)
+                    bufs[i].zero_()
+                    outs[i].zero_()
+    finally:
+        lib.bsq_batch_destroy(batch)
