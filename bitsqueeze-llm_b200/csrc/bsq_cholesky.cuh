@@ -12,12 +12,12 @@
 //     subnormal arguments and stores to global memory in between: 230).
 //   * The block row is a forward substitution right behind the pivots, eight at a time (named barriers), the block of the next
 //     pivots is updated right behind that, and all other updates run beside the chain.  From about 200 columns on those are
-//     what an SM's multiply-adds take: 53 us at 256 columns for 8 blocks, 17 us at 128 for 4.
+//     what an SM's multiply-adds take: 53 us at 256 columns for 8 blocks, 16 us at 128 for 4.
 //   * R and the inverses of its diagonal blocks go out block row by block row, and other CTAs make the rows of the inverse
 //     from them while the factor goes on: T_IJ = -(sum_{L=I..J-1} T_IL R_LJ) T_JJ from left to right.
 // Every value is the same sum in the same order whatever the number of CTAs or launches.  Back to back, factor and inverse, against the
-// two kernels (one CTA; one per block row) and, up to 64 columns, the single CTA that did this before: k = 256 64 against 99 us,
-// 192 41 / 67, 128 25 / 41, 64 14.6 / 18.7, 32 6.5 / 10.5; the factor alone 53 / 79 us at 256, 17 / 30 us at 128.
+// two kernels (one CTA; one per block row) and, up to 64 columns, the single CTA that did this before, ordinary launches: k = 256 63 against
+// 99 us, 192 41 / 67, 128 25 / 41, 64 15 / 18.7, 32 7 / 10.5; the factor alone 53 / 79 us at 256, 16.4 / 30 us at 128.
 #pragma once
 
 #include "bsq_device.cuh"
@@ -582,8 +582,8 @@ __device__ __forceinline__ void cholesky_inverse_row(int I, int k, const float *
 
 // What a launch does.  kCholBoth: the CTA that starts first factors, the others follow with the rows of the inverse: the shortest
 // time for one matrix.  kCholFactor (and the diagonal blocks of T if T is given), then kCholInverse: nobody waits for anybody, which is
-// less time of all SMs together where other work wants them (k = 256: 64 us on 8 SMs against 54 us on 1 and 28 us on 7; eight compress and
-// decompress calls of 4096 x 14336 side by side 11.88 ms in two launches, 12.05 ms in one).
+// less time of all SMs together where other work wants them (k = 256: 63 us on 8 SMs against 57 us on 1 and 23 us on 7; six compress calls of
+// 8192 x 4096 side by side 5.31 ms in two launches, 5.34 in one, eight of 4096 x 14336 9.97 and 9.96).
 enum CholeskyPart { kCholBoth, kCholFactor, kCholInverse };
 __host__ __device__ constexpr int cholesky_grid(int k, CholeskyPart part) {
     return part == kCholFactor || chol_blocks(k) == 1 ? 1 : chol_blocks(k) - (part == kCholInverse ? 1 : 0);

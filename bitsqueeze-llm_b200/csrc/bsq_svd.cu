@@ -17,7 +17,7 @@
 //   * the small SVD works on a k x k core: B^T = Q2 C with C = R2 R1 the product of the two
 //     triangular factors, C = Uc S Vc^T, V_hat = Q2 Uc, U = Q Vc.
 // The SVD of the k x k core is a one-sided Jacobi kernel of this library up to 256 columns (bsq_jacobi.cuh; where the factors
-// are coded afterwards bsq_ring_jacobi.cuh, below 48 columns the one-CTA kernel here); larger cores, and devices that cannot place the cluster, go to cuSOLVER's gesvdj on
+// are coded afterwards bsq_ring_jacobi.cuh, up to 48 columns the one-CTA kernel here); larger cores, and devices that cannot place the cluster, go to cuSOLVER's gesvdj on
 // the k x k core.  Everything that touches an M- or N-sized array is a kernel of this library.
 // Omega comes from cuRAND's XORWOW generator like the reference's (svd_lowrank_cuda.cu:143,289-291),
 // seeded per call, column-major N x k.
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(256, 1) jacobi_svd_kernel(const float *C, int 
     float *M = sm, *V = M + (size_t)kp * LEN, *nrm = V + (size_t)kp * LEN;
     int *rank_of = reinterpret_cast<int *>(nrm + kp);
     const int tid = threadIdx.x, nt = blockDim.x;
-    const int slot = tid >> 3, l = tid & 7;                   // 8 lanes per pair, 64 pair slots
+    const int slot = tid >> 3, l = tid & 7;                   // 8 lanes per pair, up to 24 pairs
     constexpr int F4 = LEN / 32;                              // float4 per lane and column
     for (int e0 = tid; e0 < kp * LEN; e0 += 4 * nt) {        // four global loads in flight per thread
         float v[4];
