@@ -240,6 +240,7 @@ struct Runtime {
     TopkBufs outlier, err;
     SvdWorkspace *svd = nullptr;
     unsigned *h_status = nullptr;                        // pinned mirror of the device status words
+    bool words_clear = false;                            // the device status words are zero: the kernel that ended the last call has left them so
     uint8_t *h_stage = nullptr;                          // pinned: section headers of a device-resident object on their way in
     DevicePack pack;
     CompressJob job;
@@ -509,13 +510,14 @@ bool emit_topk_section(Runtime &rt, const CompressJob &job, const TopkBufs &t, u
 
 // Quantise `d_src` (n elements) into q; d_deq (nullable, may alias d_src) receives the dequantised values, or, with
 // d_error_flag, what they are off by.
-bool run_quantize(Runtime &rt, int method, const float *d_src, QuantBufs &q, float *d_deq, unsigned *d_error_flag = nullptr) {
+// max_word: the status word that takes an NF4_DQ section's largest magnitude.
+bool run_quantize(Runtime &rt, int method, const float *d_src, QuantBufs &q, int max_word, float *d_deq, unsigned *d_error_flag = nullptr) {
     cudaError_t err;
     if (method == NF4)
         err = nf4_quantize(d_src, q.n, q.scales_f32.as<float>(), q.data.as<uint8_t>(), d_deq, rt.sm_count, rt.stream, d_error_flag);
     else
         err = nf4dq_quantize(d_src, q.n, q.dq.as<float>(), q.scale_codes.as<uint8_t>(), q.data.as<uint8_t>(), d_deq,
-                             rt.scratch.p, rt.sm_count, rt.stream, d_error_flag);
+                             rt.scratch.p, rt.sm_count, rt.stream, d_error_flag, rt.status.as<unsigned>() + max_word);
     return err == cudaSuccess;
 }
 
@@ -609,7 +611,7 @@ int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_p
     const uint32_t ko = rt.outlier.k, ke = rt.err.k;
     const uint32_t rank = (uint32_t)rt.rank;
     cudaStream_t st = rt.stream;
-    unsigned *d_status = rt.status.as<unsigned>();      // [0] kernel status bits, [1] error-nonzero flag
+    unsigned *d_status = rt.status.as<unsigned>();
     if (input_location == BITSQZ_LLM_INPUT_HOST && !rt.input_stage.p) return 1;
 
     job.total = plan_sections(rt, job);
@@ -641,7 +643,8 @@ int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_p
     job.prof = want_profile;
     auto mark = [&]() { if (job.prof && job.nev < 8) cudaEventRecord(rt.ev[job.nev++], st); };
 
-    if (cudaMemsetAsync(d_status, 0, 64, st) != cudaSuccess) return fail();
+    if (!rt.words_clear && cudaMemsetAsync(d_status, 0, 4 * kStatusWords, st) != cudaSuccess) return fail();
+    rt.words_clear = false;
     if (rt.inject_status) {                                             // test hook: as if a kernel had reported these bits
         rt.h_status[8] = rt.inject_status;
         rt.inject_status = 0;
@@ -657,19 +660,19 @@ int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_p
     // ---- stages ----
     const float *d_src = d_input;          // what SVD / the quantiser sees (outliers zeroed)
     bool fused_front = false;
-    bool residual_bound = false;                                        // d_status[8] holds an upper bound of |residual|
+    bool residual_bound = false;                                        // d_status[kWordBound] holds an upper bound of |residual|
     if (!has_svd && rt.q_format != quantization_NONE && ko > 0 && !error_path && frontend_supported(rows, cols, ko) &&
         (reinterpret_cast<uintptr_t>(d_input) % 16) == 0) {
         fused_front = true;
         if (frontend_quantize(rt.q_format, d_input, rows, cols, ko, rt.outlier.idx.as<uint16_t>(), rt.outlier.val.as<float>(),
                               rt.q_direct.scales_f32.as<float>(), rt.q_direct.dq.as<float>(),
                               rt.q_direct.scale_codes.as<uint8_t>(), rt.q_direct.data.as<uint8_t>(), rt.scratch.p, d_status,
-                              rt.sm_count, st) != cudaSuccess)
+                              rt.sm_count, st, nullptr, d_status + kWordFront) != cudaSuccess)
             return fail();
     } else if (ko > 0) {
         // (the largest k-th |x| bounds what is left in the residual: the SVD's products take their FP16 scale from it)
         if (topk_rows(d_input, rt.residual.as<float>(), rows, cols, ko, rt.outlier.idx.as<uint16_t>(),
-                      rt.outlier.val.as<float>(), d_status, rt.sm_count, st, d_status + 8, &residual_bound) != cudaSuccess)
+                      rt.outlier.val.as<float>(), d_status, rt.sm_count, st, d_status + kWordBound, &residual_bound) != cudaSuccess)
             return fail();
         d_src = rt.residual.as<float>();
     }
@@ -688,27 +691,28 @@ int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_p
         // 4.45 / 4.53), 6 x 4096 x 14336 8.05 / 8.14, 8 x 4096 x 14336 10.11 / 10.30.
         svd_workspace_device_full(rt.svd, in_flight >= 3 && (uint64_t)in_flight * n >= 150000000ull);
         if (svd_lowrank(rt.svd, d_src, rt.u.as<float>(), rt.s.as<float>(), rt.v.as<float>(), 1234ULL, d_status, st, omega_offset,
-                        residual_bound ? d_status + 8 : nullptr) != cudaSuccess)
+                        residual_bound ? d_status + kWordBound : nullptr) != cudaSuccess)
             return fail();
         mark(); job.ev_svd = job.nev - 1;
         // quantised factors replace U, S, V in place for the error stage (src/bitsqz_llm.cu:1078-1139)
         if (rt.uv_format != quantization_NONE) {
-            if (!run_quantize(rt, rt.uv_format, rt.u.as<float>(), rt.q_u, error_path ? rt.u.as<float>() : nullptr)) return fail();
-            if (!run_quantize(rt, rt.uv_format, rt.v.as<float>(), rt.q_v, error_path ? rt.v.as<float>() : nullptr)) return fail();
+            if (!run_quantize(rt, rt.uv_format, rt.u.as<float>(), rt.q_u, kWordMaxU, error_path ? rt.u.as<float>() : nullptr)) return fail();
+            if (!run_quantize(rt, rt.uv_format, rt.v.as<float>(), rt.q_v, kWordMaxV, error_path ? rt.v.as<float>() : nullptr)) return fail();
         }
         if (rt.s_format != quantization_NONE)
-            if (!run_quantize(rt, rt.s_format, rt.s.as<float>(), rt.q_s, error_path ? rt.s.as<float>() : nullptr)) return fail();
+            if (!run_quantize(rt, rt.s_format, rt.s.as<float>(), rt.q_s, kWordMaxOne, error_path ? rt.s.as<float>() : nullptr)) return fail();
         mark(); job.ev_quant = job.nev - 1;
         if (error_path) {
             if (reconstruct_lowrank(rt.u.as<float>(), rt.s.as<float>(), rt.v.as<float>(), rows, cols, (int)rank, d_src,
-                                    rt.error.as<float>(), d_status + 1, d_status, rt.recon_ws.as<float>(), rt.recon_ws_bytes, rt.sm_count,
+                                    rt.error.as<float>(), d_status + kWordError, d_status, rt.recon_ws.as<float>(), rt.recon_ws_bytes, rt.sm_count,
                                     st) != cudaSuccess)
                 return fail();
             mark(); job.ev_recon = job.nev - 1;
         }
     } else if (rt.q_format != quantization_NONE && !fused_front) {
         // (the error stage's input comes out of the quantiser: no dequantised matrix, no pass to subtract it)
-        if (!run_quantize(rt, rt.q_format, d_src, rt.q_direct, error_path ? rt.error.as<float>() : nullptr, error_path ? d_status + 1 : nullptr))
+        if (!run_quantize(rt, rt.q_format, d_src, rt.q_direct, kWordMaxOne, error_path ? rt.error.as<float>() : nullptr,
+                          error_path ? d_status + kWordError : nullptr))
             return fail();
         mark(); job.ev_quant = job.nev - 1;
     }
@@ -766,6 +770,7 @@ int compress_end(Runtime &rt, bitsqz_llm_array_t **out, bitsqz_llm_array_t *head
     if (!job.active) return 1;
     cudaStream_t st = rt.stream;
     const bool done = cudaStreamSynchronize(st) == cudaSuccess;
+    rt.words_clear = done && job.by_kernel;                   // (pack_object was the last kernel)
     if (!done || rt.h_status[0] != 0) {
         if (done && job.to_device && !job.by_kernel) {            // as the pack kernel does; abandon_job waits for it
             std::memset(rt.h_stage, 0, sizeof(bitsqz_llm_array_t));

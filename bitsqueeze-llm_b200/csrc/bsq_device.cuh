@@ -170,7 +170,7 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, unsigned parity
 //   * Outside every branch, and nothing in memory is read or written before it.
 //   * What the kernel before may write comes in through plain pointers: `const` with __restrict__, or __ldg, says that nobody writes the
 //     data while the kernel runs -- which is not so while it waits -- and lets loads move in front of the wait.  (The caller's matrix in
-//     the front end is read that way: the encoder comes behind the selection, the selection behind a memset.)
+//     the front end is read that way: the encoder comes behind the selection, the selection is launched the ordinary way.)
 //   * No kernel lets the next one's CTAs come early (griddepcontrol.launch_dependents): they come as its own CTAs leave, into places that
 //     are free anyway.  Let in at the start they waited on their SMs for as long as the kernel ran, up to 1.1 ms of a core's SVD, and kept
 //     other streams' kernels out.  Compress calls, ms, let in at the start / when CTAs leave / ordinary launches: four of 2048 x 4096 at rank 256

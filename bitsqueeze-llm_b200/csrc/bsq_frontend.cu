@@ -267,13 +267,13 @@ cudaError_t persistent_grid(K kernel, int threads, size_t smem, int sm_count, un
 template <int G>
 cudaError_t launch_front(int method, const float *d_in, uint32_t rows, uint32_t cols, uint32_t k, uint16_t *d_idx,
                          float *d_val, float *d_scales_f32, float *d_dq, uint8_t *d_scale_codes, uint8_t *d_data,
-                         void *d_scratch, int sm_count, cudaStream_t stream, cudaEvent_t *events) {
-    // scratch words: [0] global maximum, [1] row counter of kernel 1, [2] row counter of kernel 2 (cleared per call),
-    // [3] the selection bound carried from call to call (never cleared; see carried_hint)
-    unsigned *gmax = static_cast<unsigned *>(d_scratch);
+                         void *d_scratch, int sm_count, cudaStream_t stream, cudaEvent_t *events, unsigned *d_words) {
+    // scratch words: [0] global maximum, [1] row counter of kernel 1, [2] row counter of kernel 2 (the caller's, which are zero,
+    // or cleared per call), [3] the selection bound carried from call to call (never cleared; see carried_hint)
+    unsigned *gmax = d_words ? d_words : static_cast<unsigned *>(d_scratch), *hint = static_cast<unsigned *>(d_scratch) + 3;
     float *absmax = reinterpret_cast<float *>(static_cast<uint8_t *>(d_scratch) + 16);
     unsigned grid = 0;
-    cudaError_t err = cudaMemsetAsync(gmax, 0, 12, stream);
+    cudaError_t err = d_words ? cudaSuccess : cudaMemsetAsync(gmax, 0, 4 * kFrontWords, stream);
     if (err != cudaSuccess) return err;
     if (method == 11) {
         const FrontGeometry f = front_geometry(cols, 2);
@@ -281,7 +281,7 @@ cudaError_t launch_front(int method, const float *d_in, uint32_t rows, uint32_t 
         if (err != cudaSuccess) return err;
         if (events) cudaEventRecord(events[0], stream);
         frontend_nf4_kernel<G><<<grid, f.threads, f.smem, stream>>>(d_in, rows, cols, k, d_idx, d_val, d_scales_f32, d_data,
-                                                                    gmax + 1, gmax + 3);
+                                                                    gmax + 1, hint);
         if (events) { cudaEventRecord(events[1], stream); cudaEventRecord(events[2], stream); }
         return cudaGetLastError();
     }
@@ -290,7 +290,7 @@ cudaError_t launch_front(int method, const float *d_in, uint32_t rows, uint32_t 
     if (err != cudaSuccess) return err;
     if (events) cudaEventRecord(events[0], stream);
     frontend_select_kernel<G><<<grid, f1.threads, f1.smem, stream>>>(d_in, rows, cols, k, d_idx, d_val, absmax, gmax, gmax + 1,
-                                                                     gmax + 3);
+                                                                     hint);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     if (events) cudaEventRecord(events[1], stream);
@@ -314,7 +314,7 @@ size_t frontend_scratch_bytes(uint32_t rows, uint32_t cols) { return 16 + (size_
 cudaError_t frontend_quantize(int method, const float *d_in, uint32_t rows, uint32_t cols, uint32_t k, uint16_t *d_idx,
                               float *d_val, float *d_scales_f32, float *d_dq, uint8_t *d_scale_codes, uint8_t *d_data,
                               void *d_scratch, unsigned *d_status, int sm_count, cudaStream_t stream,
-                              cudaEvent_t *events) {
+                              cudaEvent_t *events, unsigned *d_words) {
     (void)d_status;                                          // these kernels wait on nothing
     if (!frontend_supported(rows, cols, k) || (method != 10 && method != 11)) return cudaErrorInvalidValue;
     if (!d_in || !d_data || (k > 0 && (!d_idx || !d_val))) return cudaErrorInvalidValue;
@@ -323,7 +323,7 @@ cudaError_t frontend_quantize(int method, const float *d_in, uint32_t rows, uint
     if (method == 11 && !d_scales_f32) return cudaErrorInvalidValue;
 #define BSQ_FRONT(G_)                                                                                               \
     launch_front<G_>(method, d_in, rows, cols, k, d_idx, d_val, d_scales_f32, d_dq, d_scale_codes, d_data, d_scratch, \
-                     sm_count, stream, events)
+                     sm_count, stream, events, d_words)
     switch (front_geometry(cols, 2).G) {
         case 1: return BSQ_FRONT(1);
         case 2: return BSQ_FRONT(2);

@@ -16,8 +16,10 @@ namespace bsq {
 cudaError_t nf4_quantize(const float *d_x, uint64_t n, float *d_scales, uint8_t *d_data, float *d_deq_out, int sm_count,
                          cudaStream_t stream, unsigned *d_error_flag = nullptr);
 size_t nf4dq_scratch_bytes(uint64_t n);
+// d_gmax (nullable): a device word that is zero, for the largest magnitude; without it the call clears one in d_scratch.
 cudaError_t nf4dq_quantize(const float *d_x, uint64_t n, float *d_dq, uint8_t *d_scale_codes, uint8_t *d_data,
-                           float *d_deq_out, void *d_scratch, int sm_count, cudaStream_t stream, unsigned *d_error_flag = nullptr);
+                           float *d_deq_out, void *d_scratch, int sm_count, cudaStream_t stream, unsigned *d_error_flag = nullptr,
+                           unsigned *d_gmax = nullptr);
 // Variant for callers that must not allocate: scratch is a fixed array inside the library.
 uint64_t nf4dq_static_max_elements();
 cudaError_t nf4dq_quantize_static(const float *d_x, uint64_t n, float *d_dq, uint8_t *d_scale_codes, uint8_t *d_data,
@@ -40,8 +42,8 @@ int topk_num_columns(uint16_t cols, float ratio);
 // ranking below every number.  d_idx / d_val are [rows][k].  d_residual (nullable): receives
 // the row with the selected entries set to +0.0f; may alias d_in (in-place separation).
 // d_status: device word that receives kStatus* bits.
-// d_bound (nullable device word) receives, where the shared-memory path runs (*bound_written says so), the bits of the
-// largest k-th |x| over the rows: an upper bound of every |x| that is left in d_residual.
+// d_bound (nullable device word, zero when the call runs) receives, where the shared-memory path runs (*bound_written says
+// so), the bits of the largest k-th |x| over the rows: an upper bound of every |x| that is left in d_residual.
 cudaError_t topk_rows(const float *d_in, float *d_residual, uint32_t rows, uint32_t cols, uint32_t k, uint16_t *d_idx,
                       float *d_val, unsigned *d_status, int sm_count, cudaStream_t stream, unsigned *d_bound = nullptr,
                       bool *bound_written = nullptr);
@@ -61,10 +63,13 @@ cudaError_t topk_apply_two(const uint16_t *d_idx0, const float *d_val0, uint32_t
 bool frontend_supported(uint32_t rows, uint32_t cols, uint32_t k);
 size_t frontend_scratch_bytes(uint32_t rows, uint32_t cols);
 // method: 11 = NF4 (d_scales_f32 used), 10 = NF4_DQ (d_dq, d_scale_codes used).
+// d_words (nullable): kFrontWords device words that are zero; without them the call clears words in d_scratch.
 cudaError_t frontend_quantize(int method, const float *d_in, uint32_t rows, uint32_t cols, uint32_t k, uint16_t *d_idx,
                               float *d_val, float *d_scales_f32, float *d_dq, uint8_t *d_scale_codes, uint8_t *d_data,
                               void *d_scratch, unsigned *d_status, int sm_count, cudaStream_t stream,
-                              cudaEvent_t *events = nullptr);   // events[3]: before pass 1, between, after pass 2
+                              cudaEvent_t *events = nullptr,    // events[3]: before pass 1, between, after pass 2
+                              unsigned *d_words = nullptr);
+constexpr int kFrontWords = 3;
 
 // ---- residual / error helpers ---------------------------------------------------------------
 // e = a - b and *d_flag |= 1 when some |e| > FLT_EPSILON (reference src/bitsqz_llm.cu:164-184).
@@ -73,7 +78,19 @@ cudaError_t residual_error(const float *d_a, const float *d_b, uint64_t n, float
 
 // ---- device-resident objects (bsq_pack.cu) ---------------------------------------------------
 constexpr int kMaxCopySegments = 12, kMaxHeads = 6;
-constexpr int kStatusWords = 16;                             // [0] kernel status bits, [1] error-nonzero flag, [8] bound of the SVD's products
+// The words of a runtime's status block.  All are zero when a call's first kernel starts: the kernel that ends a call hands
+// them to the host and clears them for the next one, where a memset in front of each of them cost the chain of a call
+// 4.3 us (its own 1.6 and the gap to the next operation).
+constexpr int kStatusWords = 16;
+enum : int {
+    kWordStatus = 0,                                         // kernel status bits
+    kWordError = 1,                                          // something is left for the error list
+    kWordFront = 2,                                          // kFrontWords of the fused front end
+    kWordMaxU = 5,                                           // NF4_DQ: the largest magnitude of a section
+    kWordMaxV = 6,
+    kWordMaxOne = 7,                                         // (the matrix or S)
+    kWordBound = 8                                           // bound of the residual for the SVD's products
+};
 struct CopySegment {
     void *dst;
     const void *src;
@@ -108,8 +125,8 @@ enum class Reach {
 Reach memory_reach(const void *p, uint64_t bytes);
 // Copies up to kMaxCopySegments pieces of device memory, of any alignment, in one launch.
 cudaError_t copy_segments(const CopySegment *segments, int count, cudaStream_t stream);
-// The same together with the headers and, into page-locked `mirror`, the status words.
-cudaError_t pack_object(const CopySegment *segments, int count, const PackHeaders &headers, const unsigned *d_status, unsigned *mirror,
+// The same together with the headers and, into page-locked `mirror`, the status words, which it clears.
+cudaError_t pack_object(const CopySegment *segments, int count, const PackHeaders &headers, unsigned *d_status, unsigned *mirror,
                         cudaStream_t stream);
 // Small headers out of a device-resident payload into page-locked `host`, 64 bytes apart; clears the status words.
 cudaError_t fetch_heads(const HeadList &heads, uint8_t *host, unsigned *d_status, cudaStream_t stream);

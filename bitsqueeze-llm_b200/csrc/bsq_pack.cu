@@ -9,7 +9,7 @@
 //   * the section headers and the object's header travel in the kernel's parameters; the error section's entry and flag
 //     are dropped on the device when the error flag says so, and the whole header is zeroed when a kernel of the call has
 //     reported an error (the call fails then, and nothing that could pass for an object is left in the buffer);
-//   * the status words go to the caller's page-locked mirror.
+//   * the status words go to the caller's page-locked mirror and are cleared for the next call.
 // Bound by launch latency up to a few MB, by memory above (9.7 MB of a 4096 x 4096 NF4_DQ object: 6.7 us).  Measured with
 // the calls around it: compress 256 x 1024 NF4_DQ 71 -> 40 us, 4096 x 4096 114 -> 75 us; decompress 4096 x 4096, which also
 // reads aligned sections where they lie, 78 -> 56 us.
@@ -99,7 +99,7 @@ __device__ __forceinline__ void copy_all(const CopyArgs &c) {
 __global__ void __launch_bounds__(kCopyThreads) copy_segments_kernel(const __grid_constant__ CopyArgs c) { copy_all(c); }
 
 __global__ void __launch_bounds__(kCopyThreads) pack_object_kernel(const __grid_constant__ CopyArgs c, const __grid_constant__ PackHeaders h,
-                                                                   const unsigned *status, unsigned *mirror) {
+                                                                   unsigned *status, unsigned *mirror) {
     chain_begin();
     copy_all(c);
     if (blockIdx.x != gridDim.x - 1) return;
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kCopyThreads) pack_object_kernel(const __grid_
             q.dst[i] = b;
         }
     }
-    const bool failed = status[0] != 0, no_error = status[1] == 0;
+    const bool failed = status[kWordStatus] != 0, no_error = status[kWordError] == 0;
     for (int i = threadIdx.x; i < (int)sizeof(h.object); i += kCopyThreads) {
         uint8_t b = failed ? 0 : h.object[i];
         if (no_error) {
@@ -121,7 +121,11 @@ __global__ void __launch_bounds__(kCopyThreads) pack_object_kernel(const __grid_
         }
         h.object_dst[i] = b;
     }
-    if (threadIdx.x < kStatusWords) reinterpret_cast<volatile unsigned *>(mirror)[threadIdx.x] = status[threadIdx.x];
+    __syncthreads();                                         // (everybody has read the two words above)
+    if (threadIdx.x < kStatusWords) {
+        reinterpret_cast<volatile unsigned *>(mirror)[threadIdx.x] = status[threadIdx.x];
+        status[threadIdx.x] = 0;
+    }
 }
 
 // One CTA: the small headers inside a device-resident payload into page-locked host memory, 64 bytes apart; clears the
@@ -181,7 +185,7 @@ cudaError_t copy_segments(const CopySegment *segments, int count, cudaStream_t s
     return cudaGetLastError();
 }
 
-cudaError_t pack_object(const CopySegment *segments, int count, const PackHeaders &headers, const unsigned *d_status, unsigned *mirror,
+cudaError_t pack_object(const CopySegment *segments, int count, const PackHeaders &headers, unsigned *d_status, unsigned *mirror,
                         cudaStream_t stream) {
     if (count < 0 || count > kMaxCopySegments) return cudaErrorInvalidValue;
     CopyArgs c;

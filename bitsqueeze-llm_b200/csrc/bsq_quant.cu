@@ -323,16 +323,15 @@ cudaError_t nf4_quantize(const float *d_x, uint64_t n, float *d_scales, uint8_t 
 size_t nf4dq_scratch_bytes(uint64_t n) { return (size_t)((n + 63) / 64) * sizeof(float) + 16; }
 
 cudaError_t nf4dq_quantize(const float *d_x, uint64_t n, float *d_dq, uint8_t *d_scale_codes, uint8_t *d_data,
-                           float *d_deq_out, void *d_scratch, int sm_count, cudaStream_t stream, unsigned *d_error_flag) {
+                           float *d_deq_out, void *d_scratch, int sm_count, cudaStream_t stream, unsigned *d_error_flag, unsigned *d_gmax) {
     // scratch layout: [0,16) global-max word (+ padding), then one float per block
-    unsigned *gmax = static_cast<unsigned *>(d_scratch);
+    unsigned *gmax = d_gmax ? d_gmax : static_cast<unsigned *>(d_scratch);
     float *absmax = reinterpret_cast<float *>(static_cast<uint8_t *>(d_scratch) + 16);
     const bool vec = aligned(d_x, 16) && aligned(d_data, 4) && (!d_deq_out || aligned(d_deq_out, 16));
     const int grid = grid_for(n, sm_count);
-    cudaError_t err = cudaMemsetAsync(gmax, 0, 16, stream);
+    cudaError_t err = d_gmax ? cudaSuccess : cudaMemsetAsync(gmax, 0, 4, stream);
     if (err != cudaSuccess) return err;
-    absmax_flat_kernel<<<grid, kThreads, 0, stream>>>(d_x, n, vec, absmax, gmax);
-    if ((err = cudaGetLastError()) != cudaSuccess) return err;
+    if ((err = launch_chained(absmax_flat_kernel, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax)) != cudaSuccess) return err;
     if (d_deq_out && d_error_flag)
         return launch_chained(encode_flat_kernel<true, kWriteError>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
                                                                         d_dq, d_data, d_deq_out, d_error_flag);

@@ -376,11 +376,7 @@ cudaError_t topk_rows(const float *d_in, float *d_residual, uint32_t rows, uint3
     if (!d_idx || !d_val) return cudaErrorInvalidValue;
     const bool bulk = bulk_rows(d_in, d_residual, cols);
     if (topk_rows_fit_smem(cols, k) && (bulk || ragged_rows_fit(rows, cols, k))) {
-        if (d_bound) {
-            const cudaError_t e = cudaMemsetAsync(d_bound, 0, sizeof(unsigned), stream);
-            if (e != cudaSuccess) return e;
-            if (bound_written) *bound_written = true;
-        }
+        if (d_bound && bound_written) *bound_written = true;
 #define BSQ_TOPK(G_)                                                                                                             \
     (bulk ? launch_group<G_, true>(d_in, d_residual, rows, cols, k, d_idx, d_val, d_status, sm_count, stream, d_bound) \
           : launch_group<G_, false>(d_in, d_residual, rows, cols, k, d_idx, d_val, d_status, sm_count, stream, d_bound))
