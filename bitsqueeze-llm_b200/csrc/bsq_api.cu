@@ -245,6 +245,7 @@ struct Runtime {
     DevicePack pack;
     CompressJob job;
     bool decompress_active = false;
+    unsigned head_number = 0;                            // of the last HeadCheck (even)
     unsigned inject_status = 0;                          // test hook: OR-ed into the status word of the next call
 
     void release() {
@@ -290,6 +291,7 @@ bool common_setup(Runtime &rt) {
     if (cudaHostAlloc(reinterpret_cast<void **>(&rt.h_status), 64, cudaHostAllocPortable) != cudaSuccess) return false;
     std::memset(rt.h_status, 0, 64);
     if (cudaHostAlloc(reinterpret_cast<void **>(&rt.h_stage), kStageBytes, cudaHostAllocPortable) != cudaSuccess) return false;
+    std::memset(rt.h_stage, 0, kStageBytes);
     return true;
 }
 
@@ -1066,6 +1068,98 @@ bool apply_lists(Runtime &rt, const bitsqz_llm_array_t *c, const Lists &l, float
     return err == cudaSuccess;
 }
 
+// What the headers inside the payload have to say, worked out from the object's header (sizes, methods and list lengths follow from
+// it); false where that already decides that the object is refused.
+bool expect_heads(Runtime &rt, const bitsqz_llm_array_t *c, HeadCheck *check, uint32_t *k_err, uint32_t *k_out) {
+    const uint8_t *payload = static_cast<const uint8_t *>(c->payload);
+    auto add = [&](const bitsqz_section_t &s, const void *want, size_t bytes, uint64_t mask) {
+        const int i = check->count++;
+        check->src[i] = payload + s.offset;
+        check->length[i] = (uint8_t)bytes;
+        check->mask[i] = mask;
+        std::memcpy(check->want[i], want, bytes);
+    };
+    auto span = [](size_t at, size_t bytes) { return ((1ull << bytes) - 1) << at; };
+    auto quant = [&](const bitsqz_section_t &s, int method, uint64_t count) {
+        if (s.storage != BITSQZ_SECTION_QUANT || s.size != quant_section_bytes(method, count)) return false;
+        QuantHeader h{};
+        h.magic = kQuantMagic;
+        h.version = 1;
+        h.method = method;
+        h.num_elements = count;
+        h.num_blocks = (count + 63) / 64;
+        h.block_size = 64;
+        add(s, &h, sizeof(h), span(offsetof(QuantHeader, magic), 6) | span(offsetof(QuantHeader, method), 4) | span(offsetof(QuantHeader, num_elements), 24));
+        return true;
+    };
+    auto topk = [&](const bitsqz_section_t &s, const TopkBufs &cap, uint32_t *k) {
+        const uint64_t row = 6ull * c->num_rows, body = s.size - sizeof(TopkHeader);
+        if (s.size < sizeof(TopkHeader) || body % row != 0 || body / row > c->num_columns) return false;
+        *k = (uint32_t)(body / row);
+        const TopkHeader h{c->num_rows, c->num_columns, (uint16_t)*k, 0};
+        if (!topk_section_ok(cap, c, s, h)) return false;
+        add(s, &h, sizeof(h), span(0, 6));
+        return true;
+    };
+    check->answer = reinterpret_cast<unsigned *>(rt.h_stage + kStageBytes) - 1;
+    check->number = rt.head_number += 2;
+    return quant(c->section_direct, c->quantization_only_format, c->num_elements) &&
+           (!(c->flags & kFlagError) || topk(c->section_error_topk, rt.err, k_err)) &&
+           (!(c->flags & kFlagOutlier) || topk(c->section_outlier_topk, rt.outlier, k_out));
+}
+// Waits for what the kernel launched with `check` has found (it has hardly begun then).
+bool heads_as_expected(Runtime &rt, const HeadCheck &check) {
+    const volatile unsigned *answer = check.answer;
+    for (unsigned i = 1; (*answer | 1u) != (check.number | 1u); ++i) {
+        if (i % 4096 != 0) continue;
+        const cudaError_t q = cudaStreamQuery(rt.stream);
+        if (q == cudaErrorNotReady) continue;
+        if (q != cudaSuccess || (*answer | 1u) != (check.number | 1u)) return false;
+    }
+    return *answer == check.number;
+}
+SectionSource quant_source(const bitsqz_llm_array_t *c, const bitsqz_section_t &s, int method, uint64_t count) {
+    const uint8_t *at = static_cast<const uint8_t *>(c->payload) + s.offset;
+    const uint64_t nb = (count + 63) / 64;
+    SectionSource q;
+    q.scales = at + sizeof(QuantHeader);
+    q.dq = method == NF4 ? nullptr : at + offsetof(QuantHeader, dq_scale);
+    q.data = q.scales + (method == NF4 ? nb * 4 : nb);
+    q.n = count;
+    return q;
+}
+ListSource list_source(const bitsqz_llm_array_t *c, const bitsqz_section_t &s, uint32_t k) {
+    ListSource l;
+    l.idx = static_cast<const uint8_t *>(c->payload) + s.offset + sizeof(TopkHeader);
+    l.val = l.idx + 2ull * c->num_rows * k;
+    l.k = k;
+    return l;
+}
+
+// A quantised matrix with its lists, device-resident, all of it within reach of kernels and apart from the result: one kernel
+// checks the headers, decodes, adds the lists and reports.
+int decompress_begin_one_kernel(Runtime &rt, const bitsqz_llm_array_t *c, float *d_dst) {
+    cudaStream_t st = rt.stream;
+    HeadCheck check{};
+    uint32_t k_err = 0, k_out = 0;
+    if (!expect_heads(rt, c, &check, &k_err, &k_out)) return 1;
+    auto fail = [&]() {
+        cudaStreamSynchronize(st);
+        cudaGetLastError();
+        return 1;
+    };
+    rt.h_status[0] = rt.inject_status;                        // (the stream is idle: one call at a time, and the last one has been waited for)
+    rt.inject_status = 0;
+    // error list first, outliers second (src/bitsqz_llm.cu:1372-1387)
+    if (decode_matrix(quant_source(c, c->section_direct, c->quantization_only_format, c->num_elements), c->num_rows, c->num_columns,
+                      list_source(c, c->section_error_topk, k_err), list_source(c, c->section_outlier_topk, k_out), d_dst, rt.h_status, check,
+                      rt.sm_count, st) != cudaSuccess)
+        return fail();
+    if (!heads_as_expected(rt, check)) return fail();
+    rt.decompress_active = true;
+    return 0;
+}
+
 // Enqueue one decompress call (src/bitsqz_llm.cu:1304-1393).  `c` is the 200-byte header in host memory; its payload
 // pointer may be host memory (the reference's objects) or, with payload_on_device, device memory.
 int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_device, float *d_dst) {
@@ -1084,6 +1178,9 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
     for (const bitsqz_section_t *s : {&c->section_u, &c->section_s, &c->section_v, &c->section_direct, &c->section_outlier_topk, &c->section_error_topk})
         kernels_read = kernels_read || s->storage == BITSQZ_SECTION_QUANT || s->storage == BITSQZ_SECTION_TOPK;
     const Reach reach = payload_on_device && kernels_read ? memory_reach(c->payload, payload_bytes) : Reach::kCopies;
+    const bool over_object = ranges_overlap(d_dst, (uint64_t)c->num_elements * 4, c->payload, payload_bytes);
+    if (reach == Reach::kKernels && !over_object && c->section_direct.storage == BITSQZ_SECTION_QUANT)
+        return decompress_begin_one_kernel(rt, c, d_dst);
     if (!fetch_heads(rt, c, payload_on_device, reach, &heads)) return fail();
     const bool has_out = c->flags & kFlagOutlier, has_err = c->flags & kFlagError;
     if (has_out && !topk_section_ok(rt.outlier, c, c->section_outlier_topk, heads.outlier)) return 1;
@@ -1100,7 +1197,6 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
     // lists come last: of a host object the largest copy is then under way while the small ones are queued.)
     PayloadAccess how;
     how.on_device = reach == Reach::kKernels;
-    const bool over_object = ranges_overlap(d_dst, (uint64_t)c->num_elements * 4, c->payload, payload_bytes);
     how.in_place = how.on_device && !over_object;
     Lists lists;
     lists.k[0] = has_err ? heads.err.num_topk_columns : 0;

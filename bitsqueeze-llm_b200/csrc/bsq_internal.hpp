@@ -9,6 +9,22 @@
 
 namespace bsq {
 
+// ---- a call's first and last kernel -------------------------------------------------------------
+constexpr int kMaxHeads = 6;
+// The headers inside a device-resident payload, checked by the kernel that reads the sections: it is launched before the host has seen
+// them (a wait of 12 us between a small kernel that fetched them and the one that decodes), writes nothing unless every byte under
+// `mask` is the one that the host expects, and its first CTA leaves the outcome in page-locked memory, where the host waits for it
+// before it goes on.
+constexpr int kMaxHeadBytes = 48;
+struct HeadCheck {
+    const uint8_t *src[kMaxHeads];
+    uint64_t mask[kMaxHeads];                                // bit i: byte i has to match
+    uint8_t length[kMaxHeads];
+    uint8_t want[kMaxHeads][kMaxHeadBytes];
+    int count = 0;
+    unsigned *answer = nullptr, number = 0;                  // receives `number` (even), + 1 where a header differs
+};
+
 // ---- NF4 / NF4_DQ over a flat array (bsq_quant.cu) ----------------------------------------
 // d_deq_out (nullable): also write the dequantised values, which is what the reference's
 // compress path feeds into its error-correction stage (src/bitsqz_llm.cu:506-511).  With d_error_flag (a device word) the
@@ -28,6 +44,23 @@ cudaError_t nf4_dequantize(const float *d_scales, const uint8_t *d_data, uint64_
                            cudaStream_t stream);
 cudaError_t nf4dq_dequantize(const float *d_dq, const uint8_t *d_scale_codes, const uint8_t *d_data, uint64_t n,
                              float *d_out, int sm_count, cudaStream_t stream);
+// A section as it lies in a device-resident object, whatever its alignment.
+struct SectionSource {
+    const uint8_t *scales = nullptr;      // NF4: FP32, NF4_DQ: E4M3
+    const uint8_t *dq = nullptr;          // NF4_DQ only
+    const uint8_t *data = nullptr;        // nibbles, or FP32 values where scales is null
+    uint64_t n = 0;
+};
+// A row-wise top-k list as it lies in an object (idx: u16, val: f32, any alignment).
+struct ListSource {
+    const uint8_t *idx = nullptr, *val = nullptr;
+    uint32_t k = 0;
+};
+// A quantised matrix section -> d_out, and its lists (k > 0), one after the other, added in the same pass: the whole decompress call
+// of such an object.  Nothing is written where the object's headers are not what `heads` expects.  mirror: page-locked, zero; receives
+// kStatusBadIndex where a list names a column that the matrix does not have.
+cudaError_t decode_matrix(const SectionSource &q, uint32_t rows, uint32_t cols, const ListSource &first, const ListSource &second, float *d_out,
+                          unsigned *mirror, const HeadCheck &heads, int sm_count, cudaStream_t stream);
 // Dequantise a rows x cols matrix and add a row-wise top-k list in one pass; d_scales (NF4) or d_dq + d_scale_codes (NF4_DQ).
 cudaError_t nf4_dequantize_add_topk(const float *d_scales, const float *d_dq, const uint8_t *d_scale_codes, const uint8_t *d_data,
                                     uint32_t rows, uint32_t cols, const uint16_t *d_idx, const float *d_val, uint32_t k,
@@ -77,7 +110,7 @@ cudaError_t residual_error(const float *d_a, const float *d_b, uint64_t n, float
                            cudaStream_t stream);
 
 // ---- device-resident objects (bsq_pack.cu) ---------------------------------------------------
-constexpr int kMaxCopySegments = 12, kMaxHeads = 6;
+constexpr int kMaxCopySegments = 12;
 // The words of a runtime's status block.  All are zero when a call's first kernel starts: the kernel that ends a call hands
 // them to the host and clears them for the next one, where a memset in front of each of them cost the chain of a call
 // 4.3 us (its own 1.6 and the gap to the next operation).

@@ -11,6 +11,7 @@
 // per-block scale work (IEEE reciprocal, E4M3 coding) is done once per block by lanes 0..15
 // and handed to the owning lanes by shuffle.  Codes come from the bucket-table encoder in
 // bsq_device.cuh.  HBM-bound: 4 B read + 0.5 B + (4 or 1)/64 B written per element.
+#include "bsq_call.cuh"
 #include "bsq_device.cuh"
 #include "bsq_internal.hpp"
 
@@ -211,89 +212,155 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // ---- decode ----------------------------------------------------------------------------------
-// Optional (idx non-null): a row-wise top-k list to add onto the decoded rows x cols matrix in the same pass.
+// Row-wise top-k lists to add onto the decoded rows x cols matrix in the same pass, one after the other (idx: u16, val: f32, any
+// alignment; k = 0: none).
 struct TopkList {
-    const uint16_t *idx;
-    const float *val;
-    unsigned cols, k;
-    unsigned *status;
+    const uint8_t *idx, *val;
+    unsigned k;
 };
+struct TopkLists {
+    TopkList list[2];
+    unsigned cols;
+    unsigned *status;
+    bool status_on_host;
+};
+// What a batch of kBatch elements needs from memory.  The first 64 entries of each list's row come with it.
+struct DecodeBatch {
+    unsigned w[4];
+    float scale;
+    unsigned c[2][2];
+    float v[2][2];
+};
+
+// A warp decodes kBatch consecutive elements into shared memory, adds the lists' entries there and sends the batch out by one bulk
+// store; what the next batch needs is on its way meanwhile.  scales (NF4: f32), dq_in and data may lie at any address
+// (vec_in: data at a multiple of 4); out off a 16-byte boundary, and the last batch, go out by lanes.
+// Bound by the bytes written (a plain fill of as many: 10.1 us) and the trip for the first batch.  4096 x 4096 NF4_DQ with a list of 41
+// per row 16.9 us, without 14.9, 19 with the check of the headers; two buffers and three CTAs per SM 17.9, five and six CTAs 17.9 and
+// 20.1; entries added in global memory behind the batch's own stores 17.1.  As a whole call, against a kernel that fetches the headers,
+// a wait, this kernel and a copy of the status words: 56.3 -> 40.1 us; 2505 x 3085 with two lists, off its alignment, 69.1 -> 34.5.
+constexpr int kDecodeCtas = 4;
+constexpr size_t kDecodeSmem = (size_t)(kThreads / 32) * kBatch * sizeof(float);
 template <bool DQ>
-__global__ void __launch_bounds__(kThreads)
-    decode_flat_kernel(const float *__restrict__ scales_f32, const uint8_t *__restrict__ scale_codes,
-                       const float *__restrict__ dq_in, const uint8_t *__restrict__ data, uint64_t n, bool vec,
-                       float *out, TopkList add) {
+__global__ void __launch_bounds__(kThreads, kDecodeCtas)
+    decode_flat_kernel(const uint8_t *__restrict__ scales_f32, const uint8_t *__restrict__ scale_codes,
+                       const uint8_t *__restrict__ dq_in, const uint8_t *__restrict__ data, uint64_t n, bool vec_in, bool bulk_out,
+                       float *out, const __grid_constant__ TopkLists add, const __grid_constant__ HeadCheck heads) {
+    extern __shared__ __align__(128) float stage_raw[];
     const int lane = threadIdx.x & 31;
     const uint64_t warp = (uint64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     const uint64_t nwarps = (uint64_t)gridDim.x * (kThreads / 32);
     const uint64_t nb = (n + 63) / 64;
+    float *const stage = stage_raw + (threadIdx.x >> 5) * kBatch;
     Nf4Lut lut;
     lut.load();
     float dq = 1.0f;
     if (DQ) {
-        dq = *dq_in;
+        dq = load_f32_any(dq_in);
         if (dq == 0.0f || !isfinite(dq)) dq = 1.0f;   // quantization_cuda.cu:325-328
     }
-    for (uint64_t base = warp * kBatch; base < n; base += nwarps * kBatch) {
-        const uint64_t blk = base / 64 + lane;
-        float scale = 1.0f;
-        if (lane < 16 && blk < nb) {
-            scale = DQ ? __fmul_rn(dq, e4m3_decode(scale_codes[blk])) : scales_f32[blk];
-            if (scale == 0.0f || !isfinite(scale)) scale = 1.0f;
-        }
-        unsigned w[4];
+    const bool listed = add.list[0].k + add.list[1].k != 0, small = n <= 0xFFFFFFFFull;
+    const auto row_of = [&](uint64_t e) { return small ? (uint64_t)((unsigned)e / add.cols) : e / add.cols; };
+    auto fetch = [&](uint64_t base, DecodeBatch &b) {
+        if (base >= n) return;
 #pragma unroll
         for (int it = 0; it < 4; ++it) {
             const uint64_t e = base + it * 256 + lane * 8;
-            if (vec && e + 8 <= n) {
-                w[it] = __ldcs(reinterpret_cast<const unsigned *>(data + e / 2));
+            if (vec_in && e + 8 <= n) {
+                b.w[it] = __ldcs(reinterpret_cast<const unsigned *>(data + e / 2));
             } else {
-                w[it] = 0;
+                b.w[it] = 0;
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    if (e + 2 * q < n) w[it] |= (unsigned)data[e / 2 + q] << (8 * q);
+                    if (e + 2 * q < n) b.w[it] |= (unsigned)data[e / 2 + q] << (8 * q);
             }
         }
-#pragma unroll
-        for (int it = 0; it < 4; ++it) {
-            const uint64_t e = base + it * 256 + lane * 8;
-            const float sb = __shfl_sync(kFullMask, scale, it * 4 + (lane >> 3));
-            float d[8];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const unsigned byte = (w[it] >> (8 * q)) & 0xFFu;
-                d[2 * q] = __fmul_rn(sb, lut.decode(byte >> 4));
-                d[2 * q + 1] = __fmul_rn(sb, lut.decode(byte & 0xFu));
-            }
-            if (vec && e + 8 <= n) {
-                __stcs(reinterpret_cast<float4 *>(out + e), make_float4(d[0], d[1], d[2], d[3]));
-                __stcs(reinterpret_cast<float4 *>(out + e) + 1, make_float4(d[4], d[5], d[6], d[7]));
-            } else {
-#pragma unroll
-                for (int q = 0; q < 8; ++q)
-                    if (e + q < n) out[e + q] = d[q];
-            }
+        const uint64_t blk = base / 64 + lane;
+        b.scale = 1.0f;
+        if (lane < 16 && blk < nb) {
+            b.scale = DQ ? __fmul_rn(dq, e4m3_decode(scale_codes[blk])) : load_f32_any(scales_f32 + 4 * blk);
+            if (b.scale == 0.0f || !isfinite(b.scale)) b.scale = 1.0f;
         }
-        if (add.idx) {
-            // dense[row, idx] += value (topk_cuda.cuh:83-86) for the entries that fall into the kBatch elements this
-            // warp has just written: the row(s) of the batch, k entries each, a few per lane
-            __syncwarp();                                     // the warp's stores are ordered before its reads below
-            const uint64_t last = (base + kBatch <= n ? base + kBatch : n) - 1;
-            for (uint64_t r = base / add.cols; r <= last / add.cols; ++r) {
-                for (unsigned j = lane; j < add.k; j += 32) {
-                    const unsigned c = add.idx[r * add.k + j];
-                    if (c < add.cols) {
-                        const uint64_t pos = r * add.cols + c;
-                        if (pos >= base && pos <= last) out[pos] = out[pos] + add.val[r * add.k + j];
-                    } else if (add.status) {
-                        atomicOr(add.status, kStatusBadIndex);
-                    }
+        if (!listed) return;
+        const uint64_t r = row_of(base);
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+            const TopkList t = add.list[l];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const unsigned j = lane + 32 * u;
+                if (j < t.k) {
+                    b.c[l][u] = load_u16_any(t.idx + 2 * (r * t.k + j));
+                    b.v[l][u] = load_f32_any(t.val + 4 * (r * t.k + j));
                 }
             }
         }
+    };
+    DecodeBatch now, next;
+    fetch(warp * kBatch, now);                                // (all inside the object, whatever its headers say)
+    if (!heads_match(heads)) n = 0;                           // (uniform over the CTA)
+    for (uint64_t base = warp * kBatch; base < n; base += nwarps * kBatch) {
+        fetch(base + nwarps * kBatch, next);
+        if (lane == 0) bulk_wait_read_all();                  // the batch before has left the buffer
+        __syncwarp();
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+            const float sb = __shfl_sync(kFullMask, now.scale, it * 4 + (lane >> 3));
+            float d[8];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const unsigned byte = (now.w[it] >> (8 * q)) & 0xFFu;
+                d[2 * q] = __fmul_rn(sb, lut.decode(byte >> 4));
+                d[2 * q + 1] = __fmul_rn(sb, lut.decode(byte & 0xFu));
+            }
+            float4 *to = reinterpret_cast<float4 *>(stage + it * 256 + lane * 8);
+            to[0] = make_float4(d[0], d[1], d[2], d[3]);
+            to[1] = make_float4(d[4], d[5], d[6], d[7]);
+        }
+        __syncwarp();
+        const uint64_t end = base + kBatch <= n ? base + kBatch : n;
+        if (listed) {
+            // dense[row, idx] += value (topk_cuda.cuh:83-86) for the entries that fall into this batch: its row or rows, in full
+            const uint64_t r0 = row_of(base), r1 = row_of(end - 1);
+#pragma unroll
+            for (int l = 0; l < 2; ++l) {
+                const TopkList t = add.list[l];
+                if (t.k == 0) continue;
+                // at: where the entry's row starts, counted from the batch's first element (modulo 2^32)
+                auto put = [&](unsigned at, unsigned c, float v) {
+                    if (c >= add.cols) {
+                        report_bad_index(add.status, add.status_on_host);
+                    } else if (at + c < (unsigned)(end - base)) {
+                        stage[at + c] += v;
+                    }
+                };
+                unsigned at = (unsigned)(r0 * add.cols - base);
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+                    if (lane + 32 * u < t.k) put(at, now.c[l][u], now.v[l][u]);
+                for (uint64_t r = r0; r <= r1; ++r, at += add.cols)
+                    for (unsigned j = lane + (r == r0 ? 64u : 0u); j < t.k; j += 32)
+                        put(at, load_u16_any(t.idx + 2 * (r * t.k + j)), load_f32_any(t.val + 4 * (r * t.k + j)));
+                __syncwarp();
+            }
+        }
+        if (bulk_out && end - base == kBatch) {
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                bulk_s2g(out + base, stage, kBatch * sizeof(float));
+                bulk_commit();
+            }
+        } else {
+            for (unsigned i = lane; i < (unsigned)(end - base); i += 32) out[base + i] = stage[i];
+            __syncwarp();
+        }
+        now = next;
     }
+    if (lane == 0) bulk_wait_all();
 }
 
+inline const uint8_t *bytes(const void *p) { return static_cast<const uint8_t *>(p); }
 inline bool aligned(const void *p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
 inline int grid_for(uint64_t n, int sm_count) {
@@ -374,20 +441,28 @@ cudaError_t nf4dq_quantize_static(const float *d_x, uint64_t n, float *d_dq, uin
     return nf4dq_quantize(d_x, n, d_dq, d_scale_codes, d_data, nullptr, scratch, sm_count, stream);
 }
 
+static cudaError_t launch_decode(const SectionSource &q, const TopkLists &add, float *d_out, const HeadCheck &heads, int sm_count,
+                                 cudaStream_t stream) {
+    const bool vec_in = aligned(q.data, 4), bulk_out = aligned(d_out, 16);
+    const auto go = [&](auto kernel, const uint8_t *f32, const uint8_t *codes) {
+        const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDecodeSmem);
+        if (err != cudaSuccess) return err;
+        const uint64_t ctas = (q.n + (uint64_t)kBatch * (kThreads / 32) - 1) / ((uint64_t)kBatch * (kThreads / 32));
+        const uint64_t most = (uint64_t)sm_count * kDecodeCtas;
+        kernel<<<(unsigned)(ctas < most ? ctas : most), kThreads, kDecodeSmem, stream>>>(f32, codes, q.dq, q.data, q.n, vec_in, bulk_out, d_out, add, heads);
+        return cudaGetLastError();
+    };
+    return q.dq ? go(decode_flat_kernel<true>, nullptr, q.scales) : go(decode_flat_kernel<false>, q.scales, nullptr);
+}
+
 cudaError_t nf4_dequantize(const float *d_scales, const uint8_t *d_data, uint64_t n, float *d_out, int sm_count,
                            cudaStream_t stream) {
-    const bool vec = aligned(d_data, 4) && aligned(d_out, 16);
-    decode_flat_kernel<false><<<grid_for(n, sm_count), kThreads, 0, stream>>>(d_scales, nullptr, nullptr, d_data, n, vec,
-                                                                                d_out, TopkList{});
-    return cudaGetLastError();
+    return launch_decode(SectionSource{bytes(d_scales), nullptr, d_data, n}, TopkLists{}, d_out, HeadCheck{}, sm_count, stream);
 }
 
 cudaError_t nf4dq_dequantize(const float *d_dq, const uint8_t *d_scale_codes, const uint8_t *d_data, uint64_t n,
                              float *d_out, int sm_count, cudaStream_t stream) {
-    const bool vec = aligned(d_data, 4) && aligned(d_out, 16);
-    decode_flat_kernel<true><<<grid_for(n, sm_count), kThreads, 0, stream>>>(nullptr, d_scale_codes, d_dq, d_data, n, vec,
-                                                                               d_out, TopkList{});
-    return cudaGetLastError();
+    return launch_decode(SectionSource{d_scale_codes, bytes(d_dq), d_data, n}, TopkLists{}, d_out, HeadCheck{}, sm_count, stream);
 }
 
 // Dequantise a rows x cols matrix and add its row-wise top-k list in the same pass (quantization_cuda_decompress
@@ -398,14 +473,15 @@ cudaError_t nf4_dequantize_add_topk(const float *d_scales, const float *d_dq, co
                                     float *d_out, unsigned *d_status, int sm_count, cudaStream_t stream) {
     if (!d_data || !d_out || !d_idx || !d_val || rows == 0 || cols == 0 || k == 0) return cudaErrorInvalidValue;
     if ((d_scales != nullptr) == (d_dq != nullptr && d_scale_codes != nullptr)) return cudaErrorInvalidValue;
-    const uint64_t n = (uint64_t)rows * cols;
-    const bool vec = aligned(d_data, 4) && aligned(d_out, 16);
-    const TopkList add{d_idx, d_val, cols, k, d_status};
-    if (d_scales)
-        decode_flat_kernel<false><<<grid_for(n, sm_count), kThreads, 0, stream>>>(d_scales, nullptr, nullptr, d_data, n, vec, d_out, add);
-    else
-        decode_flat_kernel<true><<<grid_for(n, sm_count), kThreads, 0, stream>>>(nullptr, d_scale_codes, d_dq, d_data, n, vec, d_out, add);
-    return cudaGetLastError();
+    const SectionSource q{d_scales ? bytes(d_scales) : d_scale_codes, d_scales ? nullptr : bytes(d_dq), d_data, (uint64_t)rows * cols};
+    return launch_decode(q, TopkLists{{{bytes(d_idx), bytes(d_val), k}, {}}, cols, d_status, false}, d_out, HeadCheck{}, sm_count, stream);
+}
+
+cudaError_t decode_matrix(const SectionSource &q, uint32_t rows, uint32_t cols, const ListSource &first, const ListSource &second, float *d_out,
+                          unsigned *mirror, const HeadCheck &heads, int sm_count, cudaStream_t stream) {
+    if (!q.scales || !q.data || !d_out || q.n != (uint64_t)rows * cols || q.n == 0) return cudaErrorInvalidValue;
+    const TopkLists add{{{first.idx, first.val, first.k}, {second.idx, second.val, second.k}}, cols, mirror, true};
+    return launch_decode(q, add, d_out, heads, sm_count, stream);
 }
 
 }  // namespace bsq

@@ -1,0 +1,87 @@
+"""A device-resident quantised matrix is checked, decoded and completed with its lists by one kernel (csrc/bsq_quant.cu): the bits of the
+host object's route, at sizes around the kernel's batches of 1024 elements, with lists shorter and longer than what a batch brings with it."""
+import ctypes as C
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+# rows, cols, outlier, error: one batch and a little less or more, several rows in a batch, several batches in a row, ragged rows (lists and
+# codes off their alignment), lists of 1, 64, 65 and more than 128 entries, lists that name the same elements, more batches than warps
+CASES = [
+    (1, 1023, 0.01, 0.0), (1, 1025, 0.01, 0.02), (3, 341, 0.3, 0.3), (33, 31, 0.0, 0.1), (64, 64, 1.0, 1.0), (5, 2049, 0.04, 0.001),
+    (16, 6400, 0.01, 0.0102), (7, 14335, 0.005, 0.01), (300, 14336, 0.0, 0.02), (1501, 3001, 0.005, 0.01),
+]
+
+
+@pytest.mark.parametrize("q", [10, 11])
+@pytest.mark.parametrize("case", CASES)
+def test_one_launch_gives_the_host_objects_bits(pkg, lib, case, q):
+    rows, cols, outlier, error = case
+    x = torch.randn(rows, cols, device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows + cols))
+    lane = lib.bsq_lane_create(rows, cols, outlier, error, -1, 1, -1, -1, q)
+    assert lane
+    try:
+        cap = int(lib.bsq_lane_packed_capacity(lane))
+        buf = torch.empty(cap, dtype=torch.uint8, device="cuda")
+        room = torch.full((rows * cols + 8,), 7.0, device="cuda")
+        torch.cuda.synchronize()
+        hdr, out = pkg.Array(), C.c_void_p(None)
+        assert lib.bsq_lane_compress_begin(lane, x.data_ptr(), 1, buf.data_ptr(), cap) == 0
+        assert lib.bsq_lane_compress_end(lane, None, C.byref(hdr), None) == 0
+        assert lib.bsq_lane_compress_begin(lane, x.data_ptr(), 1, None, 0) == 0
+        assert lib.bsq_lane_compress_end(lane, C.byref(out), None, None) == 0
+        want = torch.empty_like(x)
+        torch.cuda.synchronize()
+        assert lib.bsq_lane_decompress_begin(lane, out, 0, want.data_ptr(), rows * cols) == 0
+        assert lib.bsq_lane_decompress_end(lane) == 0
+        for off in (4, 1):                                    # on a 16-byte boundary and off it
+            y = room[off: off + rows * cols]
+            assert lib.bsq_lane_decompress_begin(lane, C.byref(hdr), 1, y.data_ptr(), rows * cols) == 0
+            assert lib.bsq_lane_decompress_end(lane) == 0
+            torch.cuda.synchronize()
+            assert torch.equal(y.view(torch.int32), want.view(torch.int32).reshape(-1)), off
+            assert (room[:off] == 7.0).all() and (room[off + rows * cols:] == 7.0).all()
+            room.fill_(7.0)
+            torch.cuda.synchronize()
+        lib.bsq_free(out)
+    finally:
+        lib.bsq_lane_destroy(lane)
+
+
+def test_refused_object_leaves_the_result_alone(pkg, lib):
+    """The kernel is launched before the host knows what the payload's headers say; a header that differs in any checked byte keeps
+    it from writing, and a column that the matrix does not have fails the call."""
+    rows, cols = 96, 640
+    x = torch.randn(rows, cols, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    lane = lib.bsq_lane_create(rows, cols, 0.02, 0.02, -1, 1, -1, -1, 10)
+    assert lane
+    try:
+        cap = int(lib.bsq_lane_packed_capacity(lane))
+        buf = torch.empty(cap, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        hdr = pkg.Array()
+        assert lib.bsq_lane_compress_begin(lane, x.data_ptr(), 1, buf.data_ptr(), cap) == 0
+        assert lib.bsq_lane_compress_end(lane, None, C.byref(hdr), None) == 0
+        y = torch.full_like(x, 7.0)
+        direct, err = 200 + hdr.section_direct.offset, 200 + hdr.section_error_topk.offset
+        for at in (direct + 3, direct + 4, direct + 8, direct + 17, direct + 39, 200 + hdr.section_outlier_topk.offset, err + 2, err + 5):
+            good = int(buf[at])
+            buf[at] = good ^ 0x10
+            torch.cuda.synchronize()
+            assert lib.bsq_lane_decompress_begin(lane, C.byref(hdr), 1, y.data_ptr(), rows * cols) == 1, at
+            torch.cuda.synchronize()
+            assert (y == 7.0).all(), at
+            buf[at] = good
+        good = buf[err + 8: err + 10].clone()
+        buf[err + 8: err + 10] = 0xFF                         # column 65535 of 640
+        torch.cuda.synchronize()
+        assert lib.bsq_lane_decompress_begin(lane, C.byref(hdr), 1, y.data_ptr(), rows * cols) == 0
+        assert lib.bsq_lane_decompress_end(lane) == 1
+        buf[err + 8: err + 10] = good
+        torch.cuda.synchronize()
+        assert lib.bsq_lane_decompress_begin(lane, C.byref(hdr), 1, y.data_ptr(), rows * cols) == 0
+        assert lib.bsq_lane_decompress_end(lane) == 0
+    finally:
+        lib.bsq_lane_destroy(lane)
