@@ -244,7 +244,7 @@ struct Runtime {
     uint8_t *h_stage = nullptr;                          // pinned: section headers of a device-resident object on their way in
     DevicePack pack;
     CompressJob job;
-    bool decompress_active = false;
+    bool decompress_active = false, ends_by_kernel = false;   // ends_by_kernel: the call's last kernel clears the status words
     unsigned head_number = 0;                            // of the last HeadCheck (even)
     unsigned inject_status = 0;                          // test hook: OR-ed into the status word of the next call
 
@@ -360,6 +360,8 @@ bool setup_runtime(Runtime &rt, bool compress, uint16_t rows, uint16_t cols, flo
     }
     if (rt.uses_quant) {
         size_t scratch = nf4dq_scratch_bytes(n);
+        if (compress && has_svd)                            // (both factors at once)
+            scratch = std::max(scratch, nf4dq_scratch_bytes((uint64_t)rows * rt.rank) + nf4dq_scratch_bytes((uint64_t)cols * rt.rank));
         scratch = std::max(scratch, frontend_scratch_bytes(rows, cols));
         if (!rt.scratch.alloc(scratch)) return false;
         if (cudaMemset(rt.scratch.p, 0, 16) != cudaSuccess) return false;      // the front end's carried selection bound starts empty
@@ -521,6 +523,31 @@ bool run_quantize(Runtime &rt, int method, const float *d_src, QuantBufs &q, int
         err = nf4dq_quantize(d_src, q.n, q.dq.as<float>(), q.scale_codes.as<uint8_t>(), q.data.as<uint8_t>(), d_deq,
                              rt.scratch.p, rt.sm_count, rt.stream, d_error_flag, rt.status.as<unsigned>() + max_word);
     return err == cudaSuccess;
+}
+
+// U and V into q_u and q_v at once; with an error stage behind it they become the dequantised values, and the status words take the
+// maxima that the reconstruction's scales come from (S is what that stage will use).
+bool run_quantize_factors(Runtime &rt, bool error_path) {
+    unsigned *words = rt.status.as<unsigned>();
+    const auto target = [&](DevBuf &x, QuantBufs &q, int gmax_word, int max_word) {
+        QuantTarget t;
+        t.x = x.as<float>();
+        t.n = q.n;
+        t.scales = q.scales_f32.as<float>();
+        t.dq = q.dq.as<float>();
+        t.scale_codes = q.scale_codes.as<uint8_t>();
+        t.data = q.data.as<uint8_t>();
+        t.gmax = words + gmax_word;
+        if (error_path) {
+            t.deq = x.as<float>();
+            t.max_bits = words + max_word;
+        }
+        return t;
+    };
+    QuantTarget u = target(rt.u, rt.q_u, kWordMaxU, kWordMaxUS);
+    u.colscale = rt.s.as<float>();
+    u.cols = (uint32_t)rt.rank;
+    return quantize_pair(rt.uv_format, u, target(rt.v, rt.q_v, kWordMaxV, kWordMaxVR), rt.scratch.p, rt.sm_count, rt.stream) == cudaSuccess;
 }
 
 double ms_between(cudaEvent_t a, cudaEvent_t b) {
@@ -697,17 +724,14 @@ int compress_begin(Runtime &rt, const float *x, int input_location, uint8_t *d_p
             return fail();
         mark(); job.ev_svd = job.nev - 1;
         // quantised factors replace U, S, V in place for the error stage (src/bitsqz_llm.cu:1078-1139)
-        if (rt.uv_format != quantization_NONE) {
-            if (!run_quantize(rt, rt.uv_format, rt.u.as<float>(), rt.q_u, kWordMaxU, error_path ? rt.u.as<float>() : nullptr)) return fail();
-            if (!run_quantize(rt, rt.uv_format, rt.v.as<float>(), rt.q_v, kWordMaxV, error_path ? rt.v.as<float>() : nullptr)) return fail();
-        }
         if (rt.s_format != quantization_NONE)
             if (!run_quantize(rt, rt.s_format, rt.s.as<float>(), rt.q_s, kWordMaxOne, error_path ? rt.s.as<float>() : nullptr)) return fail();
+        if (rt.uv_format != quantization_NONE && !run_quantize_factors(rt, error_path)) return fail();
         mark(); job.ev_quant = job.nev - 1;
         if (error_path) {
             if (reconstruct_lowrank(rt.u.as<float>(), rt.s.as<float>(), rt.v.as<float>(), rows, cols, (int)rank, d_src,
                                     rt.error.as<float>(), d_status + kWordError, d_status, rt.recon_ws.as<float>(), rt.recon_ws_bytes, rt.sm_count,
-                                    st) != cudaSuccess)
+                                    st, rt.uv_format != quantization_NONE ? d_status + kWordMaxUS : nullptr, d_status + kWordMaxVR) != cudaSuccess)
                 return fail();
             mark(); job.ev_recon = job.nev - 1;
         }
@@ -1101,14 +1125,23 @@ bool expect_heads(Runtime &rt, const bitsqz_llm_array_t *c, HeadCheck *check, ui
         add(s, &h, sizeof(h), span(0, 6));
         return true;
     };
+    const auto fp32 = [&](const bitsqz_section_t &s, uint64_t count) { return s.storage == BITSQZ_SECTION_FP32 && s.size == 4 * count; };
     check->answer = reinterpret_cast<unsigned *>(rt.h_stage + kStageBytes) - 1;
     check->number = rt.head_number += 2;
-    return quant(c->section_direct, c->quantization_only_format, c->num_elements) &&
-           (!(c->flags & kFlagError) || topk(c->section_error_topk, rt.err, k_err)) &&
+    if (c->flags & kFlagSvd) {
+        const uint64_t rank = (uint16_t)c->effective_rank, u = c->num_rows * rank, v = c->num_columns * rank;
+        if (c->section_u.storage == BITSQZ_SECTION_QUANT ? !quant(c->section_u, c->svd_uv_format, u) : !fp32(c->section_u, u)) return false;
+        if (c->section_v.storage == BITSQZ_SECTION_QUANT ? !quant(c->section_v, c->svd_uv_format, v) : !fp32(c->section_v, v)) return false;
+        if (!fp32(c->section_s, rank)) return false;
+    } else if (!quant(c->section_direct, c->quantization_only_format, c->num_elements)) {
+        return false;
+    }
+    return (!(c->flags & kFlagError) || topk(c->section_error_topk, rt.err, k_err)) &&
            (!(c->flags & kFlagOutlier) || topk(c->section_outlier_topk, rt.outlier, k_out));
 }
 // Waits for what the kernel launched with `check` has found (it has hardly begun then).
 bool heads_as_expected(Runtime &rt, const HeadCheck &check) {
+    if (check.count == 0) return true;
     const volatile unsigned *answer = check.answer;
     for (unsigned i = 1; (*answer | 1u) != (check.number | 1u); ++i) {
         if (i % 4096 != 0) continue;
@@ -1118,14 +1151,18 @@ bool heads_as_expected(Runtime &rt, const HeadCheck &check) {
     }
     return *answer == check.number;
 }
-SectionSource quant_source(const bitsqz_llm_array_t *c, const bitsqz_section_t &s, int method, uint64_t count) {
+SectionSource section_source(const bitsqz_llm_array_t *c, const bitsqz_section_t &s, int method, uint64_t count) {
     const uint8_t *at = static_cast<const uint8_t *>(c->payload) + s.offset;
     const uint64_t nb = (count + 63) / 64;
     SectionSource q;
+    q.n = count;
+    if (s.storage == BITSQZ_SECTION_FP32) {
+        q.data = at;
+        return q;
+    }
     q.scales = at + sizeof(QuantHeader);
     q.dq = method == NF4 ? nullptr : at + offsetof(QuantHeader, dq_scale);
     q.data = q.scales + (method == NF4 ? nb * 4 : nb);
-    q.n = count;
     return q;
 }
 ListSource list_source(const bitsqz_llm_array_t *c, const bitsqz_section_t &s, uint32_t k) {
@@ -1136,9 +1173,10 @@ ListSource list_source(const bitsqz_llm_array_t *c, const bitsqz_section_t &s, u
     return l;
 }
 
-// A quantised matrix with its lists, device-resident, all of it within reach of kernels and apart from the result: one kernel
-// checks the headers, decodes, adds the lists and reports.
-int decompress_begin_one_kernel(Runtime &rt, const bitsqz_llm_array_t *c, float *d_dst) {
+// A device-resident object, all of it within reach of kernels and apart from the result.  A quantised matrix: one kernel checks the
+// headers, decodes, adds the lists and reports.  Factors: one opens them beside the check, two make the product, and once the headers
+// are known to be good one adds the lists and reports.
+int decompress_begin_in_place(Runtime &rt, const bitsqz_llm_array_t *c, float *d_dst) {
     cudaStream_t st = rt.stream;
     HeadCheck check{};
     uint32_t k_err = 0, k_out = 0;
@@ -1148,14 +1186,35 @@ int decompress_begin_one_kernel(Runtime &rt, const bitsqz_llm_array_t *c, float 
         cudaGetLastError();
         return 1;
     };
+    unsigned *d_status = rt.status.as<unsigned>();
+    const ListSource err = list_source(c, c->section_error_topk, k_err), out = list_source(c, c->section_outlier_topk, k_out);
     rt.h_status[0] = rt.inject_status;                        // (the stream is idle: one call at a time, and the last one has been waited for)
     rt.inject_status = 0;
-    // error list first, outliers second (src/bitsqz_llm.cu:1372-1387)
-    if (decode_matrix(quant_source(c, c->section_direct, c->quantization_only_format, c->num_elements), c->num_rows, c->num_columns,
-                      list_source(c, c->section_error_topk, k_err), list_source(c, c->section_outlier_topk, k_out), d_dst, rt.h_status, check,
-                      rt.sm_count, st) != cudaSuccess)
+    // (both ways: error list first, outliers second, src/bitsqz_llm.cu:1372-1387)
+    if (!(c->flags & kFlagSvd)) {
+        if (decode_matrix(section_source(c, c->section_direct, c->quantization_only_format, c->num_elements), c->num_rows, c->num_columns, err, out,
+                          d_dst, rt.h_status, check, rt.sm_count, st) != cudaSuccess ||
+            !heads_as_expected(rt, check))
+            return fail();
+        rt.decompress_active = true;
+        return 0;
+    }
+    const uint32_t rank = (uint16_t)c->effective_rank;
+    const bool words_clear = rt.words_clear;
+    rt.words_clear = false;
+    if (!words_clear && cudaMemsetAsync(d_status, 0, 4 * kStatusWords, st) != cudaSuccess) return fail();
+    if (open_factors(section_source(c, c->section_u, c->svd_uv_format, (uint64_t)c->num_rows * rank),
+                     section_source(c, c->section_v, c->svd_uv_format, (uint64_t)c->num_columns * rank),
+                     static_cast<const uint8_t *>(c->payload) + c->section_s.offset, rank, rt.u.as<float>(), rt.v.as<float>(), rt.s.as<float>(),
+                     d_status + kWordMaxUS, d_status + kWordMaxVR, check, rt.sm_count, st) != cudaSuccess ||
+        !heads_as_expected(rt, check))
         return fail();
-    if (!heads_as_expected(rt, check)) return fail();
+    if (reconstruct_lowrank(rt.u.as<float>(), rt.s.as<float>(), rt.v.as<float>(), c->num_rows, c->num_columns, (int)rank, nullptr, d_dst, nullptr,
+                            d_status, rt.recon_ws.as<float>(), rt.recon_ws_bytes, rt.sm_count, st, d_status + kWordMaxUS, d_status + kWordMaxVR) !=
+            cudaSuccess ||
+        apply_lists_end(err, out, c->num_rows, c->num_columns, d_dst, d_status, rt.h_status, st) != cudaSuccess)
+        return fail();
+    rt.ends_by_kernel = true;
     rt.decompress_active = true;
     return 0;
 }
@@ -1177,10 +1236,15 @@ int decompress_begin(Runtime &rt, const bitsqz_llm_array_t *c, bool payload_on_d
     bool kernels_read = false;
     for (const bitsqz_section_t *s : {&c->section_u, &c->section_s, &c->section_v, &c->section_direct, &c->section_outlier_topk, &c->section_error_topk})
         kernels_read = kernels_read || s->storage == BITSQZ_SECTION_QUANT || s->storage == BITSQZ_SECTION_TOPK;
-    const Reach reach = payload_on_device && kernels_read ? memory_reach(c->payload, payload_bytes) : Reach::kCopies;
+    // (FP32 factors are opened by a kernel too where one reaches them; other objects without headers in them move by copies wherever they are)
+    Reach reach = payload_on_device && (kernels_read || (c->flags & kFlagSvd)) ? memory_reach(c->payload, payload_bytes) : Reach::kCopies;
+    if (!kernels_read && reach == Reach::kNone) reach = Reach::kCopies;
     const bool over_object = ranges_overlap(d_dst, (uint64_t)c->num_elements * 4, c->payload, payload_bytes);
-    if (reach == Reach::kKernels && !over_object && c->section_direct.storage == BITSQZ_SECTION_QUANT)
-        return decompress_begin_one_kernel(rt, c, d_dst);
+    rt.ends_by_kernel = false;
+    if (reach == Reach::kKernels && !over_object &&
+        ((c->flags & kFlagSvd) ? c->section_s.storage == BITSQZ_SECTION_FP32 : c->section_direct.storage == BITSQZ_SECTION_QUANT))
+        return decompress_begin_in_place(rt, c, d_dst);
+    rt.words_clear = false;
     if (!fetch_heads(rt, c, payload_on_device, reach, &heads)) return fail();
     const bool has_out = c->flags & kFlagOutlier, has_err = c->flags & kFlagError;
     if (has_out && !topk_section_ok(rt.outlier, c, c->section_outlier_topk, heads.outlier)) return 1;
@@ -1237,6 +1301,7 @@ int decompress_end(Runtime &rt) {
         cudaGetLastError();
         return 1;
     }
+    if (rt.ends_by_kernel) rt.words_clear = true;
     return rt.h_status[0] == 0 ? 0 : 1;
 }
 

@@ -297,15 +297,16 @@ size_t gemm_workspace_bytes(int M, int N, int max_splits) { return (size_t)M * N
 cudaError_t gemm(bool a_kmajor, bool b_kmajor, const float *A, long lda, const float *B, long ldb, float *C, long ldc, int M,
                  int N, int K, const float *kscale, const float *minuend, long ldm, unsigned *flag, unsigned *status,
                  float *workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream, const unsigned *a_absmax_bits, float b_bound,
-                 bool device_full) {
+                 bool device_full, const unsigned *b_absmax_bits) {
     return gemm_select(tensor_cores_enabled(), a_kmajor, b_kmajor, A, lda, B, ldb, C, ldc, M, N, K, kscale, minuend, ldm, flag,
-                       status, workspace, workspace_bytes, sm_count, stream, a_absmax_bits, b_bound, device_full);
+                       status, workspace, workspace_bytes, sm_count, stream, a_absmax_bits, b_bound, device_full, b_absmax_bits);
 }
 
 cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, const float *A, long lda, const float *B, long ldb,
                         float *C, long ldc, int M, int N, int K, const float *kscale, const float *minuend, long ldm,
                         unsigned *flag, unsigned *status, float *workspace, size_t workspace_bytes, int sm_count,
-                        cudaStream_t stream, const unsigned *a_absmax_bits, float b_bound, bool device_full) {
+                        cudaStream_t stream, const unsigned *a_absmax_bits, float b_bound, bool device_full,
+                        const unsigned *b_absmax_bits) {
     if (M <= 0 || N <= 0 || K <= 0) return cudaErrorInvalidValue;
     if (allow_tensor_cores) {
         // tensor-core path: one 128-row tile per CTA, two CTAs per SM up to N = 128; K is split so that the tiles fill
@@ -373,14 +374,15 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
                         t.n_tile = 256;                                 // (B's images were given room for 256-column tiles above)
                         t.wide_tiles = true;
                         // ... and both operands as FP16 halves (low halves without their factor: the tile's products share
-                        // one accumulator); the scales come from the largest |A kscale| and |B|, found by a pass over each
-                        // (they are small); the FP16 images take half the room, its last words hold the two maxima
+                        // one accumulator); the scales come from the largest |A kscale| and |B|, the caller's or found by a
+                        // pass over each (the FP16 images take half the room, its last words hold the two maxima)
                         if (f16_mode() >= 1 && K % 8 == 0) {
                             unsigned *words = reinterpret_cast<unsigned *>(reinterpret_cast<unsigned char *>(workspace) + a_room - 256);
                             t.f16 = true;
                             t.lo_unscaled = true;
-                            t.a_absmax_bits = words;
-                            t.b_absmax_bits = words + 1;
+                            t.maxima_given = a_absmax_bits && b_absmax_bits;
+                            t.a_absmax_bits = t.maxima_given ? a_absmax_bits : words;
+                            t.b_absmax_bits = t.maxima_given ? b_absmax_bits : words + 1;
                         }
                     }
                 }

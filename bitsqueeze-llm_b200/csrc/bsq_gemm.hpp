@@ -37,6 +37,7 @@ struct GemmArgs {
     bool f16;                      // TMA-fed kernel: operands split into two FP16 halves (bsq_gemm_tc.cuh) instead of two TF32
     const unsigned *a_absmax_bits; // halves; device words with the bits of the largest |A| and |B| (finite), from which the
     const unsigned *b_absmax_bits; // power-of-two scales of the split come
+    bool maxima_given;             // with a_image: both words are the caller's and hold their values when the call runs
     float b_scale_fixed;           // > 0: the scale of B given by the caller (from a bound it knows) instead of *b_absmax_bits
     bool lo_unscaled;              // the low halves are fp16(x s - hi) without the factor 2^11, so that all three products of a
                                    // term can share ONE accumulator (the persistent product's 256-column tiles); elements more

@@ -547,15 +547,21 @@ __global__ void __launch_bounds__(256) absmax_bits_kernel(const float *x, long l
 // The FP16 form of presplit_b_kernel: one thread per (chunk of 32 k, unit of 8 k, column): the eight values
 // B(32 c + 8 kc .. + 7, n0 + r), scaled, as the hi and the lo unit of the chunk's image (same unit order and image size
 // as the TF32 images, which hold 16 k per chunk).  k past K gives zeros.
+struct PresplitB16 {
+    const float *B;
+    long ldb;
+    int N, K, n_tile, chunks;
+    uint4 *image;
+    const unsigned *absmax_bits;
+    float fixed_scale, lo_scale;
+};
 template <bool B_KMAJOR>
-__global__ void __launch_bounds__(256) presplit_b16_kernel(const float *B, long ldb, int N, int K, int n_tile, int chunks,
-                                                           uint4 *__restrict__ image, const unsigned *absmax_bits, float fixed_scale,
-                                                           float lo_scale) {
-    chain_begin();
-    const int n0 = blockIdx.y * n_tile;
-    const int Nt = min(n_tile, N - n0);
-    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long)chunks * 4 * Nt) return;
+__device__ __forceinline__ void presplit_b16_unit(const PresplitB16 &p, int tile, long idx) {
+    const int n0 = tile * p.n_tile, K = p.K;
+    const int Nt = min(p.n_tile, p.N - n0);
+    const long ldb = p.ldb;
+    const float *B = p.B;
+    if (idx >= (long)p.chunks * 4 * Nt) return;
     int kc, r;
     if (B_KMAJOR) {
         kc = (int)(idx % 4);
@@ -568,47 +574,68 @@ __global__ void __launch_bounds__(256) presplit_b16_kernel(const float *B, long 
     const long k = c * 32 + kc * 8;
     float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (B_KMAJOR) {
-        const float *p = B + (long)(n0 + r) * ldb + k;
+        const float *q = B + (long)(n0 + r) * ldb + k;
         if (k + 7 < K) {
-            const float4 q0 = *reinterpret_cast<const float4 *>(p), q1 = *reinterpret_cast<const float4 *>(p + 4);
+            const float4 q0 = *reinterpret_cast<const float4 *>(q), q1 = *reinterpret_cast<const float4 *>(q + 4);
             v[0] = q0.x; v[1] = q0.y; v[2] = q0.z; v[3] = q0.w; v[4] = q1.x; v[5] = q1.y; v[6] = q1.z; v[7] = q1.w;
         } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-                if (k + j < K) v[j] = p[j];
+                if (k + j < K) v[j] = q[j];
         }
     } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
             if (k + j < K) v[j] = B[(k + j) * ldb + n0 + r];
     }
-    uint4 *img = image + ((size_t)blockIdx.y * chunks + c) * image_units(n_tile);
+    uint4 *img = p.image + ((size_t)tile * p.chunks + c) * image_units(p.n_tile);
     const unsigned u = image_unit_index(kc, r, Nt);
-    split16_store8(make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]), fixed_scale > 0.0f ? fixed_scale : split16_scale(*absmax_bits), img + u,
-                   img + image_half_units(Nt) + u, lo_scale);
+    split16_store8(make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]),
+                   p.fixed_scale > 0.0f ? p.fixed_scale : split16_scale(*p.absmax_bits), img + u, img + image_half_units(Nt) + u, p.lo_scale);
+}
+template <bool B_KMAJOR>
+__global__ void __launch_bounds__(256) presplit_b16_kernel(PresplitB16 p) {
+    chain_begin();
+    presplit_b16_unit<B_KMAJOR>(p, blockIdx.y, (long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // The FP16 form of presplit_a_kernel: two row-major rows_pad x K matrices of FP16 values, hi then lo, eight k per thread;
-// the scale comes from *absmax_bits, the largest |A(m, k) kscale(k)| (absmax_bits_kernel with the same kscale).
-__global__ void __launch_bounds__(256) presplit_a16_kernel(const float *A, long lda, int M, int K, const float *kscale,
-                                                           uint4 *__restrict__ image, int rows_pad, const unsigned *absmax_bits,
-                                                           float lo_scale) {
-    chain_begin();
-    const int k8 = K / 8;
-    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (long)rows_pad * k8) return;
+// the scale comes from *absmax_bits, the largest |A(m, k) kscale(k)|.
+struct PresplitA16 {
+    const float *A;
+    long lda;
+    int M, K;
+    const float *kscale;
+    uint4 *image;
+    int rows_pad;
+    const unsigned *absmax_bits;
+    float lo_scale;
+};
+__device__ __forceinline__ void presplit_a16_unit(const PresplitA16 &p, long idx) {
+    const int k8 = p.K / 8;
+    const float *kscale = p.kscale;
+    if (idx >= (long)p.rows_pad * k8) return;
     const int m = (int)(idx / k8), k = (int)(idx % k8) * 8;
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-    if (m < M) {
-        a = *reinterpret_cast<const float4 *>(A + (long)m * lda + k);
-        b = *reinterpret_cast<const float4 *>(A + (long)m * lda + k + 4);
+    if (m < p.M) {
+        a = *reinterpret_cast<const float4 *>(p.A + (long)m * p.lda + k);
+        b = *reinterpret_cast<const float4 *>(p.A + (long)m * p.lda + k + 4);
         if (kscale) {
             a.x *= kscale[k]; a.y *= kscale[k + 1]; a.z *= kscale[k + 2]; a.w *= kscale[k + 3];
             b.x *= kscale[k + 4]; b.y *= kscale[k + 5]; b.z *= kscale[k + 6]; b.w *= kscale[k + 7];
         }
     }
-    uint4 *hi = image + idx;
-    split16_store8(a, b, split16_scale(*absmax_bits), hi, hi + (long)rows_pad * k8, lo_scale);
+    uint4 *hi = p.image + idx;
+    split16_store8(a, b, split16_scale(*p.absmax_bits), hi, hi + (long)p.rows_pad * k8, p.lo_scale);
+}
+// Both operands of a reconstruction in one launch: CTAs up to b_ctas * n_tiles make B's images.  (4096 x 14336 at rank 256 7.4 us, as two
+// launches 5.8 + 3.6 and the gap between them; 2048 x 5120 at rank 64 2.5 against 2.3 + 2.0.)
+__global__ void __launch_bounds__(256) presplit_pair16_kernel(PresplitB16 b, PresplitA16 a, unsigned b_ctas, unsigned n_tiles) {
+    chain_begin();
+    if (blockIdx.x < b_ctas * n_tiles)
+        presplit_b16_unit<true>(b, blockIdx.x / b_ctas, (long)(blockIdx.x % b_ctas) * blockDim.x + threadIdx.x);
+    else
+        presplit_a16_unit(a, (long)(blockIdx.x - b_ctas * n_tiles) * blockDim.x + threadIdx.x);
 }
 
 template <bool A_KMAJOR, int NMAX>
@@ -797,29 +824,34 @@ cudaError_t launch_image(const GemmArgs &g, bool b_kmajor, unsigned *status, cud
     if (g.f16) {
         // the scale of B's split comes from its largest magnitude (B is a panel: a pass over it costs microseconds)
         // (unless the caller knows a bound: FP16 is floating point, so a loose bound costs range, not precision)
-        unsigned *bmax = const_cast<unsigned *>(g.b_absmax_bits);
-        if (!(g.b_scale_fixed > 0.0f)) {
-            if ((err = cudaMemsetAsync(bmax, 0, sizeof(unsigned), stream)) != cudaSuccess) return err;
-            const int b_rows = b_kmajor ? g.N : g.K, b_cols = b_kmajor ? g.K : g.N;
-            absmax_bits_kernel<<<592, 256, 0, stream>>>(g.B, g.ldb, b_rows, b_cols, bmax);
-        }
-        uint4 *image16 = reinterpret_cast<uint4 *>(image);
         const float lo_scale = g.lo_unscaled ? 1.0f : kSplit16LoScale;
-        if (b_kmajor) launch_chained(presplit_b16_kernel<true>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image16, bmax, g.b_scale_fixed, lo_scale);
-        else launch_chained(presplit_b16_kernel<false>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image16, bmax, g.b_scale_fixed, lo_scale);
+        const PresplitB16 pb{g.B, g.ldb, g.N, g.K, g.n_tile, chunks, reinterpret_cast<uint4 *>(image), g.b_absmax_bits, g.b_scale_fixed, lo_scale};
+        const PresplitA16 pa{g.A, g.lda, g.M, g.K, g.kscale, reinterpret_cast<uint4 *>(g.a_image), g.a_image_rows, g.a_absmax_bits, lo_scale};
+        const bool with_a = g.use_tma && g.a_image;
+        const unsigned a_ctas = with_a ? (unsigned)(((long)g.a_image_rows * (g.K / 8) + 255) / 256) : 0;
+        if (with_a && !g.maxima_given) {
+            // the largest |B| and |A kscale| for the scales (words side by side)
+            unsigned *amax = const_cast<unsigned *>(g.a_absmax_bits), *bmax = const_cast<unsigned *>(g.b_absmax_bits);
+            if ((err = cudaMemsetAsync(amax, 0, 2 * sizeof(unsigned), stream)) != cudaSuccess) return err;
+            absmax_bits_kernel<<<592, 256, 0, stream>>>(g.B, g.ldb, b_kmajor ? g.N : g.K, b_kmajor ? g.K : g.N, bmax);
+            absmax_bits_kernel<<<592, 256, 0, stream>>>(g.A, g.lda, g.M, g.K, amax, g.kscale);
+        } else if (!with_a && !(g.b_scale_fixed > 0.0f)) {
+            unsigned *bmax = const_cast<unsigned *>(g.b_absmax_bits);
+            if ((err = cudaMemsetAsync(bmax, 0, sizeof(unsigned), stream)) != cudaSuccess) return err;
+            absmax_bits_kernel<<<592, 256, 0, stream>>>(g.B, g.ldb, b_kmajor ? g.N : g.K, b_kmajor ? g.K : g.N, bmax);
+        }
+        if (with_a && b_kmajor) {
+            launch_chained(presplit_pair16_kernel, pgrid.x * n_tiles + a_ctas, 256, 0, stream, pb, pa, pgrid.x, n_tiles);
+        } else {
+            if (b_kmajor) launch_chained(presplit_b16_kernel<true>, pgrid, 256, 0, stream, pb);
+            else launch_chained(presplit_b16_kernel<false>, pgrid, 256, 0, stream, pb);
+            if (with_a) launch_chained(presplit_pair16_kernel, a_ctas, 256, 0, stream, pb, pa, 0u, 0u);
+        }
     } else if (b_kmajor) launch_chained(presplit_b_kernel<true>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image);
     else launch_chained(presplit_b_kernel<false>, pgrid, 256, 0, stream, g.B, g.ldb, g.N, g.K, g.n_tile, chunks, image);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
-    if (g.use_tma && g.a_image && g.f16) {
-        // the largest |A kscale| for the scale, then the two FP16 matrices
-        unsigned *amax = const_cast<unsigned *>(g.a_absmax_bits);
-        if ((err = cudaMemsetAsync(amax, 0, sizeof(unsigned), stream)) != cudaSuccess) return err;
-        absmax_bits_kernel<<<592, 256, 0, stream>>>(g.A, g.lda, g.M, g.K, amax, g.kscale);
-        const long units = (long)g.a_image_rows * (g.K / 8);
-        presplit_a16_kernel<<<(unsigned)((units + 255) / 256), 256, 0, stream>>>(g.A, g.lda, g.M, g.K, g.kscale, reinterpret_cast<uint4 *>(g.a_image),
-                                                                                  g.a_image_rows, amax, g.lo_unscaled ? 1.0f : kSplit16LoScale);
-        if ((err = cudaGetLastError()) != cudaSuccess) return err;
+    if (g.f16) {
     } else if (g.use_tma && g.a_image) {
         const long quads = (long)g.a_image_rows * (g.K / 4);
         presplit_a_kernel<<<(unsigned)((quads + 255) / 256), 256, 0, stream>>>(g.A, g.lda, g.M, g.K, g.kscale, g.a_image, g.a_image_rows);

@@ -44,6 +44,23 @@ cudaError_t nf4_dequantize(const float *d_scales, const uint8_t *d_data, uint64_
                            cudaStream_t stream);
 cudaError_t nf4dq_dequantize(const float *d_dq, const uint8_t *d_scale_codes, const uint8_t *d_data, uint64_t n,
                              float *d_out, int sm_count, cudaStream_t stream);
+// Two arrays of one format at once (the factors U and V), each with what it is quantised into; NF4_DQ: gmax is a device word that is
+// zero, scratch holds nf4dq_scratch_bytes of both.  deq (nullable, may be x): the dequantised values; max_bits (nullable, with deq; zero before)
+// receives the bits of the largest |deq(i) colscale(i mod cols)|, colscale nullable.
+struct QuantTarget {
+    const float *x = nullptr;
+    uint64_t n = 0;
+    float *scales = nullptr;              // NF4
+    float *dq = nullptr;                  // NF4_DQ
+    uint8_t *scale_codes = nullptr;
+    uint8_t *data = nullptr;
+    float *deq = nullptr;
+    unsigned *gmax = nullptr;
+    const float *colscale = nullptr;
+    uint32_t cols = 1;
+    unsigned *max_bits = nullptr;
+};
+cudaError_t quantize_pair(int method, const QuantTarget &a, const QuantTarget &b, void *d_scratch, int sm_count, cudaStream_t stream);
 // A section as it lies in a device-resident object, whatever its alignment.
 struct SectionSource {
     const uint8_t *scales = nullptr;      // NF4: FP32, NF4_DQ: E4M3
@@ -65,6 +82,11 @@ cudaError_t decode_matrix(const SectionSource &q, uint32_t rows, uint32_t cols, 
 cudaError_t nf4_dequantize_add_topk(const float *d_scales, const float *d_dq, const uint8_t *d_scale_codes, const uint8_t *d_data,
                                     uint32_t rows, uint32_t cols, const uint16_t *d_idx, const float *d_val, uint32_t k,
                                     float *d_out, unsigned *d_status, int sm_count, cudaStream_t stream);
+
+// The factors U (rows x rank), V and S (rank FP32 values) of an object into 16-byte aligned buffers, in one launch; *d_max_us and *d_max_v
+// (zero before) receive the bits of the largest |U(i, t) S(t)| and |V|.  What the buffers hold is of no use where `heads` finds a difference.
+cudaError_t open_factors(const SectionSource &u, const SectionSource &v, const uint8_t *s, uint32_t rank, float *d_u, float *d_v, float *d_s,
+                         unsigned *d_max_us, unsigned *d_max_v, const HeadCheck &heads, int sm_count, cudaStream_t stream);
 
 // ---- per-row top-k (bsq_topk.cu) ------------------------------------------------------------
 // k = (uint16)roundf(cols * ratio) clamped to cols, at least 1 for ratio > 0; -1 for a ratio
@@ -88,6 +110,10 @@ cudaError_t topk_apply(const uint16_t *d_idx, const float *d_val, uint32_t rows,
 // Two lists, the first before the second where they name the same element, in one launch or two.
 cudaError_t topk_apply_two(const uint16_t *d_idx0, const float *d_val0, uint32_t k0, const uint16_t *d_idx1, const float *d_val1,
                            uint32_t k1, uint32_t rows, uint32_t cols, float *d_dense, unsigned *d_status, cudaStream_t stream);
+// The same with the lists where they lie in an object, either or both possibly empty, as the end of a decompress call: status words of the
+// call's earlier kernels, and columns out of range, are reported in the page-locked, zero `mirror`; the words are cleared.
+cudaError_t apply_lists_end(const ListSource &a, const ListSource &b, uint32_t rows, uint32_t cols, float *d_dense, unsigned *d_status,
+                            unsigned *mirror, cudaStream_t stream);
 
 // ---- fused front end of the no-SVD path (bsq_frontend.cu) -----------------------------------
 // outlier separation + NF4 or NF4_DQ of the remainder, reading the input once from HBM (the
@@ -122,7 +148,9 @@ enum : int {
     kWordMaxU = 5,                                           // NF4_DQ: the largest magnitude of a section
     kWordMaxV = 6,
     kWordMaxOne = 7,                                         // (the matrix or S)
-    kWordBound = 8                                           // bound of the residual for the SVD's products
+    kWordBound = 8,                                          // bound of the residual for the SVD's products
+    kWordMaxUS = 9,                                          // the largest |U S| and |V|: scales of the reconstruction's operands
+    kWordMaxVR = 10
 };
 struct CopySegment {
     void *dst;
@@ -181,14 +209,17 @@ void *host_block_take(size_t bytes);
 cudaError_t gemm(bool a_kmajor, bool b_kmajor, const float *A, long lda, const float *B, long ldb, float *C, long ldc, int M,
                  int N, int K, const float *kscale, const float *minuend, long ldm, unsigned *flag, unsigned *status,
                  float *workspace, size_t workspace_bytes, int sm_count, cudaStream_t stream, const unsigned *a_absmax_bits = nullptr,
-                 float b_bound = 0.0f, bool device_full = false);
+                 float b_bound = 0.0f, bool device_full = false,
+                 const unsigned *b_absmax_bits = nullptr);
 // The same with the kernel choice explicit: allow_tensor_cores = false keeps the product on the FP32 pipes.
 cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, const float *A, long lda, const float *B, long ldb,
                         float *C, long ldc, int M, int N, int K, const float *kscale, const float *minuend, long ldm,
                         unsigned *flag, unsigned *status, float *workspace, size_t workspace_bytes, int sm_count,
-                        cudaStream_t stream, const unsigned *a_absmax_bits = nullptr, float b_bound = 0.0f, bool device_full = false);
+                        cudaStream_t stream, const unsigned *a_absmax_bits = nullptr, float b_bound = 0.0f, bool device_full = false,
+                        const unsigned *b_absmax_bits = nullptr);
 // (a_absmax_bits: device word with the bits of an upper bound of |A|, b_bound: an upper bound of |B| known on the host,
-// 0 = none -- with a bound on |A| the 256-column products split their operands into FP16 halves, bsq_gemm_tc.cuh)
+// 0 = none -- with a bound on |A| the 256-column products split their operands into FP16 halves, bsq_gemm_tc.cuh;
+// a_absmax_bits and b_absmax_bits together: the largest |A kscale| and |B| for a wide product's split)
 
 struct SvdWorkspace;
 // sums `count` floats at `buf` over all ranks, enqueued on `stream`
@@ -219,9 +250,12 @@ cudaError_t svd_workspace_finish(SvdWorkspace *ws, cudaStream_t stream);
 // (the output is then incomplete).
 // d_workspace (nullable, reconstruct_workspace_bytes, 128-byte aligned): room for V and U diag(S) split once into the
 // tensor cores' operand format, shared by all tiles; without it every tile splits its pieces itself.
+// d_max_us, d_max_v (nullable): device words with the bits of the largest |U(i, t) S(t)| and |V|; without them the call makes a pass
+// over each.
 size_t reconstruct_workspace_bytes(int m, int n, int k);
 cudaError_t reconstruct_lowrank(const float *d_U, const float *d_S, const float *d_V, int m, int n, int k,
                                 const float *d_minuend, float *d_out, unsigned *d_flag, unsigned *d_status, float *d_workspace,
-                                size_t workspace_bytes, int sm_count, cudaStream_t stream);
+                                size_t workspace_bytes, int sm_count, cudaStream_t stream, const unsigned *d_max_us = nullptr,
+                                const unsigned *d_max_v = nullptr);
 
 }  // namespace bsq

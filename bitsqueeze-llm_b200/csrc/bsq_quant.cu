@@ -73,14 +73,40 @@ __device__ __forceinline__ float gather_block_value(const float (&am)[4], int la
     return s;
 }
 
+// One array of a launch, or two side by side: CTAs from `second` on take the second.
+struct EncodeJob {
+    const float *x;
+    uint64_t n;
+    bool vec;
+    const float *absmax_in;
+    unsigned *gmax_bits;
+    float *scales_f32;
+    uint8_t *scale_codes;
+    float *dq_out;
+    uint8_t *data;
+    float *deq_out;                                           // may alias x (in-place write-back)
+    unsigned *flag;
+    const float *colscale;
+    unsigned cols;
+    unsigned *max_bits;
+};
+struct EncodeJobs {
+    EncodeJob job[2];
+    unsigned second;
+};
+
 // ---- NF4_DQ pass 1: per-block absmax (1.0 for an all-zero block) and the global maximum ----
-__global__ void __launch_bounds__(kThreads) absmax_flat_kernel(const float *x, uint64_t n, bool vec,
-                                                               float *__restrict__ absmax_out,
-                                                               unsigned *__restrict__ gmax_bits) {
+__global__ void __launch_bounds__(kThreads) absmax_flat_kernel(const __grid_constant__ EncodeJobs jobs) {
     chain_begin();
     const int lane = threadIdx.x & 31;
-    const uint64_t warp = (uint64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-    const uint64_t nwarps = (uint64_t)gridDim.x * (kThreads / 32);
+    const bool other = blockIdx.x >= jobs.second;
+    const EncodeJob &job = jobs.job[other];
+    const float *x = job.x;
+    const uint64_t n = job.n;
+    const bool vec = job.vec;
+    float *absmax_out = const_cast<float *>(job.absmax_in);
+    const uint64_t warp = (uint64_t)(blockIdx.x - (other ? jobs.second : 0u)) * (kThreads / 32) + (threadIdx.x >> 5);
+    const uint64_t nwarps = (uint64_t)(other ? gridDim.x - jobs.second : jobs.second) * (kThreads / 32);
     const uint64_t nb = (n + 63) / 64;
     float run = 0.0f;
     for (uint64_t base = warp * kBatch; base < n; base += nwarps * kBatch) {
@@ -99,7 +125,7 @@ __global__ void __launch_bounds__(kThreads) absmax_flat_kernel(const float *x, u
         }
     }
     run = warp_max(run);
-    if (lane == 0 && run > 0.0f) atomicMax(gmax_bits, __float_as_uint(run));
+    if (lane == 0 && run > 0.0f) atomicMax(job.gmax_bits, __float_as_uint(run));
 }
 
 // ---- encode: NF4 (DQ == false: computes its own absmax) or NF4_DQ pass 2 -----------------
@@ -108,23 +134,27 @@ __global__ void __launch_bounds__(kThreads) absmax_flat_kernel(const float *x, u
 // src/bitsqz_llm.cu:164-184: without a pass of its own over two matrices).
 enum : int { kWriteNone = 0, kWriteDeq = 1, kWriteError = 2 };
 template <bool DQ, int WRITE>
-__global__ void __launch_bounds__(kThreads)
-    encode_flat_kernel(const float *x, uint64_t n, bool vec, const float *absmax_in,
-                       const unsigned *gmax_bits, float *__restrict__ scales_f32,
-                       uint8_t *__restrict__ scale_codes, float *__restrict__ dq_out, uint8_t *__restrict__ data,
-                       float *deq_out, unsigned *flag) {   // deq_out may alias x (in-place write-back)
+__global__ void __launch_bounds__(kThreads) encode_flat_kernel(const __grid_constant__ EncodeJobs jobs) {
     chain_begin();
     bool any = false;
+    unsigned largest = 0;
     const int lane = threadIdx.x & 31;
-    const uint64_t warp = (uint64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-    const uint64_t nwarps = (uint64_t)gridDim.x * (kThreads / 32);
+    const bool other = blockIdx.x >= jobs.second;
+    const EncodeJob &job = jobs.job[other];
+    const float *x = job.x;
+    const uint64_t n = job.n;
+    const bool vec = job.vec;
+    float *scales_f32 = job.scales_f32, *deq_out = job.deq_out;
+    uint8_t *scale_codes = job.scale_codes, *data = job.data;
+    const uint64_t warp = (uint64_t)(blockIdx.x - (other ? jobs.second : 0u)) * (kThreads / 32) + (threadIdx.x >> 5);
+    const uint64_t nwarps = (uint64_t)(other ? gridDim.x - jobs.second : jobs.second) * (kThreads / 32);
     const uint64_t nb = (n + 63) / 64;
     Nf4Lut lut;
     lut.load();
     float dq = 1.0f;
     if (DQ) {
-        dq = dq_from_max(__uint_as_float(*gmax_bits));
-        if (warp == 0 && lane == 0) *dq_out = dq;
+        dq = dq_from_max(__uint_as_float(*job.gmax_bits));
+        if (warp == 0 && lane == 0) *job.dq_out = dq;
     }
     for (uint64_t base = warp * kBatch; base < n; base += nwarps * kBatch) {
         Lane8 r[4];
@@ -143,7 +173,7 @@ __global__ void __launch_bounds__(kThreads)
             if (owns_block) scales_f32[blk] = scale;
         } else {
             if (owns_block) {
-                blk_absmax = absmax_in[blk];
+                blk_absmax = job.absmax_in[blk];
                 unsigned code;
                 scale = dq_block_scale(blk_absmax, dq, &code);
                 scale_codes[blk] = (uint8_t)code;
@@ -179,6 +209,15 @@ __global__ void __launch_bounds__(kThreads)
                         any |= e + q < n && fabsf(d[q]) > 1.1920928955078125e-07f;
                     }
                 }
+                if (WRITE == kWriteDeq && job.max_bits && e < n) {
+                    unsigned c = job.colscale ? (unsigned)e % job.cols : 0u;   // (a factor has fewer than 2^32 elements)
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const float v = job.colscale ? d[q] * job.colscale[c] : d[q];
+                        if (e + q < n) largest = max(largest, __float_as_uint(v) & 0x7fffffffu);
+                        if (++c == job.cols) c = 0;
+                    }
+                }
                 if (vec && e + 8 <= n) {
                     reinterpret_cast<float4 *>(deq_out + e)[0] = make_float4(d[0], d[1], d[2], d[3]);
                     reinterpret_cast<float4 *>(deq_out + e)[1] = make_float4(d[4], d[5], d[6], d[7]);
@@ -208,7 +247,11 @@ __global__ void __launch_bounds__(kThreads)
             }
         }
     }
-    if (WRITE == kWriteError && __any_sync(kFullMask, any) && lane == 0) atomicOr(flag, 1u);
+    if (WRITE == kWriteError && __any_sync(kFullMask, any) && lane == 0) atomicOr(job.flag, 1u);
+    if (WRITE == kWriteDeq && job.max_bits) {
+        largest = __reduce_max_sync(kFullMask, largest);
+        if (lane == 0 && largest) atomicMax(job.max_bits, largest);
+    }
 }
 
 // ---- decode ----------------------------------------------------------------------------------
@@ -360,6 +403,122 @@ __global__ void __launch_bounds__(kThreads, kDecodeCtas)
     if (lane == 0) bulk_wait_all();
 }
 
+// ---- the factors of a low-rank object --------------------------------------------------------------
+struct FactorArgs {
+    SectionSource f[2];                                       // U, V
+    float *out[2];
+    unsigned *max_bits[2];
+    const uint8_t *s;
+    float *s_out;
+    unsigned rank, first_cta_v;
+};
+constexpr unsigned kSharedS = 1024;                          // singular values kept in shared memory
+// U, V and S out of an object, and the two maxima that the reconstruction's scales come from.  Bound by latency (4096 x 14336 at rank 256: 3 MB
+// of codes in, 19 MB out, 9.8 us; 7.2 to 7.6 us where there is next to nothing to do), so it is one launch: with the split of both operands
+// behind it 18 us to the product, where a fetch of the headers and a wait, two decoding kernels, a copy of S, two memsets, two passes for the
+// maxima and two for the split took 60.  Whole decompress calls of that shape 209 -> 171 us.
+__global__ void __launch_bounds__(kThreads) open_factors_kernel(const __grid_constant__ FactorArgs a, const __grid_constant__ HeadCheck heads) {
+    __shared__ float s_s[kSharedS];
+    const int lane = threadIdx.x & 31, which = blockIdx.x >= a.first_cta_v;
+    const unsigned first = which ? a.first_cta_v : 0u, ctas = which ? gridDim.x - a.first_cta_v : a.first_cta_v;
+    const SectionSource &f = a.f[which];
+    const uint64_t n = f.n, nb = (n + 63) / 64;
+    const bool coded = f.scales != nullptr, coded_dq = f.dq != nullptr;
+    const bool words = (reinterpret_cast<uintptr_t>(f.data) & 3u) == 0, pairs = (reinterpret_cast<uintptr_t>(f.data) & 7u) == 0;
+    Nf4Lut lut;
+    lut.load();
+    float dq = 1.0f;
+    if (coded_dq) {
+        dq = load_f32_any(f.dq);
+        if (dq == 0.0f || !isfinite(dq)) dq = 1.0f;           // as decode_flat_kernel
+    }
+    struct Coded {
+        unsigned w[4];
+        float scale;
+    };
+    const auto fetch = [&](uint64_t base, Coded &c) {
+        c.scale = 1.0f;
+        if (!coded || base >= n) return;
+        const uint64_t blk = base / 64 + lane;
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+            const uint64_t e = base + it * 256 + lane * 8;
+            c.w[it] = 0u;
+            if (words && e + 8 <= n) {
+                c.w[it] = *reinterpret_cast<const unsigned *>(f.data + e / 2);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (e + 2 * q < n) c.w[it] |= (unsigned)f.data[e / 2 + q] << (8 * q);
+            }
+        }
+        if (lane < 16 && blk < nb) {
+            c.scale = coded_dq ? __fmul_rn(dq, e4m3_decode(f.scales[blk])) : load_f32_any(f.scales + 4 * blk);
+            if (c.scale == 0.0f || !isfinite(c.scale)) c.scale = 1.0f;
+        }
+    };
+    // what the CTA reads first is on its way while the headers are checked (all inside the object, whatever its headers say)
+    const uint64_t step = (uint64_t)ctas * (kThreads / 32) * kBatch;
+    uint64_t base = ((uint64_t)(blockIdx.x - first) * (kThreads / 32) + (threadIdx.x >> 5)) * kBatch;
+    Coded now, next;
+    fetch(base, now);
+    if (!which)
+        for (unsigned t = threadIdx.x; t < a.rank && t < kSharedS; t += kThreads) s_s[t] = load_f32_any(a.s + 4 * t);
+    if (!heads_match(heads)) return;
+    if (which && blockIdx.x == first)
+        for (unsigned t = threadIdx.x; t < a.rank; t += kThreads) a.s_out[t] = load_f32_any(a.s + 4ull * t);
+    __syncthreads();
+    unsigned largest = 0;
+    for (; base < n; base += step) {
+        fetch(base + step, next);
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+            const uint64_t e = base + it * 256 + lane * 8;
+            float d[8];
+            if (coded) {
+                const float sb = __shfl_sync(kFullMask, now.scale, it * 4 + (lane >> 3));
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const unsigned byte = (now.w[it] >> (8 * q)) & 0xFFu;
+                    d[2 * q] = __fmul_rn(sb, lut.decode(byte >> 4));
+                    d[2 * q + 1] = __fmul_rn(sb, lut.decode(byte & 0xFu));
+                }
+            } else if (pairs && e + 8 <= n) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float2 v = reinterpret_cast<const float2 *>(f.data + 4 * e)[q];
+                    d[2 * q] = v.x;
+                    d[2 * q + 1] = v.y;
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) d[q] = e + q < n ? load_f32_any(f.data + 4 * (e + q)) : 0.0f;
+            }
+            if (e + 8 <= n) {
+                float4 *to = reinterpret_cast<float4 *>(a.out[which] + e);
+                to[0] = make_float4(d[0], d[1], d[2], d[3]);
+                to[1] = make_float4(d[4], d[5], d[6], d[7]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (e + q < n) a.out[which][e + q] = d[q];
+            }
+            unsigned c = which ? 0u : (unsigned)e % a.rank;   // (a factor has fewer than 2^32 elements)
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                if (!which) {
+                    d[q] *= a.rank <= kSharedS ? s_s[c] : load_f32_any(a.s + 4ull * c);
+                    if (++c == a.rank) c = 0;
+                }
+                if (e + q < n) largest = max(largest, __float_as_uint(d[q]) & 0x7fffffffu);
+            }
+        }
+        now = next;
+    }
+    largest = __reduce_max_sync(kFullMask, largest);
+    if (lane == 0 && largest) atomicMax(a.max_bits[which], largest);
+}
+
 inline const uint8_t *bytes(const void *p) { return static_cast<const uint8_t *>(p); }
 inline bool aligned(const void *p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
@@ -372,19 +531,42 @@ inline int grid_for(uint64_t n, int sm_count) {
 
 }  // namespace
 
+// Both arrays of `jobs` (the second possibly empty) in one launch per pass.
+static cudaError_t launch_encode(bool dq, EncodeJobs &jobs, int sm_count, cudaStream_t stream) {
+    unsigned grid = 0;
+    for (int i = 0; i < 2; ++i) {
+        EncodeJob &j = jobs.job[i];
+        if (i == 1) jobs.second = grid;
+        if (j.n == 0) continue;
+        j.vec = aligned(j.x, 16) && aligned(j.data, 4) && (!j.deq_out || aligned(j.deq_out, 16));
+        grid += (unsigned)grid_for(j.n, sm_count);
+    }
+    if (dq) {
+        const cudaError_t err = launch_chained(absmax_flat_kernel, grid, kThreads, 0, stream, jobs);
+        if (err != cudaSuccess) return err;
+    }
+    const EncodeJob &j = jobs.job[0];
+    if (j.deq_out && j.flag)
+        return dq ? launch_chained(encode_flat_kernel<true, kWriteError>, grid, kThreads, 0, stream, jobs)
+                  : launch_chained(encode_flat_kernel<false, kWriteError>, grid, kThreads, 0, stream, jobs);
+    if (j.deq_out)
+        return dq ? launch_chained(encode_flat_kernel<true, kWriteDeq>, grid, kThreads, 0, stream, jobs)
+                  : launch_chained(encode_flat_kernel<false, kWriteDeq>, grid, kThreads, 0, stream, jobs);
+    return dq ? launch_chained(encode_flat_kernel<true, kWriteNone>, grid, kThreads, 0, stream, jobs)
+              : launch_chained(encode_flat_kernel<false, kWriteNone>, grid, kThreads, 0, stream, jobs);
+}
+
 cudaError_t nf4_quantize(const float *d_x, uint64_t n, float *d_scales, uint8_t *d_data, float *d_deq_out, int sm_count,
                          cudaStream_t stream, unsigned *d_error_flag) {
-    const bool vec = aligned(d_x, 16) && aligned(d_data, 4) && (!d_deq_out || aligned(d_deq_out, 16));
-    const int grid = grid_for(n, sm_count);
-    if (d_deq_out && d_error_flag)
-        return launch_chained(encode_flat_kernel<false, kWriteError>, grid, kThreads, 0, stream, d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
-                                                                         nullptr, d_data, d_deq_out, d_error_flag);
-    else if (d_deq_out)
-        return launch_chained(encode_flat_kernel<false, kWriteDeq>, grid, kThreads, 0, stream, d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
-                                                                         nullptr, d_data, d_deq_out, nullptr);
-    else
-        return launch_chained(encode_flat_kernel<false, kWriteNone>, grid, kThreads, 0, stream, d_x, n, vec, nullptr, nullptr, d_scales, nullptr,
-                                                                          nullptr, d_data, nullptr, nullptr);
+    EncodeJobs jobs{};
+    EncodeJob &j = jobs.job[0];
+    j.x = d_x;
+    j.n = n;
+    j.scales_f32 = d_scales;
+    j.data = d_data;
+    j.deq_out = d_deq_out;
+    j.flag = d_error_flag;
+    return launch_encode(false, jobs, sm_count, stream);
 }
 
 size_t nf4dq_scratch_bytes(uint64_t n) { return (size_t)((n + 63) / 64) * sizeof(float) + 16; }
@@ -393,21 +575,50 @@ cudaError_t nf4dq_quantize(const float *d_x, uint64_t n, float *d_dq, uint8_t *d
                            float *d_deq_out, void *d_scratch, int sm_count, cudaStream_t stream, unsigned *d_error_flag, unsigned *d_gmax) {
     // scratch layout: [0,16) global-max word (+ padding), then one float per block
     unsigned *gmax = d_gmax ? d_gmax : static_cast<unsigned *>(d_scratch);
-    float *absmax = reinterpret_cast<float *>(static_cast<uint8_t *>(d_scratch) + 16);
-    const bool vec = aligned(d_x, 16) && aligned(d_data, 4) && (!d_deq_out || aligned(d_deq_out, 16));
-    const int grid = grid_for(n, sm_count);
-    cudaError_t err = d_gmax ? cudaSuccess : cudaMemsetAsync(gmax, 0, 4, stream);
-    if (err != cudaSuccess) return err;
-    if ((err = launch_chained(absmax_flat_kernel, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax)) != cudaSuccess) return err;
-    if (d_deq_out && d_error_flag)
-        return launch_chained(encode_flat_kernel<true, kWriteError>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
-                                                                        d_dq, d_data, d_deq_out, d_error_flag);
-    else if (d_deq_out)
-        return launch_chained(encode_flat_kernel<true, kWriteDeq>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
-                                                                        d_dq, d_data, d_deq_out, nullptr);
-    else
-        return launch_chained(encode_flat_kernel<true, kWriteNone>, grid, kThreads, 0, stream, d_x, n, vec, absmax, gmax, nullptr, d_scale_codes,
-                                                                         d_dq, d_data, nullptr, nullptr);
+    if (!d_gmax) {
+        const cudaError_t err = cudaMemsetAsync(gmax, 0, 4, stream);
+        if (err != cudaSuccess) return err;
+    }
+    EncodeJobs jobs{};
+    EncodeJob &j = jobs.job[0];
+    j.x = d_x;
+    j.n = n;
+    j.absmax_in = reinterpret_cast<float *>(static_cast<uint8_t *>(d_scratch) + 16);
+    j.gmax_bits = gmax;
+    j.scale_codes = d_scale_codes;
+    j.dq_out = d_dq;
+    j.data = d_data;
+    j.deq_out = d_deq_out;
+    j.flag = d_error_flag;
+    return launch_encode(true, jobs, sm_count, stream);
+}
+
+cudaError_t quantize_pair(int method, const QuantTarget &a, const QuantTarget &b, void *d_scratch, int sm_count, cudaStream_t stream) {
+    const bool dq = method == 10;
+    EncodeJobs jobs{};
+    uint8_t *room = static_cast<uint8_t *>(d_scratch);
+    for (int i = 0; i < 2; ++i) {
+        const QuantTarget &t = i ? b : a;
+        EncodeJob &j = jobs.job[i];
+        if (!t.x || !t.n || !t.data || (dq ? !t.dq || !t.scale_codes || !t.gmax || !d_scratch : !t.scales) || (t.deq == nullptr) != (a.deq == nullptr))
+            return cudaErrorInvalidValue;
+        j.x = t.x;
+        j.n = t.n;
+        j.scales_f32 = t.scales;
+        j.scale_codes = t.scale_codes;
+        j.dq_out = t.dq;
+        j.data = t.data;
+        j.deq_out = t.deq;
+        j.gmax_bits = t.gmax;
+        j.colscale = t.colscale;
+        j.cols = t.cols;
+        j.max_bits = t.max_bits;
+        if (dq) {
+            j.absmax_in = reinterpret_cast<float *>(room + 16);
+            room += nf4dq_scratch_bytes(t.n);
+        }
+    }
+    return launch_encode(dq, jobs, sm_count, stream);
 }
 
 uint64_t nf4dq_static_max_elements() { return kStaticMaxElems; }
@@ -482,6 +693,26 @@ cudaError_t decode_matrix(const SectionSource &q, uint32_t rows, uint32_t cols, 
     if (!q.scales || !q.data || !d_out || q.n != (uint64_t)rows * cols || q.n == 0) return cudaErrorInvalidValue;
     const TopkLists add{{{first.idx, first.val, first.k}, {second.idx, second.val, second.k}}, cols, mirror, true};
     return launch_decode(q, add, d_out, heads, sm_count, stream);
+}
+
+cudaError_t open_factors(const SectionSource &u, const SectionSource &v, const uint8_t *s, uint32_t rank, float *d_u, float *d_v, float *d_s,
+                         unsigned *d_max_us, unsigned *d_max_v, const HeadCheck &heads, int sm_count, cudaStream_t stream) {
+    if (!u.n || !v.n || !u.data || !v.data || !s || !rank || !aligned(d_u, 16) || !aligned(d_v, 16)) return cudaErrorInvalidValue;
+    FactorArgs a{};
+    a.f[0] = u; a.f[1] = v;
+    a.out[0] = d_u; a.out[1] = d_v;
+    a.max_bits[0] = d_max_us; a.max_bits[1] = d_max_v;
+    a.s = s;
+    a.s_out = d_s;
+    a.rank = rank;
+    // a warp per batch up to four CTAs per SM for each factor: all of them are in flight at once
+    const auto ctas = [&](uint64_t n) {
+        const uint64_t c = (n + kBatch * (kThreads / 32) - 1) / (kBatch * (kThreads / 32));
+        return (unsigned)(c < (uint64_t)sm_count * 4 ? c : (uint64_t)sm_count * 4);
+    };
+    a.first_cta_v = ctas(u.n);
+    open_factors_kernel<<<a.first_cta_v + ctas(v.n), kThreads, 0, stream>>>(a, heads);
+    return cudaGetLastError();
 }
 
 }  // namespace bsq

@@ -758,10 +758,11 @@ size_t reconstruct_workspace_bytes(int m, int n, int k) {
 
 cudaError_t reconstruct_lowrank(const float *d_U, const float *d_S, const float *d_V, int m, int n, int k,
                                 const float *d_minuend, float *d_out, unsigned *d_flag, unsigned *d_status, float *d_workspace,
-                                size_t workspace_bytes, int sm_count, cudaStream_t st) {
+                                size_t workspace_bytes, int sm_count, cudaStream_t st, const unsigned *d_max_us, const unsigned *d_max_v) {
     if (!d_U || !d_S || !d_V || !d_out || m <= 0 || n <= 0 || k <= 0) return cudaErrorInvalidValue;
     // out(i, j) = sum_t (U(i, t) S(t)) V(j, t): A = U as stored with a per-k scale, B = V^T (K-major)
-    return gemm(true, true, d_U, k, d_V, k, d_out, n, m, n, k, d_S, d_minuend, n, d_flag, d_status, d_workspace, workspace_bytes, sm_count, st);
+    return gemm(true, true, d_U, k, d_V, k, d_out, n, m, n, k, d_S, d_minuend, n, d_flag, d_status, d_workspace, workspace_bytes, sm_count, st,
+                d_max_us, 0.0f, false, d_max_v);
 }
 
 }  // namespace bsq

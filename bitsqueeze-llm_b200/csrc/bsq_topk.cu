@@ -10,6 +10,7 @@
 // sorted there (bsq_topk.cuh), and only the k pairs -- and, for separation, the row with the
 // selected entries zeroed -- are written back.  HBM-bound: 4 B read per element, 6k B written
 // per row (+ 4 B per element when the zeroed copy is wanted).
+#include "bsq_call.cuh"
 #include "bsq_internal.hpp"
 #include "bsq_rowgroup.cuh"
 #include "bsq_topk.cuh"
@@ -203,14 +204,33 @@ __global__ void __launch_bounds__(kGenericThreads)
 }
 
 // ---- scatter-add ----------------------------------------------------------------------------------
-__global__ void topk_apply_kernel(const uint16_t *__restrict__ idx, const float *__restrict__ val, unsigned rows,
-                                  unsigned cols, unsigned k, float *dense, unsigned *status) {
+// Lists may lie at any address.  The last kernel of a decompress call also takes the words of its earlier kernels: what they reported goes
+// to the host's mirror, all are cleared (the one report that this kernel can make goes there directly).
+struct ApplyReport {
+    unsigned *status;                                        // nullable; device word, or the mirror itself (on_host)
+    bool on_host;
+    unsigned *words;                                         // nullable: this is not a call's last kernel
+};
+__device__ __forceinline__ void end_call(const ApplyReport &r) {
+    if (r.words == nullptr || blockIdx.x != 0 || threadIdx.x >= kStatusWords) return;
+    const unsigned w = r.words[threadIdx.x];
+    if (threadIdx.x == kWordStatus && w) *reinterpret_cast<volatile unsigned *>(r.status) = w;
+    r.words[threadIdx.x] = 0;
+}
+__global__ void __launch_bounds__(32) end_call_kernel(ApplyReport report) {
+    chain_begin();
+    end_call(report);
+}
+__global__ void topk_apply_kernel(ListSource list, unsigned rows, unsigned cols, float *dense, ApplyReport report) {
+    chain_begin();
+    end_call(report);
+    const unsigned k = list.k;
     const size_t total = (size_t)rows * k;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const unsigned r = (unsigned)(e / k);
-        const unsigned c = idx[e];
-        if (c < cols) dense[(size_t)r * cols + c] += val[e];
-        else if (status) atomicOr(status, kStatusBadIndex);
+        const unsigned c = load_u16_any(list.idx + 2 * e);
+        if (c < cols) dense[(size_t)r * cols + c] += load_f32_any(list.val + 4 * e);
+        else report_bad_index(report.status, report.on_host);
     }
 }
 
@@ -219,15 +239,16 @@ __global__ void topk_apply_kernel(const uint16_t *__restrict__ idx, const float 
 // sectors are fetched while everything about both lists is.  Four entries of each list in flight per lane; a trip of a warp
 // (128 entries of a list) is a chain of two loads and a store, 1 us, which is what bounds it while the device has rows to
 // spare for few warps.  topk_apply_two says where it stands in for two launches.
-__device__ __forceinline__ void apply_row(const uint16_t *idx, const float *val, unsigned cols, unsigned k, float *row, unsigned lane,
-                                          unsigned *status) {
+__device__ __forceinline__ void apply_row(const ListSource &list, unsigned r, unsigned cols, float *row, unsigned lane, const ApplyReport &report) {
+    const unsigned k = list.k;
+    const uint8_t *idx = list.idx + 2 * (size_t)r * k, *val = list.val + 4 * (size_t)r * k;
     for (unsigned j0 = lane; j0 < k; j0 += 128) {
         unsigned c[4];
         float v[4], d[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            c[u] = j0 + 32 * u < k ? idx[j0 + 32 * u] : 0xFFFFFFFFu;
-            v[u] = j0 + 32 * u < k ? val[j0 + 32 * u] : 0.0f;
+            c[u] = j0 + 32 * u < k ? load_u16_any(idx + 2 * (j0 + 32 * u)) : 0xFFFFFFFFu;
+            v[u] = j0 + 32 * u < k ? load_f32_any(val + 4 * (j0 + 32 * u)) : 0.0f;
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) d[u] = c[u] < cols ? row[c[u]] : 0.0f;
@@ -236,19 +257,20 @@ __device__ __forceinline__ void apply_row(const uint16_t *idx, const float *val,
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             if (c[u] < cols) row[c[u]] = d[u] + v[u];
-            else if (c[u] != 0xFFFFFFFFu && status) atomicOr(status, kStatusBadIndex);
+            else if (c[u] != 0xFFFFFFFFu) report_bad_index(report.status, report.on_host);
         }
     }
 }
-__global__ void __launch_bounds__(256) topk_apply_two_kernel(const uint16_t *__restrict__ idx0, const float *__restrict__ val0, unsigned k0,
-                                                             const uint16_t *__restrict__ idx1, const float *__restrict__ val1, unsigned k1,
-                                                             unsigned rows, unsigned cols, float *dense, unsigned *status) {
+__global__ void __launch_bounds__(256) topk_apply_two_kernel(ListSource first, ListSource second, unsigned rows, unsigned cols, float *dense,
+                                                             ApplyReport report) {
+    chain_begin();
+    end_call(report);
     const unsigned lane = threadIdx.x & 31, r = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (r >= rows) return;
     float *row = dense + (size_t)r * cols;
-    apply_row(idx0 + (size_t)r * k0, val0 + (size_t)r * k0, cols, k0, row, lane, status);
+    apply_row(first, r, cols, row, lane, report);
     __syncwarp();
-    apply_row(idx1 + (size_t)r * k1, val1 + (size_t)r * k1, cols, k1, row, lane, status);
+    apply_row(second, r, cols, row, lane, report);
 }
 
 // ---- e = a - b, flag |= any(|e| > FLT_EPSILON) ----------------------------------------------------
@@ -393,40 +415,65 @@ cudaError_t topk_rows(const float *d_in, float *d_residual, uint32_t rows, uint3
     return cudaGetLastError();
 }
 
+static cudaError_t launch_apply(const ListSource &list, uint32_t rows, uint32_t cols, float *d_dense, const ApplyReport &report, cudaStream_t stream) {
+    const size_t total = (size_t)rows * list.k;
+    size_t grid = (total + 255) / 256;
+    if (grid > 148 * 16) grid = 148 * 16;
+    return launch_chained(topk_apply_kernel, (unsigned)grid, 256, 0, stream, list, rows, cols, d_dense, report);
+}
+static ListSource as_list(const uint16_t *d_idx, const float *d_val, uint32_t k) {
+    ListSource l;
+    l.idx = reinterpret_cast<const uint8_t *>(d_idx);
+    l.val = reinterpret_cast<const uint8_t *>(d_val);
+    l.k = k;
+    return l;
+}
+
 cudaError_t topk_apply(const uint16_t *d_idx, const float *d_val, uint32_t rows, uint32_t cols, uint32_t k,
                        float *d_dense, unsigned *d_status, cudaStream_t stream) {
     if (!d_dense || rows == 0 || cols == 0) return cudaErrorInvalidValue;
     if (k == 0) return cudaSuccess;
     if (!d_idx || !d_val) return cudaErrorInvalidValue;
-    const size_t total = (size_t)rows * k;
-    size_t grid = (total + 255) / 256;
-    if (grid > 148 * 16) grid = 148 * 16;
-    topk_apply_kernel<<<(unsigned)grid, 256, 0, stream>>>(d_idx, d_val, rows, cols, k, d_dense, d_status);
-    return cudaGetLastError();
+    return launch_apply(as_list(d_idx, d_val, k), rows, cols, d_dense, ApplyReport{d_status, false, nullptr}, stream);
 }
 
-cudaError_t topk_apply_two(const uint16_t *d_idx0, const float *d_val0, uint32_t k0, const uint16_t *d_idx1, const float *d_val1,
-                           uint32_t k1, uint32_t rows, uint32_t cols, float *d_dense, unsigned *d_status, cudaStream_t stream) {
-    if (!d_dense || rows == 0 || cols == 0) return cudaErrorInvalidValue;
-    if ((k0 && (!d_idx0 || !d_val0)) || (k1 && (!d_idx1 || !d_val1))) return cudaErrorInvalidValue;
+static cudaError_t launch_apply_two(const ListSource &a, const ListSource &b, uint32_t rows, uint32_t cols, float *d_dense, const ApplyReport &report,
+                                    cudaStream_t stream) {
     // A decompress call is 2 to 6 us shorter with one launch than with two, until a warp's trips take longer than that (few
     // rows), or a matrix beyond the L2 wants the two launches' larger grids; and lists that name a good part of a row find it in
     // the L1 cache when one warp walks it.  us a call, one / two launches, calls of either taken in turn: 300 x 4096
     // with 41 + 20 entries a row 38 / 41, 64 x 8192 with 82 + 164 39 / 41; 4001 x 4096 with 41 + 82 56 / 59; 2048 x 4096 with
     // 41 + 819 55 / 67, 1000 x 8192 with 3277 + 3277 112 / 189; on the other side 8 x 14336 with 5734 + 5734 125 / 39, 64 x 14336 with
     // 717 + 717 43 / 41, 4001 x 14336 with 717 + 717 267 / 225, 6144 x 8192 with 82 + 1638 352 / 281.
-    const uint64_t listed = (uint64_t)k0 + k1, entries = rows * listed, elements = (uint64_t)rows * cols;
-    const uint32_t trips = (k0 + 127) / 128 + (k1 + 127) / 128;
+    const uint64_t listed = (uint64_t)a.k + b.k, entries = rows * listed, elements = (uint64_t)rows * cols;
+    const uint32_t trips = (a.k + 127) / 128 + (b.k + 127) / 128;
     bool one_launch;
     if (rows >= 512 && 5 * listed >= cols) one_launch = elements <= (32u << 20) || 2 * listed >= cols;
     else if (entries > 1400000) one_launch = trips <= 3;
     else one_launch = trips <= (rows >= 512 ? 8u : 5u);
     if (!one_launch) {
-        const cudaError_t err = topk_apply(d_idx0, d_val0, rows, cols, k0, d_dense, d_status, stream);
-        return err != cudaSuccess ? err : topk_apply(d_idx1, d_val1, rows, cols, k1, d_dense, d_status, stream);
+        // (the words are for the call's last kernel; the first one reports where that one does)
+        const cudaError_t err = launch_apply(a, rows, cols, d_dense, ApplyReport{report.status, report.on_host, nullptr}, stream);
+        return err != cudaSuccess ? err : launch_apply(b, rows, cols, d_dense, report, stream);
     }
-    topk_apply_two_kernel<<<(rows + 7) / 8, 256, 0, stream>>>(d_idx0, d_val0, k0, d_idx1, d_val1, k1, rows, cols, d_dense, d_status);
-    return cudaGetLastError();
+    return launch_chained(topk_apply_two_kernel, (rows + 7) / 8, 256, 0, stream, a, b, rows, cols, d_dense, report);
+}
+
+cudaError_t topk_apply_two(const uint16_t *d_idx0, const float *d_val0, uint32_t k0, const uint16_t *d_idx1, const float *d_val1,
+                           uint32_t k1, uint32_t rows, uint32_t cols, float *d_dense, unsigned *d_status, cudaStream_t stream) {
+    if (!d_dense || rows == 0 || cols == 0) return cudaErrorInvalidValue;
+    if ((k0 && (!d_idx0 || !d_val0)) || (k1 && (!d_idx1 || !d_val1))) return cudaErrorInvalidValue;
+    if (k0 == 0) return topk_apply(d_idx1, d_val1, rows, cols, k1, d_dense, d_status, stream);
+    if (k1 == 0) return topk_apply(d_idx0, d_val0, rows, cols, k0, d_dense, d_status, stream);
+    return launch_apply_two(as_list(d_idx0, d_val0, k0), as_list(d_idx1, d_val1, k1), rows, cols, d_dense, ApplyReport{d_status, false, nullptr}, stream);
+}
+
+cudaError_t apply_lists_end(const ListSource &a, const ListSource &b, uint32_t rows, uint32_t cols, float *d_dense, unsigned *d_status,
+                            unsigned *mirror, cudaStream_t stream) {
+    const ApplyReport report{mirror, true, d_status};
+    if (a.k && b.k) return launch_apply_two(a, b, rows, cols, d_dense, report, stream);
+    if (a.k || b.k) return launch_apply(a.k ? a : b, rows, cols, d_dense, report, stream);
+    return launch_chained(end_call_kernel, 1, 32, 0, stream, report);
 }
 
 cudaError_t residual_error(const float *d_a, const float *d_b, uint64_t n, float *d_e, unsigned *d_flag, int sm_count,

@@ -85,3 +85,53 @@ def test_refused_object_leaves_the_result_alone(pkg, lib):
         assert lib.bsq_lane_decompress_end(lane) == 0
     finally:
         lib.bsq_lane_destroy(lane)
+
+
+# rows, cols, outlier, error, rank, uv: factors coded both ways and kept in FP32, off 8-byte boundaries, a rank with more singular values than
+# the kernel keeps in shared memory, factors of less than a batch, with no, one and two lists
+FACTOR_CASES = [
+    (777, 1031, 0.005, 0.0, 48, -1), (1024, 640, 0.0, 0.0, 64, -1), (1100, 1090, 0.01, 0.0, 1030, -1), (96, 70, 0.02, 0.02, 7, 11),
+    (1024, 1536, 0.01, 0.02, 64, 10), (640, 2048, 0.0, 0.02, 40, 11), (515, 1001, 0.01, 0.01, 33, 10), (1024, 1024, 0.0, 0.02, 32, -1),
+]
+
+
+@pytest.mark.parametrize("case", FACTOR_CASES)
+def test_opened_factors_give_the_host_objects_bits(pkg, lib, case):
+    """Factors opened in place by one kernel, their maxima taken on the way, against the route of a host object, which copies and decodes
+    section by section and finds the maxima in passes of their own."""
+    rows, cols, outlier, error, rank, uv = case
+    x = torch.randn(rows, cols, device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows + rank))
+    lane = lib.bsq_lane_create(rows, cols, outlier, error, rank, 1, uv, -1, -1)
+    assert lane
+    try:
+        cap = int(lib.bsq_lane_packed_capacity(lane))
+        buf = torch.empty(cap, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        hdr, out = pkg.Array(), C.c_void_p(None)
+        assert lib.bsq_lane_compress_begin(lane, x.data_ptr(), 1, buf.data_ptr(), cap) == 0
+        assert lib.bsq_lane_compress_end(lane, None, C.byref(hdr), None) == 0
+        host = buf.cpu().numpy()
+        out = lib.bsq_load_from_buffer(host.ctypes.data, host.size)
+        assert out
+        want, got = torch.empty_like(x), torch.full_like(x, 7.0)
+        torch.cuda.synchronize()
+        assert lib.bsq_lane_decompress_begin(lane, out, 0, want.data_ptr(), rows * cols) == 0
+        assert lib.bsq_lane_decompress_end(lane) == 0
+        if uv != -1:                                          # V's block count: refused before the result is touched
+            at = 200 + hdr.section_v.offset + 24
+            buf[at] ^= 1
+            torch.cuda.synchronize()
+            assert lib.bsq_lane_decompress_begin(lane, C.byref(hdr), 1, got.data_ptr(), rows * cols) == 1
+            buf[at] ^= 1
+            torch.cuda.synchronize()
+            assert (got == 7.0).all()
+        for _ in range(2):                                    # (the second call finds the words as the first one left them)
+            torch.cuda.synchronize()
+            assert lib.bsq_lane_decompress_begin(lane, C.byref(hdr), 1, got.data_ptr(), rows * cols) == 0
+            assert lib.bsq_lane_decompress_end(lane) == 0
+            torch.cuda.synchronize()
+            assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+            got.fill_(7.0)
+        lib.bsq_free(out)
+    finally:
+        lib.bsq_lane_destroy(lane)
