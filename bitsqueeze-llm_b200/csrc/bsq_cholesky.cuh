@@ -1,4 +1,5 @@
-// Cholesky factor and its inverse for the Gram matrices of the randomized SVD, k <= kCholeskyBlockedMaxK (sm_100a).
+// Cholesky factor and its inverse for the Gram matrices of the randomized SVD, k <= kCholeskyBlockedMaxK (sm_100a); above 32 columns
+// usually by way of bsq_cholesky_cluster.cuh.
 //
 // Stands where the reference orthonormalises with cusolverDnSgeqrf + Sorgqr (svd_lowrank_cuda.cu:196-281): a panel Y
 // with Gram matrix G = Y^T Y is multiplied by R^-1, G + s I = R^T R.  The shift (s = 1e-5 max(diag G)) and a floor of
@@ -15,9 +16,9 @@
 //     what an SM's multiply-adds take: 53 us at 256 columns for 8 blocks, 16 us at 128 for 4.
 //   * R and the inverses of its diagonal blocks go out block row by block row, and other CTAs make the rows of the inverse
 //     from them while the factor goes on: T_IJ = -(sum_{L=I..J-1} T_IL R_LJ) T_JJ from left to right.
-// Every value is the same sum in the same order whatever the number of CTAs or launches.  Back to back, factor and inverse, against the
-// two kernels (one CTA; one per block row) and, up to 64 columns, the single CTA that did this before, ordinary launches: k = 256 63 against
-// 99 us, 192 41 / 67, 128 25 / 41, 64 15 / 18.7, 32 7 / 10.5; the factor alone 53 / 79 us at 256, 16.4 / 30 us at 128.
+// Every value is the same sum in the same order whatever the number of CTAs.  Above 32 columns the kernel of bsq_cholesky_cluster.cuh takes the
+// place of this one wherever its cluster can be placed; both share what is above cholesky_factor.  Back to back, factor and inverse, this
+// kernel / that one, us: k = 256 71 / 32, 128 31.5 / 20, 64 14.4 / 11.2, 48 15.3 / 10.7; up to 32 columns 7.
 #pragma once
 
 #include "bsq_device.cuh"
@@ -206,9 +207,9 @@ __device__ __forceinline__ float chol_rsqrt_ftz(float x) {
 // The pivots of a diagonal block, one warp: lane c keeps column c.  Row j of R goes to dia, 1 / R(j, j) to dinv; every kCholStep rows the
 // warps of the block row (panel threads with this one) are let on.  The row in front of dia is zero.
 // kNormal: the floor under the pivots is a normal number, so every pivot is, and its root needs no scaling.
-// Rows move up after every kCholStep pivots, in a lane and in what is read of dia.
+// Rows move up after every kCholStep pivots, in a lane and in what is read of dia.  steps: times kCholStep pivots.
 template <bool kNormal>
-__device__ __forceinline__ void factor_diagonal(int at_d, int at_dia, int at_dinv, float half, int panel) {
+__device__ __forceinline__ void factor_diagonal(int at_d, int at_dia, int at_dinv, float half, int panel, int steps = kCB / kCholStep) {
     const float *D = chol_smem() + at_d;
     float *dia = chol_smem() + at_dia, *dinv = chol_smem() + at_dinv;
     const int lane = threadIdx.x & 31;
@@ -218,7 +219,7 @@ __device__ __forceinline__ void factor_diagonal(int at_d, int at_dia, int at_din
     float d = a[0].x, v = 0.0f;                             // the next pivot before its root, valid in its lane
     const unsigned dia_at = smem_u32(dia);
 #pragma unroll 1
-    for (int j0 = 0; j0 < kCB; j0 += kCholStep) {
+    for (int j0 = 0; j0 < kCholStep * steps; j0 += kCholStep) {
 #pragma unroll
         for (int j = 0; j < kCholStep; ++j) {
             d = fmaxf(d, half);                             // (a NaN as well)
@@ -247,10 +248,10 @@ __device__ __forceinline__ void factor_diagonal(int at_d, int at_dia, int at_din
     }
 }
 
-// kCols columns of a block row per thread (in blocks beside one another): forward substitution with R_JJ^T, behind the pivots.  X: the
-// columns, in place.
-template <int kCols>
-__device__ __forceinline__ void block_row(int at_x, int at_dia, int at_dinv, int panel, bool first) {
+// kCols columns of a block row per thread (in blocks beside one another): forward substitution with R_JJ^T, behind the pivots (await(s)
+// waits for the s-th eight).  X: the columns, in place.
+template <int kCols, class Await>
+__device__ __forceinline__ void block_row(int at_x, int at_dia, int at_dinv, bool first, Await await) {
     float *X = chol_smem() + at_x;
     const unsigned dia_at = smem_u32(chol_smem() + at_dia), dinv_at = smem_u32(chol_smem() + at_dinv);
     float2 y[kCols][kCB / 2];
@@ -260,7 +261,7 @@ __device__ __forceinline__ void block_row(int at_x, int at_dia, int at_dinv, int
         for (int i = 0; i < kCB / 2; ++i) y[u][i] = make_float2(X[u * kCBB + 2 * i * kCB], X[u * kCBB + (2 * i + 1) * kCB]);
 #pragma unroll 1
     for (int j0 = 0; j0 < kCB; j0 += kCholStep) {
-        bar_sync(1 + j0 / kCholStep, panel);
+        await(j0 / kCholStep);
         const float4 d0 = lds4(dinv_at + 4 * j0), d1 = lds4(dinv_at + 4 * j0 + 16);
         const float dv[kCholStep] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
 #pragma unroll
@@ -443,8 +444,9 @@ __device__ __forceinline__ void cholesky_factor(const float *G, int k, float *R,
             if (wi < panel_warps) {
                 const int b = wi == 0 ? 1 : 2 * wi;         // first block, counted from the diagonal
                 const int at_x = blk_id(J, J + b, nb) * kCBB + lane;
-                if (wi > 0 && b < rest) block_row<2>(at_x, at_dia, at_dinv, panel, false);
-                else block_row<1>(at_x, at_dia, at_dinv, panel, wi == 0);
+                const auto await = [panel](int s) { bar_sync(1 + s, panel); };
+                if (wi > 0 && b < rest) block_row<2>(at_x, at_dia, at_dinv, false, await);
+                else block_row<1>(at_x, at_dia, at_dinv, wi == 0, await);
             } else if (wi >= kCholPanel && rest) {
                 // ---- then the blocks below, that of the next pivots before all others ----
                 constexpr int kTasks = 2 * kCholTrail;      // at a time
@@ -488,7 +490,7 @@ __device__ __forceinline__ void cholesky_factor(const float *G, int k, float *R,
 // factor's block rows and the diagonal blocks of T.  The transposes of T_IL and of the sums are what is kept, so that every product
 // has the form A^T B of block_mac:
 //   T_IJ^T = -(T_JJ)^T S_J^T with S_J = sum_L T_IL R_LJ, and S_C^T += (R_JC)^T T_IJ^T for the columns C still to come.
-// sync: waited on for the block rows (null: they are there).  Gives up if they do not come.
+// sync: waited on for the block rows.  Gives up if they do not come.
 __device__ __forceinline__ void cholesky_inverse_row(int I, int k, const float *R, float *T, CholeskySync *sync, unsigned *status) {
     const int nb = chol_blocks(k);
     float *rb = chol_smem();                               // block row J of R right of its diagonal block
@@ -502,7 +504,7 @@ __device__ __forceinline__ void cholesky_inverse_row(int I, int k, const float *
                 if (row * kCB + i < k) T[(size_t)(row * kCB + i) * k + c] = 0.0f;
     for (int J = I; J < nb; ++J) {
         bool here = true;
-        if (sync && tid == 0) {
+        if (tid == 0) {
             unsigned rows = 0;
             for (unsigned i = 0; i < kMbarSpinLimit; ++i) {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(rows) : "l"(&sync->rows) : "memory");
@@ -580,27 +582,20 @@ __device__ __forceinline__ void cholesky_inverse_row(int I, int k, const float *
     }
 }
 
-// What a launch does.  kCholBoth: the CTA that starts first factors, the others follow with the rows of the inverse: the shortest
-// time for one matrix.  kCholFactor (and the diagonal blocks of T if T is given), then kCholInverse: nobody waits for anybody, which is
-// less time of all SMs together where other work wants them (k = 256: 63 us on 8 SMs against 57 us on 1 and 23 us on 7; six compress calls of
-// 8192 x 4096 side by side 5.31 ms in two launches, 5.34 in one, eight of 4096 x 14336 9.97 and 9.96).
-enum CholeskyPart { kCholBoth, kCholFactor, kCholInverse };
-__host__ __device__ constexpr int cholesky_grid(int k, CholeskyPart part) {
-    return part == kCholFactor || chol_blocks(k) == 1 ? 1 : chol_blocks(k) - (part == kCholInverse ? 1 : 0);
-}
+// The CTA that starts first factors; where the inverse is wanted there is a CTA per block, and the others follow with its rows.
 __global__ void __launch_bounds__(kCholThreads, 1) cholesky_kernel(const float *G, int k, float *R, float *T, CholeskySync *sync,
-                                                                   unsigned *status, CholeskyPart part) {
+                                                                   unsigned *status) {
     __shared__ unsigned s_role;
     chain_begin();
-    int role = part == kCholInverse ? (int)blockIdx.x + 1 : 0;
-    const bool together = part == kCholBoth && gridDim.x > 1;
+    int role = 0;
+    const bool together = gridDim.x > 1;
     if (together) {
         if (threadIdx.x == 0) s_role = atomicAdd(&sync->ticket, 1u);
         __syncthreads();
         role = (int)s_role;
     }
     if (role == 0) cholesky_factor(G, k, R, T, together ? sync : nullptr);
-    else cholesky_inverse_row(role - 1, k, R, T, together ? sync : nullptr, status);
+    else cholesky_inverse_row(role - 1, k, R, T, sync, status);
     if (!together) return;
     // The factor's last row is still on its way out when this thread gets here: if the other CTAs have given up on it, this CTA is the last
     // to leave, and a row announced behind the clearing would stand as the next launch's.

@@ -134,6 +134,21 @@ __device__ __forceinline__ unsigned smem_u32(const void *p) {
     return (unsigned)__cvta_generic_to_shared(p);
 }
 
+// The shared::cluster address of `smem_addr` (a shared::cta address of this CTA) in CTA `rank` of the cluster.
+__device__ __forceinline__ unsigned cluster_addr(unsigned smem_addr, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
+    return r;
+}
+
+// Stores into another CTA's shared memory that count themselves off on that CTA's mbarrier when they have landed:
+// the receiver waits for the bytes, no fence and no cluster-wide barrier on the sender's side.
+__device__ __forceinline__ void st_async_f4(unsigned dst, float x, float y, float z, float w, unsigned mbar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "f"(x),
+                 "f"(y), "f"(z), "f"(w), "r"(mbar)
+                 : "memory");
+}
+
 __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
 }

@@ -38,19 +38,6 @@ __host__ __device__ constexpr int ring_warps(int k) { return (ring_pairs(k) + kR
 constexpr int kRingWarps = 4;                                // of a CTA, but for the one CTA that takes up to 64 columns
 __host__ __device__ constexpr int ring_max_threads(int len) { return len == 64 ? 256 : 32 * kRingWarps; }
 
-// The shared::cluster address of `smem_addr` (a shared::cta address of this CTA) in CTA `rank` of the cluster.
-__device__ __forceinline__ unsigned cluster_addr(unsigned smem_addr, unsigned rank) {
-    unsigned r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-    return r;
-}
-// Stores into another CTA's shared memory that count themselves off on that CTA's mbarrier when they have landed:
-// the receiver waits for the bytes, no fence and no cluster-wide barrier on the sender's side.
-__device__ __forceinline__ void st_async_f4(unsigned dst, float x, float y, float z, float w, unsigned mbar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst), "f"(x),
-                 "f"(y), "f"(z), "f"(w), "r"(mbar)
-                 : "memory");
-}
 // ... and stores of some of a warp's lanes, without a branch
 __device__ __forceinline__ void st1_async_if(unsigned at, float v, unsigned mbar, unsigned on) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t@p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0], %1, [%2];\n\t}" ::"r"(at),

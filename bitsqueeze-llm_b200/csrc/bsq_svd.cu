@@ -22,6 +22,7 @@
 // Omega comes from cuRAND's XORWOW generator like the reference's (svd_lowrank_cuda.cu:143,289-291),
 // seeded per call, column-major N x k.
 #include "bsq_cholesky.cuh"
+#include "bsq_cholesky_cluster.cuh"
 #include "bsq_device.cuh"
 #include "bsq_gemm.hpp"
 #include "bsq_internal.hpp"
@@ -55,6 +56,7 @@ struct SvdWorkspace {
     float *uc = nullptr, *vc = nullptr; // k x k outputs of the core SVD
     float *rfac = nullptr;              // k x k factor that nobody asked for
     CholeskySync *chol_sync = nullptr;  // zero between launches
+    bool chol_cluster = false;          // Gram matrices go to cholesky_cluster_kernel
     float *gemm_ws = nullptr;
     size_t gemm_ws_bytes = 0;
     float *solver_work = nullptr;
@@ -444,15 +446,16 @@ cudaError_t orthonormalise(SvdWorkspace *ws, float *Y, float *tmp, int rows, int
         if (k <= kCholeskyBlockedMaxK) {
             float *r_out = pass == 0 ? r_a : r_b;
             if (!r_out) r_out = ws->rfac;
-            const auto launch = [&](CholeskyPart part) {
-                launch_chained(cholesky_kernel, cholesky_grid(k, part), kCholThreads, cholesky_blocked_smem_bytes(k), st,
-                               ws->g, k, r_out, factor_only ? nullptr : ws->t, ws->chol_sync, ws->status, part);
-            };
-            if (factor_only || ws->device_full) {
-                launch(kCholFactor);
-                if (!factor_only && chol_blocks(k) > 1) launch(kCholInverse);
+            if (ws->chol_cluster) {
+                cudaLaunchConfig_t cfg;
+                cudaLaunchAttribute attr[2];
+                cholesky_cluster_config(&cfg, attr, k, st);
+                const float *g = ws->g;
+                if ((err = cudaLaunchKernelEx(&cfg, cholesky_cluster_kernel, g, k, r_out, factor_only ? (float *)nullptr : ws->t, ws->status)) != cudaSuccess)
+                    return err;
             } else {
-                launch(kCholBoth);
+                launch_chained(cholesky_kernel, factor_only ? 1 : chol_blocks(k), kCholThreads, cholesky_blocked_smem_bytes(k), st, ws->g, k, r_out,
+                               factor_only ? nullptr : ws->t, ws->chol_sync, ws->status);
             }
         } else if (k <= kCholeskySmemMaxK) {
             cholesky_inverse_smem_kernel<<<1, 1024, cholesky_smem_bytes(k), st>>>(ws->g, k, ws->t, pass == 0 ? r_a : r_b);
@@ -593,6 +596,17 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
             }
         }
     }
+    if (ok && ws->k > kCB && ws->k <= kCholeskyBlockedMaxK &&
+        cudaFuncSetAttribute(cholesky_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cholesky_cluster_smem_bytes(kCholeskyBlockedMaxK)) ==
+            cudaSuccess) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[2];
+        cholesky_cluster_config(&cfg, attr, ws->k, nullptr);
+        int clusters = 0;
+        // (a device, or a partition of one, that cannot place the cluster keeps the kernel of up to 32 columns)
+        ws->chol_cluster = cudaOccupancyMaxActiveClusters(&clusters, cholesky_cluster_kernel, &cfg) == cudaSuccess && clusters >= 1;
+    }
+    if (ok && !ws->chol_cluster) cudaGetLastError();
     if (ok && ws->k <= kCholeskyBlockedMaxK)
         ok = cudaFuncSetAttribute(cholesky_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)cholesky_blocked_smem_bytes(ws->k)) == cudaSuccess;
