@@ -12,14 +12,14 @@
 // kJacobiLastSweepCos) and leaves the vectors that much closer to orthogonal.
 //
 // What bounds it is one dependent chain -- dot product, angle, rotation -- per round of disjoint pairs, k - 1 rounds per
-// sweep and 7 to 9 sweeps whatever the split.  So the columns, not the rows, are dealt over the CTAs: CTA c of a cluster
-// of ceil(k / 32) holds two blocks of 16 whole columns, and the blocks move on over distributed shared memory only after
-// 16 rounds of one against the other.  (Rows dealt over the CTAs, as before, needs the partial dot products of every round
+// sweep and 6 to 9 sweeps whatever the split.  So the columns, not the rows, are dealt over the CTAs: CTA c of a cluster
+// holds two blocks of whole columns, most often 16 (block_jacobi_shape), and the blocks move on over distributed shared memory only after
+// as many rounds of one against the other.  (Rows dealt over the CTAs, as before, needs the partial dot products of every round
 // from every CTA.)  Inside a CTA a warp holds two columns of one block and two of the other in registers and does two
 // rounds on them (the straight pairs, then the crossed ones), each round two independent rotations whose angles are worked
 // out side by side in the halves of the warp: half as many trips through shared memory and CTA barriers per round, which
 // otherwise cost as much as the rotations (16 lanes per pair and a trip per round: 0.46 us per round at 256 columns).
-// A sweep: the pairs inside the blocks (a tournament of 8 column pairs), then 2 x CTAs - 1 steps of a tournament of the blocks.
+// A sweep: the pairs inside the blocks (a tournament of their column pairs), then 2 x CTAs - 1 steps of a tournament of the blocks.
 //   Measured against the kernels that deal rows over the CTAs (above 64 columns) or keep the core in one CTA, on 50 cores per
 //   rank (flat, 1/i, geometric, rank-3 and 1e-9-scaled spectra), time and distance from 64 bits of the singular values:
 //     k = 256 1323 -> 800 us, 2.3e-5 -> 5.4e-8; k = 128 461 -> 287 us, 1.3e-5 -> 5.7e-8; k = 64 222 -> 129 us, 5.3e-6 -> 5.5e-8;
@@ -36,19 +36,30 @@ namespace bsq {
 namespace {
 
 constexpr int kBlockJacobiMaxK = 256;
-constexpr int kJbCols = 16;                                  // columns of a block
-constexpr int kJbThreads = 32 * kJbCols / 2;                 // a warp per pair of columns of a block
 constexpr int kJacobiMaxSweeps = 30;
 // A sweep in which no visited pair had |cos(m_p, m_q)| above this is the last one: Jacobi converges quadratically,
 // so what such a sweep's rotations leave between the columns is of the order of the square of what it met
 // (<= 1e-8, below tol), and the sweep that would only confirm it (a full sweep's time for no rotation) is not run.
 // Pairs between tol and this bound are still rotated when they are met.
 constexpr float kJacobiLastSweepCos = 1.0e-4f;
-__host__ __device__ constexpr int block_jacobi_ctas(int k) { return (k + 2 * kJbCols - 1) / (2 * kJbCols); }
-__host__ __device__ constexpr int block_jacobi_len(int ctas) { return (ctas + 1) / 2 * 64; }       // padded column length: two floats per lane
-__host__ __device__ constexpr size_t block_jacobi_smem_bytes(int ctas, bool with_v) {
+__host__ __device__ constexpr int block_jacobi_len(int k) { return (k + 63) / 64 * 64; }           // padded column length: two floats per lane
+// How a core is dealt: CTAs of the cluster, columns of a block (two blocks per CTA, a warp per pair of a block's columns).
+struct BlockShape {
+    int ctas, cols;
+};
+// A sweep takes as many rounds as the blocks have columns, padding among them, so the shape follows the rank where 16 columns per block leave
+// much of that: us, 16 columns per block / as it is: k = 48 122 / 89, 24 61 / 47, 20 59 / 46, 72 185 / 166, 16 28 / 26.  Not taken, because
+// twice the CTAs gain little: 32 on 2 x 8 63 / 58, 96 on 6 x 8 218 / 210, 128 on 8 x 8 289 / 277; slower: 48 on 2 x 12 105, 64 on 4 x 8 136
+// against 124, 144 on 8 x 12 502 against 422.
+constexpr BlockShape block_jacobi_shape(int k) {
+    if (k <= 24) return {1, k <= 16 ? 8 : 12};
+    if (k > 32 && k <= 48) return {3, 8};
+    if (k > 64 && k <= 72) return {3, 12};
+    return {(k + 31) / 32, 16};
+}
+__host__ __device__ constexpr size_t block_jacobi_smem_bytes(BlockShape b, int len, bool with_v) {
     // two parities x two blocks of columns and of squared norms, all singular values, votes and largest entries, ranks
-    return ((size_t)4 * kJbCols * block_jacobi_len(ctas) * (with_v ? 2 : 1) + 4 * kJbCols + 32 * ctas + 2 * 8 + 8 + 2 * kJbCols) * sizeof(float);
+    return ((size_t)4 * b.cols * len * (with_v ? 2 : 1) + 4 * b.cols + 2 * b.cols * b.ctas + 2 * 8 + 8 + 2 * b.cols) * sizeof(float);
 }
 
 // two FP32 multiplications / multiply-adds per instruction; each half rounds as the scalar instruction does
@@ -181,12 +192,12 @@ __device__ __forceinline__ bool rotate_two(float2 (&p0)[kPairs], float2 (&q0)[kP
     return turn && gg > kJacobiLastSweepCos * kJacobiLastSweepCos * ab;
 }
 
-template <int kCtas, bool kWithV>
-__global__ void __launch_bounds__(kJbThreads, 1) block_jacobi_kernel(const float *C, int k, float *__restrict__ S,
+template <int kLen, int kCtas, int kJbCols, bool kWithV>
+__global__ void __launch_bounds__(16 * kJbCols, 1) block_jacobi_kernel(const float *C, int k, float *__restrict__ S,
                                                                    float *__restrict__ Ucol, float *__restrict__ Vcol) {
-    constexpr int kLen = block_jacobi_len(kCtas), kCol = kLen * (kWithV ? 2 : 1);      // rows of M; floats per column (V's below M's)
+    constexpr int kJbThreads = 16 * kJbCols, kCol = kLen * (kWithV ? 2 : 1);           // floats per column (V's below M's)
     constexpr int kPairs = kLen / 64;                                    // float2 per lane and column
-    constexpr int kBlock = kJbCols * kCol, kAll = 32 * kCtas;
+    constexpr int kBlock = kJbCols * kCol, kAll = 2 * kJbCols * kCtas;
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     const int cr = kCtas > 1 ? (int)cluster.block_rank() : 0;
@@ -272,7 +283,7 @@ __global__ void __launch_bounds__(kJbThreads, 1) block_jacobi_kernel(const float
         if (l < 2) norm[l] = l ? n[1] : n[0];
     };
     int cur = 0;
-    const int steps = k > kJbCols ? 2 * kCtas - 1 : 0;        // up to 16 columns there is one block and nothing to pair it with
+    const int steps = k > kJbCols ? 2 * kCtas - 1 : 0;        // (one block has nothing to pair it with)
     // where a CTA's blocks go after a step: block 0 ("top") of CTA 0 stays, the others move one place around the ring
     //   top of CTA 1, 2, .. , last, bottom of the last, .. , 1, 0, top of CTA 1
     const int top_cta = (cr == 0 || cr == kCtas - 1) ? cr : cr + 1, top_blk = (cr == 0 || cr != kCtas - 1) ? 0 : 1;
@@ -306,17 +317,18 @@ __global__ void __launch_bounds__(kJbThreads, 1) block_jacobi_kernel(const float
             if (!any || sweep == kJacobiMaxSweeps) break;     // the same votes in every CTA: all of them leave here
         }
         bool big = false;
-        // ---- inside the blocks: a tournament of each block's 8 column pairs, warps 0-3 on the first block, 4-7 on the second ----
+        // ---- inside the blocks: a tournament of each block's column pairs, half the warps on either block ----
         {
-            float *B = X + (size_t)(w >> 2) * kBlock, *nb = nx + (w >> 2) * kJbCols;
-            const int m = w & 3;                              // match of the round
-            for (int r = 0; r < 7; ++r) {
-                int p = 7, q = r;
+            constexpr int kTeams = kJbCols / 2, kMatches = kTeams / 2;
+            float *B = X + (size_t)(w / kMatches) * kBlock, *nb = nx + (w / kMatches) * kJbCols;
+            const int m = w % kMatches;                       // match of the round
+            for (int r = 0; r < kTeams - 1; ++r) {
+                int p = kTeams - 1, q = r;
                 if (m) {
                     p = r + m;
-                    q = r + 7 - m;
-                    p -= p >= 7 ? 7 : 0;
-                    q -= q >= 7 ? 7 : 0;
+                    q = r + kTeams - 1 - m;
+                    p -= p >= kTeams - 1 ? kTeams - 1 : 0;
+                    q -= q >= kTeams - 1 ? kTeams - 1 : 0;
                 }
                 take(c4.a, c4.av, c4.na, B + (size_t)(2 * p) * kCol, nb + 2 * p);
                 take(c4.b, c4.bv, c4.nb, B + (size_t)(2 * q) * kCol, nb + 2 * q);
@@ -419,27 +431,43 @@ __global__ void __launch_bounds__(kJbThreads, 1) block_jacobi_kernel(const float
 }
 
 typedef void (*BlockJacobiFn)(const float *, int, float *, float *, float *);
-template <int kCtas>
-BlockJacobiFn block_jacobi_fn_for(int ctas, bool with_v) {
-    if (ctas == kCtas) return with_v ? block_jacobi_kernel<kCtas, true> : block_jacobi_kernel<kCtas, false>;
-    if constexpr (kCtas > 1) return block_jacobi_fn_for<kCtas - 1>(ctas, with_v);
+// The instance for a core of k columns (k <= kBlockJacobiMaxK; null: there is none).
+template <int kLen, int kCtas, int kJbCols>
+BlockJacobiFn block_jacobi_instance(bool with_v) {
+    return with_v ? block_jacobi_kernel<kLen, kCtas, kJbCols, true> : block_jacobi_kernel<kLen, kCtas, kJbCols, false>;
+}
+BlockJacobiFn block_jacobi_fn(int k, bool with_v) {
+    const BlockShape b = block_jacobi_shape(k);
+    if (b.cols == 8) return b.ctas == 1 ? block_jacobi_instance<64, 1, 8>(with_v) : block_jacobi_instance<64, 3, 8>(with_v);
+    if (b.cols == 12) return b.ctas == 1 ? block_jacobi_instance<64, 1, 12>(with_v) : block_jacobi_instance<128, 3, 12>(with_v);
+    switch (b.ctas) {
+        case 1: return block_jacobi_instance<64, 1, 16>(with_v);
+        case 2: return block_jacobi_instance<64, 2, 16>(with_v);
+        case 3: return block_jacobi_instance<128, 3, 16>(with_v);
+        case 4: return block_jacobi_instance<128, 4, 16>(with_v);
+        case 5: return block_jacobi_instance<192, 5, 16>(with_v);
+        case 6: return block_jacobi_instance<192, 6, 16>(with_v);
+        case 7: return block_jacobi_instance<256, 7, 16>(with_v);
+        case 8: return block_jacobi_instance<256, 8, 16>(with_v);
+    }
     return nullptr;
 }
-// The instance for a core of k columns (k <= kBlockJacobiMaxK).
-BlockJacobiFn block_jacobi_fn(int k, bool with_v) { return block_jacobi_fn_for<block_jacobi_ctas(kBlockJacobiMaxK)>(block_jacobi_ctas(k), with_v); }
 
-// Launch configuration: one cluster.
-void block_jacobi_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, int k, bool with_v, cudaStream_t st) {
-    cfg->gridDim = dim3(block_jacobi_ctas(k), 1, 1);
-    cfg->blockDim = dim3(kJbThreads, 1, 1);
-    cfg->dynamicSmemBytes = block_jacobi_smem_bytes(block_jacobi_ctas(k), with_v);
+// Launch configuration: one cluster, behind the kernel before as launch_chained has it.
+void block_jacobi_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute (&attr)[2], int k, bool with_v, cudaStream_t st) {
+    const BlockShape b = block_jacobi_shape(k);
+    cfg->gridDim = dim3(b.ctas, 1, 1);
+    cfg->blockDim = dim3(16 * b.cols, 1, 1);
+    cfg->dynamicSmemBytes = block_jacobi_smem_bytes(b, block_jacobi_len(k), with_v);
     cfg->stream = st;
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = block_jacobi_ctas(k);
+    attr[0].val.clusterDim.x = b.ctas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg->attrs = attr;
-    cfg->numAttrs = 1;
+    cfg->numAttrs = 2;
 }
 
 }  // namespace

@@ -19,8 +19,8 @@
 // four dot products in one butterfly whose halves end with different slots, so the four angles are worked out side by side.
 // (Rows dealt over the CTAs: every column through shared memory in every round, and the partial products of every round from and to every CTA.)
 // Four warps per CTA, one per scheduler: eight measured 10 to 20 % slower, sixteen on one CTA 45 % (128 columns).
-//   Against the kernels that it stands for, core alone: k = 256 1545 -> 1138 us, 200 1199 -> 893, 131 799 -> 568, 128 517 -> 410, 65 258 -> 210,
-//   64 249 -> 218.  Up to kRingMinK columns jacobi_svd_kernel is as fast or faster (48 160 / 158, 16 48 / 44).
+//   Against the kernels that it stands for, core alone: k = 256 1545 -> 1008 us, 192 1150 -> 761, 131 799 -> 563, 128 517 -> 413, 65 258 -> 221,
+//   64 249 -> 199.  Up to kRingMinK columns jacobi_svd_kernel is as fast or faster (48 160 / 158, 16 48 / 44).
 #pragma once
 
 #include "bsq_device.cuh"
@@ -285,6 +285,15 @@ __global__ void __launch_bounds__(ring_max_threads(kLen), 1) ring_jacobi_kernel(
         }
         if (!(vote & 1) || (vote & 2) || sweep == kJacobiMaxSweeps) break;
         float seen = 0.0f;                                    // 1: this lane's slot met a pair above the bound of the last sweep
+        // The sums of the pairs that stay inside the warp are begun in front of the round's barrier, while the columns of the others are on their
+        // way (256 columns 1084 -> 1023 us), at 128 columns what only the end of a sweep wants comes last (375 -> 366 at rank 100), and rounds are unrolled where that helps: two
+        // at 256 columns (1008), four at 64 (216 -> 199), none at 128 (two 413 -> 459).  Not so: columns that leave rotated and sent
+        // before the others (128 columns 418 -> 447), what comes in taken from shared memory before the vote on the waits (462).
+        constexpr int kUnroll = kLen == 64 ? 4 : kLen == 256 ? 2 : 1;
+        float inner_a[2], inner_b[2];
+        dot4(P[1], Q[1], inner_a[0], inner_b[0]);
+        dot4(P[2], Q[2], inner_a[1], inner_b[1]);
+#pragma unroll kUnroll
         for (int r = 0; r < rounds; ++r, ++it) {
             const unsigned par = it & 1, phase = (it >> 1) & 1;
             if (works) {
@@ -293,8 +302,10 @@ __global__ void __launch_bounds__(ring_max_threads(kLen), 1) ring_jacobi_kernel(
                 float g;
                 {
                     float ta[kS], tb[kS];
-                    dot4(P[1], Q[1], ta[1], tb[1]);           // (the columns that have just come in last)
-                    dot4(P[2], Q[2], ta[2], tb[2]);
+                    ta[1] = inner_a[0];
+                    tb[1] = inner_b[0];
+                    ta[2] = inner_a[1];
+                    tb[2] = inner_b[1];
                     dot4(P[0], Q[0], ta[0], tb[0]);
                     dot4(P[3], Q[3], ta[3], tb[3]);
                     float g2[2], o[2];
@@ -347,7 +358,7 @@ __global__ void __launch_bounds__(ring_max_threads(kLen), 1) ring_jacobi_kernel(
                     sj[j] = __shfl_sync(kFullMask, sn, lane_of(j));
                 }
                 const float pn = turn ? fmaxf(alpha - t * g, 0.0f) : alpha, qn = turn ? beta + t * g : beta;
-                seen = turn && g * g > kJacobiLastSweepCos * kJacobiLastSweepCos * alpha * beta ? 1.0f : seen;
+                if (kLen != 128) seen = turn && g * g > kJacobiLastSweepCos * kJacobiLastSweepCos * alpha * beta ? 1.0f : seen;
                 constexpr unsigned kAll = 1u << lane_of(0) | 1u << lane_of(1) | 1u << lane_of(2) | 1u << lane_of(3);
                 if ((turns & kAll) == kAll) {
                     rotate(P[0], Q[0], cj[0], sj[0]);
@@ -396,6 +407,7 @@ __global__ void __launch_bounds__(ring_max_threads(kLen), 1) ring_jacobi_kernel(
                 } else {
                     put(up_to + par * box_par, Q[kS - 1]);
                 }
+                if (kLen == 128) seen = turn && g * g > kJacobiLastSweepCos * kJacobiLastSweepCos * alpha * beta ? 1.0f : seen;
                 // everything moves one slot on
 #pragma unroll
                 for (int j = 0; j + 1 < kS; ++j)
@@ -406,6 +418,8 @@ __global__ void __launch_bounds__(ring_max_threads(kLen), 1) ring_jacobi_kernel(
 #pragma unroll
                     for (int u = 0; u < kN2; ++u) Q[j][u] = Q[j - 1][u];
             }
+            dot4(P[1], Q[1], inner_a[0], inner_b[0]);
+            dot4(P[2], Q[2], inner_a[1], inner_b[1]);
             __syncthreads();
             if (works) {
                 if (kCluster) {
@@ -500,7 +514,7 @@ RingLaunch ring_jacobi_launch(int k, bool with_v) {
     }
     return r;
 }
-void ring_jacobi_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, const RingLaunch &r, cudaStream_t st) {
+void ring_jacobi_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute (&attr)[2], const RingLaunch &r, cudaStream_t st) {
     cfg->gridDim = dim3(r.ctas, 1, 1);
     cfg->blockDim = dim3(32 * r.warps, 1, 1);
     cfg->dynamicSmemBytes = r.smem;
@@ -509,8 +523,10 @@ void ring_jacobi_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, cons
     attr[0].val.clusterDim.x = r.ctas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg->attrs = attr;
-    cfg->numAttrs = 1;
+    cfg->numAttrs = 2;
 }
 
 }  // namespace

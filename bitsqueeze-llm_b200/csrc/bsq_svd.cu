@@ -562,11 +562,11 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
         const char *v = getenv("BSQ_JACOBI_V");
         ws->jc_with_v = v ? v[0] == '1' : ws->k <= kCoreWithVMaxK;
         cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         block_jacobi_config(&cfg, attr, ws->k, ws->jc_with_v, nullptr);
         const BlockJacobiFn fn = block_jacobi_fn(ws->k, ws->jc_with_v);
         int clusters = 0;
-        ws->block_core = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) == cudaSuccess &&
+        ws->block_core = fn && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) == cudaSuccess &&
                          cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters >= 1;
         if (!ws->block_core) {                               // a device (or partition of one) that cannot place the cluster
             cudaGetLastError();
@@ -586,7 +586,7 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
         if (ok && ws->ring.ctas > 1) {
             // a device (or partition of one) that cannot place the cluster keeps the library solver
             cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute attr[1];
+            cudaLaunchAttribute attr[2];
             ring_jacobi_config(&cfg, attr, ws->ring, nullptr);
             int clusters = 0;
             const cudaError_t q = cudaOccupancyMaxActiveClusters(&clusters, ws->ring.fn, &cfg);
@@ -732,14 +732,14 @@ cudaError_t svd_lowrank(SvdWorkspace *ws, const float *d_A, float *d_U, float *d
     // The row-major C read as column-major is C^T = Vc S Uc^T: the solver's "U" is Vc, its "V" is Uc.
     if (ws->block_core) {
         cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         block_jacobi_config(&cfg, attr, k, ws->jc_with_v, st);
         const float *core = ws->core;
         float *vc = ws->vc, *uc = ws->uc;
         if ((err = cudaLaunchKernelEx(&cfg, block_jacobi_fn(k, ws->jc_with_v), core, k, d_S, vc, uc)) != cudaSuccess) return err;
     } else if (ws->own_core_svd && k > kRingMinK) {
         cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         ring_jacobi_config(&cfg, attr, ws->ring, st);
         const float *core = ws->core;
         float *vc = ws->vc, *uc = ws->uc;
