@@ -13,7 +13,8 @@ namespace {
 
 constexpr int TM = 128;          // output rows per CTA (UMMA M)
 constexpr int TK = 16;           // K per shared-memory stage (two k-steps of 8)
-constexpr int NT = 256;          // threads: all stage operands, one issues the MMAs, two per accumulator row in the epilogue
+constexpr int NT = 256;          // threads that stage operands, two per accumulator row in the epilogue
+constexpr int NT2 = NT + 32;     // and a control warp, which issues the MMAs
 constexpr int DEPTH = 3;         // chunks of K in flight in registers per thread
 constexpr int STAGES = 2;        // operand stages in shared memory (three measured slower: less L1 left for the loads)
 
