@@ -15,7 +15,7 @@
 //     and lo*hi + hi*lo into a second one, added in the epilogue (the dropped lo*lo term and the
 //     rounding of lo are ~2^-22 relative; the tensor core truncates when it accumulates, which leaves
 //     an error of a few 1e-7 of sum |a||b| for K in the thousands, against a few 1e-8 on the FP32 pipes);
-//   * 256 threads stage 16 of K at a time and keep the global loads of three such chunks in flight in
+//   * 256 threads stage 16 of K at a time and keep the global loads of one or two such chunks in flight in
 //     registers, so HBM latency hides behind the staging of earlier chunks; two shared-memory stages:
 //     the splits of chunk c+1 overlap the MMAs of chunk c; tcgen05.commit on an mbarrier tells when a
 //     stage may be overwritten and when the tile is done; two CTAs share an SM when N <= 128;
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(NT2, NMAX <= 128 ? 2 : 1) gemm_tc_kernel(GemmA
     __shared__ __align__(8) uint64_t bar_free[STAGES];
     __shared__ __align__(8) uint64_t bar_done;
     __shared__ unsigned tmem_base_slot;
-    constexpr int ITEMS = NMAX / (NT - TM);                   // slots of B per serving thread: 1 (N <= 128) or 2
+    constexpr int ITEMS = NMAX / (NT - TM), DEPTH = tc_depth(NMAX);      // slots of B per serving thread: 1 (N <= 128) or 2
     const int tid = threadIdx.x, warp = tid >> 5;
     const bool control = warp == NT / 32;                     // the ninth warp issues the MMAs
     const int n0 = blockIdx.y * g.n_tile;                     // this CTA's columns: n0 .. n0 + N

@@ -15,7 +15,10 @@ constexpr int TM = 128;          // output rows per CTA (UMMA M)
 constexpr int TK = 16;           // K per shared-memory stage (two k-steps of 8)
 constexpr int NT = 256;          // threads that stage operands, two per accumulator row in the epilogue
 constexpr int NT2 = NT + 32;     // and a control warp, which issues the MMAs
-constexpr int DEPTH = 3;         // chunks of K in flight in registers per thread
+// Chunks of K in flight in registers per thread, by tile width.  What is in flight hides the loads, what is unrolled costs instruction fetches and
+// registers: us at 1 / 2 / 3 chunks, tiles up to 128 columns: 8192 x 128 x 4096 67.8 / 74.7 / 76.4, its transpose 60.6 / 63.1 / 62.4, 8192 x 256 x 256
+// 14.4 / 15.3 / 16.1, Gram matrix of 4096 x 256 13.0 / 13.4 / 13.7; wider: 14336 x 256 x 256 22.4 / 19.5 / 21.1, Gram matrix 22.0 / 19.5 / 21.3.
+__host__ __device__ constexpr int tc_depth(int nmax) { return nmax <= 128 ? 1 : 2; }
 constexpr int STAGES = 2;        // operand stages in shared memory (three measured slower: less L1 left for the loads)
 
 __device__ __forceinline__ uint64_t smem_desc(unsigned addr_bytes, unsigned lbo_bytes, unsigned sbo_bytes) {
