@@ -101,6 +101,7 @@ SIGNATURES = {
     "bsq_lane_destroy": (None, [_vp]),
     "bsq_lane_packed_capacity": (_u64, [_vp]),
     "bsq_lane_stream": (_vp, [_vp, _i]),
+    "bsq_lane_order_after": (_i, [_vp, _i, _vp]),
     "bsq_lane_compress_begin": (_i, [_vp, _vp, _i, _vp, _u64]),
     "bsq_lane_compress_end": (_i, [_vp, C.POINTER(_vp), _vp, C.POINTER(_u64)]),
     "bsq_lane_decompress_begin": (_i, [_vp, _vp, _i, _vp, _u64]),

@@ -234,6 +234,7 @@ struct Runtime {
     int sm_count = 148;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[8] = {};
+    cudaEvent_t order = nullptr;                         // bsq_lane_order_after
     DevBuf input_stage, residual, error, u, s, v, scratch, status, recon_ws;
     size_t recon_ws_bytes = 0;
     QuantBufs q_direct, q_u, q_s, q_v;
@@ -256,6 +257,7 @@ struct Runtime {
         outlier.release(); err.release();
         if (svd) { svd_workspace_destroy(svd); svd = nullptr; }
         for (auto &e : ev) { if (e) cudaEventDestroy(e); e = nullptr; }
+        if (order) { cudaEventDestroy(order); order = nullptr; }
         if (h_status) { cudaFreeHost(h_status); h_status = nullptr; }
         if (h_stage) { cudaFreeHost(h_stage); h_stage = nullptr; }
         if (job.active && !job.to_device && job.block) {
@@ -1146,7 +1148,10 @@ bool heads_as_expected(Runtime &rt, const HeadCheck &check) {
     for (unsigned i = 1; (*answer | 1u) != (check.number | 1u); ++i) {
         if (i % 4096 != 0) continue;
         const cudaError_t q = cudaStreamQuery(rt.stream);
-        if (q == cudaErrorNotReady) continue;
+        if (q == cudaErrorNotReady) {
+            cudaGetLastError();                              // (an answer, but noted as an error)
+            continue;
+        }
         if (q != cudaSuccess || (*answer | 1u) != (check.number | 1u)) return false;
     }
     return *answer == check.number;
@@ -1456,6 +1461,28 @@ uint64_t bsq_lane_packed_capacity(bsq_lane *lane) {
 void *bsq_lane_stream(bsq_lane *lane, int decompress_side) {
     if (!lane) return nullptr;
     return decompress_side ? lane->decompress.stream : lane->compress.stream;
+}
+
+// (An event of its own per call, created, recorded, waited for and destroyed from Python, was 4 us of a 36 us call, and the wait for one
+// that has long passed still holds the lane's first kernel up.)
+int bsq_lane_order_after(bsq_lane *lane, int decompress_side, void *stream) {
+    if (!lane) return 1;
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return 1;
+    const bool elsewhere = device != lane->device;
+    if (elsewhere && cudaSetDevice(lane->device) != cudaSuccess) return 1;
+    Runtime &rt = decompress_side ? lane->decompress : lane->compress;
+    const cudaStream_t st = static_cast<cudaStream_t>(stream);
+    cudaError_t err = cudaStreamQuery(st);
+    if (err == cudaErrorNotReady) {
+        cudaGetLastError();                                  // (an answer, but noted as an error)
+        err = rt.order ? cudaSuccess : cudaEventCreateWithFlags(&rt.order, cudaEventDisableTiming);
+        if (err == cudaSuccess) err = cudaEventRecord(rt.order, st);
+        if (err == cudaSuccess) err = cudaStreamWaitEvent(rt.stream, rt.order, 0);
+    }
+    if (err != cudaSuccess) cudaGetLastError();
+    if (elsewhere) cudaSetDevice(device);
+    return err == cudaSuccess ? 0 : 1;
 }
 
 int bsq_lane_compress_begin(bsq_lane *lane, const float *matrix, int input_location, void *d_packed, uint64_t capacity) {

@@ -63,8 +63,6 @@ class Compressor:
         if not self._lane:
             raise RuntimeError("bsq_lane_create failed (invalid settings or out of device memory)")
         self.capacity = int(self._lib.bsq_lane_packed_capacity(self._lane))
-        self._c_stream = torch.cuda.ExternalStream(self._lib.bsq_lane_stream(self._lane, 0), device=self._device)
-        self._d_stream = torch.cuda.ExternalStream(self._lib.bsq_lane_stream(self._lane, 1), device=self._device)
 
     def close(self):
         if self._lane:
@@ -77,6 +75,11 @@ class Compressor:
         except Exception:
             pass
 
+    def _order_after(self, side):
+        """What is begun next on that side comes behind the work on PyTorch's current stream."""
+        if self._lib.bsq_lane_order_after(self._lane, side, torch.cuda.current_stream(self._device).cuda_stream) != 0:
+            raise RuntimeError("bsq_lane_order_after failed")
+
     # ---- compress ----
     def compress_async(self, x, out=None):
         """Queues the compression of `x` behind the work on PyTorch's current stream and returns a handle whose wait()
@@ -88,7 +91,7 @@ class Compressor:
         elif out.dtype != torch.uint8 or out.numel() < self.capacity or not out.is_cuda or not out.is_contiguous():
             raise ValueError("out must be a contiguous uint8 CUDA tensor of at least %d bytes" % self.capacity)
         location = INPUT_DEVICE if x.is_cuda else INPUT_HOST
-        self._c_stream.wait_stream(torch.cuda.current_stream(self._device))      # x and out may still be written there
+        self._order_after(0)                                  # x and out may still be written on PyTorch's stream
         if self._lib.bsq_lane_compress_begin(self._lane, x.data_ptr(), location, out.data_ptr(), out.numel()) != 0:
             raise RuntimeError("bsq_lane_compress_begin failed")
         # x and out are kept alive by this closure until wait() has seen the lane's stream finish, so the caching
@@ -112,7 +115,7 @@ class Compressor:
             out = torch.empty((self.rows, self.cols), dtype=torch.float32, device=torch.device("cuda", self._device))
         elif out.dtype != torch.float32 or out.numel() < self.rows * self.cols or not out.is_cuda or not out.is_contiguous():
             raise ValueError("out must be a contiguous float32 CUDA tensor of rows x cols elements")
-        self._d_stream.wait_stream(torch.cuda.current_stream(self._device))
+        self._order_after(1)
         host_obj = None
         if isinstance(packed, PackedMatrix):
             rc = self._lib.bsq_lane_decompress_begin(self._lane, C.byref(packed.header), 1, out.data_ptr(), out.numel())
