@@ -185,9 +185,14 @@ void launch_fp32(const GemmArgs &g, cudaStream_t stream) {
 // small product is the way of its few steps from memory: copies that are waited for one by one and 128 x 128 tiles for everything took
 // 14 to 18 us for each product of 777 x 1031 at rank 48, whole compress and decompress calls of that shape 0.79 ms, now 0.64;
 // 2048 x 5120 at rank 64, whose Gram matrices run here, 1.14 and 1.08 ms.
+// Wider products, reconstructions above all, take 64 x 64 tiles as well where those of 128 x 128 are no more than half the SMs: us, 128 / 64,
+// 396 x 557 x 19 7.5 / 3.8, 777 x 1031 x 48 9.6 / 6.1, 777 x 1031 x 200 32.0 / 18.6, 65 x 8000 x 20 6.7 / 4.6 (63 tiles and fewer); 144 tiles, on the
+// other side: 1500 x 1500 x 48 9.9 / 10.8, 2000 x 1030 x 33 10.3 / 12.3.
 template <bool A_KMAJOR, bool B_KMAJOR>
 void launch_fp32(const GemmArgs &g, int sm_count, cudaStream_t stream) {
-    if (g.N > 64) launch_fp32<A_KMAJOR, B_KMAJOR, 128, 128, 2>(g, stream);
+    const long tiles = (long)((g.M + 127) / 128) * ((g.N + 127) / 128) * g.splits;
+    if (g.N > 64 && 2 * tiles > sm_count) launch_fp32<A_KMAJOR, B_KMAJOR, 128, 128, 2>(g, stream);
+    else if (g.N > 64) launch_fp32<A_KMAJOR, B_KMAJOR, 64, 64, 4>(g, stream);
     else if (g.M <= 64 || (long)((g.M + 127) / 128) * g.splits < sm_count) launch_fp32<A_KMAJOR, B_KMAJOR, 64, 64, 4>(g, stream);
     else launch_fp32<A_KMAJOR, B_KMAJOR, 128, 64, 3>(g, stream);
 }
