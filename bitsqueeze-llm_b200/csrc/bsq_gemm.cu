@@ -398,8 +398,8 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
             }
         }
         const int slots = (t.use_tma ? 1 : with_image ? gemm_tc_image_ctas_per_sm(t.n_tile) : (t.n_tile <= 128 ? 2 : 1)) * sm_count;
-        // the FP16 form of the split (BSQ_GEMM_F16=1; =2 also without a given bound on |A|: it is then worked out here,
-        // a pass over A): 256-column products with A contiguous along K on the TMA-fed kernel
+        // the FP16 form of the split (BSQ_GEMM_F16=1, products whose caller gives a bound on |A|; =2 also 256-column products without one:
+        // it is then worked out here, a pass over A)
         if (t.use_tma && !t.persistent && !kscale && !minuend && workspace_bytes >= 4096 &&
             (halves16 || (t.n_tile == 256 && (f16_mode() == 2 || (f16_mode() == 1 && a_absmax_bits))))) {
             unsigned *words = reinterpret_cast<unsigned *>(workspace);      // [0]: |B| max, [1]: |A| max when not given
@@ -415,7 +415,8 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
                 t.a_absmax_bits = words + 1;
             }
         }
-        if (t.use_tma) gemm_tc_tma_rings(t.n_tile, a_kmajor, &t.raw_stages, &t.a_stages, &t.b_stages, t.f16 && !t.a_image);
+        t.boxed_c = t.wide_tiles && t.f16;
+        if (t.use_tma) gemm_tc_tma_rings(t.n_tile, a_kmajor, &t.raw_stages, &t.a_stages, &t.b_stages, t.f16 && !t.a_image, t.boxed_c);
         else if (with_image) gemm_tc_image_rings(t.n_tile, &t.a_stages, &t.b_stages);
         if (workspace && !minuend && !kscale && tiles_tc < slots) {
             const int max_by_k = max(1, K / 256);             // a split below 256 of K costs more in the reduction than it gains

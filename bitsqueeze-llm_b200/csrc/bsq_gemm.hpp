@@ -33,6 +33,7 @@ struct GemmArgs {
                                // then fit tensor memory), their epilogue shared by the warps that have nothing to split: per
                                // column of C half as many barrier waits, descriptors and commits for the one thread that issues
                                // the MMAs, which is what bounds a product with a short K
+    bool boxed_c;              // wide_tiles and f16: tiles of C leave through boxes in shared memory
     int sm_count;
     bool f16;                      // TMA-fed kernel: operands split into two FP16 halves (bsq_gemm_tc.cuh) instead of two TF32
     const unsigned *a_absmax_bits; // halves; device words with the bits of the largest |A| and |B| (finite), from which the
@@ -63,7 +64,7 @@ cudaError_t gemm_tc_launch(const GemmArgs &g, bool a_kmajor, bool b_kmajor, unsi
 // BSQ_GEMM_TMA switch; gemm_tc_tma_rings gives the ring lengths for raw_stages / a_stages / b_stages.
 bool gemm_tc_tma_enabled();
 bool gemm_tc_tma_usable(const GemmArgs &g, bool a_kmajor);
-void gemm_tc_tma_rings(int n_tile, bool a_kmajor, int *nraw, int *nr, int *nb, bool f16 = false);
+void gemm_tc_tma_rings(int n_tile, bool a_kmajor, int *nraw, int *nr, int *nb, bool f16 = false, bool boxed_c = false);
 cudaError_t gemm_tc_tma_launch(const GemmArgs &g, bool a_kmajor, unsigned *status, cudaStream_t stream);
 
 }  // namespace bsq

@@ -57,6 +57,10 @@ __device__ __forceinline__ void tma_load_2d(void *dst_smem, const CUtensorMap *m
                  "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
                  : "memory");
 }
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, int x, int y, const void *src_smem) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x), "r"(y), "r"(smem_u32(src_smem))
+                 : "memory");
+}
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -86,6 +90,8 @@ __device__ __forceinline__ void tc_commit(uint64_t *bar) {
 
 constexpr unsigned RAW_BOX = 32 * 32 * 4;       // A contiguous along M: one box of 32 k x 32 rows, four per slot
 constexpr unsigned RAW_SLOT = 4 * RAW_BOX;
+constexpr unsigned C_BOX = 32 * 32 * 4;         // 32 rows x 32 columns of C on their way out (EPI_STORE, EPI_MINUEND: one box for each of the 8 epilogue warps)
+constexpr int EPI_LANES = 0, EPI_STORE = 1, EPI_MINUEND = 2;   // how a tile leaves: each lane its own row; wide FP16 tiles, without and with a minuend
 
 struct TmaBars {
     uint64_t full_a[MAXR], ready_a[MAXR], empty_a[MAXR], full_b[MAXR], empty_b[MAXR];
@@ -135,8 +141,9 @@ struct TileWalk {
 // all layouts keep their BYTES (a 128-byte operand row now holds 64 of K, an image of B 32 of K), so descriptors, rings
 // and the MMA issue loop are the same; the caller's FP32 boxes go through the raw ring in both orientations, because
 // the 16-bit images cannot be made in place.
-template <bool A_KMAJOR, int NMAX, bool F16 = false>
-__global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_constant__ CUtensorMap tmap_a, GemmArgs g, unsigned *status) {
+template <bool A_KMAJOR, int NMAX, bool F16 = false, int EPI = EPI_LANES>
+__global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_c, GemmArgs g,
+                                                             unsigned *status) {
     chain_begin();
     extern __shared__ unsigned char smem_dyn[];
     unsigned char *base = smem_dyn + ((1024u - (smem_u32(smem_dyn) & 1023u)) & 1023u);      // the swizzle wants 1024-byte aligned slots
@@ -146,15 +153,16 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
     constexpr unsigned RAW_SLOT = F16 ? 2u * bsq::RAW_SLOT : bsq::RAW_SLOT;
     const int NR = g.a_stages, NB = g.b_stages, NRAW = (USES_RAW && g.a_image == nullptr) ? g.raw_stages : 0;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool a_img = A_KMAJOR && g.a_image != nullptr;           // A split beforehand: both halves of a slot come in by TMA
+    const bool a_img = EPI != EPI_LANES || (!F16 && A_KMAJOR && g.a_image != nullptr);    // A split beforehand: both halves of a slot come in by TMA
     const unsigned b_stride = 2u * image_half_units(g.n_tile) * 16u;
     unsigned char *raw_slots = base;
     unsigned char *a_slots = raw_slots + (size_t)NRAW * RAW_SLOT;
     unsigned char *b_slots = a_slots + (size_t)NR * A_SLOT;
-    TmaBars &bars = *reinterpret_cast<TmaBars *>(b_slots + (size_t)NB * b_stride);
+    unsigned char *c_boxes = b_slots + (size_t)NB * b_stride;
+    TmaBars &bars = *reinterpret_cast<TmaBars *>(c_boxes + (EPI != EPI_LANES ? 8 * C_BOX : 0));
     // accumulator columns of one set (hi*hi chain and, acc_cols further on, the cross terms), and how many sets
     const unsigned acc_cols = g.n_tile <= 16 ? 16u : (g.n_tile <= 32 ? 32u : (g.n_tile <= 64 ? 64u : (g.n_tile <= 128 ? 128u : 256u)));
-    const bool one_acc = a_img && g.wide_tiles;                    // the cross terms go into the hi * hi accumulator
+    const bool one_acc = EPI != EPI_LANES || (a_img && g.wide_tiles);                    // the cross terms go into the hi * hi accumulator
     const unsigned acc_stride = one_acc ? acc_cols : 2u * acc_cols;  // tensor-memory columns of one set
     const int acc_sets = (g.persistent && acc_stride <= 256u) ? 2 : 1;
     // Tensor memory has room for a second hi * hi accumulator beside those of a narrow tile: slots of A go to one and the other in turn.
@@ -468,6 +476,22 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
         const bool wide32 = ((reinterpret_cast<uintptr_t>(g.C) | (uintptr_t)(g.ldc * 4) | (uintptr_t)(g.split_stride * 4)) % 32 == 0) &&
                             (!g.minuend || (reinterpret_cast<uintptr_t>(g.minuend) | (uintptr_t)(g.ldm * 4)) % 32 == 0);
         bool any = false;
+        // (EPI_MINUEND) this warp's 32 x 32 piece `s32` of the minuend of tile i: eight lanes a row
+        float4 mn[2][8];
+        auto ask_minuend = [&](int i, int s32, float4 (&m)[8]) {
+            if (i >= walk.count) return;
+            int mt, nt, z;
+            walk.at(i, &mt, &nt, &z);
+            const int row = mt * TM + quarter * 32 + (lane >> 3), col = nt * g.n_tile + cb + 32 * s32 + 4 * (lane & 7);
+            if (col >= g.N) return;                                      // (n_tile is 256: only the matrix ends inside a tile)
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (row + 4 * j < g.M) m[j] = *reinterpret_cast<const float4 *>(g.minuend + (long)(row + 4 * j) * g.ldm + col);
+        };
+        if (EPI == EPI_MINUEND) {
+            ask_minuend(0, 0, mn[0]);
+            ask_minuend(0, 1, mn[1]);
+        }
         Ring rs(acc_sets);
         for (int i = 0; i < walk.count && ok; ++i, rs.next()) {
             int mt, nt, z;
@@ -481,7 +505,7 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
             // the wait for the accumulators, so that its HBM latency passes while the tensor core still works on the
             // tile (fetched 16 columns at a time inside the loop below, every step would wait for memory on its own).
             const int ce = one_acc ? min(N, cb + 128) : N;                // this thread's columns of the tile: cb .. ce - 1
-            const bool pre = g.minuend != nullptr && ce - cb == 128 && row < g.M;
+            const bool pre = !F16 && g.minuend != nullptr && ce - cb == 128 && row < g.M;
             float4 mn_pre[32];
             if (pre) {
                 const float *mn = g.minuend + (long)row * g.ldm + n0 + cb;
@@ -494,9 +518,75 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
                 }
             }
             ok = mbar_wait_bounded(&bars.acc_full[set], rs.par, status);
+            if (EPI != EPI_LANES) ok = __all_sync(0xffffffffu, ok);               // (its lanes go on together or not at all)
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (pre) {
+            if (EPI == EPI_STORE) {
+                // 32 columns at a time into this warp's box in shared memory (16-byte pieces swizzled: no bank conflicts), which leaves by one
+                // TMA store: whole 128-byte lines, and the warp goes on.  Stores of 32 bytes per lane and row took 7 to 8.5 us per tile
+                // whatever its K, which was what bounded the reconstructions (4096 x 14336 at rank 256 97.4 -> 82.2 us, 8192 x 4096 60 -> 46.6;
+                // one box of 128 rows for four warps, which then met at barriers: 88.4).
+                unsigned char *box = c_boxes + (warp - 3) * C_BOX;
+                for (int s32 = 0; s32 < 4 && cb + 32 * s32 < N; ++s32) {
+                    unsigned r[32];
+                    const unsigned taddr = tmem_d + (unsigned)set * acc_stride + ((unsigned)(quarter * 32) << 16) + (unsigned)(cb + s32 * 32);
+                    tmem_ld16(taddr, reinterpret_cast<unsigned(&)[16]>(r[0]));
+                    if (cb + 32 * s32 + 16 < N) tmem_ld16(taddr + 16, reinterpret_cast<unsigned(&)[16]>(r[16]));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    float4 o4[8];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        o4[j] = make_float4(__fmul_rn(__uint_as_float(r[4 * j]), inv16), __fmul_rn(__uint_as_float(r[4 * j + 1]), inv16),
+                                            __fmul_rn(__uint_as_float(r[4 * j + 2]), inv16), __fmul_rn(__uint_as_float(r[4 * j + 3]), inv16));
+                    }
+                    if (lane == 0) bulk_wait_read_all();                // the box's last store has read it
+                    __syncwarp();
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) reinterpret_cast<float4 *>(box)[lane * 8 + (j ^ (lane & 7))] = o4[j];
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0 && mt * TM + quarter * 32 < g.M) {
+                        tma_store_2d(&tmap_c, n0 + cb + 32 * s32, mt * TM + quarter * 32, box);
+                        bulk_commit();
+                    }
+                }
+            } else if (EPI == EPI_MINUEND) {
+                // The same way out, but back from the box to the lanes, eight of them a row: the minuend's pieces come in the same layout, asked
+                // for two blocks of 32 columns ahead (64 KB of it in flight per SM, through the wait for the accumulators), and the
+                // differences leave, as whole 128-byte lines.  8192 x 4096 at rank 256 99.6 -> 75.4 us; the minuend of the whole tile asked for
+                // before the wait, a row per lane, took 128 registers (spills) and 32 bytes of each line at a time.
+                float4 *box = reinterpret_cast<float4 *>(c_boxes + (warp - 3) * C_BOX);
+#pragma unroll
+                for (int s32 = 0; s32 < 4; ++s32) {
+                    if (cb + 32 * s32 < N) {
+                        unsigned r[32];
+                        const unsigned taddr = tmem_d + (unsigned)set * acc_stride + ((unsigned)(quarter * 32) << 16) + (unsigned)(cb + s32 * 32);
+                        tmem_ld16(taddr, reinterpret_cast<unsigned(&)[16]>(r[0]));
+                        if (cb + 32 * s32 + 16 < N) tmem_ld16(taddr + 16, reinterpret_cast<unsigned(&)[16]>(r[16]));
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        __syncwarp();                                    // the box's last block has been read
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            box[lane * 8 + (j ^ (lane & 7))] =
+                                make_float4(__fmul_rn(__uint_as_float(r[4 * j]), inv16), __fmul_rn(__uint_as_float(r[4 * j + 1]), inv16),
+                                            __fmul_rn(__uint_as_float(r[4 * j + 2]), inv16), __fmul_rn(__uint_as_float(r[4 * j + 3]), inv16));
+                        __syncwarp();
+                        const int col = cb + 32 * s32 + 4 * (lane & 7);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const int rr = 4 * j + (lane >> 3), at = mt * TM + quarter * 32 + rr;
+                            const float4 m4 = mn[s32 & 1][j], v = box[rr * 8 + ((lane & 7) ^ (rr & 7))];
+                            const float4 o = make_float4(__fsub_rn(m4.x, v.x), __fsub_rn(m4.y, v.y), __fsub_rn(m4.z, v.z), __fsub_rn(m4.w, v.w));
+                            if (at < g.M && col < N) {
+                                any |= fabsf(o.x) > 1.1920928955078125e-07f || fabsf(o.y) > 1.1920928955078125e-07f ||
+                                       fabsf(o.z) > 1.1920928955078125e-07f || fabsf(o.w) > 1.1920928955078125e-07f;
+                                *reinterpret_cast<float4 *>(C + (long)at * g.ldc + n0 + col) = o;
+                            }
+                        }
+                    }
+                    ask_minuend(s32 < 2 ? i : i + 1, (s32 + 2) & 3, mn[s32 & 1]);
+                }
+            } else if (pre) {
                 float4 *dst = reinterpret_cast<float4 *>(C + (long)row * g.ldc + n0 + cb);
 #pragma unroll
                 for (int s16 = 0; s16 < 8; ++s16) {
@@ -587,6 +677,7 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             mbar_arrive(&bars.acc_empty[set]);
         }
+        if (EPI == EPI_STORE && lane == 0) bulk_wait_all();
         if (!ok) atomicOr(&bars.failed, 1u);
         if (g.flag && __any_sync(0xffffffffu, any) && lane == 0) atomicOr(g.flag, 1u);
     }
@@ -623,22 +714,22 @@ bool tma_enabled() {
     return on;
 }
 
-size_t tma_smem_bytes(int n_tile, int nraw, int nr, int nb, bool f16 = false) {
-    return 1024 + (size_t)nraw * (f16 ? 2 : 1) * RAW_SLOT + (size_t)nr * A_SLOT + (size_t)nb * 2 * image_half_units(n_tile) * 16 + sizeof(TmaBars) + 64;
+size_t tma_smem_bytes(int n_tile, int nraw, int nr, int nb, bool f16 = false, bool boxed_c = false) {
+    return 1024 + (boxed_c ? 8 * C_BOX : 0) + (size_t)nraw * (f16 ? 2 : 1) * RAW_SLOT + (size_t)nr * A_SLOT + (size_t)nb * 2 * image_half_units(n_tile) * 16 + sizeof(TmaBars) + 64;
 }
 
-template <bool AK, int NMAX, bool F16 = false>
-cudaError_t launch_tma(const CUtensorMap &map, const GemmArgs &g, dim3 grid, size_t smem, unsigned *status, cudaStream_t stream) {
-    cudaError_t err = cudaFuncSetAttribute(gemm_tc_tma_kernel<AK, NMAX, F16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <bool AK, int NMAX, bool F16 = false, int EPI = EPI_LANES>
+cudaError_t launch_tma(const CUtensorMap &map, const CUtensorMap &map_c, const GemmArgs &g, dim3 grid, size_t smem, unsigned *status, cudaStream_t stream) {
+    cudaError_t err = cudaFuncSetAttribute(gemm_tc_tma_kernel<AK, NMAX, F16, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (err != cudaSuccess) return err;
-    return launch_chained(gemm_tc_tma_kernel<AK, NMAX, F16>, grid, NTH, smem, stream, map, g, status);
+    return launch_chained(gemm_tc_tma_kernel<AK, NMAX, F16, EPI>, grid, NTH, smem, stream, map, map_c, g, status);
 }
 
 }  // namespace
 
 // Ring lengths.  A contiguous along K: as many slots of A (split in place) as fit beside three images of B (four up to
 // 128 columns).  A contiguous along M: two operand stages, and as many raw slots as fit for the copies' head start.
-void gemm_tc_tma_rings(int n_tile, bool a_kmajor, int *nraw, int *nr, int *nb, bool f16) {
+void gemm_tc_tma_rings(int n_tile, bool a_kmajor, int *nraw, int *nr, int *nb, bool f16, bool boxed_c) {
     *nb = n_tile > 128 ? 3 : 4;
     if (f16) {                                             // raw boxes of 64 k (32 KB), operand stages, images of B
         *nr = 2;
@@ -649,7 +740,7 @@ void gemm_tc_tma_rings(int n_tile, bool a_kmajor, int *nraw, int *nr, int *nb, b
     }
     if (a_kmajor) {
         int r = MAXR;
-        while (r > 2 && tma_smem_bytes(n_tile, 0, r, *nb) > (size_t)227 * 1024) --r;
+        while (r > 2 && tma_smem_bytes(n_tile, 0, r, *nb, false, boxed_c) > (size_t)227 * 1024) --r;
         *nr = r;
         *nraw = 0;
     } else {
@@ -685,15 +776,26 @@ cudaError_t gemm_tc_tma_launch(const GemmArgs &g, bool a_kmajor, unsigned *statu
                        l2 == 256 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : (l2 == 0 ? CU_TENSOR_MAP_L2_PROMOTION_NONE : CU_TENSOR_MAP_L2_PROMOTION_L2_128B),
                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
-    const size_t smem = tma_smem_bytes(g.n_tile, ((a_kmajor && !g.f16) || a_img) ? 0 : g.raw_stages, g.a_stages, g.b_stages, g.f16);
+    CUtensorMap map_c = map;                                     // (not looked at without boxed_c)
+    if (g.boxed_c) {
+        const cuuint64_t dims_c[2] = {(cuuint64_t)g.N, (cuuint64_t)g.M}, strides_c[1] = {(cuuint64_t)g.ldc * sizeof(float)};
+        const cuuint32_t box_c[2] = {32u, 32u};
+        if (encode_tiled()(&map_c, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, g.C, dims_c, strides_c, box_c, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return cudaErrorInvalidValue;
+    }
+    const size_t smem = tma_smem_bytes(g.n_tile, ((a_kmajor && !g.f16) || a_img) ? 0 : g.raw_stages, g.a_stages, g.b_stages, g.f16, g.boxed_c);
     dim3 grid((g.M + TM - 1) / TM, (g.N + g.n_tile - 1) / g.n_tile, g.splits);
     if (g.persistent) {
         const int tiles = (int)(grid.x * grid.y);
         grid = dim3((unsigned)(tiles < g.sm_count ? tiles : g.sm_count), 1, 1);
     }
-    if (g.f16) return a_kmajor ? launch_tma<true, 256, true>(map, g, grid, smem, status, stream) : launch_tma<false, 256, true>(map, g, grid, smem, status, stream);
-    if (a_kmajor) return g.n_tile <= 128 ? launch_tma<true, 128>(map, g, grid, smem, status, stream) : launch_tma<true, 256>(map, g, grid, smem, status, stream);
-    return g.n_tile <= 128 ? launch_tma<false, 128>(map, g, grid, smem, status, stream) : launch_tma<false, 256>(map, g, grid, smem, status, stream);
+    if (g.boxed_c)                                               // (wide tiles: A contiguous along K)
+        return g.minuend ? launch_tma<true, 256, true, EPI_MINUEND>(map, map_c, g, grid, smem, status, stream)
+                         : launch_tma<true, 256, true, EPI_STORE>(map, map_c, g, grid, smem, status, stream);
+    if (g.f16) return a_kmajor ? launch_tma<true, 256, true>(map, map_c, g, grid, smem, status, stream) : launch_tma<false, 256, true>(map, map_c, g, grid, smem, status, stream);
+    if (a_kmajor) return g.n_tile <= 128 ? launch_tma<true, 128>(map, map_c, g, grid, smem, status, stream) : launch_tma<true, 256>(map, map_c, g, grid, smem, status, stream);
+    return g.n_tile <= 128 ? launch_tma<false, 128>(map, map_c, g, grid, smem, status, stream) : launch_tma<false, 256>(map, map_c, g, grid, smem, status, stream);
 }
 
 }  // namespace bsq
