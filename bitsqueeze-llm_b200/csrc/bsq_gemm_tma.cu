@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
             if (EPI == EPI_STORE) {
                 // 32 columns at a time into this warp's box in shared memory (16-byte pieces swizzled: no bank conflicts), which leaves by one
                 // TMA store: whole 128-byte lines, and the warp goes on.  Stores of 32 bytes per lane and row took 7 to 8.5 us per tile
-                // whatever its K, which was what bounded the reconstructions (4096 x 14336 at rank 256 97.4 -> 82.2 us, 8192 x 4096 60 -> 46.6;
+                // whatever its K, which was what bounded the reconstructions (4096 x 14336 at rank 256 97.4 -> 78.3 us, 8192 x 4096 60 -> 46.6;
                 // one box of 128 rows for four warps, which then met at barriers: 88.4).
                 unsigned char *box = c_boxes + (warp - 3) * C_BOX;
                 for (int s32 = 0; s32 < 4 && cb + 32 * s32 < N; ++s32) {
@@ -729,8 +729,10 @@ cudaError_t launch_tma(const CUtensorMap &map, const CUtensorMap &map_c, const G
 
 // Ring lengths.  A contiguous along K: as many slots of A (split in place) as fit beside three images of B (four up to
 // 128 columns).  A contiguous along M: two operand stages, and as many raw slots as fit for the copies' head start.
+// With boxes for C two slots of A (64 of K each) and four images of B (32 of K each) fit: three and three left B only 96 of K
+// ahead and took 78.3 us for 4096 x 14336 at rank 256, this 71.6.
 void gemm_tc_tma_rings(int n_tile, bool a_kmajor, int *nraw, int *nr, int *nb, bool f16, bool boxed_c) {
-    *nb = n_tile > 128 ? 3 : 4;
+    *nb = n_tile > 128 && !boxed_c ? 3 : 4;
     if (f16) {                                             // raw boxes of 64 k (32 KB), operand stages, images of B
         *nr = 2;
         int r = 4;
