@@ -1473,7 +1473,10 @@ int bsq_lane_order_after(bsq_lane *lane, int decompress_side, void *stream) {
     if (elsewhere && cudaSetDevice(lane->device) != cudaSuccess) return 1;
     Runtime &rt = decompress_side ? lane->decompress : lane->compress;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
-    cudaError_t err = cudaStreamQuery(st);
+    // (a stream that is being captured must not be asked for its state)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t err = cudaStreamIsCapturing(st, &capture);
+    err = err == cudaSuccess && capture == cudaStreamCaptureStatusNone ? cudaStreamQuery(st) : cudaErrorNotReady;
     if (err == cudaErrorNotReady) {
         cudaGetLastError();                                  // (an answer, but noted as an error)
         err = rt.order ? cudaSuccess : cudaEventCreateWithFlags(&rt.order, cudaEventDisableTiming);
