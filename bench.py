@@ -47,10 +47,10 @@ import __graft_entry__ as entry  # noqa: E402
 METRIC = "FP32-input GB/s, compress+decompress of 32 x (4096x14336) FP32 matrices, full pipeline"
 WORKLOAD = ("configs[4]: 32 independent 4096x14336 FP32 matrices, outlier_topk=0.005, SVD rank 256 (2 power iterations), "
             "U/V NF4, S FP32, error_correction_topk=0.01, compress+decompress, matrix i on rank i % N")
-# kernels this library launches per matrix in this configuration, counted from an ncu launch list of
-# `python bench.py --single C5A` (all launches of the run, minus the decompress calls', divided by the compress calls)
-LAUNCHES_PER_COMPRESS = 67
-LAUNCHES_PER_DECOMPRESS = 9
+# kernels this library launches per matrix in this configuration, counted from a CUPTI trace (torch.profiler) of the batch calls on
+# device-resident objects, eight matrices in flight
+LAUNCHES_PER_COMPRESS = 56
+LAUNCHES_PER_DECOMPRESS = 4
 # DRAM bytes of one 4096x14336x256 product launch of gemm_tc_tma_kernel (ncu, read + write): 239.8-242.7 MB for W X (matrix
 # read along M), 250.0-251.9 MB for W^T X (read along K); the matrix itself is 234.9 MB, so it is read once.
 PRODUCT_DRAM_BYTES_PER_LAUNCH = 245.7e6
