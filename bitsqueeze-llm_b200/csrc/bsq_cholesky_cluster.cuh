@@ -292,6 +292,7 @@ __global__ void __launch_bounds__(kCholThreads, 1) cholesky_cluster_kernel(const
             __syncthreads();                               // the sums of the next column are whole, tij may be overwritten
         }
     }
+    __syncthreads();                                       // every warp's waits are behind it (without T nothing else is between the roles and here)
     if (tid == 0 && bars->failed) {
         // a wait ran out: what may still be on its way into this CTA's shared memory has to land before it goes away
         bars->failed = 0;

@@ -110,3 +110,18 @@ def test_ring_waits_for_stores_in_flight_before_it_leaves():
     leave = body[body.index("float *sv = "):]
     drain, last = leave.find("if (failed)"), leave.rfind("cluster.sync()")
     assert 0 <= drain < last and leave[drain: last].count("mbar_wait_bounded(") == 2
+
+
+def test_cholesky_cluster_drains_behind_every_wait_that_may_run_out():
+    """The thread that looks whether a wait ran out belongs to one warp, the waits to others: without a barrier of the CTA in front it may
+    look too early, and a copy that is still under way lands in shared memory that the CTA has given back."""
+    body = KERNELS["cholesky_cluster_kernel"][1]
+    roles = block(body, body.index("if (warp == 0)"))
+    at = body.index("    } else {", body.index(roles))        # the last role
+    drain, last = body.index("&& bars->failed)"), body.rindex("cluster.sync()")
+    assert at < drain < last
+    between = body[body.index("    if (T) {", at): drain]
+    inverse = block(between, 0)
+    behind = between[between.index(inverse) + len(inverse):]
+    assert "__syncthreads();" in behind
+    assert block(body, drain).count("cc_wait(") == 4
