@@ -1473,10 +1473,14 @@ int bsq_lane_order_after(bsq_lane *lane, int decompress_side, void *stream) {
     if (elsewhere && cudaSetDevice(lane->device) != cudaSuccess) return 1;
     Runtime &rt = decompress_side ? lane->decompress : lane->compress;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
-    // (a stream that is being captured must not be asked for its state)
+    // A stream that is being captured must not be asked for its state, and a blocking stream answers for its own work only, where an event
+    // also comes behind what is on the legacy default stream; that stream's answer does cover the blocking ones.
+    unsigned flags = cudaStreamDefault;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     cudaError_t err = cudaStreamIsCapturing(st, &capture);
-    err = err == cudaSuccess && capture == cudaStreamCaptureStatusNone ? cudaStreamQuery(st) : cudaErrorNotReady;
+    bool ask = err == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+    if (ask && st != nullptr && st != cudaStreamLegacy) ask = cudaStreamGetFlags(st, &flags) == cudaSuccess && (flags & cudaStreamNonBlocking) != 0;
+    err = ask ? cudaStreamQuery(st) : cudaErrorNotReady;
     if (err == cudaErrorNotReady) {
         cudaGetLastError();                                  // (an answer, but noted as an error)
         err = rt.order ? cudaSuccess : cudaEventCreateWithFlags(&rt.order, cudaEventDisableTiming);

@@ -217,7 +217,8 @@ uint64_t bsq_lane_packed_capacity(bsq_lane_t *lane);
 /* the lane's cudaStream_t (compress side or decompress side), e.g. to make other work wait for it with an event */
 void *bsq_lane_stream(bsq_lane_t *lane, int decompress_side);
 /* What is begun next on that side of the lane comes behind the work that is on `stream` (a cudaStream_t of the lane's device; null: the legacy
- * default stream) now.  Where `stream` has nothing left to do there is nothing to wait for. */
+ * default stream) now, as an event recorded there would: legacy default and blocking streams wait for one another.  Where `stream` has nothing
+ * left to do there is nothing to wait for. */
 int bsq_lane_order_after(bsq_lane_t *lane, int decompress_side, void *stream);
 /* matrix: host (input_location 0; pinned memory makes the copy asynchronous) or device (1) */
 int bsq_lane_compress_begin(bsq_lane_t *lane, const float *matrix, int input_location, void *d_packed, uint64_t capacity);
