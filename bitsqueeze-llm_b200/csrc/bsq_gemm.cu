@@ -327,14 +327,10 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
         // (measured: the products are then bound by what the CTAs draw from L2, A once and B's images once per row
         // tile; that pays for tiles wider than 128 columns, where splitting B in every CTA is two thirds of the
         // staging work, and for long K)
-        // (up to 128 columns and with TF32 halves the register-staged kernel with two CTAs per SM measured faster than either image
-        // kernel: 67 against 80-88 us for 8192 x 128 x 4096; FP16 halves, TMA-fed: 45)
-        // A caller that gives a bound on |A| gets FP16 halves at any width: whole compress calls of FP32 factors, TF32 / FP16 halves, the pass for
-        // the bound included: 8192 x 4096 at rank 16 635 / 566 us, 64 808 / 715, 128 1176 / 1062, 240 1941 / 1777; 2048 x 2048 at 16
-        // 284 / 275, 128 806 / 799; 512 x 1024 at 16 268 / 257.  Error over the result's norm, 8192 x 128 x 4096: 2.43e-6 / 1.25e-6.
-        const bool halves16 = a_absmax_bits && f16_mode() >= 1 && !kscale && !minuend && N <= 256;
+        // (up to 128 columns the register-staged kernel with two CTAs per SM measured faster than either image kernel:
+        // 67 against 80-88 us for 8192 x 128 x 4096)
         bool with_image = workspace && image_bytes + 128 <= workspace_bytes &&
-                          (b_image_mode() == 2 ? M >= 256 : (b_image_mode() == 1 && M >= 512 && (t.n_tile > 128 || halves16) && K >= 1024));
+                          (b_image_mode() == 2 ? M >= 256 : (b_image_mode() == 1 && M >= 512 && t.n_tile > 128 && K >= 1024));
         // a wide product (the reconstruction: N = a matrix dimension, K = the rank) in 256-column tiles, B's images
         // made once and shared by all row tiles, when the workspace has room for them; otherwise every CTA of a
         // 128-column tile splits its piece of B itself
@@ -398,10 +394,12 @@ cudaError_t gemm_select(bool allow_tensor_cores, bool a_kmajor, bool b_kmajor, c
             }
         }
         const int slots = (t.use_tma ? 1 : with_image ? gemm_tc_image_ctas_per_sm(t.n_tile) : (t.n_tile <= 128 ? 2 : 1)) * sm_count;
-        // the FP16 form of the split (BSQ_GEMM_F16=1, products whose caller gives a bound on |A|; =2 also 256-column products without one:
-        // it is then worked out here, a pass over A)
-        if (t.use_tma && !t.persistent && !kscale && !minuend && workspace_bytes >= 4096 &&
-            (halves16 || (t.n_tile == 256 && (f16_mode() == 2 || (f16_mode() == 1 && a_absmax_bits))))) {
+        // the FP16 form of the split (BSQ_GEMM_F16=1; =2 also without a given bound on |A|: it is then worked out here, a pass over A):
+        // 256-column products on the TMA-fed kernel.  Narrower ones keep TF32 halves: 8192 x 128 x 4096 takes 67 us with them and 45 with FP16 halves, but one
+        // scale for the whole of A leaves rows far below its largest element fewer bits (error over the row's own norm 4e-5 at 2^-24, 2e-2 at 2^-32;
+        // 7e-7 with TF32 halves), and U and V of such rows with them.
+        if (t.use_tma && !t.persistent && t.n_tile == 256 && !kscale && !minuend && workspace_bytes >= 4096 &&
+            (f16_mode() == 2 || (f16_mode() == 1 && a_absmax_bits))) {
             unsigned *words = reinterpret_cast<unsigned *>(workspace);      // [0]: |B| max, [1]: |A| max when not given
             workspace += 64;
             workspace_bytes -= 256;

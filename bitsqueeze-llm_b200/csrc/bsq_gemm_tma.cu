@@ -165,11 +165,7 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
     const bool one_acc = EPI != EPI_LANES || (a_img && g.wide_tiles);                    // the cross terms go into the hi * hi accumulator
     const unsigned acc_stride = one_acc ? acc_cols : 2u * acc_cols;  // tensor-memory columns of one set
     const int acc_sets = (g.persistent && acc_stride <= 256u) ? 2 : 1;
-    // Tensor memory has room for a second hi * hi accumulator beside those of a narrow tile: slots of A go to one and the other in turn.
-    // The tensor core truncates when it accumulates, which is most of what these products are off by, and chains half as long halve it
-    // (8192 x 128 x 4096, K in two parts, error over the result's norm 2.46e-6 with one).
-    const bool two_acc = F16 && !g.persistent && g.n_tile <= 128;
-    const unsigned tmem_cols = two_acc ? 4u * acc_cols : acc_stride * (unsigned)acc_sets;
+    const unsigned tmem_cols = acc_stride * (unsigned)acc_sets;
     const int epi_groups = one_acc ? 2 : 1;                        // wide tiles: the transform warps take the tile's second 128 columns
     const TileWalk walk(g);
     const int chunks_total = (g.K + TK - 1) / TK;
@@ -313,8 +309,6 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const unsigned a_addr = smem_u32(a_slots + (size_t)s * A_SLOT);
                     const uint64_t da_hi = smem_desc_sw128(a_addr), da_lo = smem_desc_sw128(a_addr + A_HALF);
-                    const unsigned acc_h = two_acc && (c & 1) ? acc + 2u * acc_cols : acc;
-                    const bool begun = two_acc ? c > 1 : c > 0;                  // this accumulator holds something
                     for (int h = 0; h < 2 && ok; ++h) {
                         if (2 * c + h >= chunks_b) break;                // K ends inside this slot: its second half is zeros
                         const int sb = rb.pos;
@@ -328,7 +322,7 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
                             const uint64_t dah = da_hi + (uint64_t)(kk * 2), dal = da_lo + (uint64_t)(kk * 2);
                             const uint64_t dbh = db0 + (uint64_t)(ks * b_kstep), dbl = dbh + b_units;
                             if (F16) {
-                                mma_f16(acc_h, dah, dbh, idesc, begun || kk > 0);
+                                mma_f16(acc, dah, dbh, idesc, c > 0 || kk > 0);
                                 mma_f16(acc_x, dal, dbh, idesc, one_acc || c > 0 || kk > 0);
                                 mma_f16(acc_x, dah, dbl, idesc, true);
                             } else {
@@ -499,7 +493,6 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
             const int n0 = nt * g.n_tile, N = min(g.n_tile, g.N - n0);
             const int row = mt * TM + quarter * 32 + lane;
             const int set = rs.pos;
-            const bool both_acc = two_acc && min(g.K, (z + 1) * g.k_per_split) - z * g.k_per_split > KS;
             float *C = g.C + (long)z * g.split_stride;
             // A full 128-column tile with a minuend: the thread's whole row segment of the minuend is asked for before
             // the wait for the accumulators, so that its HBM latency passes while the tensor core still works on the
@@ -627,15 +620,7 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
                 const unsigned taddr = tmem_d + (unsigned)set * acc_stride + ((unsigned)(quarter * 32) << 16) + (unsigned)c0;
                 tmem_ld16(taddr, r);
                 if (!one_acc) tmem_ld16(taddr + acc_cols, q);
-                if (both_acc) {
-                    unsigned r2[16];
-                    tmem_ld16(taddr + 2u * acc_cols, r2);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(r[j]), __uint_as_float(r2[j])));
-                } else {
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                }
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (F16 && one_acc) {                                // one accumulator (low halves without their factor): the scales taken out
 #pragma unroll
                     for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__fmul_rn(__uint_as_float(r[j]), inv16));
@@ -795,7 +780,7 @@ cudaError_t gemm_tc_tma_launch(const GemmArgs &g, bool a_kmajor, unsigned *statu
     if (g.boxed_c)                                               // (wide tiles: A contiguous along K)
         return g.minuend ? launch_tma<true, 256, true, EPI_MINUEND>(map, map_c, g, grid, smem, status, stream)
                          : launch_tma<true, 256, true, EPI_STORE>(map, map_c, g, grid, smem, status, stream);
-    if (g.f16) return a_kmajor ? launch_tma<true, 256, true>(map, map_c, g, grid, smem, status, stream) : launch_tma<false, 256, true>(map, map_c, g, grid, smem, status, stream);
+    if (g.f16 && g.n_tile > 128) return a_kmajor ? launch_tma<true, 256, true>(map, map_c, g, grid, smem, status, stream) : launch_tma<false, 256, true>(map, map_c, g, grid, smem, status, stream);
     if (a_kmajor) return g.n_tile <= 128 ? launch_tma<true, 128>(map, map_c, g, grid, smem, status, stream) : launch_tma<true, 256>(map, map_c, g, grid, smem, status, stream);
     return g.n_tile <= 128 ? launch_tma<false, 128>(map, map_c, g, grid, smem, status, stream) : launch_tma<false, 256>(map, map_c, g, grid, smem, status, stream);
 }

@@ -73,7 +73,6 @@ struct SvdWorkspace {
     unsigned *a_absmax = nullptr;       // bits of the largest |A| of the current call (scale of the FP16 split of the big products)
     bool a_absmax_valid = false;
     const unsigned *a_absmax_use = nullptr;
-    bool halves16 = false;              // the products with A split their operands into FP16 halves
     RingLaunch ring = {};               // the core's kernel for coded factors above kRingMinK columns
     bool jc_with_v = false;             // ... and whether it accumulates the right factor (else that comes from the panel)
     bool device_full = false;           // other work fills the device beside this (chooses tile widths, not results)
@@ -515,8 +514,6 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
     ws->allreduce_ctx = allreduce_ctx;
     ws->k = std::max(1, std::min(k, std::min(allreduce ? m_total : m, n)));
     ws->transposed = allreduce ? false : m < n;
-    // Below 256 columns the halves change last bits that codes and error lists would show, so only FP32 factors take them.
-    ws->halves16 = ws->k >= 256 || (!coded_factors && ws->k % 16 == 0);
     ws->M = ws->transposed ? n : m;
     ws->N = ws->transposed ? m : n;
     const size_t kk = (size_t)ws->k * ws->k;
@@ -702,12 +699,12 @@ cudaError_t svd_lowrank(SvdWorkspace *ws, const float *d_A, float *d_U, float *d
 
     cudaError_t err;
     float *q = nullptr, *qz = nullptr, *spare = nullptr;
-    // the largest |A|, once per call: the six products with A split it into FP16 halves scaled by a power of two from it
-    // (or a bound that the caller already has)
+    // the largest |A|, once per call: from 256 columns on the six products with A split it into FP16 halves scaled by a power of two
+    // from it (or a bound that the caller already has)
     ws->a_absmax_use = d_abs_bound ? d_abs_bound : ws->a_absmax;
-    ws->a_absmax_valid = ws->halves16 && (d_abs_bound != nullptr ||
-                                     (ws->n % 4 == 0 && reinterpret_cast<uintptr_t>(d_A) % 16 == 0 &&
-                                      gemm_absmax_bits(d_A, ws->n, ws->m, ws->n, ws->a_absmax, st) == cudaSuccess));
+    ws->a_absmax_valid = k >= 256 && (d_abs_bound != nullptr ||
+                                      (ws->n % 4 == 0 && reinterpret_cast<uintptr_t>(d_A) % 16 == 0 &&
+                                       gemm_absmax_bits(d_A, ws->n, ws->m, ws->n, ws->a_absmax, st) == cudaSuccess));
     // Y = W Omega, Q = orth(Y).  Panels ping-pong between the two buffers of their size.
     if ((err = times_w(ws, d_A, false, ws->omega, true, ws->y, st)) != cudaSuccess) return err;
     const int last_passes = 2;
