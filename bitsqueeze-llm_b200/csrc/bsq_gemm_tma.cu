@@ -596,11 +596,10 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const float4 m4 = mn_pre[s16 * 4 + j];
-                        float p0 = __fadd_rn(__uint_as_float(r[4 * j]), __uint_as_float(q[4 * j]));
-                        float p1 = __fadd_rn(__uint_as_float(r[4 * j + 1]), __uint_as_float(q[4 * j + 1]));
-                        float p2 = __fadd_rn(__uint_as_float(r[4 * j + 2]), __uint_as_float(q[4 * j + 2]));
-                        float p3 = __fadd_rn(__uint_as_float(r[4 * j + 3]), __uint_as_float(q[4 * j + 3]));
-                        if (F16) { p0 = __fmul_rn(p0, inv16); p1 = __fmul_rn(p1, inv16); p2 = __fmul_rn(p2, inv16); p3 = __fmul_rn(p3, inv16); }
+                        const float p0 = __fadd_rn(__uint_as_float(r[4 * j]), __uint_as_float(q[4 * j]));
+                        const float p1 = __fadd_rn(__uint_as_float(r[4 * j + 1]), __uint_as_float(q[4 * j + 1]));
+                        const float p2 = __fadd_rn(__uint_as_float(r[4 * j + 2]), __uint_as_float(q[4 * j + 2]));
+                        const float p3 = __fadd_rn(__uint_as_float(r[4 * j + 3]), __uint_as_float(q[4 * j + 3]));
                         const float4 o = make_float4(__fsub_rn(m4.x, p0), __fsub_rn(m4.y, p1), __fsub_rn(m4.z, p2), __fsub_rn(m4.w, p3));
                         any |= fabsf(o.x) > 1.1920928955078125e-07f || fabsf(o.y) > 1.1920928955078125e-07f ||
                                fabsf(o.z) > 1.1920928955078125e-07f || fabsf(o.w) > 1.1920928955078125e-07f;
@@ -621,10 +620,7 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
                 tmem_ld16(taddr, r);
                 if (!one_acc) tmem_ld16(taddr + acc_cols, q);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (F16 && one_acc) {                                // one accumulator (low halves without their factor): the scales taken out
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__fmul_rn(__uint_as_float(r[j]), inv16));
-                } else if (F16) {                                    // hi * hi + (cross terms) / 2^11, and the operands' scales taken out
+                if (F16) {                                           // hi * hi + (cross terms) / 2^11, and the operands' scales taken out
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
                         r[j] = __float_as_uint(__fmul_rn(__fmaf_rn(__uint_as_float(q[j]), 1.0f / kSplit16LoScale, __uint_as_float(r[j])), inv16));
