@@ -498,7 +498,8 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
             // the wait for the accumulators, so that its HBM latency passes while the tensor core still works on the
             // tile (fetched 16 columns at a time inside the loop below, every step would wait for memory on its own).
             const int ce = one_acc ? min(N, cb + 128) : N;                // this thread's columns of the tile: cb .. ce - 1
-            const bool pre = !F16 && g.minuend != nullptr && ce - cb == 128 && row < g.M;
+            // (A warp takes it as a whole or not at all: its loads from tensor memory are executed by all lanes together.)
+            const bool pre = !F16 && g.minuend != nullptr && ce - cb == 128 && row - lane + 32 <= g.M;
             float4 mn_pre[32];
             if (pre) {
                 const float *mn = g.minuend + (long)row * g.ldm + n0 + cb;
@@ -510,8 +511,7 @@ __global__ void __launch_bounds__(NTH, 1) gemm_tc_tma_kernel(const __grid_consta
                     for (int j = 0; j < 32; ++j) mn_pre[j] = reinterpret_cast<const float4 *>(mn)[j];
                 }
             }
-            ok = mbar_wait_bounded(&bars.acc_full[set], rs.par, status);
-            if (EPI != EPI_LANES) ok = __all_sync(0xffffffffu, ok);               // (its lanes go on together or not at all)
+            ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bars.acc_full[set], rs.par, status));      // (its lanes go on together or not at all)
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (EPI == EPI_STORE) {

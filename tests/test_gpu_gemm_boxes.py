@@ -36,3 +36,9 @@ def test_boxes_at_the_edges_of_tiles(pkg, lib, rows, cols, rank):
     product = y[:rows].clone()
     round_trip(1.0)
     assert bool(((y[:rows] - x).abs() <= 2.0 ** -23 * (x.abs() + product.abs())).all())
+
+
+@pytest.mark.parametrize("rows,cols,rank", [(515, 3856, 68), (1001, 2592, 100), (2050, 1328, 76)])
+def test_wide_tiles_of_tf32_halves_at_the_edges(pkg, lib, rows, cols, rank):
+    """Ranks that are not multiples of 8 keep TF32 halves and leave a row per lane; the last rows fill part of a warp."""
+    test_boxes_at_the_edges_of_tiles(pkg, lib, rows, cols, rank)

@@ -125,3 +125,11 @@ def test_cholesky_cluster_drains_behind_every_wait_that_may_run_out():
     behind = between[between.index(inverse) + len(inverse):]
     assert "__syncthreads();" in behind
     assert block(body, drain).count("cc_wait(") == 4
+
+
+def test_tensor_memory_is_read_by_whole_warps():
+    """tcgen05.ld is executed by all lanes of a warp together: what decides on the way to one is the same in all of them."""
+    text = dict(sources())["bsq_gemm_tma.cu"]
+    pre = re.search(r"const bool pre = ([^;]*);", text).group(1)
+    assert "row - lane + 32 <= g.M" in pre and not re.search(r"\brow <", pre)
+    assert "__all_sync(0xffffffffu, mbar_wait_bounded(&bars.acc_full[set]" in text
