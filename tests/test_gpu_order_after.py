@@ -2,11 +2,15 @@
 the legacy default stream and blocking streams wait for one another.  Producers are still running when the call is made."""
 import ctypes as C
 import importlib
+import subprocess
+import sys
 
 import pytest
 
 pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
+
+from conftest import ROOT  # noqa: E402
 
 ROWS, COLS = 256, 1024
 
@@ -74,3 +78,28 @@ def test_a_stream_that_is_being_captured_stays_so(comp, lib):
     assert torch.equal(b, 2 * a)
     x = torch.randn(ROWS, COLS, device="cuda")                # the lane goes on as before
     assert torch.equal(comp.compress(x).data[200:1200], comp.compress(x).data[200:1200])
+
+
+def test_waiting_for_other_work_is_left_to_the_device_flags():
+    """A process whose context asks for waits that sleep: a decompress call behind 0.3 s of other work does not keep a core busy until its kernel's answer
+    comes.  (The limit of a quarter: such a wait takes next to none of it, polling takes all.)"""
+    code = """
+import ctypes, time
+cuda = ctypes.CDLL("libcuda.so.1")
+assert cuda.cuInit(0) == 0 and cuda.cuDevicePrimaryCtxSetFlags_v2(0, 4) == 0         # CU_CTX_SCHED_BLOCKING_SYNC
+import importlib, torch, __graft_entry__
+pkg = __graft_entry__.load_package()
+comp = importlib.import_module(pkg.__name__ + ".torch_api").Compressor(256, 1024, outlier=0.01, q=pkg.NF4_DQ)
+x = torch.randn(256, 1024, device="cuda")
+packed = comp.compress(x)
+want = comp.decompress(packed)
+torch.cuda.synchronize()
+torch.cuda._sleep(600_000_000)
+wall, cpu = time.perf_counter(), time.thread_time()
+got = comp.decompress(packed)
+wall, cpu = time.perf_counter() - wall, time.thread_time() - cpu
+assert torch.equal(got, want) and wall > 0.1, wall
+assert cpu < 0.25 * wall, (cpu, wall)
+"""
+    done = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
