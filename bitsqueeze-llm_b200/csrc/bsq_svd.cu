@@ -596,7 +596,8 @@ SvdWorkspace *svd_workspace_create_sharded(int m, int n, int k, int niter, int s
             }
         }
     }
-    if (ok && ws->k > kCB && ws->k <= kCholeskyBlockedMaxK &&
+    const char *chol = getenv("BSQ_CHOL_CLUSTER");           // 0: as a device that cannot place the cluster (A/B comparisons)
+    if (ok && ws->k > kCB && ws->k <= kCholeskyBlockedMaxK && !(chol && chol[0] == '0') &&
         cudaFuncSetAttribute(cholesky_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cholesky_cluster_smem_bytes(kCholeskyBlockedMaxK)) ==
             cudaSuccess) {
         cudaLaunchConfig_t cfg;
