@@ -81,6 +81,16 @@ def test_rotations_of_fp32_factors_keep_lengths(lib, k, kind):
     assert np.linalg.norm(s - exact) <= 2e-6 * np.linalg.norm(exact)
 
 
+@pytest.mark.parametrize("k", [7, 9, 23, 24, 25, 34, 47, 49, 71, 72, 73])
+def test_shapes_of_blocks_follow_the_rank(lib, k):
+    """Full blocks of 8 and 12 columns, and the ranks on either side of each line of block_jacobi_shape."""
+    for kind in ("noise", "small"):
+        test_core_edges(lib, k, kind)
+    test_core_of_deficient_and_zero_matrices(lib, k)
+    for kind in ("1/i", "flat"):
+        test_rotations_of_fp32_factors_keep_lengths(lib, k, kind)
+
+
 class CodedFactors:
     """The library with bsq_svd_lowrank standing for the kernels of coded factors."""
 
