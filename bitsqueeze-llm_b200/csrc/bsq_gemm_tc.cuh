@@ -88,10 +88,12 @@ __device__ __forceinline__ void split_store(float4 v, float4 *hi, float4 *lo) {
                       tf32_rna(__fsub_rn(v.w, h.w)));
 }
 
-// The FP16 form of the split: x * s = hi + lo' / 2^11 (+ e, |e| <= 2^-22 |x * s|) with hi = fp16(x * s) and
-// lo' = fp16((x * s - hi) * 2^11), s a power of two that brings the operand's largest magnitude into [2^14, 2^15):
-// hi carries 11 significant bits and lo' the next 11, like the two TF32 halves, and lo' has hi's magnitude, so both sit
-// in FP16's range (elements below 2^-28 of the largest lose bits, an absolute error below FP32's on the largest).
+// The FP16 form of the split: x * s = hi + lo' / 2^11 + e with hi = fp16(x * s) and lo' = fp16((x * s - hi) * 2^11), s a power of two that
+// brings the operand's largest magnitude into [2^14, 2^15): hi carries 11 significant bits and lo' the next 11, like the two TF32
+// halves, and lo' has hi's magnitude, so both sit in FP16's range.  |e| <= 2^-22 |x * s| down to |x * s| = 2^-14, 2^-28 of the largest; below that hi
+// is subnormal, the conversion rounds it a second time and lo' does not know of it: |e| up to 2^-25, far below what the largest element itself
+// is off by, but not small against a row that lies there as a whole (error of its products over its own norm, by the row's scale against
+// the operand's: 2^-20 7e-7, 2^-24 4e-5, 2^-28 1e-3, 2^-36 0.3).  Only products of 256 columns and more take it.
 // hi * hi goes into one accumulator, lo' * hi + hi * lo' into the other, which the epilogue scales by 2^-11.
 constexpr float kSplit16LoScale = 2048.0f;
 // The scale from the bits of the operand's largest |x|: 2^(14 - exponent), kept within 2^+-60 so that the product of
