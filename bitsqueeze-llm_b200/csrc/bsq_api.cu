@@ -1141,18 +1141,29 @@ bool expect_heads(Runtime &rt, const bitsqz_llm_array_t *c, HeadCheck *check, ui
     return (!(c->flags & kFlagError) || topk(c->section_error_topk, rt.err, k_err)) &&
            (!(c->flags & kFlagOutlier) || topk(c->section_outlier_topk, rt.outlier, k_out));
 }
-// Waits for what the kernel launched with `check` has found.  With nothing in front of it that takes as long as a launch, and polling the word
-// is the short way.  Behind other work (the caller's, other lanes') it takes as long as that does: then as any wait for the stream, in the
-// way that the device's flags ask for, and the answer is there when the stream is done.
+// Waits for what the kernel launched with `check` has found.  With nothing in front of it that takes as long as a launch; behind other work (the
+// caller's, other lanes') it takes as long as that does, and where the device's flags ask for waits that sleep or yield it is then one for
+// the stream: the answer is there when that is done.  (Otherwise such a wait polls too, and comes back later: batches of eight 4096 x 14336 against
+// polling alone 0.992x with waits for the stream in every process, 1.001x and 1.011x like this.)
 constexpr std::chrono::microseconds kAnswerPoll(100);
 bool heads_as_expected(Runtime &rt, const HeadCheck &check) {
     if (check.count == 0) return true;
     const volatile unsigned *answer = check.answer;
     const auto here = [&]() { return (*answer | 1u) == (check.number | 1u); };
     const auto start = std::chrono::steady_clock::now();
+    bool asked = false;
     for (unsigned i = 1; !here(); ++i) {
-        if (i % 256 != 0 || std::chrono::steady_clock::now() - start < kAnswerPoll) continue;
-        if (cudaStreamSynchronize(rt.stream) != cudaSuccess || !here()) return false;
+        if (i % 4096 != 0) continue;
+        cudaError_t state = cudaStreamQuery(rt.stream);
+        if (state == cudaErrorNotReady) {
+            cudaGetLastError();                              // (an answer, but noted as an error)
+            if (asked || std::chrono::steady_clock::now() - start < kAnswerPoll) continue;
+            asked = true;
+            unsigned flags = 0;
+            if (cudaGetDeviceFlags(&flags) != cudaSuccess || (flags & (cudaDeviceScheduleBlockingSync | cudaDeviceScheduleYield)) == 0) continue;
+            state = cudaStreamSynchronize(rt.stream);
+        }
+        if (state != cudaSuccess || !here()) return false;
     }
     return *answer == check.number;
 }
