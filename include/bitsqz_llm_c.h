@@ -155,7 +155,7 @@ int bsq_gemm(int a_kmajor, int b_kmajor, const float *d_A, long lda, const float
 /* The same product when the caller knows an upper bound of |A| (a device word holding the bits of a finite, non-negative
  * float): 256-column products on the TMA-fed kernel then split their operands into two FP16 halves, scaled by powers of
  * two taken from that bound and from the largest |B|, instead of two TF32 halves (same accuracy class, twice the
- * tensor rate); every other shape runs as in bsq_gemm.  A bound below the true maximum overflows FP16: the result
+ * tensor rate; rows more than 2^-20 below the bound keep fewer bits); every other shape runs as in bsq_gemm.  A bound below the true maximum overflows FP16: the result
  * holds Inf / NaN then. */
 int bsq_gemm_bounded(int a_kmajor, int b_kmajor, const float *d_A, long lda, const float *d_B, long ldb, float *d_C, long ldc, int M,
                      int N, int K, float *d_workspace, size_t workspace_bytes, const uint32_t *d_a_absmax_bits, uint32_t *d_status,
