@@ -1190,7 +1190,7 @@ ListSource list_source(const bitsqz_llm_array_t *c, const bitsqz_section_t &s, u
 }
 
 // A device-resident object, all of it within reach of kernels and apart from the result.  A quantised matrix: one kernel checks the
-// headers, decodes, adds the lists and reports.  Factors: one opens them beside the check, two make the product, and once the headers
+// headers, decodes, adds the lists and reports; long lists (decode_lists_apart) are added behind it as those of factors are.  Factors: one opens them beside the check, two make the product, and once the headers
 // are known to be good one adds the lists and reports.
 int decompress_begin_in_place(Runtime &rt, const bitsqz_llm_array_t *c, float *d_dst) {
     cudaStream_t st = rt.stream;
@@ -1208,9 +1208,11 @@ int decompress_begin_in_place(Runtime &rt, const bitsqz_llm_array_t *c, float *d
     rt.inject_status = 0;
     // (both ways: error list first, outliers second, src/bitsqz_llm.cu:1372-1387)
     if (!(c->flags & kFlagSvd)) {
-        if (decode_matrix(section_source(c, c->section_direct, c->quantization_only_format, c->num_elements), c->num_rows, c->num_columns, err, out,
-                          d_dst, rt.h_status, check, rt.sm_count, st) != cudaSuccess ||
-            !heads_as_expected(rt, check))
+        const bool apart = decode_lists_apart(c->num_rows, c->num_columns, k_err, k_out, rt.sm_count);
+        if (decode_matrix(section_source(c, c->section_direct, c->quantization_only_format, c->num_elements), c->num_rows, c->num_columns,
+                          apart ? ListSource{} : err, apart ? ListSource{} : out, d_dst, rt.h_status, check, rt.sm_count, st) != cudaSuccess ||
+            !heads_as_expected(rt, check) ||
+            (apart && apply_lists_end(err, out, c->num_rows, c->num_columns, d_dst, nullptr, rt.h_status, st) != cudaSuccess))
             return fail();
         rt.decompress_active = true;
         return 0;

@@ -78,6 +78,8 @@ struct ListSource {
 // kStatusBadIndex where a list names a column that the matrix does not have.
 cudaError_t decode_matrix(const SectionSource &q, uint32_t rows, uint32_t cols, const ListSource &first, const ListSource &second, float *d_out,
                           unsigned *mirror, const HeadCheck &heads, int sm_count, cudaStream_t stream);
+// Whether lists of k0 and k1 entries a row are better added behind that pass (apply_lists_end).
+bool decode_lists_apart(uint32_t rows, uint32_t cols, uint32_t k0, uint32_t k1, int sm_count);
 // Dequantise a rows x cols matrix and add a row-wise top-k list in one pass; d_scales (NF4) or d_dq + d_scale_codes (NF4_DQ).
 cudaError_t nf4_dequantize_add_topk(const float *d_scales, const float *d_dq, const uint8_t *d_scale_codes, const uint8_t *d_data,
                                     uint32_t rows, uint32_t cols, const uint16_t *d_idx, const float *d_val, uint32_t k,
@@ -111,7 +113,8 @@ cudaError_t topk_apply(const uint16_t *d_idx, const float *d_val, uint32_t rows,
 cudaError_t topk_apply_two(const uint16_t *d_idx0, const float *d_val0, uint32_t k0, const uint16_t *d_idx1, const float *d_val1,
                            uint32_t k1, uint32_t rows, uint32_t cols, float *d_dense, unsigned *d_status, cudaStream_t stream);
 // The same with the lists where they lie in an object, either or both possibly empty, as the end of a decompress call: status words of the
-// call's earlier kernels, and columns out of range, are reported in the page-locked, zero `mirror`; the words are cleared.
+// call's earlier kernels (d_status, null where they report to the mirror themselves), and columns out of range, are reported in the page-locked, zero
+// `mirror`; the words are cleared.
 cudaError_t apply_lists_end(const ListSource &a, const ListSource &b, uint32_t rows, uint32_t cols, float *d_dense, unsigned *d_status,
                             unsigned *mirror, cudaStream_t stream);
 

@@ -15,6 +15,7 @@
 #include "bsq_device.cuh"
 #include "bsq_internal.hpp"
 
+#include <algorithm>
 #include <mutex>
 
 namespace bsq {
@@ -686,6 +687,19 @@ cudaError_t nf4_dequantize_add_topk(const float *d_scales, const float *d_dq, co
     if ((d_scales != nullptr) == (d_dq != nullptr && d_scale_codes != nullptr)) return cudaErrorInvalidValue;
     const SectionSource q{d_scales ? bytes(d_scales) : d_scale_codes, d_scales ? nullptr : bytes(d_dq), d_data, (uint64_t)rows * cols};
     return launch_decode(q, TopkLists{{{bytes(d_idx), bytes(d_val), k}, {}}, cols, d_status, false}, d_out, HeadCheck{}, sm_count, stream);
+}
+
+// In the pass a warp looks through the whole lists of a row for each batch that it decodes there, 32 entries a trip of 0.25 to 0.4 us; behind it the
+// lists cost a launch and a wait, of which 6 us show, and about 8 us for a million entries, each read once.  us a call, in the pass / behind
+// it: 8 x 9216 with 68 + 14 entries a row 22.6 / 29.7, 384 x 1792 with 46 + 270 27.6 / 33.1, 4928 x 768 with one list of 489 31.0 / 47.8, 1856 x 4608 with
+// one of 1781 71 / 95; on the other side 64 x 3136 with 343 + 1040 41.7 / 28.7, 158 x 14175 with one of 1113 51.0 / 27.8, 2897 x 5492 with one of 446 73 / 46,
+// 69 x 11924 with 4664 + 3463 143 / 37, 3673 x 5182 with 1900 + 2380 468 / 254.  Of 400 shapes the choice costs 1.3 % in the mean.
+bool decode_lists_apart(uint32_t rows, uint32_t cols, uint32_t k0, uint32_t k1, int sm_count) {
+    const uint64_t batches = ((uint64_t)rows * cols + kBatch - 1) / kBatch, warps = (uint64_t)sm_count * kDecodeCtas * (kThreads / 32);
+    const double per_warp = batches > warps ? (double)batches / warps : 1.0;
+    const double rows_of_batch = cols < kBatch ? std::min<uint32_t>(rows, (kBatch - 1) / cols + 2) : 1.0 + (double)(kBatch - 1) / cols;
+    const double trips = ((k0 + 31) / 32 + (k1 + 31) / 32) * rows_of_batch * per_warp;
+    return 0.25 * trips > 6.0 + 8.0e-6 * rows * ((double)k0 + k1);
 }
 
 cudaError_t decode_matrix(const SectionSource &q, uint32_t rows, uint32_t cols, const ListSource &first, const ListSource &second, float *d_out,

@@ -1,6 +1,7 @@
 """A device-resident quantised matrix is checked, decoded and completed with its lists by one kernel (csrc/bsq_quant.cu): the bits of the
 host object's route, at sizes around the kernel's batches of 1024 elements, with lists shorter and longer than what a batch brings with it."""
 import ctypes as C
+import importlib
 
 import pytest
 
@@ -13,6 +14,8 @@ CASES = [
     (1, 1023, 0.01, 0.0), (1, 1025, 0.01, 0.02), (3, 341, 0.3, 0.3), (33, 31, 0.0, 0.1), (64, 64, 1.0, 1.0), (5, 2049, 0.04, 0.001),
     (16, 6400, 0.01, 0.0102), (7, 14335, 0.005, 0.01), (300, 14336, 0.0, 0.02), (1501, 3001, 0.005, 0.01),
 ]
+# lists that a kernel of their own adds: one and two of them, in one launch and in two, ragged, all of a row
+LONG_CASES = [(8, 11200, 0.036, 0.253), (64, 3136, 0.11, 0.33), (11, 5879, 0.0, 0.2), (33, 2047, 1.0, 0.0), (512, 1601, 0.4, 0.6), (5, 14335, 0.5, 1.0)]
 
 
 @pytest.mark.parametrize("q", [10, 11])
@@ -50,12 +53,45 @@ def test_one_launch_gives_the_host_objects_bits(pkg, lib, case, q):
         lib.bsq_lane_destroy(lane)
 
 
+@pytest.mark.parametrize("q", [10, 11])
+@pytest.mark.parametrize("case", LONG_CASES)
+def test_long_lists_behind_the_decode_give_the_host_objects_bits(pkg, lib, case, q):
+    test_one_launch_gives_the_host_objects_bits(pkg, lib, case, q)
+
+
+@pytest.mark.parametrize("case,apart", [(c, True) for c in LONG_CASES] + [((8, 9216, 0.0074, 0.0015), False), ((256, 1024, 0.01, 0.0), False),
+                                                                          ((1024, 4096, 0.01, 0.01), False)])
+def test_long_lists_take_a_kernel_of_their_own(pkg, lib, case, apart):
+    """A warp that looks through thousands of entries for each of its batches takes up to four times as long as the lists added behind the decode."""
+    rows, cols, outlier, error = case
+    x = torch.randn(rows, cols, device="cuda")
+    comp = importlib.import_module(pkg.__name__ + ".torch_api").Compressor(rows, cols, outlier=outlier, error=error, q=10)
+    packed = comp.compress(x)
+    comp.decompress(packed)
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as trace:
+        comp.decompress(packed)
+        torch.cuda.synchronize()
+    names = [e.key for e in trace.key_averages()]
+    comp.close()
+    assert any("decode_flat_kernel" in n for n in names) and any("topk_apply" in n for n in names) == apart, names
+
+
 def test_refused_object_leaves_the_result_alone(pkg, lib):
     """The kernel is launched before the host knows what the payload's headers say; a header that differs in any checked byte keeps
     it from writing, and a column that the matrix does not have fails the call."""
+    refused(pkg, lib, 0.02)
+
+
+def test_refused_object_with_long_lists_leaves_the_result_alone(pkg, lib):
+    """Here the lists' kernel is launched when the headers are known to be good."""
+    refused(pkg, lib, 0.7)
+
+
+def refused(pkg, lib, ratio):
     rows, cols = 96, 640
     x = torch.randn(rows, cols, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
-    lane = lib.bsq_lane_create(rows, cols, 0.02, 0.02, -1, 1, -1, -1, 10)
+    lane = lib.bsq_lane_create(rows, cols, ratio, ratio, -1, 1, -1, -1, 10)
     assert lane
     try:
         cap = int(lib.bsq_lane_packed_capacity(lane))
