@@ -1190,8 +1190,8 @@ ListSource list_source(const bitsqz_llm_array_t *c, const bitsqz_section_t &s, u
 }
 
 // A device-resident object, all of it within reach of kernels and apart from the result.  A quantised matrix: one kernel checks the
-// headers, decodes, adds the lists and reports; long lists (decode_lists_apart) are added behind it as those of factors are.  Factors: one opens them beside the check, two make the product, and once the headers
-// are known to be good one adds the lists and reports.
+// headers, decodes, adds the lists and reports; long lists (decode_lists_apart) are added behind it as those of factors are.  Factors:
+// one opens them beside the check, two make the product, and once the headers are known to be good one adds the lists and reports.
 int decompress_begin_in_place(Runtime &rt, const bitsqz_llm_array_t *c, float *d_dst) {
     cudaStream_t st = rt.stream;
     HeadCheck check{};
